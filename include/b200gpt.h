@@ -41,6 +41,9 @@ int b200_device_info(int* sm_count, int* cc_major, int* cc_minor);
 int b200_set_pdl(int enabled);
 /* number of kernels launched by this library since load (the `gpu_launches` evidence of bench.py) */
 int64_t b200_launch_count(void);
+/* Reads (synchronising `stream`) and clears the current device's error word: non-zero when a kernel gave up a bounded wait on its
+ * own copies or matrix products since the last call; the outputs of that launch are then invalid. */
+int b200_wait_error(b200_stream_t stream, unsigned int* code);
 /* tuning override for the fast GEMV: ksteps in {0(auto),1,2,4}, ctas_per_sm in {0(auto),1,2,3,4}; returns 0 */
 int b200_qgemv_tune(int ksteps, int ctas_per_sm, int force_generic);
 

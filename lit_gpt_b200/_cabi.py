@@ -232,7 +232,7 @@ _CORE_SIGNATURES = {
                                 c_void_p]),
 }
 _CORE_SHARED = ("b200_abi_version", "b200_last_error", "b200_device_info", "b200_set_pdl", "b200_launch_count", "b200_rmsnorm", "b200_swiglu",
-                "b200_embedding", "b200_argmax", "b200_sample", "b200_attn_prefill")
+                "b200_embedding", "b200_argmax", "b200_sample", "b200_attn_prefill", "b200_wait_error")
 
 _SIGNATURES = {
     "b200_abi_version": (c_int, []),
@@ -240,6 +240,7 @@ _SIGNATURES = {
     "b200_device_info": (c_int, [ctypes.POINTER(c_int)] * 3),
     "b200_set_pdl": (c_int, [c_int]),
     "b200_launch_count": (c_int64, []),
+    "b200_wait_error": (c_int, [c_void_p, ctypes.POINTER(ctypes.c_uint)]),
     "b200_qgemv_tune": (c_int, [c_int, c_int, c_int]),
     "b200_quantize_4bit": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "b200_dequantize_4bit": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_int, c_void_p]),

@@ -26,9 +26,37 @@ int sm_count() {
   return cached[dev];
 }
 
+// Raised by a kernel that gave up a bounded wait (tc05.cuh); one word per device, as every __device__ variable.
+__device__ unsigned d_wait_error;
+
+unsigned* wait_error_word() {
+  static std::atomic<unsigned*> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  unsigned* p = cached[dev].load(std::memory_order_acquire);
+  if (!p) {
+    void* a = nullptr;
+    if (cudaGetSymbolAddress(&a, d_wait_error) != cudaSuccess) return nullptr;
+    p = static_cast<unsigned*>(a);
+    cached[dev].store(p, std::memory_order_release);
+  }
+  return p;
+}
+
 }  // namespace b200
 
 extern "C" {
+
+int b200_wait_error(b200_stream_t stream, unsigned int* code) {
+  B200_CHECK_ARG(code, "b200_wait_error: null argument");
+  unsigned* word = b200::wait_error_word();
+  B200_CHECK_ARG(word, "b200_wait_error: no device");
+  cudaStream_t st = (cudaStream_t)stream;
+  B200_CUDA(cudaMemcpyAsync(code, word, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  B200_CUDA(cudaStreamSynchronize(st));
+  if (*code) B200_CUDA(cudaMemsetAsync(word, 0, sizeof(unsigned), st));
+  return B200_OK;
+}
 
 int b200_abi_version(void) { return B200GPT_ABI_VERSION; }
 

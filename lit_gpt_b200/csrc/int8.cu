@@ -7,12 +7,12 @@
 //                CA = rint(x * 127 / absmax_row), SCA = absmax_row
 //   y = f16( int32(CA . CB^T) * (SCA * SCB / 127^2) )  [+ bias -> f16]  [+ f16(x_out . f16(CB_out * SCB / 127)^T) -> f16]
 //
-// The int8 x int8 -> int32 products run on the tensor cores (mma.sync m16n8k32 s8: exact, order-free), weights as the
-// A operand loaded straight from HBM in fragment order (16 contiguous bytes of one row per lane; the K permutation
-// this implies is applied to both operands).  Two mappings over the same fragments:
-//   rows <= 16 (decode): one CTA per 16 weight rows, its 8 warps split K, int32 partials meet in shared memory;
-//   rows  > 16 (prefill): a CTA holds 128 weight rows x 64 activation rows, each warp 16 x 64 over all of K.
-#include "common.cuh"
+// The int8 x int8 -> int32 products are exact and order-free.  Two mappings:
+//   rows <= 16 (decode): mma.sync m16n8k32 s8, the weights loaded straight from HBM in fragment order (16 contiguous bytes of one row per
+//   lane; the K permutation this implies is applied to both operands); one CTA per 16 weight rows, its 8 warps split K, int32 partials
+//   meet in shared memory;
+//   rows  > 16 (prefill): tcgen05.mma kind::i8 over TMA-fed tiles of both operands, int32 accumulators in tensor memory (int8_gemm_kernel).
+#include "tc05.cuh"
 
 namespace b200 {
 
@@ -57,52 +57,108 @@ __global__ void __launch_bounds__(256) dequantize_int8_rows_kernel(const int8_t*
 }
 
 // ---- activation side ------------------------------------------------------------------------------------------
-// flags[k] = 1 when any row has |x[m,k]| >= threshold
-__global__ void __launch_bounds__(256) int8_outlier_flags_kernel(const __half* __restrict__ x, int64_t M, int64_t K, float threshold,
-                                                                 int* __restrict__ flags) {
+// flags[k] = 1 when any row has |x[m,k]| >= threshold.  A thread looks at eight neighbouring columns of `block_rows` rows; with one row block
+// the flags are written outright, with more they start at zero and only hits are written.  (One thread per column walking every row kept
+// 16 CTAs busy for 4096 columns: 250 us of the 750 at 777 rows.)
+__global__ void __launch_bounds__(128) int8_outlier_flags_kernel(const __half* __restrict__ x, int64_t M, int64_t K, float threshold, int block_rows, int* __restrict__ flags) {
+  griddep_launch();
   griddep_wait();
-  const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int64_t k = ((int64_t)blockIdx.x * 128 + threadIdx.x) * 8;
   if (k >= K) return;
-  int f = 0;
+  const int64_t m0 = (int64_t)blockIdx.y * block_rows;
+  const int rows = (int)(M - m0 < block_rows ? M - m0 : block_rows);
+  const __half* px = x + m0 * K + k;
+  unsigned hit = 0;
   if (threshold > 0.f) {
-    for (int64_t m = 0; m < M; ++m) f |= fabsf(__half2float(x[m * K + k])) >= threshold;
+#pragma unroll 8
+    for (int r = 0; r < rows; ++r) {
+      const uint4 v = *reinterpret_cast<const uint4*>(px + (int64_t)r * K);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+        hit |= (fabsf(f.x) >= threshold ? 1u : 0u) << (2 * j) | (fabsf(f.y) >= threshold ? 1u : 0u) << (2 * j + 1);
+      }
+    }
   }
-  flags[k] = f;
+  if (gridDim.y == 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) flags[k + j] = (hit >> j) & 1u;
+  } else if (hit) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if ((hit >> j) & 1u) flags[k + j] = 1;
+  }
 }
 
 // ordered compaction of the flagged columns (ascending k: the fp32 side product is summed in this order)
 __global__ void __launch_bounds__(1024) int8_compact_kernel(const int* __restrict__ flags, int64_t K, int* __restrict__ idx,
                                                             int* __restrict__ count) {
-  __shared__ int s_cnt[1024];
+  __shared__ int s_sum[32];
+  griddep_launch();
   griddep_wait();
-  const int t = threadIdx.x;
-  const int64_t per = (K + 1023) / 1024, beg = t * per, end = beg + per < K ? beg + per : K;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int64_t per = (K + 1023) / 1024, beg = t * per < K ? t * per : K, end = beg + per < K ? beg + per : K;
   int c = 0;
   for (int64_t k = beg; k < end; ++k) c += flags[k];
-  s_cnt[t] = c;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {  // inclusive scan
-    const int v = t >= o ? s_cnt[t - o] : 0;
-    __syncthreads();
-    s_cnt[t] += v;
-    __syncthreads();
+  int incl = c;   // inclusive scan over the warp, then over the warps' sums
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
   }
-  int pos = s_cnt[t] - c;
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  int before = 0;
+  for (int w = 0; w < warp; ++w) before += s_sum[w];
+  int pos = before + incl - c;
   for (int64_t k = beg; k < end; ++k) {
     if (flags[k]) idx[pos++] = (int)k;
   }
-  if (t == 1023) *count = s_cnt[1023];
+  if (t == 1023) *count = before + incl;
 }
 
 // one CTA per activation row: SCA = absmax over the non-outlier columns, CA = rint(x * 127 / SCA) (0 in outlier columns)
+// (K is a multiple of 64 and the rows start on 16-byte boundaries: eight columns per access, the first 8192 kept in registers between
+// the maximum and the rounding)
 __global__ void __launch_bounds__(256) int8_rowquant_kernel(const __half* __restrict__ x, int64_t K, const int* __restrict__ flags,
                                                             int8_t* __restrict__ ca, float* __restrict__ sca) {
   __shared__ float s_max[8];
+  constexpr int KEEP = 4;
+  griddep_launch();
   griddep_wait();
   const int64_t m = blockIdx.x;
   const __half* row = x + m * K;
+  const int nv = (int)(K >> 3);
+  auto load = [&](int i, float (&f)[8]) {   // eight columns, outliers as 0
+    const uint4 v = reinterpret_cast<const uint4*>(row)[i];
+    const int4 fa = reinterpret_cast<const int4*>(flags)[2 * i], fb = reinterpret_cast<const int4*>(flags)[2 * i + 1];
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const int fl[8] = {fa.x, fa.y, fa.z, fa.w, fb.x, fb.y, fb.z, fb.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+      f[2 * j] = fl[2 * j] ? 0.f : h.x;
+      f[2 * j + 1] = fl[2 * j + 1] ? 0.f : h.y;
+    }
+  };
+  float kept[KEEP][8];
   float mx = 0.f;
-  for (int64_t k = threadIdx.x; k < K; k += 256) mx = fmaxf(mx, flags[k] ? 0.f : fabsf(__half2float(row[k])));
+#pragma unroll
+  for (int u = 0; u < KEEP; ++u) {
+    const int i = (int)threadIdx.x + u * 256;
+    if (i < nv) {
+      load(i, kept[u]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(kept[u][j]));
+    }
+  }
+  for (int i = (int)threadIdx.x + KEEP * 256; i < nv; i += 256) {
+    float f[8];
+    load(i, f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(f[j]));
+  }
   mx = warp_max(mx);
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
   __syncthreads();
@@ -111,9 +167,25 @@ __global__ void __launch_bounds__(256) int8_rowquant_kernel(const __half* __rest
   for (int i = 1; i < 8; ++i) mx = fmaxf(mx, s_max[i]);
   if (threadIdx.x == 0) sca[m] = mx;
   const float inv = __fdiv_rn(127.0f, mx);
-  for (int64_t k = threadIdx.x; k < K; k += 256) {
-    const float v = __fmul_rn(flags[k] ? 0.f : __half2float(row[k]), inv);
-    ca[m * K + k] = (v != v) ? (int8_t)0 : (int8_t)__float2int_rn(v);
+  auto store = [&](int i, const float (&f)[8]) {
+    uint32_t o[2] = {0u, 0u};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float v = __fmul_rn(f[j], inv);
+      const int8_t q = (v != v) ? (int8_t)0 : (int8_t)__float2int_rn(v);
+      o[j >> 2] |= (uint32_t)(uint8_t)q << (8 * (j & 3));
+    }
+    *reinterpret_cast<uint2*>(ca + m * K + (int64_t)i * 8) = make_uint2(o[0], o[1]);
+  };
+#pragma unroll
+  for (int u = 0; u < KEEP; ++u) {
+    const int i = (int)threadIdx.x + u * 256;
+    if (i < nv) store(i, kept[u]);
+  }
+  for (int i = (int)threadIdx.x + KEEP * 256; i < nv; i += 256) {
+    float f[8];
+    load(i, f);
+    store(i, f);
   }
 }
 
@@ -213,56 +285,223 @@ __global__ void __launch_bounds__(kI8Threads) int8_gemv_kernel(const I8Params p)
   }
 }
 
-// ---- prefill: M > 16.  grid = (ceil(N / 128), ceil(M / 64)); warp w: weight rows [n0 + 16 w, +16) x 64 activation rows
-__global__ void __launch_bounds__(kI8Threads) int8_gemm_kernel(const I8Params p) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int64_t n0 = (int64_t)blockIdx.x * 128 + warp * 16, m0 = (int64_t)blockIdx.y * 64;
-  if (n0 >= p.N) return;
-  const int64_t ra = n0 + g < p.N ? n0 + g : p.N - 1, rb = n0 + g + 8 < p.N ? n0 + g + 8 : p.N - 1;
-  const int8_t* wa = p.cb + ra * p.K + 16 * t;
-  const int8_t* wb = p.cb + rb * p.K + 16 * t;
-  const int8_t* xr[8];
-  bool xv_ok[8];
-#pragma unroll
-  for (int mb = 0; mb < 8; ++mb) {
-    const int64_t m = m0 + mb * 8 + g;
-    xv_ok[mb] = m < p.M;
-    xr[mb] = p.ca + (xv_ok[mb] ? m : 0) * p.K + 16 * t;
+// ---- prefill: M > 16 ----------------------------------------------------------------------------------------------
+// Persistent CTAs, one per SM, over (128 rows x BN features) output tiles, neighbouring CTAs on the same weight rows.  One thread loads
+// 128-byte-wide boxes of both operands by TMA into a ring of stages, one issues tcgen05.mma kind::i8 (M = 128, N = BN, K = 32) into one of
+// two tensor-memory accumulators, and eight epilogue warps scale, round and store the other: the epilogue (a division, three roundings
+// and the outlier columns per output) hides behind the next tile's products.  Bound: the int8 tensor pipe (BN = 256 reads 96 bytes of
+// shared memory per clock, BN = 128 the full 128).
+constexpr int kI8EpiWarps = 8, kI8GemmThreads = (kI8EpiWarps + 2) * 32;
+constexpr int kI8KB = 128;   // int8 columns per stage: one 128-byte swizzle row
+
+template <int BN>
+struct I8Tile {
+  static constexpr int kStage = (128 + BN) * kI8KB;
+  static constexpr int kStages = BN == 256 ? 4 : 6;
+  static constexpr int kSmem = kStages * kStage + 1024;
+  // kind::i8: D = int32, A = B = signed 8 bit, both K-major, N = BN, M = 128
+  static constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+};
+
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kI8GemmThreads, 1)
+int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int m_tiles, int n_tiles, unsigned* err) {
+  using C = I8Tile<BN>;
+  extern __shared__ __align__(1024) uint8_t i8_smem[];
+  __shared__ __align__(8) uint64_t s_bars[2 * C::kStages + 4];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t tiles = (tc::smem_u32(i8_smem) + 1023u) & ~1023u;
+  const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]);
+  const uint32_t acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_empty = acc_full + 16;
+  if (tid == 0) {
+    for (int s = 0; s < C::kStages; ++s) { tc::mbar_init(full + 8 * s, 1); tc::mbar_init(empty + 8 * s, 1); }
+    for (int a = 0; a < 2; ++a) { tc::mbar_init(acc_full + 8 * a, 1); tc::mbar_init(acc_empty + 8 * a, kI8EpiWarps); }
+    tc::mbar_init_fence();
+    tc::prefetch_map(&map_a);
+    tc::prefetch_map(&map_b);
   }
-  const int nchunks = (int)(p.K >> 6);
-  int acc[8][4];
-#pragma unroll
-  for (int mb = 0; mb < 8; ++mb) acc[mb][0] = acc[mb][1] = acc[mb][2] = acc[mb][3] = 0;
+  if (warp == kI8EpiWarps) tc::tmem_alloc<2 * BN>(tc::smem_u32(&s_tmem));
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = s_tmem;
   griddep_launch();
   griddep_wait();
-  uint4 an = *reinterpret_cast<const uint4*>(wa), bn = *reinterpret_cast<const uint4*>(wb);
-  for (int c = 0; c < nchunks; ++c) {
-    const uint4 av = an, bv = bn;
-    if (c + 1 < nchunks) {
-      an = *reinterpret_cast<const uint4*>(wa + (int64_t)(c + 1) * 64);
-      bn = *reinterpret_cast<const uint4*>(wb + (int64_t)(c + 1) * 64);
+  const int nkb = (int)((p.K + kI8KB - 1) / kI8KB), total = m_tiles * n_tiles;
+  bool ok = true;
+
+  if (warp == kI8EpiWarps) {
+    // ---- copies ----
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 1;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        const int m0 = (t % m_tiles) * 128, n0 = (t / m_tiles) * BN;
+        for (int kb = 0; kb < nkb && ok; ++kb) {
+          ok = tc::mbar_wait(empty + 8 * s, ph);
+          if (!ok) break;
+          const uint32_t st = tiles + s * C::kStage;
+          tc::mbar_expect_tx(full + 8 * s, C::kStage);
+          tc::tma_load_2d(st, &map_a, kb * kI8KB, m0, full + 8 * s);
+          tc::tma_load_2d(st + 128 * kI8KB, &map_b, kb * kI8KB, n0, full + 8 * s);
+          if (++s == C::kStages) { s = 0; ph ^= 1u; }
+        }
+      }
+      if (!ok)   // given up: no copy may still be on its way when the CTA leaves
+        for (int i = 0; i < C::kStages; ++i) tc::mbar_wait(full + 8 * i, i < s ? ph ^ 1u : ph);
     }
-    uint4 xv[8];
+  } else if (warp == kI8EpiWarps + 1) {
+    // ---- products ----
+    if (lane == 0) {
+      int s = 0, acc = 0;
+      uint32_t ph = 0, aph = 1;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        ok = tc::mbar_wait(acc_empty + 8 * acc, aph);
+        tc::fence_after();
+        for (int kb = 0; kb < nkb && ok; ++kb) {
+          ok = tc::mbar_wait(full + 8 * s, ph);
+          if (!ok) break;
+          tc::fence_after();
+          const uint32_t st = tiles + s * C::kStage;
+          const uint64_t da = tc::desc_sw128(st), db = tc::desc_sw128(st + 128 * kI8KB);
 #pragma unroll
-    for (int mb = 0; mb < 8; ++mb) {
-      xv[mb] = make_uint4(0u, 0u, 0u, 0u);
-      if (xv_ok[mb]) xv[mb] = *reinterpret_cast<const uint4*>(xr[mb] + (int64_t)c * 64);
+          for (int k = 0; k < kI8KB / 32; ++k) umma_i8(tmem + acc * BN, da + 2 * k, db + 2 * k, C::kIdesc, (kb | k) != 0);
+          tc::commit(empty + 8 * s);
+          if (++s == C::kStages) { s = 0; ph ^= 1u; }
+        }
+        if (ok) tc::commit(acc_full + 8 * acc);
+        acc ^= 1;
+        if (acc == 0) aph ^= 1u;
+      }
     }
+  } else {
+    // ---- epilogue: warp w holds rows 32 (w % 4) .. + 31 and half of the columns ----
+    int acc = 0;
+    uint32_t ph = 0;
+    const int no = *p.count;
+    const bool vec = (p.N & 7) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+      const int64_t m = (int64_t)(t % m_tiles) * 128 + (warp & 3) * 32 + lane, n0 = (int64_t)(t / m_tiles) * BN + (warp >> 2) * (BN / 2);
+      const bool mok = m < p.M;
+      const float sca = mok ? p.sca[m] : 0.f;
+      const __half* const xr = p.x + (mok ? m : 0) * p.K;
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(acc_full + 8 * acc, ph));
+      if (!ok) break;
+      tc::fence_after();
+#pragma unroll 1
+      for (int c0 = 0; c0 < BN / 2; c0 += 32) {
+        // this lane's feature of the 32: its statistics, and its weight in each outlier column, are handed round by shuffles
+        const int64_t nl = n0 + c0 + lane;
+        const bool nok = nl < p.N;
+        const float scb_l = nok ? p.scb[nl] : 0.f;
+        const float bias_l = nok && p.bias ? __half2float(p.bias[nl]) : 0.f;
+        const float ws_l = __fdiv_rn(scb_l, 127.0f);
+        const int8_t* const cb_l = p.cb + (nok ? nl : 0) * p.K;
+        uint32_t v[32];
+        tc::ld32(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * BN + (warp >> 2) * (BN / 2) + c0));
+        tc::wait_ld();
+        float out[32];
 #pragma unroll
-    for (int mb = 0; mb < 8; ++mb) {
-      imma16832(acc[mb], av.x, bv.x, av.y, bv.y, xv[mb].x, xv[mb].y);
-      imma16832(acc[mb], av.z, bv.z, av.w, bv.w, xv[mb].z, xv[mb].w);
+        for (int e = 0; e < 32; ++e) {
+          const float scale = __fdiv_rn(__fmul_rn(sca, __shfl_sync(0xffffffffu, scb_l, e)), 127.0f * 127.0f);
+          out[e] = round_f16(__fmul_rn((float)(int)v[e], scale));
+        }
+        if (p.bias) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) out[e] = round_f16(out[e] + __shfl_sync(0xffffffffu, bias_l, e));
+        }
+        if (no > 0) {
+          float sub[32];
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sub[e] = 0.f;
+          for (int j0 = 0; j0 < no; j0 += 8) {   // ascending columns, eight columns' loads in flight
+            float xv[8], wl[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const bool jok = j0 + j < no;
+              const int k = jok ? p.idx[j0 + j] : 0;
+              xv[j] = jok ? __half2float(xr[k]) : 0.f;
+              wl[j] = jok ? (float)cb_l[k] : 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              if (j0 + j < no) {
+                const float w = round_f16(__fmul_rn(wl[j], ws_l));
+#pragma unroll
+                for (int e = 0; e < 32; ++e) sub[e] = fmaf(xv[j], __shfl_sync(0xffffffffu, w, e), sub[e]);
+              }
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 32; ++e) out[e] = round_f16(out[e] + round_f16(sub[e]));
+        }
+        if (mok) {
+          __half* const yr = p.y + m * p.N + n0 + c0;
+          if (vec) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 8) {
+              if (n0 + c0 + e < p.N) {
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const __half2 h = __floats2half2_rn(out[e + 2 * i], out[e + 2 * i + 1]);
+                  o[i] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                *reinterpret_cast<uint4*>(yr + e) = make_uint4(o[0], o[1], o[2], o[3]);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (n0 + c0 + e < p.N) yr[e] = __float2half_rn(out[e]);
+          }
+        }
+      }
+      tc::fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(acc_empty + 8 * acc);
+      acc ^= 1;
+      if (acc == 0) ph ^= 1u;
     }
   }
-#pragma unroll
-  for (int mb = 0; mb < 8; ++mb) {
-    const int64_t m = m0 + mb * 8 + 2 * t;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int64_t mm = m + (i & 1), nn = n0 + g + (i >> 1) * 8;
-      if (mm < p.M && nn < p.N) i8_store(p, mm, nn, acc[mb][i]);
-    }
+  if (!ok && err) *err = 1u;
+  tc::fence_before();
+  __syncthreads();
+  if (warp == kI8EpiWarps) tc::tmem_free<2 * BN>(tmem);
+}
+
+template <int BN>
+static cudaError_t launch_i8_gemm(const I8Params& p, cudaStream_t st) {
+  using C = I8Tile<BN>;
+  static PerDeviceOnce once;
+  if (once.need()) {
+    const cudaError_t e = cudaFuncSetAttribute(int8_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+    if (e != cudaSuccess) return e;
+    once.done();
   }
+  alignas(64) CUtensorMap ma, mb;
+  if (!tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.ca, p.M, p.K, p.K, 128) || !tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.cb, p.N, p.K, p.K, BN))
+    return cudaErrorInvalidValue;
+  const int mt = (int)((p.M + 127) / 128), nt = (int)((p.N + BN - 1) / BN);
+  const int64_t tiles = (int64_t)mt * nt;
+  const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+  return launch(int8_gemm_kernel<BN>, dim3((unsigned)grid), dim3(kI8GemmThreads), (size_t)C::kSmem, st, p, ma, mb, mt, nt, wait_error_word());
+}
+
+// Features per tile: the wider tile reads less shared memory per product (a full tile of 256 takes 1.9 x one of 128), the narrower leaves a
+// smaller remainder in the last round over the SMs -- the smaller number of rounds x tile time wins.
+static cudaError_t launch_i8_gemm(const I8Params& p, cudaStream_t st) {
+  const int64_t mt = (p.M + 127) / 128, sms = sm_count();
+  const int64_t r256 = (mt * ((p.N + 255) / 256) + sms - 1) / sms, r128 = (mt * ((p.N + 127) / 128) + sms - 1) / sms;
+  return r256 * 19 <= r128 * 10 ? launch_i8_gemm<256>(p, st) : launch_i8_gemm<128>(p, st);
 }
 
 }  // namespace b200
@@ -324,7 +563,10 @@ int b200_linear_int8(const b200_linear_int8_args* a, b200_stream_t stream) {
   int8_t* ca = reinterpret_cast<int8_t*>(ws + (size_t)a->K * 8 + 16 + (((size_t)a->M * 4 + 15) & ~(size_t)15));
   const __half* x = reinterpret_cast<const __half*>(a->x);
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = launch(int8_outlier_flags_kernel, dim3((unsigned)((a->K + 255) / 256)), dim3(256), 0, st, x, a->M, a->K, a->threshold, flags);
+  const int block_rows = a->M <= 32 * 4096 ? 32 : 64;
+  const dim3 fg((unsigned)((a->K / 8 + 127) / 128), (unsigned)((a->M + block_rows - 1) / block_rows));
+  cudaError_t e = fg.y > 1 ? cudaMemsetAsync(flags, 0, (size_t)a->K * sizeof(int), st) : cudaSuccess;
+  if (e == cudaSuccess) e = launch(int8_outlier_flags_kernel, fg, dim3(128), 0, st, x, a->M, a->K, a->threshold, block_rows, flags);
   if (e == cudaSuccess) e = launch(int8_compact_kernel, dim3(1), dim3(1024), 0, st, (const int*)flags, a->K, idx, count);
   if (e == cudaSuccess) e = launch(int8_rowquant_kernel, dim3((unsigned)a->M), dim3(256), 0, st, x, a->K, (const int*)flags, ca, sca);
   I8Params p{};
@@ -338,7 +580,7 @@ int b200_linear_int8(const b200_linear_int8_args* a, b200_stream_t stream) {
     const dim3 gv((unsigned)((a->N + 15) / 16));
     if (a->M <= 8) e = launch(int8_gemv_kernel<1>, gv, dim3(kI8Threads), 0, st, p);
     else if (a->M <= 16) e = launch(int8_gemv_kernel<2>, gv, dim3(kI8Threads), 0, st, p);
-    else e = launch(int8_gemm_kernel, dim3((unsigned)((a->N + 127) / 128), (unsigned)((a->M + 63) / 64)), dim3(kI8Threads), 0, st, p);
+    else e = launch_i8_gemm(p, st);
   }
   if (e != cudaSuccess) {
     set_error("b200_linear_int8: launch failed: %s", cudaGetErrorString(e));

@@ -352,13 +352,18 @@ def tp_gather(h: "C.TpHandoff", batch: int, n_per_rank: int, device: torch.devic
 
 
 def check_gemv_errors(device: torch.device) -> None:
-    """Raise if a GEMV kernel on `device` gave up a bounded wait (a tensor-parallel peer that never delivered its
-    packets, a stream-K partner CTA): synchronizes the current stream.  Called by generate() at its sync points."""
+    """Raise if a kernel on `device` gave up a bounded wait (a tensor-parallel peer that never delivered its packets, a
+    stream-K partner CTA, a stage of a tensor-memory kernel): synchronizes the current stream.  Called by generate() at
+    its sync points."""
+    code = ctypes.c_uint(0)
+    with torch.cuda.device(device):
+        C.check(C.load().b200_wait_error(C.stream_ptr(device), ctypes.byref(code)), "wait_error")
+    if code.value:
+        raise C.B200Error("a kernel gave up a bounded wait on its own copies or matrix products; the output of this step is invalid")
     key = ("qgemv_tiled", device.index if device.index is not None else torch.cuda.current_device())
     ws = _workspaces.get(key)
     if ws is None:
         return
-    code = ctypes.c_uint(0)
     with torch.cuda.device(device):
         C.check(C.load().b200_qgemv_tiled_error(ws.data_ptr(), C.stream_ptr(device), ctypes.byref(code)), "qgemv_tiled_error")
     if code.value:

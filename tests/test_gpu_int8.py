@@ -168,3 +168,13 @@ def test_gpt_int8_generate(K):
     with torch.no_grad():
         out = generate(model, idx[0], 16, temperature=0.0)
     assert out.shape == (16,) and torch.equal(out[:8], idx[0])
+
+
+@pytest.mark.parametrize("M,N,Kd,bias", [(17, 8, 64, False), (127, 136, 192, True), (128, 256, 128, False), (129, 250, 4096, True), (257, 520, 1088, False),
+                                         (600, 8200, 192, True), (40, 12288, 320, False)])
+def test_linear_int8_prefill_tile_edges(K, M, N, Kd, bias):
+    """Row and feature remainders of the tensor-memory tiles, a feature count that is no multiple of 8, half-filled column blocks, more
+    tiles than SMs -- without outliers every output is exact -- and outlier columns in several row blocks, more of them than one batch."""
+    assert not _check(K, M, N, Kd, 400 + M + N, bias=bias)
+    out = [(7 * j, 11 * j + 3, 6.0 + j) for j in range(19)]
+    assert _check(K, M, N, Kd, 500 + M + N, bias=bias, outliers=out)
