@@ -286,98 +286,130 @@ __global__ void __launch_bounds__(kI8Threads) int8_gemv_kernel(const I8Params p)
 }
 
 // ---- prefill: M > 16 ----------------------------------------------------------------------------------------------
-// Persistent CTAs, one per SM, over (128 rows x BN features) output tiles, neighbouring CTAs on the same weight rows.  One thread loads
-// 128-byte-wide boxes of both operands by TMA into a ring of stages, one issues tcgen05.mma kind::i8 (M = 128, N = BN, K = 32) into one of
-// two tensor-memory accumulators, and eight epilogue warps scale, round and store the other: the epilogue (a division, three roundings
-// and the outlier columns per output) hides behind the next tile's products.  Bound: the int8 tensor pipe (BN = 256 reads 96 bytes of
-// shared memory per clock, BN = 128 the full 128).
+// Persistent over output tiles, neighbouring CTAs on the same weight rows.  One thread loads 128-byte-wide boxes of both operands by TMA into a
+// ring of stages, one issues tcgen05.mma kind::i8 (K = 32) into one of two tensor-memory accumulators, and eight epilogue warps scale, round
+// and store the other: the epilogue (a division, three roundings and the outlier columns per output) hides behind the next tile's products.
+//   PAIR = true: a CTA pair on 256 rows x 256 features, each CTA holding 128 rows of either operand.  Shared memory is the limit of the
+//   int8 pipe -- a CTA alone on 128 x 128 moves 128 bytes in and 128 bytes out of it per clock at full rate, twice what it carries, the pair
+//   half as much.  777 x 4096 -> 11008 with its three preparing kernels, six outlier columns: 780 us with fragments read from L2, 100 us with
+//   128 x 128 tiles, 71 us with pairs (4096 rows -> 12288: 338 and 229 us, 1.8 POP/s; without outlier columns 2.1).
+//   PAIR = false: one CTA on 128 x 128, for up to 128 rows, where the second half of a pair's rows would be padding.
 constexpr int kI8EpiWarps = 8, kI8GemmThreads = (kI8EpiWarps + 2) * 32;
-constexpr int kI8KB = 128;   // int8 columns per stage: one 128-byte swizzle row
+constexpr int kI8KB = 128;                       // int8 columns per stage: one 128-byte swizzle row
+constexpr int kI8Stages = 6, kI8Stage = 256 * kI8KB, kI8Smem = kI8Stages * kI8Stage + 1024;   // 128 rows of either operand
 
-template <int BN>
-struct I8Tile {
-  static constexpr int kStage = (128 + BN) * kI8KB;
-  static constexpr int kStages = BN == 256 ? 4 : 6;
-  static constexpr int kSmem = kStages * kStage + 1024;
-  // kind::i8: D = int32, A = B = signed 8 bit, both K-major, N = BN, M = 128
-  static constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-};
-
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+// kind::i8: D = int32, A = B = signed 8 bit, both K-major
+template <bool PAIR>
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+  constexpr uint32_t kM = PAIR ? 256 : 128, kN = PAIR ? 256 : 128;
+  constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((kN >> 3) << 17) | ((kM >> 4) << 24);
+  if constexpr (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-template <int BN>
+// x / 127^2 rounded as the division is: the reciprocal, then one Newton step on the remainder (Markstein); beyond 1e30 the division itself
+__device__ __forceinline__ float i8_scale(float x) {
+  constexpr float d = 127.0f * 127.0f, r = 1.0f / d;
+  if (!(x < 1e30f)) return __fdiv_rn(x, d);
+  const float q = __fmul_rn(x, r);
+  return fmaf(fmaf(-q, d, x), r, q);
+}
+__device__ __forceinline__ float2 round_f16x2(float a, float b) { return __half22float2(__floats2half2_rn(a, b)); }
+
+template <bool PAIR>
 __global__ void __launch_bounds__(kI8GemmThreads, 1)
 int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int m_tiles, int n_tiles, unsigned* err) {
-  using C = I8Tile<BN>;
+  constexpr int CTAS = PAIR ? 2 : 1, BN = 128 * CTAS;
   extern __shared__ __align__(1024) uint8_t i8_smem[];
-  __shared__ __align__(8) uint64_t s_bars[2 * C::kStages + 4];
+  __shared__ __align__(8) uint64_t s_bars[2 * kI8Stages + 4];
   __shared__ uint32_t s_tmem;
+  __shared__ __align__(16) float s_feat[10][BN];               // per feature of the tile: weight scale, bias, weight in the first eight outlier columns
+  __shared__ __align__(16) float s_more[kI8EpiWarps][8][32];   // per epilogue warp: the weights of 32 features in the next eight
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t rank = PAIR ? tc::cluster_rank() : 0u;
   const uint32_t tiles = (tc::smem_u32(i8_smem) + 1023u) & ~1023u;
-  const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]);
-  const uint32_t acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_empty = acc_full + 16;
+  const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[kI8Stages]);
+  const uint32_t acc_full = tc::smem_u32(&s_bars[2 * kI8Stages]), acc_empty = acc_full + 16;
   if (tid == 0) {
-    for (int s = 0; s < C::kStages; ++s) { tc::mbar_init(full + 8 * s, 1); tc::mbar_init(empty + 8 * s, 1); }
-    for (int a = 0; a < 2; ++a) { tc::mbar_init(acc_full + 8 * a, 1); tc::mbar_init(acc_empty + 8 * a, kI8EpiWarps); }
+    for (int s = 0; s < kI8Stages; ++s) { tc::mbar_init(full + 8 * s, 1); tc::mbar_init(empty + 8 * s, 1); }
+    for (int a = 0; a < 2; ++a) { tc::mbar_init(acc_full + 8 * a, 1); tc::mbar_init(acc_empty + 8 * a, kI8EpiWarps * CTAS); }
     tc::mbar_init_fence();
     tc::prefetch_map(&map_a);
     tc::prefetch_map(&map_b);
   }
-  if (warp == kI8EpiWarps) tc::tmem_alloc<2 * BN>(tc::smem_u32(&s_tmem));
+  if (warp == kI8EpiWarps) {
+    if constexpr (PAIR) tc::tmem_alloc_pair<2 * BN>(tc::smem_u32(&s_tmem));
+    else tc::tmem_alloc<2 * BN>(tc::smem_u32(&s_tmem));
+  }
   tc::fence_before();
+  if constexpr (PAIR) tc::cluster_sync();
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = s_tmem;
   griddep_launch();
   griddep_wait();
   const int nkb = (int)((p.K + kI8KB - 1) / kI8KB), total = m_tiles * n_tiles;
+  const int first = (int)blockIdx.x / CTAS, step = (int)gridDim.x / CTAS;
   bool ok = true;
 
   if (warp == kI8EpiWarps) {
-    // ---- copies ----
+    // ---- copies: 128 rows of either operand into this CTA's stage, counted on the issuing CTA's barrier ----
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 1;
-      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        const int m0 = (t % m_tiles) * 128, n0 = (t / m_tiles) * BN;
-        for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = tc::mbar_wait(empty + 8 * s, ph);
+      for (int t = first; t < total && ok; t += step) {
+        const int m0 = (t % m_tiles) * BN + (int)rank * 128, n0 = (t / m_tiles) * BN + (int)rank * 128;
+        for (int kb = 0; kb < nkb; ++kb) {
+          ok = PAIR ? tc::mbar_wait_cluster(empty + 8 * s, ph) : tc::mbar_wait(empty + 8 * s, ph);
           if (!ok) break;
-          const uint32_t st = tiles + s * C::kStage;
-          tc::mbar_expect_tx(full + 8 * s, C::kStage);
-          tc::tma_load_2d(st, &map_a, kb * kI8KB, m0, full + 8 * s);
-          tc::tma_load_2d(st + 128 * kI8KB, &map_b, kb * kI8KB, n0, full + 8 * s);
-          if (++s == C::kStages) { s = 0; ph ^= 1u; }
+          const uint32_t st = tiles + s * kI8Stage;
+          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * kI8Stage);
+          if constexpr (PAIR) {
+            const uint32_t bar = tc::at_rank(full + 8 * s, 0);
+            tc::tma_load_2d_pair(st, &map_a, kb * kI8KB, m0, bar);
+            tc::tma_load_2d_pair(st + 128 * kI8KB, &map_b, kb * kI8KB, n0, bar);
+          } else {
+            tc::tma_load_2d(st, &map_a, kb * kI8KB, m0, full + 8 * s);
+            tc::tma_load_2d(st + 128 * kI8KB, &map_b, kb * kI8KB, n0, full + 8 * s);
+          }
+          if (++s == kI8Stages) { s = 0; ph ^= 1u; }
         }
       }
-      if (!ok)   // given up: no copy may still be on its way when the CTA leaves
-        for (int i = 0; i < C::kStages; ++i) tc::mbar_wait(full + 8 * i, i < s ? ph ^ 1u : ph);
+      if (!ok && rank == 0)   // given up: no copy may still be on its way when the CTAs leave
+        for (int i = 0; i < kI8Stages; ++i) tc::mbar_wait(full + 8 * i, i < s ? ph ^ 1u : ph);
     }
   } else if (warp == kI8EpiWarps + 1) {
     // ---- products ----
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {
       int s = 0, acc = 0;
       uint32_t ph = 0, aph = 1;
-      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        ok = tc::mbar_wait(acc_empty + 8 * acc, aph);
+      for (int t = first; t < total && ok; t += step) {
+        ok = PAIR ? tc::mbar_wait_cluster(acc_empty + 8 * acc, aph) : tc::mbar_wait(acc_empty + 8 * acc, aph);
         tc::fence_after();
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = tc::mbar_wait(full + 8 * s, ph);
+          ok = PAIR ? tc::mbar_wait_cluster(full + 8 * s, ph) : tc::mbar_wait(full + 8 * s, ph);
           if (!ok) break;
           tc::fence_after();
-          const uint32_t st = tiles + s * C::kStage;
+          const uint32_t st = tiles + s * kI8Stage;
           const uint64_t da = tc::desc_sw128(st), db = tc::desc_sw128(st + 128 * kI8KB);
 #pragma unroll
-          for (int k = 0; k < kI8KB / 32; ++k) umma_i8(tmem + acc * BN, da + 2 * k, db + 2 * k, C::kIdesc, (kb | k) != 0);
-          tc::commit(empty + 8 * s);
-          if (++s == C::kStages) { s = 0; ph ^= 1u; }
+          for (int k = 0; k < kI8KB / 32; ++k) umma_i8<PAIR>(tmem + acc * BN, da + 2 * k, db + 2 * k, (kb | k) != 0);
+          if constexpr (PAIR) tc::commit_pair(empty + 8 * s);
+          else tc::commit(empty + 8 * s);
+          if (++s == kI8Stages) { s = 0; ph ^= 1u; }
         }
-        if (ok) tc::commit(acc_full + 8 * acc);
+        if (ok) {
+          if constexpr (PAIR) tc::commit_pair(acc_full + 8 * acc);
+          else tc::commit(acc_full + 8 * acc);
+        }
         acc ^= 1;
         if (acc == 0) aph ^= 1u;
       }
@@ -388,60 +420,105 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
     uint32_t ph = 0;
     const int no = *p.count;
     const bool vec = (p.N & 7) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-      const int64_t m = (int64_t)(t % m_tiles) * 128 + (warp & 3) * 32 + lane, n0 = (int64_t)(t / m_tiles) * BN + (warp >> 2) * (BN / 2);
+    int k0[8];   // the first eight outlier columns
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k0[j] = j < no ? p.idx[j] : 0;
+    float(&more)[8][32] = s_more[warp];
+    for (int t = first; t < total; t += step) {
+      const int64_t m = (int64_t)(t % m_tiles) * BN + rank * 128 + (warp & 3) * 32 + lane, n0 = (int64_t)(t / m_tiles) * BN;
+      const int half = (warp >> 2) * (BN / 2);
       const bool mok = m < p.M;
       const float sca = mok ? p.sca[m] : 0.f;
       const __half* const xr = p.x + (mok ? m : 0) * p.K;
-      ok = __all_sync(0xffffffffu, tc::mbar_wait(acc_full + 8 * acc, ph));
-      if (!ok) break;
+      float x0[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x0[j] = j < no ? __half2float(xr[k0[j]]) : 0.f;
+      // the tile's features, one per thread, while its products are still running (a gather per 32 columns in the loop below cost more than
+      // the products: 72 us of 266 at 4096 rows with six outlier columns)
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // the last tile's readers are done
+      if (tid < BN) {
+        const int64_t n = n0 + tid;
+        const bool nok = n < p.N;
+        const float scb = nok ? p.scb[n] : 0.f, ws = __fdiv_rn(scb, 127.0f);
+        const int8_t* const cb = p.cb + (nok ? n : 0) * p.K;
+        float w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = j < no ? (float)cb[k0[j]] : 0.f;
+        s_feat[0][tid] = scb;
+        s_feat[1][tid] = nok && p.bias ? __half2float(p.bias[n]) : 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j < no) s_feat[2 + j][tid] = round_f16(__fmul_rn(w[j], ws));
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      ok = ok && __all_sync(0xffffffffu, PAIR ? tc::mbar_wait_cluster(acc_full + 8 * acc, ph) : tc::mbar_wait(acc_full + 8 * acc, ph));
       tc::fence_after();
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN / 2; c0 += 32) {
-        // this lane's feature of the 32: its statistics, and its weight in each outlier column, are handed round by shuffles
-        const int64_t nl = n0 + c0 + lane;
-        const bool nok = nl < p.N;
-        const float scb_l = nok ? p.scb[nl] : 0.f;
-        const float bias_l = nok && p.bias ? __half2float(p.bias[nl]) : 0.f;
-        const float ws_l = __fdiv_rn(scb_l, 127.0f);
-        const int8_t* const cb_l = p.cb + (nok ? nl : 0) * p.K;
+      for (int c0 = half; c0 < half + BN / 2 && ok; c0 += 32) {
         uint32_t v[32];
-        tc::ld32(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * BN + (warp >> 2) * (BN / 2) + c0));
-        tc::wait_ld();
+        tc::ld32(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * BN + c0));
+        tc::wait_ld(v);
         float out[32];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const float scale = __fdiv_rn(__fmul_rn(sca, __shfl_sync(0xffffffffu, scb_l, e)), 127.0f * 127.0f);
-          out[e] = round_f16(__fmul_rn((float)(int)v[e], scale));
+        for (int e = 0; e < 32; e += 2) {
+          const float2 sc = *reinterpret_cast<const float2*>(&s_feat[0][c0 + e]);
+          const float2 o = round_f16x2(__fmul_rn((float)(int)v[e], i8_scale(__fmul_rn(sca, sc.x))), __fmul_rn((float)(int)v[e + 1], i8_scale(__fmul_rn(sca, sc.y))));
+          out[e] = o.x;
+          out[e + 1] = o.y;
         }
         if (p.bias) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) out[e] = round_f16(out[e] + __shfl_sync(0xffffffffu, bias_l, e));
+          for (int e = 0; e < 32; e += 2) {
+            const float2 b = *reinterpret_cast<const float2*>(&s_feat[1][c0 + e]);
+            const float2 o = round_f16x2(out[e] + b.x, out[e + 1] + b.y);
+            out[e] = o.x;
+            out[e + 1] = o.y;
+          }
         }
         if (no > 0) {
           float sub[32];
 #pragma unroll
           for (int e = 0; e < 32; ++e) sub[e] = 0.f;
-          for (int j0 = 0; j0 < no; j0 += 8) {   // ascending columns, eight columns' loads in flight
-            float xv[8], wl[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const bool jok = j0 + j < no;
-              const int k = jok ? p.idx[j0 + j] : 0;
-              xv[j] = jok ? __half2float(xr[k]) : 0.f;
-              wl[j] = jok ? (float)cb_l[k] : 0.f;
-            }
+          auto add = [&](int j0, const float (&xv)[8], const float* rows, int ld) {   // ascending columns
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               if (j0 + j < no) {
-                const float w = round_f16(__fmul_rn(wl[j], ws_l));
 #pragma unroll
-                for (int e = 0; e < 32; ++e) sub[e] = fmaf(xv[j], __shfl_sync(0xffffffffu, w, e), sub[e]);
+                for (int e = 0; e < 32; e += 4) {
+                  const float4 w = *reinterpret_cast<const float4*>(rows + j * ld + e);
+                  sub[e] = fmaf(xv[j], w.x, sub[e]);
+                  sub[e + 1] = fmaf(xv[j], w.y, sub[e + 1]);
+                  sub[e + 2] = fmaf(xv[j], w.z, sub[e + 2]);
+                  sub[e + 3] = fmaf(xv[j], w.w, sub[e + 3]);
+                }
               }
             }
+          };
+          add(0, x0, &s_feat[2][c0], BN);
+          for (int j0 = 8; j0 < no; j0 += 8) {
+            const int64_t n = n0 + c0 + lane;
+            const bool nok = n < p.N;
+            const float ws = __fdiv_rn(s_feat[0][c0 + lane], 127.0f);
+            const int8_t* const cb = p.cb + (nok ? n : 0) * p.K;
+            float xv[8], w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const int k = j0 + j < no ? p.idx[j0 + j] : 0;
+              xv[j] = j0 + j < no ? __half2float(xr[k]) : 0.f;
+              w[j] = j0 + j < no ? (float)cb[k] : 0.f;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) more[j][lane] = round_f16(__fmul_rn(w[j], ws));
+            __syncwarp();
+            add(j0, xv, &more[0][0], 32);
           }
 #pragma unroll
-          for (int e = 0; e < 32; ++e) out[e] = round_f16(out[e] + round_f16(sub[e]));
+          for (int e = 0; e < 32; e += 2) {
+            const float2 r = round_f16x2(sub[e], sub[e + 1]);
+            out[e] += r.x;      // rounded by the store
+            out[e + 1] += r.y;
+          }
         }
         if (mok) {
           __half* const yr = p.y + m * p.N + n0 + c0;
@@ -467,41 +544,41 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
       }
       tc::fence_before();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(acc_empty + 8 * acc);
+      if (lane == 0) {
+        if constexpr (PAIR) tc::mbar_arrive_at(tc::at_rank(acc_empty + 8 * acc, 0));
+        else tc::mbar_arrive(acc_empty + 8 * acc);
+      }
       acc ^= 1;
       if (acc == 0) ph ^= 1u;
     }
   }
   if (!ok && err) *err = 1u;
   tc::fence_before();
+  if constexpr (PAIR) tc::cluster_sync();   // the other CTA's shared memory is read until its last product
   __syncthreads();
-  if (warp == kI8EpiWarps) tc::tmem_free<2 * BN>(tmem);
+  if (warp == kI8EpiWarps) {
+    __syncwarp();
+    if constexpr (PAIR) tc::tmem_free_pair<2 * BN>(tmem);
+    else tc::tmem_free<2 * BN>(tmem);
+  }
 }
 
-template <int BN>
+template <bool PAIR>
 static cudaError_t launch_i8_gemm(const I8Params& p, cudaStream_t st) {
-  using C = I8Tile<BN>;
   static PerDeviceOnce once;
   if (once.need()) {
-    const cudaError_t e = cudaFuncSetAttribute(int8_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+    const cudaError_t e = cudaFuncSetAttribute(int8_gemm_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI8Smem);
     if (e != cudaSuccess) return e;
     once.done();
   }
   alignas(64) CUtensorMap ma, mb;
-  if (!tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.ca, p.M, p.K, p.K, 128) || !tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.cb, p.N, p.K, p.K, BN))
+  if (!tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.ca, p.M, p.K, p.K, 128) || !tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.cb, p.N, p.K, p.K, 128))
     return cudaErrorInvalidValue;
-  const int mt = (int)((p.M + 127) / 128), nt = (int)((p.N + BN - 1) / BN);
-  const int64_t tiles = (int64_t)mt * nt;
-  const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-  return launch(int8_gemm_kernel<BN>, dim3((unsigned)grid), dim3(kI8GemmThreads), (size_t)C::kSmem, st, p, ma, mb, mt, nt, wait_error_word());
-}
-
-// Features per tile: the wider tile reads less shared memory per product (a full tile of 256 takes 1.9 x one of 128), the narrower leaves a
-// smaller remainder in the last round over the SMs -- the smaller number of rounds x tile time wins.
-static cudaError_t launch_i8_gemm(const I8Params& p, cudaStream_t st) {
-  const int64_t mt = (p.M + 127) / 128, sms = sm_count();
-  const int64_t r256 = (mt * ((p.N + 255) / 256) + sms - 1) / sms, r128 = (mt * ((p.N + 127) / 128) + sms - 1) / sms;
-  return r256 * 19 <= r128 * 10 ? launch_i8_gemm<256>(p, st) : launch_i8_gemm<128>(p, st);
+  constexpr int CTAS = PAIR ? 2 : 1, BN = 128 * CTAS;
+  const int mt = (int)((p.M + BN - 1) / BN), nt = (int)((p.N + BN - 1) / BN);
+  const int64_t tiles = (int64_t)mt * nt, most = sm_count() / CTAS;
+  const dim3 grid((unsigned)((tiles < most ? tiles : most) * CTAS));
+  return launch_cluster(int8_gemm_kernel<PAIR>, grid, dim3(kI8GemmThreads), CTAS, (size_t)kI8Smem, st, p, ma, mb, mt, nt, wait_error_word());
 }
 
 }  // namespace b200
@@ -563,7 +640,7 @@ int b200_linear_int8(const b200_linear_int8_args* a, b200_stream_t stream) {
   int8_t* ca = reinterpret_cast<int8_t*>(ws + (size_t)a->K * 8 + 16 + (((size_t)a->M * 4 + 15) & ~(size_t)15));
   const __half* x = reinterpret_cast<const __half*>(a->x);
   cudaStream_t st = (cudaStream_t)stream;
-  const int block_rows = a->M <= 32 * 4096 ? 32 : 64;
+  const int block_rows = a->M <= 8 * 65535 ? 8 : 64;   // eight loads in flight per thread, as many CTAs as the grid allows
   const dim3 fg((unsigned)((a->K / 8 + 127) / 128), (unsigned)((a->M + block_rows - 1) / block_rows));
   cudaError_t e = fg.y > 1 ? cudaMemsetAsync(flags, 0, (size_t)a->K * sizeof(int), st) : cudaSuccess;
   if (e == cudaSuccess) e = launch(int8_outlier_flags_kernel, fg, dim3(128), 0, st, x, a->M, a->K, a->threshold, block_rows, flags);
@@ -580,7 +657,7 @@ int b200_linear_int8(const b200_linear_int8_args* a, b200_stream_t stream) {
     const dim3 gv((unsigned)((a->N + 15) / 16));
     if (a->M <= 8) e = launch(int8_gemv_kernel<1>, gv, dim3(kI8Threads), 0, st, p);
     else if (a->M <= 16) e = launch(int8_gemv_kernel<2>, gv, dim3(kI8Threads), 0, st, p);
-    else e = launch_i8_gemm(p, st);
+    else e = a->M > 128 ? launch_i8_gemm<true>(p, st) : launch_i8_gemm<false>(p, st);
   }
   if (e != cudaSuccess) {
     set_error("b200_linear_int8: launch failed: %s", cudaGetErrorString(e));
