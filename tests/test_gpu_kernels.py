@@ -723,3 +723,33 @@ def test_qlinear_double_quant_modes(K, mode):
     _check_gemv(lin(x.cuda()).cpu(), x, torch.from_numpy(deq))
     xm = _randw((64, 1024), 23, std=1.0)
     _check_gemv(lin(xm.cuda()).cpu(), xm, torch.from_numpy(deq))
+
+
+@pytest.mark.parametrize("B,T,H,G,hs,n,max_seq,table,pos_dtype", [
+    (1, 5, 8, 2, 128, 128, 16, torch.float32, torch.int64),     # whole heads turned
+    (2, 3, 6, 3, 128, 64, 9, torch.bfloat16, torch.int32),      # half of each head passes through
+    (1, 7, 4, 4, 64, 16, 32, torch.float32, torch.int32),       # one turned unit, three passed through
+    (1, 2, 40, 40, 80, 32, 8, torch.bfloat16, torch.int64),     # five units per head: threads left over, more heads than lanes
+    (1, 4, 4, 2, 64, 0, 8, torch.float32, torch.int64),         # nothing turned
+    (1, 4, 4, 2, 64, 24, 8, torch.float32, torch.int64),        # a rotated part that is no whole unit: the element-wise kernel
+    (1, 4, 4, 1, 40, 40, 8, torch.bfloat16, torch.int64),       # a head that is no whole unit
+])
+@pytest.mark.parametrize("preselected", [False, True])
+def test_rope_kv_append_units(K, B, T, H, G, hs, n, max_seq, table, pos_dtype, preselected):
+    g = torch.Generator().manual_seed(hs + n)
+    qkv = torch.randn(B, T, (H + 2 * G) * hs, generator=g).bfloat16()
+    cos, sin = (torch.randn(max_seq, n, generator=g).to(table) for _ in range(2))   # arbitrary tables: both halves are read
+    pos = torch.arange(max_seq - T, max_seq)
+    kc = torch.zeros(B, G, max_seq, hs, dtype=torch.bfloat16, device="cuda")
+    vc = torch.zeros_like(kc)
+    c, s = cos[pos], sin[pos]
+    tabs = (c, s) if preselected else (cos, sin)
+    if n == 0:
+        tabs = (torch.zeros(1), torch.zeros(1))
+    q = K.rope_kv_append(qkv.cuda(), tabs[0].cuda(), tabs[1].cuda(), pos.to(pos_dtype).cuda(), kc, vc, H, G, hs, n, table_preselected=preselected)
+    qpk = H // G
+    qq, kk, vv = qkv.view(B, T, G, qpk + 2, hs).permute(0, 2, 3, 1, 4).split((qpk, 1, 1), dim=2)
+    turned = lambda x: torch.cat((M.apply_rope(x[..., :n], c, s), x[..., n:]), -1) if n else x   # noqa: E731
+    assert torch.equal(q.cpu(), turned(qq.reshape(B, H, T, hs)))
+    assert torch.equal(kc[:, :, pos].cpu(), turned(kk.reshape(B, G, T, hs))) and torch.equal(vc[:, :, pos].cpu(), vv.reshape(B, G, T, hs))
+    assert kc[:, :, : max_seq - T].abs().sum() == 0
