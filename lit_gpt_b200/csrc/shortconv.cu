@@ -64,11 +64,15 @@ __device__ __forceinline__ void load_pair<float>(const float* p, int64_t i, bool
   }
 }
 
-// NIT: 64-element pieces of the widest head; TAPS: the number of taps when it is one of the unrolled ones, else 0 (read at run time)
+// NIT: 64-element pieces of the widest head; TAPS: the number of taps when it is one of the unrolled ones, else 0 (read at run time).
+// A warp walks rows_per_warp neighbouring rows of its head: the taps' weights are read once and, with unrolled taps, the rows that earlier
+// taps need stay in registers, so a row is read once instead of once per tap (and fetched one row ahead).  Bound: instructions -- the
+// division of silu, the norm's reduction, the rotation's sine.
 template <typename T, int NIT, int TAPS>
 __global__ void __launch_bounds__(kCvThreads) short_conv_kernel(const T* __restrict__ in, int64_t ld_in, CvParams P,
                                                                  const T* __restrict__ tail, int64_t tail_slot_stride, int tail_cols,
-                                                                 const int4* __restrict__ seqs, const int* __restrict__ row_seq, int pairs) {
+                                                                 const int4* __restrict__ seqs, const int* __restrict__ row_seq, int64_t rows,
+                                                                 int rows_per_warp, int pairs) {
   griddep_launch();
   griddep_wait();
   const int lane = threadIdx.x & 31;
@@ -77,89 +81,157 @@ __global__ void __launch_bounds__(kCvThreads) short_conv_kernel(const T* __restr
   int gi = 0;
   while (gi + 1 < P.n_groups && hh >= P.g[gi].heads) { hh -= P.g[gi].heads; ++gi; }
   const CvGroup& G = P.g[gi];
-  const int64_t row = blockIdx.x;
-  const int4 sq = seqs[row_seq[row]];
-  const int r = (int)(row - sq.x);            // row within the step's part of its sequence
-  const int pos = sq.z + r;
+  const int64_t row0 = (int64_t)blockIdx.x * rows_per_warp, row1 = row0 + rows_per_warp < rows ? row0 + rows_per_warp : rows;
   const int taps = TAPS ? TAPS : P.taps;
-  const T* tl = tail + (int64_t)sq.w * tail_slot_stride;
   const T* wt = reinterpret_cast<const T*>(G.w);
   const int c_head = G.col0 + hh * G.dim;     // first channel of this head among the convolved columns
   const bool pair = (pairs & 1) != 0;
   const bool wvec = TAPS == 4 && (pairs & 2) != 0;   // the eight taps of two neighbouring channels in one 16-byte (fp32: 32-byte) access
+  const bool out_pair = (pairs & 4) != 0;
+  constexpr int HIST = TAPS ? TAPS - 1 : 0, WT = TAPS ? TAPS : 1;
 
-  float val[NIT][2];
-  float ss = 0.f;
+  float w[NIT][2][WT];                        // the taps of this lane's channels
+  if constexpr (TAPS != 0) {
 #pragma unroll
-  for (int it = 0; it < NIT; ++it) {
-    const int d = it * 64 + lane * 2;
-    float acc0 = 0.f, acc1 = 0.f;
-    if (d < G.dim) {
-      const bool second = d + 1 < G.dim;
-      const int c = c_head + d;
-      const T* wc = wt + (int64_t)(hh * G.dim + d) * taps;
-      float wf[8];
-      if (wvec) load8(wc, wf);
+    for (int it = 0; it < NIT; ++it) {
+      const int d = it * 64 + lane * 2;
 #pragma unroll
-      for (int j = 0; j < (TAPS ? TAPS : kCvMaxTaps + 1); ++j) {
-        if (!TAPS && j >= taps) break;
-        const int back = taps - 1 - j;       // how many positions before this row
-        float u0 = 0.f, u1 = 0.f;
-        if (back <= pos) {                   // else: before the sequence's first token, zero
-          if (back <= r) load_pair(in, (row - back) * ld_in + c, pair, second, u0, u1);
-          else load_pair(tl, (int64_t)(taps - 1 - (back - r)) * tail_cols + c, pair, second, u0, u1);   // tail row taps-1-k: the k-th row before the step
+      for (int j = 0; j < TAPS; ++j) w[it][0][j] = w[it][1][j] = 0.f;
+      if (d < G.dim) {
+        const T* wc = wt + (int64_t)(hh * G.dim + d) * TAPS;
+        if constexpr (TAPS == 4) {
+          if (wvec) {
+            float wf[8];
+            load8(wc, wf);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { w[it][0][j] = wf[j]; w[it][1][j] = wf[4 + j]; }
+            continue;
+          }
         }
-        if (wvec) {
-          acc0 = fmaf(wf[j & 3], u0, acc0);
-          acc1 = fmaf(wf[4 + (j & 3)], u1, acc1);
-        } else {
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+          w[it][0][j] = load_as_float(wc, j);
+          if (d + 1 < G.dim) w[it][1][j] = load_as_float(wc, TAPS + j);
+        }
+      }
+    }
+  }
+  // the value `back` positions before row `row` (whose sequence's description is sq) in this lane's channels of piece `it`
+  auto fetch = [&](int64_t row, const int4& sq, int back, int it, float& u0, float& u1) {
+    u0 = u1 = 0.f;
+    const int d = it * 64 + lane * 2;
+    if (d >= G.dim) return;
+    const bool second = d + 1 < G.dim;
+    const int c = c_head + d, r = (int)(row - sq.x);   // row within the step's part of its sequence
+    if (back > sq.z + r) return;                       // before the sequence's first token: zero
+    if (back <= r) load_pair(in, (row - back) * ld_in + c, pair, second, u0, u1);
+    else load_pair(tail + (int64_t)sq.w * tail_slot_stride, (int64_t)(taps - 1 - (back - r)) * tail_cols + c, pair, second, u0, u1);   // tail row taps-1-k: the k-th row before the step
+  };
+
+  float hist[HIST ? HIST : 1][NIT][2], next[NIT][2];   // hist[j]: the input of tap j
+  int seq = -1;
+  int4 sq = make_int4(0, 0, 0, 0);
+  for (int64_t row = row0; row < row1; ++row) {
+    const int s = row_seq[row];
+    if (s != seq) {
+      seq = s;
+      sq = seqs[s];
+      if constexpr (TAPS != 0) {
+#pragma unroll
+        for (int it = 0; it < NIT; ++it) {
+#pragma unroll
+          for (int j = 0; j < HIST; ++j) fetch(row, sq, TAPS - 1 - j, it, hist[j][it][0], hist[j][it][1]);
+          fetch(row, sq, 0, it, next[it][0], next[it][1]);
+        }
+      }
+    }
+    const int pos = sq.z + (int)(row - sq.x);
+    float val[NIT][2];
+    float ss = 0.f;
+    float cur[NIT][2];
+    if constexpr (TAPS != 0) {
+#pragma unroll
+      for (int it = 0; it < NIT; ++it) {
+        cur[it][0] = next[it][0];
+        cur[it][1] = next[it][1];
+        if (row + 1 < row1 && row + 1 < (int64_t)sq.x + sq.y) fetch(row + 1, sq, 0, it, next[it][0], next[it][1]);
+      }
+    }
+#pragma unroll
+    for (int it = 0; it < NIT; ++it) {
+      const int d = it * 64 + lane * 2;
+      float acc0 = 0.f, acc1 = 0.f;
+      if constexpr (TAPS != 0) {
+#pragma unroll
+        for (int j = 0; j < HIST; ++j) {
+          acc0 = fmaf(w[it][0][j], hist[j][it][0], acc0);
+          acc1 = fmaf(w[it][1][j], hist[j][it][1], acc1);
+        }
+        acc0 = fmaf(w[it][0][WT - 1], cur[it][0], acc0);
+        acc1 = fmaf(w[it][1][WT - 1], cur[it][1], acc1);
+#pragma unroll
+        for (int j = 0; j + 1 < HIST; ++j) { hist[j][it][0] = hist[j + 1][it][0]; hist[j][it][1] = hist[j + 1][it][1]; }
+        if constexpr (HIST > 0) { hist[HIST - 1][it][0] = cur[it][0]; hist[HIST - 1][it][1] = cur[it][1]; }
+      } else if (d < G.dim) {
+        const T* wc = wt + (int64_t)(hh * G.dim + d) * taps;
+#pragma unroll
+        for (int j = 0; j < kCvMaxTaps + 1; ++j) {
+          if (j >= taps) break;
+          float u0, u1;
+          fetch(row, sq, taps - 1 - j, it, u0, u1);
           acc0 = fmaf(load_as_float(wc, j), u0, acc0);
-          if (second) acc1 = fmaf(load_as_float(wc, taps + j), u1, acc1);
+          if (d + 1 < G.dim) acc1 = fmaf(load_as_float(wc, taps + j), u1, acc1);
         }
       }
       if (G.act == 1) {
         acc0 = acc0 / (1.0f + expf(-acc0));
         acc1 = acc1 / (1.0f + expf(-acc1));
       }
+      val[it][0] = acc0;
+      val[it][1] = acc1;
     }
-    val[it][0] = acc0;
-    val[it][1] = acc1;
-  }
-  if (G.post == 1) {
+    if (G.post == 1) {
+#pragma unroll
+      for (int it = 0; it < NIT; ++it) {
+        const int d = it * 64 + lane * 2;
+        if (d + 1 < G.rot_dims && d + 1 < G.dim) {
+          // the angle in double, reduced to [-pi, pi] before the fp32 sine and cosine: exact to fp32 at any position
+          double a = (double)pos * G.inv_freq[d >> 1];
+          a -= 6.283185307179586476925286766559 * rint(a * 0.15915494309189533576888376337251);
+          float sn, cs;
+          sincosf((float)a, &sn, &cs);
+          sn *= G.rot_mscale;
+          cs *= G.rot_mscale;
+          const float u = val[it][0], v = val[it][1];
+          val[it][0] = u * cs - v * sn;
+          val[it][1] = v * cs + u * sn;
+        }
+      }
+    }
+    if (G.post != 0) {
+#pragma unroll
+      for (int it = 0; it < NIT; ++it) ss += val[it][0] * val[it][0] + val[it][1] * val[it][1];   // lanes past dim hold zeros
+      ss = warp_sum(ss);
+    }
+    float mul = G.post_scale;
+    if (G.post == 1) mul *= 1.0f / sqrtf(ss / (float)G.dim + G.eps);
+    else if (G.post == 2) mul *= 1.0f / sqrtf(ss + G.eps);
 #pragma unroll
     for (int it = 0; it < NIT; ++it) {
       const int d = it * 64 + lane * 2;
-      if (d + 1 < G.rot_dims && d + 1 < G.dim) {
-        // the angle in double, reduced to [-pi, pi] before the fp32 sine and cosine: exact to fp32 at any position
-        double a = (double)pos * G.inv_freq[d >> 1];
-        a -= 6.283185307179586476925286766559 * rint(a * 0.15915494309189533576888376337251);
-        float sn, cs;
-        sincosf((float)a, &sn, &cs);
-        sn *= G.rot_mscale;
-        cs *= G.rot_mscale;
-        const float u = val[it][0], v = val[it][1];
-        val[it][0] = u * cs - v * sn;
-        val[it][1] = v * cs + u * sn;
+      if (d >= G.dim) continue;
+      const int64_t o = row * G.ld_out + (int64_t)hh * G.dim + d;
+      const float v0 = val[it][0] * mul, v1 = val[it][1] * mul;
+      if (out_pair) {
+        if (G.out_f32 || sizeof(T) == 4) *reinterpret_cast<float2*>(reinterpret_cast<float*>(G.out) + o) = make_float2(v0, v1);
+        else *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(G.out) + o) = pack_bf16(v0, v1);
+        continue;
       }
-    }
-  }
-  if (G.post != 0) {
 #pragma unroll
-    for (int it = 0; it < NIT; ++it) ss += val[it][0] * val[it][0] + val[it][1] * val[it][1];   // lanes past dim hold zeros
-    ss = warp_sum(ss);
-  }
-  float mul = G.post_scale;
-  if (G.post == 1) mul *= 1.0f / sqrtf(ss / (float)G.dim + G.eps);
-  else if (G.post == 2) mul *= 1.0f / sqrtf(ss + G.eps);
-#pragma unroll
-  for (int it = 0; it < NIT; ++it) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int d = it * 64 + lane * 2 + e;
-      if (d < G.dim) {
-        const int64_t o = row * G.ld_out + (int64_t)hh * G.dim + d;
-        if (G.out_f32) reinterpret_cast<float*>(G.out)[o] = val[it][e] * mul;
-        else store_from_float(reinterpret_cast<T*>(G.out), o, val[it][e] * mul);
+      for (int e = 0; e < 2; ++e) {
+        if (d + e >= G.dim) break;
+        if (G.out_f32) reinterpret_cast<float*>(G.out)[o + e] = e ? v1 : v0;
+        else store_from_float(reinterpret_cast<T*>(G.out), o + e, e ? v1 : v0);
       }
     }
   }
@@ -167,12 +239,15 @@ __global__ void __launch_bounds__(kCvThreads) short_conv_kernel(const T* __restr
 
 template <typename T, int NIT>
 cudaError_t short_conv_launch(int taps, dim3 grid, cudaStream_t st, const T* in, int64_t ld_in, const CvParams& P, const T* tail,
-                              int64_t tail_slot_stride, int tail_cols, const int4* seqs, const int* row_seq, int pairs) {
+                              int64_t tail_slot_stride, int tail_cols, const int4* seqs, const int* row_seq, int64_t rows, int rows_per_warp, int pairs) {
+  auto go = [&](auto kernel) {
+    return launch(kernel, grid, dim3(kCvThreads), 0, st, in, ld_in, P, tail, tail_slot_stride, tail_cols, seqs, row_seq, rows, rows_per_warp, pairs);
+  };
   switch (taps) {
-    case 2: return launch(short_conv_kernel<T, NIT, 2>, grid, dim3(kCvThreads), 0, st, in, ld_in, P, tail, tail_slot_stride, tail_cols, seqs, row_seq, pairs);
-    case 3: return launch(short_conv_kernel<T, NIT, 3>, grid, dim3(kCvThreads), 0, st, in, ld_in, P, tail, tail_slot_stride, tail_cols, seqs, row_seq, pairs);
-    case 4: return launch(short_conv_kernel<T, NIT, 4>, grid, dim3(kCvThreads), 0, st, in, ld_in, P, tail, tail_slot_stride, tail_cols, seqs, row_seq, pairs);
-    default: return launch(short_conv_kernel<T, NIT, 0>, grid, dim3(kCvThreads), 0, st, in, ld_in, P, tail, tail_slot_stride, tail_cols, seqs, row_seq, pairs);
+    case 2: return go(short_conv_kernel<T, NIT, 2>);
+    case 3: return go(short_conv_kernel<T, NIT, 3>);
+    case 4: return go(short_conv_kernel<T, NIT, 4>);
+    default: return go(short_conv_kernel<T, NIT, 0>);
   }
 }
 
@@ -234,26 +309,31 @@ int b200_short_conv(const void* in, int64_t ld_in, const b200_conv_group* groups
   }
   const int per = kCvThreads / 32;
   B200_CHECK_ARG((P.total_heads + per - 1) / per <= 65535, "b200_short_conv: too many heads");
-  const dim3 grid((unsigned)rows, (unsigned)((P.total_heads + per - 1) / per));
+  // Rows per warp: enough of them to spare the re-reads once the warps outnumber what the SMs hold at a time (about 32 each), else one
+  const int64_t warps = rows * P.total_heads;
+  const int rpw = warps >= (int64_t)sm_count() * 32 * 8 ? 8 : (warps >= (int64_t)sm_count() * 32 * 4 ? 4 : 1);
+  const dim3 grid((unsigned)((rows + rpw - 1) / rpw), (unsigned)((P.total_heads + per - 1) / per));
   // pairs of neighbouring channels are read with one access when every head starts on an even channel of even-pitched, aligned rows
   const size_t esz = dtype == B200_F32 ? 4 : 2;
   int pairs = (ld_in % 2 == 0) && (tail_cols % 2 == 0) && (tail_slot_stride % 2 == 0) && (reinterpret_cast<uintptr_t>(in) % (2 * esz) == 0) &&
               (reinterpret_cast<uintptr_t>(tail) % (2 * esz) == 0);
   int max_dim = 0;
-  bool w16 = true;
+  bool w16 = true, out2 = true;
   for (int i = 0; i < n_groups; ++i) {
     pairs = pairs && groups[i].dim % 2 == 0 && groups[i].col0 % 2 == 0;
     w16 = w16 && reinterpret_cast<uintptr_t>(groups[i].w) % 16 == 0;
+    out2 = out2 && groups[i].dim % 2 == 0 && groups[i].ld_out % 2 == 0 && reinterpret_cast<uintptr_t>(groups[i].out) % (groups[i].out_f32 ? 8 : 2 * esz) == 0;
     max_dim = groups[i].dim > max_dim ? groups[i].dim : max_dim;
   }
   if (pairs && w16) pairs |= 2;   // even channels times four taps: every pair's taps start on a 16-byte boundary
+  if (out2) pairs |= 4;
   cudaStream_t st = (cudaStream_t)stream;
   const int4* sq = reinterpret_cast<const int4*>(seqs);
   B200_FLOAT_TYPES(dtype, T, {
-    if (max_dim <= 64) B200_CUDA((short_conv_launch<T, 1>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, pairs)));
-    else if (max_dim <= 128) B200_CUDA((short_conv_launch<T, 2>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, pairs)));
-    else if (max_dim <= 256) B200_CUDA((short_conv_launch<T, 4>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, pairs)));
-    else B200_CUDA((short_conv_launch<T, kCvMaxIt>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, pairs)));
+    if (max_dim <= 64) B200_CUDA((short_conv_launch<T, 1>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows, rpw, pairs)));
+    else if (max_dim <= 128) B200_CUDA((short_conv_launch<T, 2>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows, rpw, pairs)));
+    else if (max_dim <= 256) B200_CUDA((short_conv_launch<T, 4>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows, rpw, pairs)));
+    else B200_CUDA((short_conv_launch<T, kCvMaxIt>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows, rpw, pairs)));
   });
   return B200_OK;
 }
