@@ -580,6 +580,11 @@ typedef struct b200_delta_rule_args {
 } b200_delta_rule_args;
 int64_t b200_delta_rule_state_floats(int dk, int dv);
 int b200_delta_rule(const b200_delta_rule_args* args, b200_stream_t stream);
+/* The same for prompts with keys of at most 128 numbers, 32 tokens at a time with matrix products instead of one by one (csrc/delta_chunk.cu).
+ * max_rows must be the longest sequence's rows.  b200_delta_rule_workspace_bytes: scratch that lets every launch cover as much as pays, 0 when
+ * the call is better served by b200_delta_rule; a smaller workspace (at least one chunk) works in more launches. */
+size_t b200_delta_rule_workspace_bytes(int max_rows, int n_seqs, int heads, int dk, int dv);
+int b200_delta_rule_chunked(const b200_delta_rule_args* args, void* workspace, size_t workspace_bytes, b200_stream_t stream);
 /* out[row, h, :] = dtype(o / sqrt(mean(o^2) + eps) * weight * gate(z) * out_scale) per head; gate 1 silu, 2 sigmoid; weight NULL: none */
 int b200_gated_rms_heads(const float* o, int64_t ldo, const void* z, int64_t ldz, const void* weight, void* out, int64_t ld_out, int64_t rows,
                          int heads, int dv, int gate, float eps, float out_scale, int dtype, b200_stream_t stream);

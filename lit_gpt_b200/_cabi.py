@@ -168,7 +168,8 @@ ACT_GELU, ACT_GELU_TANH, ACT_SILU, ACT_RELU2 = 0, 1, 2, 3
 
 # Entry points of the sources every model needs (library state, norms, sampling) and of the fp32-residual / latent-attention /
 # expert kernels: `load_core()` can serve them from a library built from those sources alone.
-_CORE_SOURCES = ("api.cu", "norm.cu", "sample.cu", "resid.cu", "latent.cu", "moe.cu", "attn_prefill.cu", "shortconv.cu", "delta.cu", "window_attn.cu",
+_CORE_SOURCES = ("api.cu", "norm.cu", "sample.cu", "resid.cu", "latent.cu", "moe.cu", "attn_prefill.cu", "shortconv.cu", "delta.cu",
+                 "delta_chunk.cu", "window_attn.cu",
                  "linear_attn.cu", "depth.cu", "rope.cu", "talk_attn.cu")
 _CORE_SIGNATURES = {
     "b200_embed_pos": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p]),
@@ -206,6 +207,8 @@ _CORE_SIGNATURES = {
     "b200_conv_tail_update": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_void_p, c_int, c_int, c_void_p]),
     "b200_delta_rule_state_floats": (c_int64, [c_int, c_int]),
     "b200_delta_rule": (c_int, [ctypes.POINTER(DeltaRuleArgs), c_void_p]),
+    "b200_delta_rule_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "b200_delta_rule_chunked": (c_int, [ctypes.POINTER(DeltaRuleArgs), c_void_p, c_size_t, c_void_p]),
     "b200_gated_rms_heads": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_float, c_float,
                                      c_int, c_void_p]),
     "b200_window_attn": (c_int, [ctypes.POINTER(WindowAttnArgs), c_void_p]),
