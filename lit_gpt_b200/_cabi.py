@@ -168,7 +168,7 @@ ACT_GELU, ACT_GELU_TANH, ACT_SILU, ACT_RELU2 = 0, 1, 2, 3
 
 # Entry points of the sources every model needs (library state, norms, sampling) and of the fp32-residual / latent-attention /
 # expert kernels: `load_core()` can serve them from a library built from those sources alone.
-_CORE_SOURCES = ("api.cu", "norm.cu", "sample.cu", "resid.cu", "latent.cu", "moe.cu", "attn_prefill.cu", "shortconv.cu", "delta.cu",
+_CORE_SOURCES = ("api.cu", "norm.cu", "sample.cu", "resid.cu", "latent.cu", "moe.cu", "attn_prefill.cu", "attn_tc05.cu", "shortconv.cu", "delta.cu",
                  "delta_chunk.cu", "window_attn.cu",
                  "linear_attn.cu", "depth.cu", "rope.cu", "talk_attn.cu")
 _CORE_SIGNATURES = {

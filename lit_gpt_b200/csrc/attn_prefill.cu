@@ -11,6 +11,7 @@
 // memory by cp.async; S = Q K^T and O += P V on mma.sync.m16n8k16 (bf16 -> fp32) with ldmatrix operand loads from
 // XOR-swizzled tiles.  The heads of one query group run in adjacent CTAs so the K/V tiles are shared through L2.
 // Output is written as (B, T, H * hs), the layout attn.proj consumes (model.py:653).
+#include "attn_tc05.cuh"
 #include "mma_tile.cuh"
 
 namespace b200 {
@@ -20,6 +21,11 @@ namespace {
 constexpr int kPfBM = 128;   // query rows per CTA
 constexpr int kPfBN = 64;    // keys per tile
 constexpr int kPfThreads = 256;
+constexpr float kLog2e = 1.4426950408889634f;
+// Plain causal (windowed, with a sink) prompts from this many rows on go to the tcgen05 kernel (attn_tc05.cu).  It starts slower -- tensor
+// memory, barriers, tiles of twice the rows and keys: 8.8 against 5.1 us for 17 rows, 8.0 against 8.2 us for 128 -- and steps faster: 18.6 against
+// 31.5 us for 600 rows of 32 heads, 230 against 589 us for 4096.
+constexpr int kTc05MinRows = 128;
 
 // Where the operands live, in elements.  The cached layout of the GQA models is (B, H or G, rows, HS); a ragged batch packs the
 // query rows of all sequences into one (rows, H * HS) matrix and gives, per sequence, seqs[b] = {first query row, query rows,
@@ -527,7 +533,13 @@ extern "C" int b200_attn_prefill(const void* q, const void* k_cache, const void*
   B200_CHECK_ARG(head_size == 64 || head_size == 128, "b200_attn_prefill: head_size must be 64 or 128 (got %d)", head_size);
   B200_CHECK_ARG(n_head <= 65535 && batch <= 65535, "b200_attn_prefill: grid too large");
   cudaStream_t st = (cudaStream_t)stream;
-  if (head_size == 128) {
+  if (T >= kTc05MinRows) {
+    const int64_t hs = head_size, plane = (int64_t)max_seq * hs;
+    const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, (__nv_bfloat16*)y, hs * n_head * T, hs * T, hs,
+                         n_groups * plane, plane, hs, n_groups * plane, plane, hs, hs * n_head * T, hs * n_head, nullptr, pos, pos_is_int64, 0, nullptr, 0, T, n_head,
+                         n_groups, max_seq, scale * kLog2e};
+    B200_CUDA(launch_attn_tc05(A, head_size, batch, st));
+  } else if (head_size == 128) {
     if (pos_is_int64) B200_CUDA((launch_prefill<128, int64_t>(q, k_cache, v_cache, pos, y, batch, T, n_head, n_groups, max_seq, scale, st)));
     else B200_CUDA((launch_prefill<128, int32_t>(q, k_cache, v_cache, pos, y, batch, T, n_head, n_groups, max_seq, scale, st)));
   } else {
@@ -548,9 +560,15 @@ extern "C" int b200_attn_prefill_ragged(const void* q, int64_t ldq, const void* 
   B200_CHECK_ARG(((ldq | ldk | ldv) & 7) == 0 && (ldy & 1) == 0, "b200_attn_prefill_ragged: leading dimensions must be multiples of 8 elements");
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(seqs)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(y) & 3) == 0, "b200_attn_prefill_ragged: operands must be 16-byte aligned");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (max_q_len >= kTc05MinRows) {
+    const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)y, 0, head_size, ldq, 0, head_size, ldk, 0, head_size,
+                         ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), nullptr, 0, 0, nullptr, 0, max_q_len, n_head, n_head, 0, scale * kLog2e};
+    B200_CUDA(launch_attn_tc05(A, head_size, n_seqs, st));
+    return B200_OK;
+  }
   const PfView vw{0, head_size, ldq, 0, head_size, ldk, 0, head_size, ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), 0, nullptr, 0,
                   nullptr, 0, nullptr, 0, 0, nullptr, 0, 0, 0, 0};
-  cudaStream_t st = (cudaStream_t)stream;
   if (head_size == 128) B200_CUDA((launch_prefill<128, int32_t>(q, k, v, nullptr, y, n_seqs, max_q_len, n_head, n_head, 0, scale, st, &vw)));
   else B200_CUDA((launch_prefill<64, int32_t>(q, k, v, nullptr, y, n_seqs, max_q_len, n_head, n_head, 0, scale, st, &vw)));
   return B200_OK;
@@ -577,6 +595,13 @@ extern "C" int b200_attn_prefill_window_ex(const void* q, int64_t ldq, const voi
   B200_CHECK_ARG(((ldq | ldk | ldv) & 7) == 0 && (ldy & 1) == 0, "b200_attn_prefill_window: leading dimensions must be multiples of 8 elements");
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(seqs)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(y) & 3) == 0, "b200_attn_prefill_window: operands must be 16-byte aligned");
+  if (!r1 && gate_mode == 0 && max_q_len >= kTc05MinRows) {
+    const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)y, 0, head_size, ldq, 0, head_size, ldk, 0, head_size,
+                         ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), nullptr, 0, window, reinterpret_cast<const __nv_bfloat16*>(sink), 1, max_q_len, n_head, n_kv_head,
+                         0, scale * kLog2e};
+    B200_CUDA(launch_attn_tc05(A, head_size, n_seqs, (cudaStream_t)stream));
+    return B200_OK;
+  }
   // every visible distance is below the window (or, without one, below the longest sequence of this step, which starts at 0)
   const int reach = window > 0 ? (window < max_q_len ? window : max_q_len) : max_q_len;
   const PfView vw{0, head_size, ldq, 0, head_size, ldk, 0, head_size, ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), window,
@@ -604,7 +629,6 @@ extern "C" int b200_window_attn_tiles(const b200_window_attn_args* a, b200_strea
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(a->q) | reinterpret_cast<uintptr_t>(a->k) | reinterpret_cast<uintptr_t>(a->v) |
                    reinterpret_cast<uintptr_t>(a->seqs)) & 15) == 0 && (reinterpret_cast<uintptr_t>(a->out) & 3) == 0,
                  "b200_window_attn_tiles: operands must be 16-byte aligned");
-  constexpr float kLog2e = 1.4426950408889634f;
   const PfView vw{0, a->dk, a->ldq, 0, a->dk, a->ldk, 0, a->dv, a->ldv, 0, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->window,
                   reinterpret_cast<const __nv_bfloat16*>(a->sink), 1, nullptr, 0, a->gate_mode ? reinterpret_cast<const __nv_bfloat16*>(a->gate) : nullptr,
                   a->ldg, a->gate_mode, nullptr, 0, 0, 0, 0, nullptr, nullptr, 0, a->dk, a->dv, a->keep, a->softcap * kLog2e,

@@ -753,3 +753,78 @@ def test_rope_kv_append_units(K, B, T, H, G, hs, n, max_seq, table, pos_dtype, p
     assert torch.equal(q.cpu(), turned(qq.reshape(B, H, T, hs)))
     assert torch.equal(kc[:, :, pos].cpu(), turned(kk.reshape(B, G, T, hs))) and torch.equal(vc[:, :, pos].cpu(), vv.reshape(B, G, T, hs))
     assert kc[:, :, : max_seq - T].abs().sum() == 0
+
+
+def _attn_exact(q, k, v, lim, low, scale, sink=None):
+    """q (T, H, hs), k and v (S, G, hs) in 64 bits: row t sees keys low[t] .. lim[t]; sink: a logit per head in the denominator"""
+    T, H, _ = q.shape
+    k, v = (t.double().repeat_interleave(H // t.shape[1], 1).transpose(0, 1) for t in (k, v))
+    s = torch.einsum("thd,hjd->htj", q.double(), k) * scale
+    j = torch.arange(k.shape[1])
+    s = s.masked_fill(((j[None] > lim[:, None]) | (j[None] < low[:, None]))[None], float("-inf"))
+    if sink is not None:
+        s = torch.cat((s, sink.double().view(H, 1, 1).expand(H, T, 1)), 2)
+    return torch.einsum("htj,hjd->thd", torch.softmax(s, -1)[..., : k.shape[1]], v).reshape(T, -1)
+
+
+def _attn_close(y, ref):
+    """Two roundings to bf16, of the weights and of the result, each at most 2^-9 of its number"""
+    d = y.double().cpu() - ref
+    assert d.norm() <= 2.0 ** -8 * ref.norm(), (d.norm() / ref.norm()).item()
+    assert d.abs().max() <= 2.0 ** -5 * ref.abs().max()
+
+
+@pytest.mark.parametrize("T,start,tail", [(128, 0, 0), (129, 0, 7), (255, 130, 0), (256, 128, 128), (257, 0, 1), (300, 1, 200), (640, 0, 0), (130, 1000, 3)])
+@pytest.mark.parametrize("B,H,G,hs,pos_dtype", [(1, 4, 4, 128, torch.int64), (2, 8, 2, 64, torch.int32)])
+def test_attn_prefill_tiles(K, T, start, tail, B, H, G, hs, pos_dtype):
+    """Rows and keys on either side of the tiles of the prompt kernel; whatever lies behind the last position must not be seen."""
+    g = torch.Generator().manual_seed(T + start)
+    S = start + T + tail
+    q, k, v = (torch.randn(B, n, r, hs, generator=g).bfloat16() for n, r in ((H, T), (G, S), (G, S)))
+    k[:, :, start + T :], v[:, :, start + T :] = float("nan"), float("nan")
+    pos = torch.arange(start, start + T)
+    y = K.attn_prefill(q.cuda(), k.cuda(), v.cuda(), pos.to(pos_dtype).cuda())
+    for b in range(B):
+        n = start + T
+        _attn_close(y[b], _attn_exact(q[b].transpose(0, 1), k[b, :, :n].transpose(0, 1), v[b, :, :n].transpose(0, 1), pos, torch.zeros_like(pos), hs ** -0.5))
+
+
+def test_attn_prefill_tiles_sharp_rows_and_any_positions(K):
+    """Scores that grow from tile to tile (every step moves the maximum, by far), and positions with gaps and out of order."""
+    H, T, S, hs = 2, 200, 700, 128
+    g = torch.Generator().manual_seed(3)
+    q = torch.randn(1, H, T, hs, generator=g).bfloat16()
+    k = (torch.randn(1, H, S, hs, generator=g) * torch.linspace(0.1, 6.0, S).view(1, 1, S, 1)).bfloat16()
+    v = torch.randn(1, H, S, hs, generator=g).bfloat16()
+    pos = torch.randperm(S, generator=g)[:T]
+    y = K.attn_prefill(q.cuda(), k.cuda(), v.cuda(), pos.cuda(), 0.5)
+    _attn_close(y[0], _attn_exact(q[0].transpose(0, 1), k[0].transpose(0, 1), v[0].transpose(0, 1), pos, torch.zeros_like(pos), 0.5))
+
+
+@pytest.mark.parametrize("window", [0, 1, 127, 128, 129, 300])
+@pytest.mark.parametrize("hs,H,G", [(128, 4, 2), (64, 3, 3)])
+def test_attn_window_tiles(K, window, hs, H, G):
+    """Packed ragged prompts with a window and a sink: windows ending on either side of a key tile, a sequence of one row, rows between heads
+    of other columns; the next sequence's rows are poisoned in turn."""
+    from lit_gpt_b200 import _cabi as C
+
+    lens = (400, 1, 257)
+    g = torch.Generator().manual_seed(window)
+    n, ld = sum(lens), (H + 2 * G) * hs + 8
+    rows = torch.randn(n, ld, generator=g).bfloat16()
+    sink = torch.randn(H, generator=g).bfloat16()
+    sink_dev = sink.cuda()
+    first = [0, 400, 401]
+    for i, m in enumerate(lens):
+        buf = torch.full_like(rows, float("nan"))
+        buf[first[i] : first[i] + m] = rows[first[i] : first[i] + m]
+        dev = buf.cuda()
+        seqs = torch.tensor([[first[i], m, 0, 0]], dtype=torch.int32, device="cuda")
+        y = torch.zeros(n, H * hs, dtype=torch.bfloat16, device="cuda")
+        C.check(C.load().b200_attn_prefill_window(dev.data_ptr(), ld, dev[:, H * hs :].data_ptr(), ld, dev[:, (H + G) * hs :].data_ptr(), ld, seqs.data_ptr(), 1,
+                                                  max(lens), y.data_ptr(), H * hs, H, G, hs, 0.3, window, sink_dev.data_ptr(), C.stream_ptr()), "window")
+        part = rows[first[i] : first[i] + m]
+        q, k, v = part[:, : H * hs].view(m, H, hs), part[:, H * hs : (H + G) * hs].view(m, G, hs), part[:, (H + G) * hs : (H + 2 * G) * hs].view(m, G, hs)
+        lim = torch.arange(m)
+        low = lim - window + 1 if window else torch.zeros_like(lim)
+        _attn_close(y[first[i] : first[i] + m], _attn_exact(q, k, v, lim, low, 0.3, sink))
