@@ -1,24 +1,22 @@
-// Prefill GEMM: y (M, N) = x (M, K) . dequant(W)^T on the 5th-generation tensor cores (tcgen05 + TMEM), DESIGN.md §5.4.
+// Prefill GEMM: y (M, N) = x (M, K) . dequant(W)^T on the 5th-generation tensor cores (tcgen05 + TMEM).
 //
 // Replaces, for T > 16 rows, bnb.nn.Linear4bit.forward's "dequantize_4bit of the WHOLE weight to bf16, then F.linear"
-// (SURVEY Q1; call sites lit_gpt/model.py:519,619,656,713,714,716): the bf16 weight is never materialised in HBM.
-// Each CTA owns a (128 * MT tokens) x (128 output features) tile and walks K in blocks of 64:
-//   * the ACTIVATION tiles (128 tokens x 64 k, bf16) are fetched by TMA (cp.async.bulk.tensor.2d over a tensor map of x,
-//     SWIZZLE_128B, rows past M zero-filled by the hardware) straight into the tensor core's K-major layout;
-//   * 16 PRODUCER warps read the packed 4-bit weights (8 B = 16 codes per thread per k-block) and their absmax /
-//     {scale, zero}, rebuild the bf16 values with exactly the dequantise kernel's arithmetic
-//     (bf16_rn(code_fp32 * absmax_fp32), resp. bf16_rn(scale * (q - zero))) and write them, together with the
-//     activation tile, into shared memory in the tensor core's K-major 128-byte-swizzled layout;
-//   * ONE thread issues tcgen05.mma (cta_group::1, kind::f16, bf16 x bf16 -> fp32, M = 128, N = 128, K = 16) over
-//     shared-memory matrix descriptors; the fp32 accumulators live in TENSOR MEMORY (128 lanes x 128 columns per
-//     M sub-tile); tcgen05.commit hands each shared-memory stage back to the producers through an mbarrier;
-//   * 4 EPILOGUE warps (the first four producer warps, once K is exhausted) read the accumulators with tcgen05.ld
-//     (32 lanes x 32 columns per warp and instruction), add the bias, round to bf16 and store rows of y.
-// With MT = 2 one dequantised weight tile feeds 256 tokens, so the CUDA-core dequant (~500 clk per k-block) is
-// hidden under the tensor-core time (2 x 256 clk).
-#include <cuda.h>  // CUtensorMap (type only; the encoder is resolved at run time through the runtime, no -lcuda)
-
-#include "common.cuh"
+// (call sites lit_gpt/model.py:519,619,656,713,714,716): the bf16 weight is never materialised in HBM.
+// Persistent over output tiles of 256 features x 256 MT tokens, a CTA PAIR each (cta_group::2; up to 128 tokens: one CTA on 128 x 128),
+// walking K in blocks of 64.  Per CTA:
+//   * warps 0-15 rebuild the bf16 values of 128 features from the packed 4-bit weights and their absmax / {scale, zero} with exactly the
+//     dequantise kernel's arithmetic (bf16_rn(code_fp32 * absmax_fp32), resp. bf16_rn(scale * (q - zero))) and write them into shared memory in
+//     the tensor core's K-major 128-byte-swizzled layout.  Even and odd k-blocks belong to eight warps each: a warp has two blocks' time
+//     for its loads, look-ups and the proxy fence, and 32 codes a thread to overlap;
+//   * warp 16 fetches the activation tiles (128 tokens x 64 k per CTA and sub-tile) by TMA, rows past M zero-filled by the hardware;
+//   * warp 17 of the pair's first CTA issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, 256 x 256 x 16) into TENSOR MEMORY; tcgen05.commit
+//     hands each stage back to both CTAs;
+//   * the sixteen warps read the accumulators with tcgen05.ld, add the bias, round to bf16 and store rows of y.
+// Bound: with MT = 2 the tensor pipe and the shared memory that feeds it (a CTA alone on 128 x 128 reads 128 bytes a clock of it for the
+// products alone, the pair 64); one dequantised tile serves 512 tokens.  What was before -- a CTA on 128 features x 384 tokens, one thread that
+// loaded the activations between its own dequantising, every warp in every k-block -- spent 1750 clocks a k-block whatever the tokens.
+// 4096 tokens, 4096 -> 14336: int4 516 -> 390 us, nf4 591 -> 410; 14336 -> 4096: int4 532 -> 334 (1440 TFLOP/s), nf4 631 -> 356.
+#include "tc05.cuh"
 
 namespace b200 {
 
@@ -30,255 +28,268 @@ struct GemmParams {
   __nv_bfloat16* y;           // (M, N)
   int64_t M, N, K;
   int qtype;
-  int ksplit;                 // > 1 (grids that would not fill the SMs): blockIdx.z owns a range of k-blocks and writes fp32 partial sums
-  float* partial;             // (ksplit, M, N) fp32, summed in split order by qgemm_splitk_reduce_kernel
+  int ksplit;                 // > 1 (too few tiles for the SMs): an item owns a range of k-blocks and writes fp32 partial sums
+  float* partial;             // (ksplit, M, N) fp32, summed in range order by qgemm_splitk_reduce_kernel
+  int n_tiles, m_tiles;
 };
 
-constexpr int kGProducers = 512;            // 16 warps: 4 per scheduler, enough to hide the look-up latency
-constexpr int kGThreads = kGProducers + 32; // + the MMA / TMEM-allocator warp
-constexpr int kGStages = 4;
-constexpr int kBN = 128, kBK = 64;
+constexpr int kGDequant = 512, kGThreads = kGDequant + 64;   // 16 dequantising warps, the copies' and the products'
+constexpr int kBK = 64;
 constexpr int kTileBytes = 128 * kBK * 2;   // one 128-row x 64-k bf16 operand tile = 16 KB
-
-__device__ __forceinline__ uint32_t g_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void g_mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void g_mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void g_mbar_wait(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  do {
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  } while (!done);
-}
-
-// Shared-memory matrix descriptor, K-major operand, 128-byte swizzle (cute::UMMA::SmemDescriptor):
-//   [0,14) start address >> 4 | [16,30) leading byte offset >> 4 (unused for swizzled K-major: 1) |
-//   [32,46) stride byte offset >> 4 (8 rows x 128 B = 1024 B) | [46,48) version = 1 | [61,64) layout = 2 (SWIZZLE_128B)
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptor (cute::UMMA::InstrDescriptor): D = f32, A = B = bf16, both K-major, N = 128, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(kIdesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {  // arrives on `bar` when all MMAs issued so far have completed
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 
 // byte offset of the 16-byte chunk `c` (0..7) of row `r` inside a 128-row K-major SWIZZLE_128B tile
 __device__ __forceinline__ uint32_t sw128(int r, int c) { return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4)); }
 
-template <int MT, bool INT4>
-__global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap_x) {
+template <int CTAS>
+__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
+  // D = f32, A = B = bf16, both K-major, N = M = 128 per CTA of the group
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 * CTAS >> 3) << 17) | ((uint32_t)(128 * CTAS >> 4) << 24);
+  if constexpr (CTAS == 2)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+template <int MT>
+struct GemmTile {
+  static constexpr int kStages = MT == 2 ? 4 : 6;          // an even number: a stage belongs to one half of the dequantising warps
+  static constexpr int kStage = (MT + 1) * kTileBytes;     // MT activation tiles + 1 weight tile
+  static constexpr int kSmem = kStages * kStage + 1024;
+};
+
+template <int CTAS, int MT, bool INT4>
+__global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_x, unsigned* err) {
+  using C = GemmTile<MT>;
   extern __shared__ __align__(1024) uint8_t g_smem[];
-  constexpr int STAGE = (MT + 1) * kTileBytes;      // MT activation tiles + 1 weight tile
-  constexpr int TMEM_COLS = MT <= 2 ? 128 * MT : 512;   // a power of two (MT = 3: 384 accumulator columns of 512)
-  constexpr int NSTAGE = MT <= 2 ? kGStages : 3;          // MT = 3: 64 KB stages, three of them fit
-  __shared__ __align__(8) uint64_t s_bars[2 * kGStages + 1];
+  constexpr int BN = 128 * CTAS, BM = BN;           // features per tile, tokens per sub-tile
+  __shared__ __align__(8) uint64_t s_bars[2 * C::kStages + 2];
   __shared__ uint32_t s_tmem;
   __shared__ float s_code[16 * 32];                 // fp32 code book, one copy per lane (conflict-free look-ups)
-
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(g_smem) + 1023) & ~(uintptr_t)1023);
-  const uint32_t tiles_a = g_smem_u32(tiles);
-  const uint32_t full0 = g_smem_u32(&s_bars[0]), empty0 = g_smem_u32(&s_bars[kGStages]), done_bar = g_smem_u32(&s_bars[2 * kGStages]);
-  const int64_t n0 = (int64_t)blockIdx.x * kBN, m0 = (int64_t)blockIdx.y * (128 * MT);
-  // split-K (short prompts: the output tiles alone would leave most SMs idle): this CTA's k-blocks are [kb0, kb0 + nkb)
-  const int nkb_all = (int)(p.K / kBK);
-  const int kb0 = (int)(((int64_t)nkb_all * blockIdx.z) / p.ksplit);
-  const int nkb = (int)(((int64_t)nkb_all * (blockIdx.z + 1)) / p.ksplit) - kb0;
-  constexpr bool int4 = INT4;
-
+  const uint32_t rank = CTAS == 2 ? tc::cluster_rank() : 0u;
+  const uint32_t tiles = (tc::smem_u32(g_smem) + 1023u) & ~1023u;
+  const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]), acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_free = acc_full + 8;
   if (tid == 0) {
-    for (int s = 0; s < NSTAGE; ++s) { g_mbar_init(full0 + s * 8, kGProducers / 32 + 1); g_mbar_init(empty0 + s * 8, 1); }
-    g_mbar_init(done_bar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int s = 0; s < C::kStages; ++s) { tc::mbar_init(full + 8 * s, 8 * CTAS + 1); tc::mbar_init(empty + 8 * s, 1); }
+    tc::mbar_init(acc_full, 1);
+    tc::mbar_init(acc_free, 16 * CTAS);
+    tc::mbar_init_fence();
+    tc::prefetch_map(&map_x);
   }
-  if (!int4) {
+  if (!INT4)
     for (int i = tid; i < 16 * 32; i += kGThreads) s_code[i] = code_value(p.qtype, i >> 5);
+  if (warp == 17) {
+    if constexpr (CTAS == 2) tc::tmem_alloc_pair<BN * MT>(tc::smem_u32(&s_tmem));
+    else tc::tmem_alloc<BN * MT>(tc::smem_u32(&s_tmem));
   }
-  if (warp == kGProducers / 32) {  // the MMA warp also owns the tensor-memory allocation
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(g_smem_u32(&s_tmem)), "n"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  tc::fence_before();
+  if constexpr (CTAS == 2) tc::cluster_sync();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  tc::fence_after();
   const uint32_t tmem = s_tmem;
   griddep_launch();
   griddep_wait();
 
-  if (warp < kGProducers / 32) {
-    // =========================================== PRODUCERS ======================================================
-    // The activation tiles of k-block kb are requested by ONE thread with TMA (no LSU work, no registers); the packed
-    // weights and scales are prefetched into registers kWLag k-blocks ahead.  full[s] collects one arrival per warp
-    // (dequantised weight tile written) plus the TMA thread's expect_tx arrival; the TMA bytes complete the phase.
-    constexpr int kWLag = 2;
-    // weight tile: thread -> (row r = tid / 4, quarter h = tid % 4): 8 packed bytes = k [16h, 16h + 16) of the k-block
-    const int wr = tid >> 2, wh = tid & 3;
-    const int64_t wn = n0 + wr;
-    const bool wvalid = wn < p.N;
-    const uint8_t* wsrc = p.packed + (wvalid ? wn : 0) * (p.K >> 1) + wh * 8;
-    const uint32_t* ssrc = p.scale + (wvalid ? wn : 0) * (int4 ? (p.K >> 7) : (p.K >> 6));
-    uint2 qn[kWLag];
-    uint32_t scn[kWLag];
-#pragma unroll
-    for (int i = 0; i < kWLag; ++i) {
-      qn[i] = make_uint2(0u, 0u);
-      scn[i] = 0u;
-      if (i < nkb) { qn[i] = ldg_stream_v2(wsrc + (int64_t)(kb0 + i) * 32); scn[i] = ssrc[int4 ? ((kb0 + i) >> 1) : (kb0 + i)]; }
-    }
-    const uint32_t wdst0 = (uint32_t)(MT * kTileBytes) + sw128(wr, wh * 2), wdst1 = (uint32_t)(MT * kTileBytes) + sw128(wr, wh * 2 + 1);
-    // running state instead of per-iteration index arithmetic (the loop is bound by its instruction count: 139 -> ~105 per k-block):
-    // ring slot / parity, the packed-weight pointer and the k-block index of the look-ahead load (rows past N read row 0: in bounds)
-    const uint8_t* wp = wsrc + (int64_t)(kb0 + kWLag) * 32;
-    int kq = kb0 + kWLag;                 // absolute k-block of the next look-ahead load
-    int s = 0;
-    uint32_t eph = 1;                     // parity of the EMPTY phase to wait for (first lap: passes at once)
-    uint32_t st_a = tiles_a;              // shared-window address of the current stage
-    for (int kb = 0; kb < nkb; ++kb) {
-      g_mbar_wait(empty0 + s * 8, eph);
-      // ---- activation tiles: MT boxes of 128 rows x 64 k by TMA, issued by one thread ------------------------------
-      if (tid == 0) {
-        const uint32_t bar = full0 + s * 8;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(MT * kTileBytes) : "memory");
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-          asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                       ::"r"(st_a + (uint32_t)(mt * kTileBytes)), "l"(&tmap_x), "r"((kb0 + kb) * kBK), "r"((int)(m0 + mt * 128)), "r"(bar)
-                       : "memory");
-      }
-      // ---- weight tile: dequantise 16 codes -> 2 chunks of 8 bf16 ----------------------------------------------------
-      const uint2 q = qn[0];
-      const uint32_t sc = scn[0];
-#pragma unroll
-      for (int i = 0; i + 1 < kWLag; ++i) { qn[i] = qn[i + 1]; scn[i] = scn[i + 1]; }
-      if (kb + kWLag < nkb) { qn[kWLag - 1] = ldg_stream_v2(wp); scn[kWLag - 1] = ssrc[int4 ? (kq >> 1) : kq]; }
-      wp += 32; ++kq;
-      const uint32_t qw[2] = {q.x, q.y};
-      if (int4) {
-        // bf16_rn(scale * (q - zero)) with three instructions per code: the nibble is moved to the top four mantissa bits of 16.0f
-        // (SHF + LOP3: f = 16 + q exactly, five significant bits), then ONE FFMA scale * f - scale * (16 + zero): both products are
-        // exact in fp32 (11-bit fp16 scale x 6-bit integer), so the result is the exact scale * (q - zero), as before -- without the
-        // quarter-rate I2F per code that bound this loop
-        const __half2 h2 = *reinterpret_cast<const __half2*>(&sc);
-        const float scale = __low2float(h2);
-        const float c0 = -scale * (16.0f + __high2float(h2));
-        auto deq = [&](uint32_t w, int e) -> float {   // element e (bits 4e .. 4e + 3) of word w
-          const uint32_t sh = e <= 4 ? w << (19 - 4 * e) : w >> (4 * e - 19);
-          return fmaf(scale, __uint_as_float((sh & 0x00780000u) | 0x41800000u), c0);
-        };
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {  // word j = k [16h + 8j, +8), element e in bits 4e
-          uint32_t o[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) o[e] = pack_bf16(deq(qw[j], 2 * e), deq(qw[j], 2 * e + 1));
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(st_a + (j ? wdst1 : wdst0)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-        }
-      } else {
-        // bf16_rn(code_fp32 * absmax_fp32): look-up offset = nibble << 7 | lane << 2 from the table's (link-time constant) address:
-        // SHF + LOP3 + LDS per code
-        const float am = __uint_as_float(sc);
-        const uint32_t lane4 = (uint32_t)lane * 4u;
-        auto deq = [&](uint32_t w, int bit) -> float {   // the nibble at bits bit .. bit + 3 of word w
-          const uint32_t sh = bit <= 7 ? w << (7 - bit) : w >> (bit - 7);
-          return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(s_code) + ((sh & 0x780u) | lane4)) * am;
-        };
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {  // word j = bytes 4j..4j+3 = k [16h + 8j, +8); even element in the HIGH nibble
-          uint32_t o[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) o[e] = pack_bf16(deq(qw[j], 8 * e + 4), deq(qw[j], 8 * e));
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(st_a + (j ? wdst1 : wdst0)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // generic-proxy writes -> visible to the tensor core
-      __syncwarp();
-      if (lane == 0) g_mbar_arrive(full0 + s * 8);                       // weight tile of kb
-      st_a += STAGE;
-      if (++s == NSTAGE) { s = 0; eph ^= 1u; st_a = tiles_a; }
-    }
-  } else if (lane == 0) {
-    // =========================================== MMA ISSUER =====================================================
-    int s = 0;
-    uint32_t fph = 0;
-    for (int kb = 0; kb < nkb; ++kb) {
-      g_mbar_wait(full0 + s * 8, fph);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sa = tiles_a + s * STAGE;
-      const uint64_t db = umma_desc_sw128(sa + MT * kTileBytes);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const uint64_t da = umma_desc_sw128(sa + mt * kTileBytes);
-#pragma unroll
-        for (int k = 0; k < kBK / 16; ++k)  // +32 B along K inside the swizzle atom = +2 in the address field
-          umma_bf16(tmem + mt * 128, da + 2 * k, db + 2 * k, (kb | k) != 0);
-      }
-      umma_commit(empty0 + s * 8);   // stage reusable once these MMAs have read it (implies fence::before_thread_sync)
-      if (++s == NSTAGE) { s = 0; fph ^= 1u; }
-    }
-    umma_commit(done_bar);           // accumulators complete
-  }
+  const int nkb_all = (int)(p.K / kBK), total = p.n_tiles * p.m_tiles * p.ksplit;
+  struct Item { int64_t m0, n0; int z, kb0, nkb, mts; };
+  auto item = [&](int i) {
+    Item t;
+    const int z = i / (p.n_tiles * p.m_tiles), r = i - z * (p.n_tiles * p.m_tiles), m = r / p.n_tiles;
+    t.z = z;
+    t.m0 = (int64_t)m * (BM * MT);
+    t.n0 = (int64_t)(r - m * p.n_tiles) * BN;
+    t.kb0 = (int)(((int64_t)nkb_all * z) / p.ksplit);
+    t.nkb = (int)(((int64_t)nkb_all * (z + 1)) / p.ksplit) - t.kb0;
+    t.mts = MT == 1 || p.M - t.m0 <= BM ? 1 : MT;     // sub-tiles with tokens in them
+    return t;
+  };
+  const int first = (int)blockIdx.x / CTAS, step = (int)gridDim.x / CTAS;
+  bool ok = true;
+  int q = 0;                                          // k-blocks so far: stage q % kStages
 
-  // =============================================== EPILOGUE =======================================================
-  if (warp < 4) {
-    g_mbar_wait(done_bar, 0);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-    for (int mt = 0; mt < MT; ++mt) {
-      const int64_t m = m0 + mt * 128 + warp * 32 + lane;        // this thread's output row (TMEM lane = row)
-#pragma unroll 1
-      for (int c0 = 0; c0 < kBN; c0 += 32) {
-        uint32_t v[32];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * 128 + c0);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
-            "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-              "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-              "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-              "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (m < p.M && p.ksplit > 1) {
-          float* dst = p.partial + ((int64_t)blockIdx.z * p.M + m) * p.N;   // raw fp32 sums of this k range; bias and rounding in the reduce kernel
+  if (warp < 16) {
+    // =========================================== DEQUANTISE, THEN STORE =========================================
+    constexpr int LAG = 2;
+    const int g = warp >> 3, tg = tid & 255, wr = tg >> 1, wh = tg & 1;   // half of the warps, feature, half of the k-block
+    uint32_t acc_ph = 0;
+    for (int i = first; i < total && ok; i += step) {
+      const Item t = item(i);
+      const int64_t wn = t.n0 + rank * 128 + wr;
+      const bool wvalid = wn < p.N;
+      const uint8_t* wp = p.packed + (wvalid ? wn : 0) * (p.K >> 1) + (int64_t)t.kb0 * 32 + wh * 16;
+      const uint32_t* sp = p.scale + (wvalid ? wn : 0) * (INT4 ? (p.K >> 7) : (p.K >> 6));
+      const int l0 = (q + g) & 1;                     // this half's first k-block of the item
+      uint4 qn[LAG];
+      uint32_t sn[LAG];
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const int64_t n = n0 + c0 + j;
-            if (n < p.N) *reinterpret_cast<uint4*>(dst + n) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      for (int e = 0; e < LAG; ++e) {
+        const int l = l0 + 2 * e;
+        qn[e] = make_uint4(0u, 0u, 0u, 0u);
+        sn[e] = 0u;
+        if (l < t.nkb) { qn[e] = ldg_stream_v4(wp + (int64_t)l * 32); sn[e] = sp[INT4 ? ((t.kb0 + l) >> 1) : (t.kb0 + l)]; }
+      }
+      for (int l = l0; l < t.nkb; l += 2) {
+        const int s = (q + l) % C::kStages;
+        const uint32_t ph = (uint32_t)((q + l) / C::kStages) & 1u;
+        const uint4 w = qn[0];
+        const uint32_t sc = sn[0];
+#pragma unroll
+        for (int e = 0; e + 1 < LAG; ++e) { qn[e] = qn[e + 1]; sn[e] = sn[e + 1]; }
+        const int ln = l + 2 * LAG;
+        if (ln < t.nkb) { qn[LAG - 1] = ldg_stream_v4(wp + (int64_t)ln * 32); sn[LAG - 1] = sp[INT4 ? ((t.kb0 + ln) >> 1) : (t.kb0 + ln)]; }
+        const uint32_t qw[4] = {w.x, w.y, w.z, w.w};
+        const uint32_t dst = tiles + s * C::kStage + MT * kTileBytes;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(empty + 8 * s, ph ^ 1u));
+        if (!ok) break;
+        if (INT4) {
+          // bf16_rn(scale * (q - zero)) with three instructions per code: the nibble is moved to the top four mantissa bits of 16.0f
+          // (SHF + LOP3: f = 16 + q exactly, five significant bits), then ONE FFMA scale * f - scale * (16 + zero): both products are
+          // exact in fp32 (11-bit fp16 scale x 6-bit integer), so the result is the exact scale * (q - zero)
+          const __half2 h2 = *reinterpret_cast<const __half2*>(&sc);
+          const float scale = __low2float(h2);
+          const float c0 = -scale * (16.0f + __high2float(h2));
+          auto deq = [&](uint32_t v, int e) -> float {   // element e (bits 4e .. 4e + 3) of word v
+            const uint32_t sh = e <= 4 ? v << (19 - 4 * e) : v >> (4 * e - 19);
+            return fmaf(scale, __uint_as_float((sh & 0x00780000u) | 0x41800000u), c0);
+          };
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {  // word j = k [32 wh + 8j, +8), element e in bits 4e
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = pack_bf16(deq(qw[j], 2 * e), deq(qw[j], 2 * e + 1));
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + sw128(wr, wh * 4 + j)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
           }
-        } else if (m < p.M) {
+        } else {
+          // bf16_rn(code_fp32 * absmax_fp32): look-up offset = nibble << 7 | lane << 2 from the table's (link-time constant) address:
+          // SHF + LOP3 + LDS per code
+          const float am = __uint_as_float(sc);
+          const uint32_t lane4 = (uint32_t)lane * 4u;
+          auto deq = [&](uint32_t v, int bit) -> float {   // the nibble at bits bit .. bit + 3 of word v
+            const uint32_t sh = bit <= 7 ? v << (7 - bit) : v >> (bit - 7);
+            return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(s_code) + ((sh & 0x780u) | lane4)) * am;
+          };
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            const int64_t n = n0 + c0 + j;
-            if (n < p.N) {  // N % 8 == 0 (host check): a chunk is either fully inside or fully outside
-              uint32_t o[4];
+          for (int j = 0; j < 4; ++j) {  // word j = bytes 4j..4j+3 = k [32 wh + 8j, +8); even element in the HIGH nibble
+            uint32_t o[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                float a = __uint_as_float(v[j + 2 * e]), b = __uint_as_float(v[j + 2 * e + 1]);
-                if (p.bias) { a += __bfloat162float(p.bias[n + 2 * e]); b += __bfloat162float(p.bias[n + 2 * e + 1]); }
-                o[e] = pack_bf16(a, b);
+            for (int e = 0; e < 4; ++e) o[e] = pack_bf16(deq(qw[j], 8 * e + 4), deq(qw[j], 8 * e));
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + sw128(wr, wh * 4 + j)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+          }
+        }
+        tc::fence_smem_async();                       // generic-proxy writes -> visible to the tensor core
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (CTAS == 2) tc::mbar_signal_at(tc::at_rank(full + 8 * s, 0));
+          else tc::mbar_arrive(full + 8 * s);
+        }
+      }
+      q += t.nkb;
+      // ---- accumulators -> y (or partial sums): warp w has rows 32 (w % 4) .. + 31 and a quarter of the columns ----
+      ok = ok && __all_sync(0xffffffffu, tc::mbar_wait(acc_full, acc_ph));
+      acc_ph ^= 1u;
+      if (!ok) break;
+      tc::fence_after();
+#pragma unroll 1
+      for (int mt = 0; mt < t.mts; ++mt) {
+        const int64_t m = t.m0 + mt * BM + rank * 128 + (warp & 3) * 32 + lane;        // this thread's output row (TMEM lane = row)
+#pragma unroll 1
+        for (int c0 = (warp >> 2) * (BN / 4); c0 < ((warp >> 2) + 1) * (BN / 4); c0 += 32) {
+          uint32_t v[32];
+          tc::ld32(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * BN + c0));
+          tc::wait_ld(v);
+          if (m < p.M && p.ksplit > 1) {
+            float* dst = p.partial + ((int64_t)t.z * p.M + m) * p.N;   // raw fp32 sums of this k range; bias and rounding in the reduce kernel
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const int64_t n = t.n0 + c0 + j;
+              if (n < p.N) *reinterpret_cast<uint4*>(dst + n) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            }
+          } else if (m < p.M) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+              const int64_t n = t.n0 + c0 + j;
+              if (n < p.N) {  // N % 8 == 0 (host check): a chunk is either fully inside or fully outside
+                uint32_t o[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  float a = __uint_as_float(v[j + 2 * e]), b = __uint_as_float(v[j + 2 * e + 1]);
+                  if (p.bias) { a += __bfloat162float(p.bias[n + 2 * e]); b += __bfloat162float(p.bias[n + 2 * e + 1]); }
+                  o[e] = pack_bf16(a, b);
+                }
+                *reinterpret_cast<uint4*>(p.y + m * p.N + n) = make_uint4(o[0], o[1], o[2], o[3]);
               }
-              *reinterpret_cast<uint4*>(p.y + m * p.N + n) = make_uint4(o[0], o[1], o[2], o[3]);
             }
           }
         }
       }
+      tc::fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if constexpr (CTAS == 2) tc::mbar_arrive_at(tc::at_rank(acc_free, 0));
+        else tc::mbar_arrive(acc_free);
+      }
+    }
+  } else if (warp == 16) {
+    // =========================================== ACTIVATIONS ====================================================
+    if (lane == 0) {
+      for (int i = first; i < total && ok; i += step) {
+        const Item t = item(i);
+        for (int l = 0; l < t.nkb; ++l, ++q) {
+          const int s = q % C::kStages;
+          ok = tc::mbar_wait(empty + 8 * s, ((uint32_t)(q / C::kStages) & 1u) ^ 1u);
+          if (!ok) break;
+          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * t.mts * kTileBytes);
+          const uint32_t st = tiles + s * C::kStage, bar = CTAS == 2 ? tc::at_rank(full + 8 * s, 0) : full + 8 * s;
+          for (int mt = 0; mt < t.mts; ++mt) {
+            const int row = (int)(t.m0 + mt * BM + rank * 128), col = (t.kb0 + l) * kBK;
+            if constexpr (CTAS == 2) tc::tma_load_2d_pair(st + mt * kTileBytes, &map_x, col, row, bar);
+            else tc::tma_load_2d(st + mt * kTileBytes, &map_x, col, row, bar);
+          }
+        }
+      }
+      if (!ok && rank == 0)   // given up: no copy may still be on its way when the CTAs leave
+        for (int i = 0; i < C::kStages; ++i) tc::mbar_wait(full + 8 * i, (uint32_t)((q + C::kStages - 1 - i) / C::kStages + 1) & 1u);
+    }
+  } else if (lane == 0 && rank == 0) {
+    // =========================================== PRODUCTS =======================================================
+    uint32_t free_ph = 1;
+    for (int i = first; i < total && ok; i += step) {
+      const Item t = item(i);
+      ok = tc::mbar_wait(acc_free, free_ph);
+      free_ph ^= 1u;
+      tc::fence_after();
+      for (int l = 0; l < t.nkb && ok; ++l, ++q) {
+        const int s = q % C::kStages;
+        ok = tc::mbar_wait(full + 8 * s, (uint32_t)(q / C::kStages) & 1u);
+        if (!ok) break;
+        tc::fence_after();
+        const uint32_t st = tiles + s * C::kStage;
+        const uint64_t db = tc::desc_sw128(st + MT * kTileBytes);
+        for (int mt = 0; mt < t.mts; ++mt) {
+          const uint64_t da = tc::desc_sw128(st + mt * kTileBytes);
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)  // +32 B along K inside the swizzle atom = +2 in the address field
+            umma_bf16<CTAS>(tmem + mt * BN, da + 2 * k, db + 2 * k, (l | k) != 0);
+        }
+        if constexpr (CTAS == 2) tc::commit_pair(empty + 8 * s);   // the stage is free once these products have read it
+        else tc::commit(empty + 8 * s);
+      }
+      if (ok) {
+        if constexpr (CTAS == 2) tc::commit_pair(acc_full);
+        else tc::commit(acc_full);
+      }
     }
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if (!ok && err) *err = 1u;
+  tc::fence_before();
+  if constexpr (CTAS == 2) tc::cluster_sync();   // the other CTA's shared memory is read until its last product
   __syncthreads();
-  if (warp == kGProducers / 32) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM_COLS) : "memory");
+  if (warp == 17) {
+    __syncwarp();
+    if constexpr (CTAS == 2) tc::tmem_free_pair<BN * MT>(tmem);
+    else tc::tmem_free<BN * MT>(tmem);
   }
 }
 
@@ -308,65 +319,65 @@ __global__ void __launch_bounds__(256) qgemm_splitk_reduce_kernel(const float* _
   *reinterpret_cast<uint4*>(y + i) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-static std::atomic<int> g_gemm_mt3{1};   // development switch (b200_qgemm_tune)
+static std::atomic<int> g_gemm_wide{1};   // development switch (b200_qgemm_tune): 0 keeps to one sub-tile of 256 tokens
 
-// k ranges for prompts whose (M tiles) x (N / 128) CTAs leave SMs idle (up to ~1000 tokens at N = 4096): enough ranges to fill ONE wave
-// (a second, partial wave costs more than the idle SMs of the first), at least one lap of the four-stage ring per range, and at
-// most 64 MB of fp32 partial sums
-static int gemm_ksplit(int64_t M, int64_t N, int64_t K) {
+struct GemmPlan {
+  int ctas, mt, ksplit;
+};
+
+// Tile and k ranges by the time of the last SM to finish, in clocks as measured over launches of one round: a k-block takes about 1500 with two
+// sub-tiles of 256 tokens, 1130 with one (the dequantisation, which a second sub-tile shares), 950 for a CTA alone on 128 tokens; a tile
+// costs 6000 more to start and to store, partial sums of k ranges 13000 and a clock per 1860 bytes.  k ranges are for launches that leave
+// SMs idle -- two at least where half of them would be: at least four k-blocks per range, at most 16 ranges and 64 MB of partial sums, and
+// no more than fill the SMs once.
+static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool split_ok) {
   const int nkb = (int)(K / kBK);
-  const int64_t mtile = M > 512 && g_gemm_mt3.load() ? 384 : M > 128 ? 256 : 128;
-  const int64_t ctas = ((N + kBN - 1) / kBN) * ((M + mtile - 1) / mtile);
-  int64_t s = sm_count() / (ctas > 0 ? ctas : 1);
-  if (s > nkb / kGStages) s = nkb / kGStages;
-  if (s > 16) s = 16;
-  while (s > 1 && s * M * N * (int64_t)sizeof(float) > (64ll << 20)) --s;
-  return s < 1 ? 1 : (int)s;
+  const int64_t sms = sm_count();
+  GemmPlan best{1, 1, 1};
+  int64_t best_t = -1;
+  for (int kind = 0; kind < 3; ++kind) {
+    const int ctas = kind ? 2 : 1, mt = kind == 2 ? 2 : 1;
+    if (kind == 0 ? M > 128 : M <= 128) continue;            // a pair's second half would be padding; a CTA alone would dequantise twice
+    if (kind == 2 && (M <= 256 || !g_gemm_wide.load())) continue;
+    const int64_t units = sms / ctas, tiles = ((N + 128 * ctas - 1) / (128 * ctas)) * ((M + 128 * ctas * mt - 1) / (128 * ctas * mt));
+    int64_t most = split_ok ? units / tiles : 1;
+    if (most > nkb / 4) most = nkb / 4;
+    if (most > 16) most = 16;
+    while (most > 1 && most * M * N * (int64_t)sizeof(float) > (64ll << 20)) --most;
+    const int64_t per = kind == 0 ? 950 : kind == 1 ? 1130 : 1500;
+    for (int64_t s = most > 1 && tiles * 2 <= units ? 2 : 1; s <= (most < 1 ? 1 : most); ++s) {
+      const int64_t t = ((tiles * s + units - 1) / units) * (((nkb + s - 1) / s) * per + 6000) + (s > 1 ? 13000 + s * M * N * 4 / 1860 : 0);
+      if (best_t < 0 || t < best_t) { best_t = t; best = GemmPlan{ctas, mt, (int)s}; }
+    }
+  }
+  return best;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
-template <int MT, bool INT4>
-static cudaError_t launch_gemm_q(const GemmParams& p, cudaStream_t st) {
-  constexpr int smem = (MT <= 2 ? kGStages : 3) * (MT + 1) * kTileBytes + 1024;
+template <int CTAS, int MT, bool INT4>
+static cudaError_t launch_gemm(GemmParams p, cudaStream_t st) {
+  constexpr int smem = GemmTile<MT>::kSmem;
   static PerDeviceOnce once;
   if (once.need()) {
-    cudaError_t e = cudaFuncSetAttribute(qgemm_tcgen05_kernel<MT, INT4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(qgemm_tcgen05_kernel<CTAS, MT, INT4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     once.done();
   }
-  // tensor map of x (M, K) bf16 row-major: dim0 = K (contiguous), dim1 = M; box 64 x 128, 128-byte swizzle, zero fill
-  EncodeTiledFn enc = encode_tiled();
-  if (!enc) return cudaErrorNotSupported;
-  alignas(64) CUtensorMap tmap;
-  const cuuint64_t gdim[2] = {(cuuint64_t)p.K, (cuuint64_t)p.M};
-  const cuuint64_t gstride[1] = {(cuuint64_t)p.K * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kBK, 128u};
-  const cuuint32_t estr[2] = {1u, 1u};
-  if (enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p.x), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return cudaErrorInvalidValue;
-  dim3 grid((unsigned)((p.N + kBN - 1) / kBN), (unsigned)((p.M + 128 * MT - 1) / (128 * MT)), (unsigned)p.ksplit);
-  cudaError_t e = launch(qgemm_tcgen05_kernel<MT, INT4>, grid, dim3(kGThreads), (size_t)smem, st, p, tmap);
+  alignas(64) CUtensorMap map;
+  if (!tensor_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.x, p.M, p.K, p.K * 2, 128)) return cudaErrorInvalidValue;
+  p.n_tiles = (int)((p.N + 128 * CTAS - 1) / (128 * CTAS));
+  p.m_tiles = (int)((p.M + 128 * CTAS * MT - 1) / (128 * CTAS * MT));
+  const int64_t items = (int64_t)p.n_tiles * p.m_tiles * p.ksplit, units = sm_count() / CTAS;
+  const cudaError_t e = launch_cluster(qgemm_tcgen05_kernel<CTAS, MT, INT4>, dim3((unsigned)((items < units ? items : units) * CTAS)), dim3(kGThreads), CTAS,
+                                       (size_t)smem, st, p, map, wait_error_word());
   if (e != cudaSuccess || p.ksplit == 1) return e;
   const int64_t MN = p.M * p.N;
   return launch(qgemm_splitk_reduce_kernel, dim3((unsigned)((MN / 8 + 255) / 256)), dim3(256), (size_t)0, st, (const float*)p.partial, p.bias, p.y, MN, p.N, p.ksplit);
 }
 
-template <int MT>
-static cudaError_t launch_gemm(const GemmParams& p, cudaStream_t st) {
-  return p.qtype == B200_Q_INT4 ? launch_gemm_q<MT, true>(p, st) : launch_gemm_q<MT, false>(p, st);
+template <bool INT4>
+static cudaError_t launch_plan(const GemmParams& p, const GemmPlan& g, cudaStream_t st) {
+  if (g.ctas == 1) return launch_gemm<1, 1, INT4>(p, st);
+  return g.mt == 2 ? launch_gemm<2, 2, INT4>(p, st) : launch_gemm<2, 1, INT4>(p, st);
 }
 
 }  // namespace b200
@@ -375,12 +386,12 @@ using namespace b200;
 
 extern "C" {
 
-int b200_qgemm_tune(int mt3) { g_gemm_mt3 = mt3 ? 1 : 0; return B200_OK; }
+int b200_qgemm_tune(int wide) { g_gemm_wide = wide ? 1 : 0; return B200_OK; }
 
 size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   // accumulators live in tensor memory; only a launch split over k ranges (short prompts: too few output tiles for the SMs) stages fp32 partial sums
   if (M <= 0 || N <= 0 || K < kBK) return 0;
-  const int s = gemm_ksplit(M, N, K);
+  const int s = gemm_plan(M, N, K, true).ksplit;
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
 }
 
@@ -395,7 +406,7 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
               a->blocksize, (long long)a->N, (long long)a->K);
     return B200_ERR_UNSUPPORTED;
   }
-  B200_CHECK_ARG(a->N <= 65535LL * kBN && a->M <= 65535LL * 128, "b200_qgemm: shape too large for the grid");
+  B200_CHECK_ARG(a->N <= 65535LL * 128 && a->M <= 65535LL * 128, "b200_qgemm: shape too large for the grid");
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(a->packed) | reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->y)) & 15) == 0,
                  "b200_qgemm: packed / x / y must be 16-byte aligned");
   GemmParams p{};
@@ -405,15 +416,14 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
   p.bias = reinterpret_cast<const __nv_bfloat16*>(a->bias);
   p.y = reinterpret_cast<__nv_bfloat16*>(a->y);
   p.M = a->M; p.N = a->N; p.K = a->K; p.qtype = a->qtype;
-  // split-K only when the caller provided the workspace b200_qgemm_workspace_bytes asks for (none: one k range, as before)
-  p.ksplit = gemm_ksplit(a->M, a->N, a->K);
-  if (p.ksplit > 1 && (a->workspace == nullptr || a->workspace_bytes < (size_t)p.ksplit * a->M * a->N * sizeof(float) ||
+  // k ranges only when the caller provided the workspace b200_qgemm_workspace_bytes asks for (none: one k range)
+  GemmPlan g = gemm_plan(a->M, a->N, a->K, true);
+  if (g.ksplit > 1 && (a->workspace == nullptr || a->workspace_bytes < (size_t)g.ksplit * a->M * a->N * sizeof(float) ||
                        (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
-    p.ksplit = 1;
+    g = gemm_plan(a->M, a->N, a->K, false);
+  p.ksplit = g.ksplit;
   p.partial = reinterpret_cast<float*>(a->workspace);
-  cudaStream_t st = (cudaStream_t)stream;
-  // tokens per dequantised weight tile: 128, 256, or 384 for long prompts (the CUDA-core dequantisation is the bound: §5.4)
-  const cudaError_t e = a->M > 512 && g_gemm_mt3.load() ? launch_gemm<3>(p, st) : a->M > 128 ? launch_gemm<2>(p, st) : launch_gemm<1>(p, st);
+  const cudaError_t e = int4 ? launch_plan<true>(p, g, (cudaStream_t)stream) : launch_plan<false>(p, g, (cudaStream_t)stream);
   if (e != cudaSuccess) {
     set_error("b200_qgemm: launch failed: %s", cudaGetErrorString(e));
     return B200_ERR_CUDA;

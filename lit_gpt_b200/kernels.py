@@ -398,7 +398,7 @@ def qgemm(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, N: int, K:
 
 
 def qgemm_tune(mt3: bool = True) -> None:
-    """development switch: 384-token tiles for long prompts (default) or the 256-token tiles of round 1"""
+    """development switch: long prompts may use tiles of 512 tokens (default) or keep to 256"""
     C.check(C.load().b200_qgemm_tune(1 if mt3 else 0), "qgemm_tune")
 
 

@@ -26,7 +26,7 @@ def main() -> None:
     ap.add_argument("--tokens", type=int, default=4096)
     ap.add_argument("--reps", type=int, default=5)
     ap.add_argument("--layers", type=int, default=None)
-    ap.add_argument("--mt3", type=int, default=1, help="0: 256-token GEMM tiles (round 1) instead of 384")
+    ap.add_argument("--mt3", type=int, default=1, help="0: GEMM tiles of 256 tokens instead of up to 512")
     args = ap.parse_args()
 
     import bench
