@@ -286,7 +286,7 @@ def qgemv_tiled(x: torch.Tensor, tiled: torch.Tensor, N: int, K: int, quant_type
     lead = x.shape[:-1]
     batch = x.numel() // K
     epilogue = C.EPI_SWIGLU if tiled2 is not None else (C.EPI_RESIDUAL if residual is not None else C.EPI_STORE)
-    y = out if out is not None else torch.empty((*lead, N), dtype=torch.bfloat16, device=x.device)
+    y = out if out is not None else x.new_empty((*lead, N))
     delta, residual, bias, bias2, norm_weight = (_bf16c(delta, "delta"), _bf16c(residual, "residual"), _bf16c(bias, "bias"),
                                                  _bf16c(bias2, "bias2"), _bf16c(norm_weight, "norm_weight"))
     ws = _ws("qgemv_tiled", x.device, C.load().b200_qgemv_tiled_workspace_bytes())
