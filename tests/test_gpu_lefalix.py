@@ -761,3 +761,43 @@ def test_prompts_on_the_tensor_cores_then_decoding_over_their_rings(dtype):
     assert_close(torch.cat(got["a"]), want["a"][70:115], dtype, "a")
     assert_close(torch.cat(got["b"]), want["b"][50:95], dtype, "b")
     assert_close(torch.cat(got["c"]), want["c"], dtype, "c")
+
+
+# ---- short convolution: a warp walks several rows once the rows are many (csrc/shortconv.cu) -----------------------
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("taps,dim,heads,rows", [(4, 64, 12, 2400), (3, 72, 40, 600), (2, 128, 40, 1203), (4, 33, 24, 1700)])
+def test_short_conv_row_groups(dtype, taps, dim, heads, rows):
+    """Sequences whose ends fall anywhere in a warp's rows, some begun before the step: every row bit-equal to the same sequence run
+    alone (few rows, one per warp), the tails too."""
+    g = torch.Generator().manual_seed(rows)
+    hq, cols = heads // 4, heads * dim
+    cuts = sorted({0, 1, 2, 5, 13, 16, 24, 31, rows // 3, rows // 2 + 3, rows - 2, rows})
+    slots = torch.randperm(len(cuts) - 1, generator=g).tolist()
+    seqs = [(a, b - a, (0, 1, 700)[i % 3], slots[i]) for i, (a, b) in enumerate(zip(cuts, cuts[1:]))]
+    inp = torch.randn(rows, cols + 6, generator=g).to(dtype).cuda()
+    w = torch.randn(cols, taps, generator=g).to(dtype).cuda()
+    fr = (10000.0 ** (-torch.arange(0, 16, dtype=torch.float64) / 16)).cuda()
+    tail0 = torch.randn(len(seqs), taps - 1, cols, generator=g).to(dtype).cuda()
+
+    def run(x, tail, descr):
+        n = x.shape[0]
+        outs = [torch.empty(n, h * dim, dtype=d, device="cuda") for h, d in ((hq, torch.float32), (hq, dtype), (heads - 2 * hq, dtype))]
+        c1, c2 = hq * dim, 2 * hq * dim
+        groups = [K().conv_group(w[:c1], outs[0], 0, hq, dim, act=1, post=2, post_scale=0.25, eps=1e-6),
+                  K().conv_group(w[c1:c2], outs[1], c1, hq, dim, post=1, rot_dims=32, inv_freq=fr, rot_mscale=1.1, eps=1e-5),
+                  K().conv_group(w[c2:], outs[2], c2, heads - 2 * hq, dim, act=1)]
+        row_seq = torch.cat([torch.full((d[1],), i, dtype=torch.int32) for i, d in enumerate(descr)]).cuda()
+        K().short_conv(x, groups, taps, tail, torch.tensor(descr, dtype=torch.int32).cuda(), row_seq)
+        return outs
+
+    tail = tail0.clone()
+    whole = run(inp, tail, seqs)
+    part = 18944 // heads // 2   # half the fewest rows that are grouped: a long sequence alone runs in parts, its tail carried
+    for first, n, start, slot in seqs:
+        t1, got = tail0[slot : slot + 1].clone(), []
+        for o in range(0, n, part):
+            m = min(part, n - o)
+            got.append(run(inp[first + o : first + o + m], t1, [(0, m, start + o, 0)]))
+        for a, parts in zip(whole, zip(*got)):
+            assert torch.equal(a[first : first + n], torch.cat(parts)), (first, n, start)
+        assert torch.equal(tail[slot], t1[0])
