@@ -369,8 +369,9 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 def stream_ptr(device: torch.device | None = None) -> int:
     """The raw handle of `device`'s current stream (0.1 us; building a torch.cuda.Stream to ask it takes 2)."""
-    index = device.index if device is not None else None
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    if isinstance(device, torch.device) and device.type == "cuda" and device.index is not None:
+        return torch._C._cuda_getCurrentRawStream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def require_cuda(*tensors: torch.Tensor | None) -> None:
