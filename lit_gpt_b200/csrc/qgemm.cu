@@ -12,6 +12,8 @@
 //   * warp 17 of the pair's first CTA issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, 256 x 256 x 16) into TENSOR MEMORY; tcgen05.commit
 //     hands each stage back to both CTAs;
 //   * the sixteen warps read the accumulators with tcgen05.ld, add the bias, round to bf16 and store rows of y.
+// SWIGLU: the pair's first CTA dequantises 128 rows of the gate projection and the second the same rows of the up projection, so that a
+// thread holds both halves of its outputs and stores silu(gate) * up, with the roundings of the separate launches.
 // Bound: with MT = 2 the tensor pipe and the shared memory that feeds it (a CTA alone on 128 x 128 reads 128 bytes a clock of it for the
 // products alone, the pair 64); one dequantised tile serves 512 tokens.  What was before -- a CTA on 128 features x 384 tokens, one thread that
 // loaded the activations between its own dequantising, every warp in every k-block -- spent 1750 clocks a k-block whatever the tokens.
@@ -23,6 +25,8 @@ namespace b200 {
 struct GemmParams {
   const uint8_t* packed;      // reference layout: nf4/fp4 bytes (N, K/2); int4 words (N, K/8)
   const uint32_t* scale;      // fp32 absmax (N, K/64) or half2 {scale, zero} (N, K/128)
+  const uint8_t* packed2;     // the up-projection beside the gate (SWIGLU)
+  const uint32_t* scale2;
   const __nv_bfloat16* x;     // (M, K)
   const __nv_bfloat16* bias;  // (N) or null
   __nv_bfloat16* y;           // (M, N)
@@ -59,7 +63,7 @@ struct GemmTile {
   static constexpr int kSmem = kStages * kStage + 1024;
 };
 
-template <int CTAS, int MT, bool INT4>
+template <int CTAS, int MT, bool INT4, bool SWIGLU>
 __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_x, unsigned* err) {
   using C = GemmTile<MT>;
   extern __shared__ __align__(1024) uint8_t g_smem[];
@@ -99,7 +103,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     const int z = i / (p.n_tiles * p.m_tiles), r = i - z * (p.n_tiles * p.m_tiles), m = r / p.n_tiles;
     t.z = z;
     t.m0 = (int64_t)m * (BM * MT);
-    t.n0 = (int64_t)(r - m * p.n_tiles) * BN;
+    t.n0 = (int64_t)(r - m * p.n_tiles) * (SWIGLU ? 128 : BN);
     t.kb0 = (int)(((int64_t)nkb_all * z) / p.ksplit);
     t.nkb = (int)(((int64_t)nkb_all * (z + 1)) / p.ksplit) - t.kb0;
     t.mts = MT == 1 || p.M - t.m0 <= BM ? 1 : MT;     // sub-tiles with tokens in them
@@ -116,10 +120,10 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     uint32_t acc_ph = 0;
     for (int i = first; i < total && ok; i += step) {
       const Item t = item(i);
-      const int64_t wn = t.n0 + rank * 128 + wr;
+      const int64_t wn = t.n0 + (SWIGLU ? 0 : rank * 128) + wr;
       const bool wvalid = wn < p.N;
-      const uint8_t* wp = p.packed + (wvalid ? wn : 0) * (p.K >> 1) + (int64_t)t.kb0 * 32 + wh * 16;
-      const uint32_t* sp = p.scale + (wvalid ? wn : 0) * (INT4 ? (p.K >> 7) : (p.K >> 6));
+      const uint8_t* wp = (SWIGLU && rank ? p.packed2 : p.packed) + (wvalid ? wn : 0) * (p.K >> 1) + (int64_t)t.kb0 * 32 + wh * 16;
+      const uint32_t* sp = (SWIGLU && rank ? p.scale2 : p.scale) + (wvalid ? wn : 0) * (INT4 ? (p.K >> 7) : (p.K >> 6));
       const int l0 = (q + g) & 1;                     // this half's first k-block of the item
       uint4 qn[LAG];
       uint32_t sn[LAG];
@@ -194,6 +198,33 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
 #pragma unroll 1
       for (int mt = 0; mt < t.mts; ++mt) {
         const int64_t m = t.m0 + mt * BM + rank * 128 + (warp & 3) * 32 + lane;        // this thread's output row (TMEM lane = row)
+        if constexpr (SWIGLU) {   // columns [0, 128) are the gate, [128, 256) the up projection of the same features
+          const int c0 = (warp >> 2) * 32;
+          uint32_t v[32], u[32];
+          const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * BN + c0);
+          tc::ld32(v, at);
+          tc::ld32(u, at + 128);
+          tc::wait_ld(v);
+          tc::wait_ld(u);
+          if (m >= p.M) continue;
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            const int64_t n = t.n0 + c0 + j;
+            if (n < p.N) {
+              uint32_t o[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                auto act = [](uint32_t g, uint32_t w) {
+                  const float a = round_bf16(__uint_as_float(g));
+                  return round_bf16(a / (1.0f + expf(-a))) * round_bf16(__uint_as_float(w));
+                };
+                o[e] = pack_bf16(act(v[j + 2 * e], u[j + 2 * e]), act(v[j + 2 * e + 1], u[j + 2 * e + 1]));
+              }
+              *reinterpret_cast<uint4*>(p.y + m * p.N + n) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+          }
+          continue;
+        }
 #pragma unroll 1
         for (int c0 = (warp >> 2) * (BN / 4); c0 < ((warp >> 2) + 1) * (BN / 4); c0 += 32) {
           uint32_t v[32];
@@ -330,6 +361,13 @@ struct GemmPlan {
 // costs 6000 more to start and to store, partial sums of k ranges 13000 and a clock per 1860 bytes.  k ranges are for launches that leave
 // SMs idle -- two at least where half of them would be: at least four k-blocks per range, at most 16 ranges and 64 MB of partial sums, and
 // no more than fill the SMs once.
+static int64_t gemm_clocks(int64_t M, int64_t N, int64_t K, const GemmPlan& g) {
+  const int64_t nkb = K / kBK, units = sm_count() / g.ctas, s = g.ksplit;
+  const int64_t tiles = ((N + 128 * g.ctas - 1) / (128 * g.ctas)) * ((M + 128 * g.ctas * g.mt - 1) / (128 * g.ctas * g.mt));
+  const int64_t per = g.ctas == 1 ? 950 : g.mt == 1 ? 1130 : 1500;
+  return ((tiles * s + units - 1) / units) * (((nkb + s - 1) / s) * per + 6000) + (s > 1 ? 13000 + s * M * N * 4 / 1860 : 0);
+}
+
 static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool split_ok) {
   const int nkb = (int)(K / kBK);
   const int64_t sms = sm_count();
@@ -344,30 +382,31 @@ static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool split_ok) {
     if (most > nkb / 4) most = nkb / 4;
     if (most > 16) most = 16;
     while (most > 1 && most * M * N * (int64_t)sizeof(float) > (64ll << 20)) --most;
-    const int64_t per = kind == 0 ? 950 : kind == 1 ? 1130 : 1500;
     for (int64_t s = most > 1 && tiles * 2 <= units ? 2 : 1; s <= (most < 1 ? 1 : most); ++s) {
-      const int64_t t = ((tiles * s + units - 1) / units) * (((nkb + s - 1) / s) * per + 6000) + (s > 1 ? 13000 + s * M * N * 4 / 1860 : 0);
-      if (best_t < 0 || t < best_t) { best_t = t; best = GemmPlan{ctas, mt, (int)s}; }
+      const GemmPlan g{ctas, mt, (int)s};
+      const int64_t t = gemm_clocks(M, N, K, g);
+      if (best_t < 0 || t < best_t) { best_t = t; best = g; }
     }
   }
   return best;
 }
 
-template <int CTAS, int MT, bool INT4>
+template <int CTAS, int MT, bool INT4, bool SWIGLU = false>
 static cudaError_t launch_gemm(GemmParams p, cudaStream_t st) {
   constexpr int smem = GemmTile<MT>::kSmem;
   static PerDeviceOnce once;
   if (once.need()) {
-    cudaError_t e = cudaFuncSetAttribute(qgemm_tcgen05_kernel<CTAS, MT, INT4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(qgemm_tcgen05_kernel<CTAS, MT, INT4, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     once.done();
   }
   alignas(64) CUtensorMap map;
   if (!tensor_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.x, p.M, p.K, p.K * 2, 128)) return cudaErrorInvalidValue;
-  p.n_tiles = (int)((p.N + 128 * CTAS - 1) / (128 * CTAS));
+  constexpr int BN = SWIGLU ? 128 : 128 * CTAS;
+  p.n_tiles = (int)((p.N + BN - 1) / BN);
   p.m_tiles = (int)((p.M + 128 * CTAS * MT - 1) / (128 * CTAS * MT));
   const int64_t items = (int64_t)p.n_tiles * p.m_tiles * p.ksplit, units = sm_count() / CTAS;
-  const cudaError_t e = launch_cluster(qgemm_tcgen05_kernel<CTAS, MT, INT4>, dim3((unsigned)((items < units ? items : units) * CTAS)), dim3(kGThreads), CTAS,
+  const cudaError_t e = launch_cluster(qgemm_tcgen05_kernel<CTAS, MT, INT4, SWIGLU>, dim3((unsigned)((items < units ? items : units) * CTAS)), dim3(kGThreads), CTAS,
                                        (size_t)smem, st, p, map, wait_error_word());
   if (e != cudaSuccess || p.ksplit == 1) return e;
   const int64_t MN = p.M * p.N;
@@ -378,6 +417,27 @@ template <bool INT4>
 static cudaError_t launch_plan(const GemmParams& p, const GemmPlan& g, cudaStream_t st) {
   if (g.ctas == 1) return launch_gemm<1, 1, INT4>(p, st);
   return g.mt == 2 ? launch_gemm<2, 2, INT4>(p, st) : launch_gemm<2, 1, INT4>(p, st);
+}
+
+// Sub-tiles of a gate / up pair in one launch, by gemm_plan's clocks; 0 where two launches and the product are the shorter way.  The product
+// costs 4000 to start and a clock per 550 elements; half of that counts, and a twentieth has to be won, since the second of two launches starts
+// on the SMs that the first one's last round leaves idle: what pays is a round of tiles saved, or small matrices.  us, two launches and the
+// product against one, nf4 / int4: 4096 -> 14336 at 4096 rows 1014 -> 904 / 981 -> 917, at 2048 538 -> 462 / 517 -> 449; 4096 -> 11008 at 1000 rows
+// 257 -> 193 / 247 -> 192; 2048 -> 5632 at 203 rows 62 -> 40 / 55 -> 30.  Left apart: 4096 -> 11008 at 203 rows 98 against 105 / 107 against 98, at 4096
+// 757 against 712 / 685 against 667; 5120 -> 13824 at 2048 515 against 515 / 494 against 527.
+static int swiglu_tiles(int64_t M, int64_t N, int64_t K) {
+  if (M <= 128) return 0;
+  const int64_t units = sm_count() / 2, n = (N + 127) / 128, nkb = K / kBK;
+  const GemmPlan one = gemm_plan(M, N, K, true);
+  int64_t apart = gemm_clocks(M, N, K, one);
+  if (one.mt == 2 && (M - 1) % 512 < 256) apart -= 370 * (nkb / one.ksplit);   // the last tiles have one sub-tile
+  const int64_t worth = (2 * apart + 2000 + M * N / 1100) / 20 * 19;
+  int64_t best = 0, best_t = worth;
+  for (int mt = 1; mt <= (M > 256 && g_gemm_wide.load() ? 2 : 1); ++mt) {
+    const int64_t t = (n * ((M + 256 * mt - 1) / (256 * mt)) + units - 1) / units * (nkb * (mt == 2 ? 1500 : 1130) + 6000);
+    if (t < best_t) { best_t = t; best = mt; }
+  }
+  return (int)best;
 }
 
 }  // namespace b200
@@ -395,7 +455,7 @@ size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
 }
 
-int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
+static int gemm_args(const b200_qgemm_args* a, GemmParams& p) {
   B200_CHECK_ARG(a != nullptr, "b200_qgemm: null args");
   B200_CHECK_ARG(a->packed && a->scale && a->x && a->y, "b200_qgemm: null packed/scale/x/y pointer");
   B200_CHECK_ARG(a->M > 0 && a->N > 0 && a->K > 0, "b200_qgemm: M, N, K must be positive");
@@ -409,13 +469,18 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
   B200_CHECK_ARG(a->N <= 65535LL * 128 && a->M <= 65535LL * 128, "b200_qgemm: shape too large for the grid");
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(a->packed) | reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->y)) & 15) == 0,
                  "b200_qgemm: packed / x / y must be 16-byte aligned");
-  GemmParams p{};
   p.packed = reinterpret_cast<const uint8_t*>(a->packed);
   p.scale = reinterpret_cast<const uint32_t*>(a->scale);
   p.x = reinterpret_cast<const __nv_bfloat16*>(a->x);
   p.bias = reinterpret_cast<const __nv_bfloat16*>(a->bias);
   p.y = reinterpret_cast<__nv_bfloat16*>(a->y);
   p.M = a->M; p.N = a->N; p.K = a->K; p.qtype = a->qtype;
+  return B200_OK;
+}
+
+int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
+  GemmParams p{};
+  if (const int rc = gemm_args(a, p)) return rc;
   // k ranges only when the caller provided the workspace b200_qgemm_workspace_bytes asks for (none: one k range)
   GemmPlan g = gemm_plan(a->M, a->N, a->K, true);
   if (g.ksplit > 1 && (a->workspace == nullptr || a->workspace_bytes < (size_t)g.ksplit * a->M * a->N * sizeof(float) ||
@@ -423,9 +488,40 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
     g = gemm_plan(a->M, a->N, a->K, false);
   p.ksplit = g.ksplit;
   p.partial = reinterpret_cast<float*>(a->workspace);
-  const cudaError_t e = int4 ? launch_plan<true>(p, g, (cudaStream_t)stream) : launch_plan<false>(p, g, (cudaStream_t)stream);
+  const cudaError_t e = a->qtype == B200_Q_INT4 ? launch_plan<true>(p, g, (cudaStream_t)stream) : launch_plan<false>(p, g, (cudaStream_t)stream);
   if (e != cudaSuccess) {
     set_error("b200_qgemm: launch failed: %s", cudaGetErrorString(e));
+    return B200_ERR_CUDA;
+  }
+  return B200_OK;
+}
+
+int b200_qgemm_swiglu_supported(int64_t M, int64_t N, int64_t K, int qtype, int blocksize) {
+  const int block = qtype == B200_Q_INT4 ? 128 : 64;
+  if ((qtype != B200_Q_NF4 && qtype != B200_Q_FP4 && qtype != B200_Q_INT4) || blocksize != block) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || K % block || N % 8 || N > 65535LL * 128 || M > 65535LL * 128) return 0;
+  return swiglu_tiles(M, N, K) > 0;
+}
+
+int b200_qgemm_swiglu(const b200_qgemm_args* a, const void* packed2, const void* scale2, b200_stream_t stream) {
+  GemmParams p{};
+  if (const int rc = gemm_args(a, p)) return rc;
+  B200_CHECK_ARG(packed2 && scale2 && (reinterpret_cast<uintptr_t>(packed2) & 15) == 0, "b200_qgemm_swiglu: null or misaligned second matrix");
+  B200_CHECK_ARG(!a->bias, "b200_qgemm_swiglu: takes no bias");
+  const int mt = swiglu_tiles(a->M, a->N, a->K);
+  if (mt == 0) {
+    set_error("b200_qgemm_swiglu: (M=%lld N=%lld K=%lld) runs as two b200_qgemm and b200_swiglu", (long long)a->M, (long long)a->N, (long long)a->K);
+    return B200_ERR_UNSUPPORTED;
+  }
+  p.packed2 = reinterpret_cast<const uint8_t*>(packed2);
+  p.scale2 = reinterpret_cast<const uint32_t*>(scale2);
+  p.ksplit = 1;
+  const bool int4 = a->qtype == B200_Q_INT4;
+  const cudaStream_t st = (cudaStream_t)stream;
+  const cudaError_t e = mt == 2 ? (int4 ? launch_gemm<2, 2, true, true>(p, st) : launch_gemm<2, 2, false, true>(p, st))
+                                : (int4 ? launch_gemm<2, 1, true, true>(p, st) : launch_gemm<2, 1, false, true>(p, st));
+  if (e != cudaSuccess) {
+    set_error("b200_qgemm_swiglu: launch failed: %s", cudaGetErrorString(e));
     return B200_ERR_CUDA;
   }
   return B200_OK;

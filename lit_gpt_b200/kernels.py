@@ -397,6 +397,27 @@ def qgemm(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, N: int, K:
     return y
 
 
+def qgemm_swiglu_supported(M: int, N: int, K: int, quant_type: str = "nf4", blocksize: int = 64) -> bool:
+    """True where one launch for both projections of a SwiGLU pair is the shorter way (asked of the library; nothing is launched)."""
+    return C.load().b200_qgemm_swiglu_supported(M, N, K, QTYPES[quant_type], blocksize) != 0
+
+
+def qgemm_swiglu(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, packed2: torch.Tensor, scale2: torch.Tensor, N: int, K: int,
+                 quant_type: str = "nf4", blocksize: int = 64) -> torch.Tensor:
+    """silu(x . dequant(W)^T) * (x . dequant(W2)^T), bf16-rounded where two ``qgemm`` and ``swiglu`` round, in one launch.
+    Raises NotImplementedError where ``qgemm_swiglu_supported`` is false."""
+    C.require_cuda(x, packed, scale, packed2, scale2)
+    x = _bf16c(x, "x")
+    M = x.numel() // K
+    if x.numel() != M * K:
+        raise C.B200Error("qgemm_swiglu: x does not hold whole rows of length K")
+    y = torch.empty(tuple(x.shape[:-1]) + (N,), dtype=torch.bfloat16, device=x.device)
+    args = C.QGemmArgs(packed=packed.data_ptr(), scale=scale.data_ptr(), qtype=QTYPES[quant_type], blocksize=blocksize, M=M, N=N, K=K,
+                       x=x.data_ptr(), y=y.data_ptr())
+    C.check(C.load().b200_qgemm_swiglu(ctypes.byref(args), packed2.data_ptr(), scale2.data_ptr(), C.stream_ptr(x.device)), "qgemm_swiglu")
+    return y
+
+
 def qgemm_tune(mt3: bool = True) -> None:
     """development switch: long prompts may use tiles of 512 tokens (default) or keep to 256"""
     C.check(C.load().b200_qgemm_tune(1 if mt3 else 0), "qgemm_tune")

@@ -398,6 +398,17 @@ def prefill_linear(q: QLinear, x: torch.Tensor) -> torch.Tensor:
     return F.linear(x, w, q.bias)
 
 
+def prefill_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
+    """True where the two projections of a gated MLP can be one launch with the product in its epilogue: plain 4-bit modules of one layout
+    without a bias or a hook (a hook wants the projections' own outputs) whose reference layouts are resident, at sizes the library calls the shorter way."""
+    if not all(isinstance(m, QLinear) and type(m).forward is QLinear.forward and m.is_quantized and not m.released and m.quant_type != "int8"
+               and m.bias is None and not (m._forward_hooks or m._forward_pre_hooks) for m in (gate, up)):
+        return False
+    return (gate.quant_type == up.quant_type and gate.blocksize == up.blocksize and gate.in_features == up.in_features
+            and gate.out_features == up.out_features
+            and K.qgemm_swiglu_supported(rows, gate.out_features, gate.in_features, gate.quant_type, gate.blocksize))
+
+
 class QuantPrecision:
     """Mirror of ``lightning.fabric.plugins.BitsandbytesPrecision(mode, dtype, ignore_modules)``."""
 

@@ -682,6 +682,69 @@ def test_qgemm_onehot_rows_read_dequantised_weights(K):
         assert torch.equal(y.cpu(), deq.to(torch.bfloat16).T.contiguous()), qt
 
 
+@pytest.mark.parametrize("qt", ["nf4", "int4"])
+@pytest.mark.parametrize("M,N,Kdim", [(129, 8, 128), (255, 264, 128), (256, 256, 128), (257, 264, 384), (511, 136, 256), (513, 520, 128),
+                                      (1025, 4104, 384), (2049, 2568, 128)])
+def test_qgemm_tile_edges(K, qt, M, N, Kdim):
+    """Rows and features on both sides of a tile of 256 and of its sub-tiles, one to three scale blocks of k, more tiles than CTA pairs:
+    one-hot rows read exactly bf16(dequant(W)), scattered so that every tile holds rows of every k block."""
+    w, _, packed, scale, bs, deq = _gemv_case(K, N, Kdim, 1, qt, seed=M)
+    hot = torch.randint(0, Kdim, (M,), generator=torch.Generator().manual_seed(N))
+    x = torch.nn.functional.one_hot(hot, Kdim).to(torch.bfloat16)
+    y = K.qgemm(x.cuda(), packed, scale, N, Kdim, qt, bs)
+    assert torch.equal(y.cpu(), deq.to(torch.bfloat16).T[hot])
+    bias = _randw((N,), 6, std=0.5)
+    y = K.qgemm(x.cuda(), packed, scale, N, Kdim, qt, bs, bias=bias.cuda())
+    assert torch.equal(y.cpu(), (deq.to(torch.bfloat16).T[hot].float() + bias.float()).to(torch.bfloat16))
+
+
+def test_qgemm_single_k_block(K):
+    w, _, packed, scale, bs, deq = _gemv_case(K, 264, 64, 1, "nf4", seed=9)
+    hot = torch.arange(300) % 64
+    x = torch.nn.functional.one_hot(hot, 64).to(torch.bfloat16)
+    assert torch.equal(K.qgemm(x.cuda(), packed, scale, 264, 64, "nf4", bs).cpu(), deq.to(torch.bfloat16).T[hot])
+
+
+@pytest.mark.parametrize("qt", ["nf4", "fp4", "int4"])
+@pytest.mark.parametrize("M,N,Kdim", [(129, 9472, 256), (203, 11008, 4096), (257, 9472, 128), (513, 9480, 384), (1281, 5504, 512), (4096, 1408, 256)])
+def test_qgemm_swiglu_is_the_separate_launches(K, qt, M, N, Kdim):
+    """Both projections and their product in one launch: bit-equal to two GEMMs and the product wherever those run without k ranges
+    (the same sums in the same order, the same roundings), at rows and features on both sides of a tile."""
+    from lit_gpt_b200 import _cabi as C
+    _, _, p1, s1, bs, _ = _gemv_case(K, N, Kdim, 1, qt, seed=M)
+    _, _, p2, s2, _, _ = _gemv_case(K, N, Kdim, 1, qt, seed=N)
+    x = _randw((M, Kdim), 5, std=3.0).cuda()
+    if not K.qgemm_swiglu_supported(M, N, Kdim, qt, bs):
+        with pytest.raises(NotImplementedError):
+            K.qgemm_swiglu(x, p1, s1, p2, s2, N, Kdim, qt, bs)
+        pytest.skip("the separate launches are the shorter way here")
+    assert C.load().b200_qgemm_workspace_bytes(M, N, Kdim) == 0
+    y = K.qgemm_swiglu(x, p1, s1, p2, s2, N, Kdim, qt, bs)
+    ref = K.swiglu(K.qgemm(x, p1, s1, N, Kdim, qt, bs), K.qgemm(x, p2, s2, N, Kdim, qt, bs))
+    assert torch.equal(y, ref)
+
+
+def test_mlp_prompt_pair_keeps_hooks(K):
+    """A gated MLP's prompt takes the one launch; a hook on a projection still sees that projection's output, with the same result."""
+    from lit_gpt_b200 import Config
+    from lit_gpt_b200.model import LLaMAMLP
+    from lit_gpt_b200.quant import QLinear, prefill_pair
+
+    mlp = LLaMAMLP(Config(n_embd=256, intermediate_size=9472, n_head=4, bias=False)).to(torch.bfloat16)
+    for name in ("fc_1", "fc_2", "proj"):
+        setattr(mlp, name, QLinear.from_linear(getattr(mlp, name).cuda(), "nf4", torch.bfloat16))
+    x = _randw((300, 256), 4, std=1.0).cuda()
+    assert prefill_pair(mlp.fc_1, mlp.fc_2, 300)
+    fused, seen = mlp(x), []
+    hook = mlp.fc_2.register_forward_hook(lambda m, a, o: seen.append(o.shape))
+    assert not prefill_pair(mlp.fc_1, mlp.fc_2, 300)
+    assert torch.equal(fused, mlp(x)) and seen == [(300, 9472)]
+    hook.remove()
+    mlp.fc_1.release_reference_layout()
+    assert not prefill_pair(mlp.fc_1, mlp.fc_2, 300) or not mlp.fc_1.released
+    assert torch.equal(fused, mlp(x))
+
+
 def test_qgemm_unsupported_shapes(K):
     w, _, packed, scale, bs, _ = _gemv_case(K, 20, 96, 1, "nf4")
     with pytest.raises(NotImplementedError):
