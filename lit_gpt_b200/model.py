@@ -289,7 +289,7 @@ class GPT(nn.Module):
             n2 = K.rmsnorm(x, block.norm_2.weight, eps, delta=h.view(B * T, -1), sum_out=x_new)   # x = h + x, then norm_2
             x = x_new
             n2 = n2.view(B, T, -1)
-            delta = m(n2).view(B * T, -1)   # LLaMAMLP.forward: fused SwiGLU (b200_swiglu, or the GEMV epilogue for <= 16 rows); its tensor-parallel hook sums the ranks' partials
+            delta = m(n2).view(B * T, -1)   # LLaMAMLP.forward: fused SwiGLU (b200_swiglu, or the epilogue of the GEMV for <= 16 rows, of the GEMM for long prompts); its tensor-parallel hook sums the ranks' partials
         xf = K.rmsnorm(x, self.transformer.ln_f.weight, eps, delta=delta)
         return self.lm_head(xf.view(B, T, -1))
 
