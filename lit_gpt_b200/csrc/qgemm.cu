@@ -11,6 +11,10 @@
 //   * warp 16 fetches the activation tiles (128 tokens x 64 k per CTA and sub-tile) by TMA, rows past M zero-filled by the hardware;
 //   * warp 17 of the pair's first CTA issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, 256 x 256 x 16) into TENSOR MEMORY; tcgen05.commit
 //     hands each stage back to both CTAs;
+//   * across the pair every hand-over has cluster scope: warp 17 of the second CTA passes its CTA's dequantised tiles on to the first CTA's
+//     barrier, and each CTA's warp 16 passes a stage's return on to its dequantising warps.  Those wait and arrive on barriers of their own
+//     CTA only -- a release or an acquire at cluster scope waits for all that a thread has under way, and their weight loads always are
+//     (700 to 1500 clocks a k-block);
 //   * the sixteen warps read the accumulators with tcgen05.ld, add the bias, round to bf16 and store rows of y.
 // SWIGLU: the pair's first CTA dequantises 128 rows of the gate projection and the second the same rows of the up projection, so that a
 // thread holds both halves of its outputs and stores silu(gate) * up, with the roundings of the separate launches.
@@ -68,15 +72,20 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   using C = GemmTile<MT>;
   extern __shared__ __align__(1024) uint8_t g_smem[];
   constexpr int BN = 128 * CTAS, BM = BN;           // features per tile, tokens per sub-tile
-  __shared__ __align__(8) uint64_t s_bars[2 * C::kStages + 2];
+  __shared__ __align__(8) uint64_t s_bars[3 * C::kStages + 2];
   __shared__ uint32_t s_tmem;
   __shared__ float s_code[16 * 32];                 // fp32 code book, one copy per lane (conflict-free look-ups)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = CTAS == 2 ? tc::cluster_rank() : 0u;
   const uint32_t tiles = (tc::smem_u32(g_smem) + 1023u) & ~1023u;
   const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]), acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_free = acc_full + 8;
+  const uint32_t room = CTAS == 2 ? acc_full + 16 : empty;   // where the dequantising warps learn that a stage is theirs
   if (tid == 0) {
-    for (int s = 0; s < C::kStages; ++s) { tc::mbar_init(full + 8 * s, 8 * CTAS + 1); tc::mbar_init(empty + 8 * s, 1); }
+    for (int s = 0; s < C::kStages; ++s) {
+      tc::mbar_init(full + 8 * s, rank == 0 ? 8 + CTAS : 8);   // half of the dequantising warps; in the first CTA the copies and the other CTA's tile
+      tc::mbar_init(empty + 8 * s, 1);
+      if (CTAS == 2) tc::mbar_init(room + 8 * s, 1);
+    }
     tc::mbar_init(acc_full, 1);
     tc::mbar_init(acc_free, 16 * CTAS);
     tc::mbar_init_fence();
@@ -112,6 +121,9 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   const int first = (int)blockIdx.x / CTAS, step = (int)gridDim.x / CTAS;
   bool ok = true;
   int q = 0;                                          // k-blocks so far: stage q % kStages
+  auto wait = [](uint32_t bar, uint32_t parity) {     // on a barrier that the other CTA of a pair arrives on
+    return CTAS == 2 ? tc::mbar_wait_cluster(bar, parity) : tc::mbar_wait(bar, parity);
+  };
 
   if (warp < 16) {
     // =========================================== DEQUANTISE, THEN STORE =========================================
@@ -145,7 +157,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
         if (ln < t.nkb) { qn[LAG - 1] = ldg_stream_v4(wp + (int64_t)ln * 32); sn[LAG - 1] = sp[INT4 ? ((t.kb0 + ln) >> 1) : (t.kb0 + ln)]; }
         const uint32_t qw[4] = {w.x, w.y, w.z, w.w};
         const uint32_t dst = tiles + s * C::kStage + MT * kTileBytes;
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(empty + 8 * s, ph ^ 1u));
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(room + 8 * s, CTAS == 2 ? ph : ph ^ 1u));
         if (!ok) break;
         if (INT4) {
           // bf16_rn(scale * (q - zero)) with three instructions per code: the nibble is moved to the top four mantissa bits of 16.0f
@@ -184,14 +196,11 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
         }
         tc::fence_smem_async();                       // generic-proxy writes -> visible to the tensor core
         __syncwarp();
-        if (lane == 0) {
-          if constexpr (CTAS == 2) tc::mbar_signal_at(tc::at_rank(full + 8 * s, 0));
-          else tc::mbar_arrive(full + 8 * s);
-        }
+        if (lane == 0) tc::mbar_arrive(full + 8 * s);
       }
       q += t.nkb;
       // ---- accumulators -> y (or partial sums): warp w has rows 32 (w % 4) .. + 31 and a quarter of the columns ----
-      ok = ok && __all_sync(0xffffffffu, tc::mbar_wait(acc_full, acc_ph));
+      ok = ok && __all_sync(0xffffffffu, wait(acc_full, acc_ph));
       acc_ph ^= 1u;
       if (!ok) break;
       tc::fence_after();
@@ -269,8 +278,9 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
         const Item t = item(i);
         for (int l = 0; l < t.nkb; ++l, ++q) {
           const int s = q % C::kStages;
-          ok = tc::mbar_wait(empty + 8 * s, ((uint32_t)(q / C::kStages) & 1u) ^ 1u);
+          ok = wait(empty + 8 * s, ((uint32_t)(q / C::kStages) & 1u) ^ 1u);
           if (!ok) break;
+          if (CTAS == 2) tc::mbar_arrive(room + 8 * s);
           if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * t.mts * kTileBytes);
           const uint32_t st = tiles + s * C::kStage, bar = CTAS == 2 ? tc::at_rank(full + 8 * s, 0) : full + 8 * s;
           for (int mt = 0; mt < t.mts; ++mt) {
@@ -288,12 +298,12 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     uint32_t free_ph = 1;
     for (int i = first; i < total && ok; i += step) {
       const Item t = item(i);
-      ok = tc::mbar_wait(acc_free, free_ph);
+      ok = wait(acc_free, free_ph);
       free_ph ^= 1u;
       tc::fence_after();
       for (int l = 0; l < t.nkb && ok; ++l, ++q) {
         const int s = q % C::kStages;
-        ok = tc::mbar_wait(full + 8 * s, (uint32_t)(q / C::kStages) & 1u);
+        ok = wait(full + 8 * s, (uint32_t)(q / C::kStages) & 1u);
         if (!ok) break;
         tc::fence_after();
         const uint32_t st = tiles + s * C::kStage;
@@ -310,6 +320,17 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
       if (ok) {
         if constexpr (CTAS == 2) tc::commit_pair(acc_full);
         else tc::commit(acc_full);
+      }
+    }
+  } else if (lane == 0 && CTAS == 2) {
+    // ============================ THE SECOND CTA'S TILES, PASSED ON TO THE FIRST ================================
+    for (int i = first; i < total && ok; i += step) {
+      const int nkb = item(i).nkb;
+      for (int l = 0; l < nkb; ++l, ++q) {
+        const int s = q % C::kStages;
+        ok = tc::mbar_wait(full + 8 * s, (uint32_t)(q / C::kStages) & 1u);
+        if (!ok) break;
+        tc::mbar_arrive_at(tc::at_rank(full + 8 * s, 0));
       }
     }
   }

@@ -107,11 +107,6 @@ __device__ __forceinline__ uint32_t at_rank(uint32_t addr, uint32_t rank) {   //
 __device__ __forceinline__ void mbar_arrive_at(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
-// The same for writes to this CTA's own shared memory that only the pair's products read (after fence_smem_async): they are in place when the
-// arrival leaves the SM, whereas a release to the cluster first waits for everything the thread has under way, loads included (1500 clocks)
-__device__ __forceinline__ void mbar_signal_at(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
 __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"

@@ -698,6 +698,22 @@ def test_qgemm_tile_edges(K, qt, M, N, Kdim):
     assert torch.equal(y.cpu(), (deq.to(torch.bfloat16).T[hot].float() + bias.float()).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("qt", ["nf4", "int4"])
+@pytest.mark.parametrize("M,N,Kdim", [(203, 11008, 4096), (700, 4096, 4096)])
+def test_qgemm_pair_handover_repeats(K, qt, M, N, Kdim):
+    """Both CTAs of a pair fill one stage, one of them issues the products: many wraps of the ring, over and over with other weights in between,
+    give the same bits every time -- those of the packed weights' dequantised copy up to the rounding of the sum."""
+    _, _, p1, s1, bs, deq = _gemv_case(K, N, Kdim, 1, qt, seed=M)
+    _, _, p2, s2, _, _ = _gemv_case(K, N, Kdim, 1, qt, seed=M + 1)
+    x = _randw((M, Kdim), 7, std=1.0)
+    xd = x.cuda()
+    first = [K.qgemm(xd, p, s, N, Kdim, qt, bs) for p, s in ((p1, s1), (p2, s2))]
+    _check_gemv(first[0].cpu(), x, deq)
+    for _ in range(40):
+        for want, (p, s) in zip(first, ((p1, s1), (p2, s2))):
+            assert torch.equal(K.qgemm(xd, p, s, N, Kdim, qt, bs), want)
+
+
 def test_qgemm_single_k_block(K):
     w, _, packed, scale, bs, deq = _gemv_case(K, 264, 64, 1, "nf4", seed=9)
     hot = torch.arange(300) % 64
