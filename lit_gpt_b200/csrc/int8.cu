@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(kI8Threads) int8_gemv_kernel(const I8Params p)
 constexpr int kI8EpiWarps = 8, kI8GemmThreads = (kI8EpiWarps + 2) * 32;
 constexpr int kI8KB = 128;                       // int8 columns per stage: one 128-byte swizzle row
 constexpr int kI8Stages = 6, kI8Stage = 256 * kI8KB, kI8Smem = kI8Stages * kI8Stage + 1024;   // 128 rows of either operand
+static_assert(kI8Smem >= tc::kPairMinSmem, "one CTA of a pair per SM");
 
 // kind::i8: D = int32, A = B = signed 8 bit, both K-major
 template <bool PAIR>
@@ -345,6 +346,8 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
     tc::prefetch_map(&map_a);
     tc::prefetch_map(&map_b);
   }
+  griddep_launch();
+  griddep_wait();
   if (warp == kI8EpiWarps) {
     if constexpr (PAIR) tc::tmem_alloc_pair<2 * BN>(tc::smem_u32(&s_tmem));
     else tc::tmem_alloc<2 * BN>(tc::smem_u32(&s_tmem));
@@ -354,8 +357,6 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = s_tmem;
-  griddep_launch();
-  griddep_wait();
   const int nkb = (int)((p.K + kI8KB - 1) / kI8KB), total = m_tiles * n_tiles;
   const int first = (int)blockIdx.x / CTAS, step = (int)gridDim.x / CTAS;
   bool ok = true;

@@ -65,6 +65,7 @@ struct GemmTile {
   static constexpr int kStages = MT == 2 ? 4 : 6;          // an even number: a stage belongs to one half of the dequantising warps
   static constexpr int kStage = (MT + 1) * kTileBytes;     // MT activation tiles + 1 weight tile
   static constexpr int kSmem = kStages * kStage + 1024;
+  static_assert(kSmem >= tc::kPairMinSmem, "one CTA of a pair per SM");
 };
 
 template <int CTAS, int MT, bool INT4, bool SWIGLU>
@@ -93,6 +94,8 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   }
   if (!INT4)
     for (int i = tid; i < 16 * 32; i += kGThreads) s_code[i] = code_value(p.qtype, i >> 5);
+  griddep_launch();
+  griddep_wait();
   if (warp == 17) {
     if constexpr (CTAS == 2) tc::tmem_alloc_pair<BN * MT>(tc::smem_u32(&s_tmem));
     else tc::tmem_alloc<BN * MT>(tc::smem_u32(&s_tmem));
@@ -102,8 +105,6 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = s_tmem;
-  griddep_launch();
-  griddep_wait();
 
   const int nkb_all = (int)(p.K / kBK), total = p.n_tiles * p.m_tiles * p.ksplit;
   struct Item { int64_t m0, n0; int z, kb0, nkb, mts; };

@@ -74,6 +74,8 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_smem_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// Tensor memory is taken after griddep_wait() only: a CTA that started early and held columns while it waited for the grid before it would
+// keep them from that grid's own CTAs.  Past the wait a CTA that blocks here waits for CTAs that run to their end.
 template <int COLS>
 __device__ __forceinline__ void tmem_alloc(uint32_t slot) {   // one whole warp; the address lands in shared memory
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "n"(COLS) : "memory");
@@ -122,6 +124,8 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(cluster_bar) : "memory");
 }
+// Two pairs that shared their SMs could each hold one half of what both need: a kernel with pairs takes more than half of an SM's shared memory.
+constexpr int kPairMinSmem = 114 * 1024 + 1;
 template <int COLS>
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t slot) {   // one warp of EACH CTA
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "n"(COLS) : "memory");

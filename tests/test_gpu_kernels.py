@@ -907,3 +907,28 @@ def test_attn_window_tiles(K, window, hs, H, G):
         lim = torch.arange(m)
         low = lim - window + 1 if window else torch.zeros_like(lim)
         _attn_close(y[first[i] : first[i] + m], _attn_exact(q, k, v, lim, low, 0.3, sink))
+
+
+def test_tensor_memory_kernels_in_turn(K):
+    """Prompt attention with heads of 64 (whose CTAs leave shared memory free), a GEMM pair and attention again, each started while the one
+    before drains: every result is that of the call alone."""
+    H, T, hs, N = 16, 700, 64, 3072
+    _, _, packed, scale, bs, _ = _gemv_case(K, N, H * hs, 1, "nf4", seed=1)
+    q, k, v = (_randw((1, H, T, hs), i, std=1.0).cuda() for i in (2, 3, 4))
+    pos = torch.arange(T, device="cuda")
+
+    def run(sync):
+        out = []
+        for _ in range(20):
+            y = K.attn_prefill(q, k, v, pos)
+            if sync:
+                torch.cuda.synchronize()
+            out += [y, K.qgemm(y, packed, scale, N, H * hs, "nf4", bs)]
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return out
+
+    alone = run(True)
+    for a, b in zip(run(False), alone):
+        assert torch.equal(a, b)
