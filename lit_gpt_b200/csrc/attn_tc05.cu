@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kAtThreads, 1)
 attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, unsigned* err) {
   using C = AtTile<HS>;
   extern __shared__ __align__(1024) uint8_t at_smem[];
-  __shared__ __align__(8) uint64_t s_bars[25];
+  __shared__ __align__(8) uint64_t s_bars[26];
   __shared__ float s_shrink[2 * kAtBM];   // per row: what its O and sum shrink by in this step
   __shared__ uint32_t s_tmem;
   __shared__ int s_max[8];
@@ -100,7 +100,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   const uint32_t sq_ = smem, sk_ = smem + 2 * C::kBytes, sv_ = smem + 4 * C::kBytes;
   const uint32_t bars = tc::smem_u32(s_bars);
   const uint32_t k_full = bars, v_full = bars + 16, k_empty = bars + 32, v_empty = bars + 48, s_full = bars + 64, p_half = bars + 80, p_full = bars + 96,
-                 o_done = bars + 112, q_full = bars + 128, shrink = bars + 136;   // shrink: one per softmax warp
+                 o_done = bars + 112, q_full = bars + 128, shrink = bars + 136, idle = bars + 200;   // shrink: one per softmax warp; idle: products that gave up
 
   griddep_launch();
   griddep_wait();
@@ -117,6 +117,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   }
   if (tid == 0) {
     tc::mbar_init(q_full, 8);
+    tc::mbar_init(idle, 1);
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(k_full + 8 * i, 1);
       tc::mbar_init(v_full + 8 * i, 1);
@@ -174,8 +175,9 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
     // the map's column and row of position 0: heads are planes of rows (a cache) or column blocks (packed rows)
     const int x0 = A.seqs ? grp * HS : 0;
     const int64_t row0 = A.seqs ? kvrow0 : ((int64_t)b * A.n_groups + grp) * A.max_seq;
-    for (int j = t_lo; j < t_hi; ++j) {
-      const int i = j - t_lo, s = i & 1;
+    int i = 0;   // tiles so far
+    for (int j = t_lo; j < t_hi; ++j, ++i) {
+      const int s = i & 1;
       ok = __all_sync(0xffffffffu, tc::mbar_wait(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u));
       if (!ok) break;
       // (what a cache holds behind the last key does not matter to the scores, which are masked there)
@@ -191,6 +193,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
         publish(full + 8 * s);
       }
     }
+    for (int e = max(i - 2, 0); e < i; ++e) ok = __all_sync(0xffffffffu, tc::mbar_wait(full + 8 * (e & 1), (uint32_t)(e >> 1) & 1u)) && ok;
   } else if (warp == 12) {
     // ================================ products ================================
     if (lane == 0) {
@@ -239,6 +242,10 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
         if (!ok) break;
         tc::commit(v_empty + 8 * s);
         if (more) tc::commit(k_empty + 8 * s1);
+      }
+      if (!ok) {
+        tc::commit(idle);
+        tc::mbar_wait(idle, 0);
       }
     }
   } else if (warp >= 8) {

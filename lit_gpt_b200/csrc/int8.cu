@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kI8GemmThreads, 1)
 int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int m_tiles, int n_tiles, unsigned* err) {
   constexpr int CTAS = PAIR ? 2 : 1, BN = 128 * CTAS;
   extern __shared__ __align__(1024) uint8_t i8_smem[];
-  __shared__ __align__(8) uint64_t s_bars[2 * kI8Stages + 4];
+  __shared__ __align__(8) uint64_t s_bars[2 * kI8Stages + 5];
   __shared__ uint32_t s_tmem;
   __shared__ __align__(16) float s_feat[10][BN];               // per feature of the tile: weight scale, bias, weight in the first eight outlier columns
   __shared__ __align__(16) float s_more[kI8EpiWarps][8][32];   // per epilogue warp: the weights of 32 features in the next eight
@@ -338,10 +338,11 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
   const uint32_t rank = PAIR ? tc::cluster_rank() : 0u;
   const uint32_t tiles = (tc::smem_u32(i8_smem) + 1023u) & ~1023u;
   const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[kI8Stages]);
-  const uint32_t acc_full = tc::smem_u32(&s_bars[2 * kI8Stages]), acc_empty = acc_full + 16;
+  const uint32_t acc_full = tc::smem_u32(&s_bars[2 * kI8Stages]), acc_empty = acc_full + 16, idle = acc_full + 32;
   if (tid == 0) {
     for (int s = 0; s < kI8Stages; ++s) { tc::mbar_init(full + 8 * s, 1); tc::mbar_init(empty + 8 * s, 1); }
     for (int a = 0; a < 2; ++a) { tc::mbar_init(acc_full + 8 * a, 1); tc::mbar_init(acc_empty + 8 * a, kI8EpiWarps * CTAS); }
+    tc::mbar_init(idle, 1);
     tc::mbar_init_fence();
     tc::prefetch_map(&map_a);
     tc::prefetch_map(&map_b);
@@ -384,8 +385,11 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
           if (++s == kI8Stages) { s = 0; ph ^= 1u; }
         }
       }
-      if (!ok && rank == 0)   // given up: no copy may still be on its way when the CTAs leave
-        for (int i = 0; i < kI8Stages; ++i) tc::mbar_wait(full + 8 * i, i < s ? ph ^ 1u : ph);
+      if (rank == 0)
+        for (int i = 0; i < kI8Stages; ++i) {
+          const uint32_t last = i < s ? ph ^ 1u : ph;   // (a stage never used: the phase before the first)
+          ok = (PAIR ? tc::mbar_wait_cluster(full + 8 * i, last) : tc::mbar_wait(full + 8 * i, last)) && ok;
+        }
     }
   } else if (warp == kI8EpiWarps + 1) {
     // ---- products ----
@@ -413,6 +417,11 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
         }
         acc ^= 1;
         if (acc == 0) aph ^= 1u;
+      }
+      if (!ok) {
+        if constexpr (PAIR) tc::commit_pair(idle);
+        else tc::commit(idle);
+        tc::mbar_wait(idle, 0);
       }
     }
   } else {

@@ -73,14 +73,14 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   using C = GemmTile<MT>;
   extern __shared__ __align__(1024) uint8_t g_smem[];
   constexpr int BN = 128 * CTAS, BM = BN;           // features per tile, tokens per sub-tile
-  __shared__ __align__(8) uint64_t s_bars[3 * C::kStages + 2];
+  __shared__ __align__(8) uint64_t s_bars[3 * C::kStages + 3];
   __shared__ uint32_t s_tmem;
   __shared__ float s_code[16 * 32];                 // fp32 code book, one copy per lane (conflict-free look-ups)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = CTAS == 2 ? tc::cluster_rank() : 0u;
   const uint32_t tiles = (tc::smem_u32(g_smem) + 1023u) & ~1023u;
-  const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]), acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_free = acc_full + 8;
-  const uint32_t room = CTAS == 2 ? acc_full + 16 : empty;   // where the dequantising warps learn that a stage is theirs
+  const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]), acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_free = acc_full + 8, idle = acc_full + 16;
+  const uint32_t room = CTAS == 2 ? idle + 8 : empty;   // where the dequantising warps learn that a stage is theirs
   if (tid == 0) {
     for (int s = 0; s < C::kStages; ++s) {
       tc::mbar_init(full + 8 * s, rank == 0 ? 8 + CTAS : 8);   // half of the dequantising warps; in the first CTA the copies and the other CTA's tile
@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     }
     tc::mbar_init(acc_full, 1);
     tc::mbar_init(acc_free, 16 * CTAS);
+    tc::mbar_init(idle, 1);
     tc::mbar_init_fence();
     tc::prefetch_map(&map_x);
   }
@@ -291,8 +292,9 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
           }
         }
       }
-      if (!ok && rank == 0)   // given up: no copy may still be on its way when the CTAs leave
-        for (int i = 0; i < C::kStages; ++i) tc::mbar_wait(full + 8 * i, (uint32_t)((q + C::kStages - 1 - i) / C::kStages + 1) & 1u);
+      if (rank == 0)
+        for (int i = 0; i < C::kStages; ++i)   // (a stage never used: the phase before the first)
+          ok = wait(full + 8 * i, (uint32_t)((q + C::kStages - 1 - i) / C::kStages + 1) & 1u) && ok;
     }
   } else if (lane == 0 && rank == 0) {
     // =========================================== PRODUCTS =======================================================
@@ -322,6 +324,11 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
         if constexpr (CTAS == 2) tc::commit_pair(acc_full);
         else tc::commit(acc_full);
       }
+    }
+    if (!ok) {
+      if constexpr (CTAS == 2) tc::commit_pair(idle);
+      else tc::commit(idle);
+      tc::mbar_wait(idle, 0);
     }
   } else if (lane == 0 && CTAS == 2) {
     // ============================ THE SECOND CTA'S TILES, PASSED ON TO THE FIRST ================================

@@ -2,6 +2,8 @@
 //
 // Every wait is bounded: after about two seconds mbar_wait() gives up and returns false, the kernel raises the word wait_error_word()
 // hands out (host: b200_wait_error) and leaves through its ordinary teardown, so that a mistake costs one wrong result and not a hung GPU.
+// Before it leaves, the thread that issues copies waits for the last one into each of its stages, and the thread that issues products, when it
+// gave up, for those issued so far: neither may still write into memory that then belongs to another CTA.
 #pragma once
 #include <cuda.h>  // CUtensorMap (type only; the encoder is resolved at run time through the runtime, no -lcuda)
 

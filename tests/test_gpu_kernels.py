@@ -932,3 +932,19 @@ def test_tensor_memory_kernels_in_turn(K):
     alone = run(True)
     for a, b in zip(run(False), alone):
         assert torch.equal(a, b)
+
+
+def test_last_copies_are_waited_for(K):
+    """The copying threads wait for the last copy into each of their stages before a CTA leaves: with fewer stages used than there are, with
+    whole wraps of the ring and parts of one, on CTAs alone and in pairs, no such wait runs out."""
+    for nkb in (1, 2, 3, 4, 5, 6, 7, 11, 12, 13):
+        w, _, packed, scale, bs, _ = _gemv_case(K, 264, 64 * nkb, 1, "nf4", seed=nkb)
+        for M in (100, 200, 600):
+            K.qgemm(_randw((M, 64 * nkb), nkb, std=1.0).cuda(), packed, scale, 264, 64 * nkb, "nf4", bs)
+        cb, scb = K.quantize_int8(w.cuda())
+        for M in (100, 200):
+            K.linear_int8(_randw((M, 64 * nkb), nkb, dtype=torch.float16, std=1.0).cuda(), cb, scb)
+    for T in (128, 200, 300, 500, 700):
+        q, k, v = (_randw((1, 2, T, 128), i, std=1.0).cuda() for i in (2, 3, 4))
+        K.attn_prefill(q, k, v, torch.arange(T, device="cuda"))
+    K.check_gemv_errors(torch.device("cuda", 0))
