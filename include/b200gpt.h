@@ -41,9 +41,14 @@ int b200_device_info(int* sm_count, int* cc_major, int* cc_minor);
 int b200_set_pdl(int enabled);
 /* number of kernels launched by this library since load (the `gpu_launches` evidence of bench.py) */
 int64_t b200_launch_count(void);
-/* Reads (synchronising `stream`) and clears the current device's error word: non-zero when a kernel gave up a bounded wait on its
- * own copies or matrix products since the last call; the outputs of that launch are then invalid. */
+/* Error words: a kernel that gives up a bounded wait on its own copies or matrix products (after about two seconds; its outputs are then
+ * invalid) raises its device's word, and the next call of such a kernel's entry point on that device fails with B200_ERR_CUDA.
+ * b200_wait_errors_take reads and clears the words of the devices in the mask (bit d: device d) without touching the devices -- the answer covers the
+ * launches that the caller has waited for; b200_wait_error does so for the current device after synchronising `stream`.
+ * b200_wait_probe launches a wait of limit_ns (at most two seconds) that nothing ends: the way a give-up is reported, to try it. */
+uint64_t b200_wait_errors_take(uint64_t devices);
 int b200_wait_error(b200_stream_t stream, unsigned int* code);
+int b200_wait_probe(uint64_t limit_ns, b200_stream_t stream);
 /* tuning override for the fast GEMV: ksteps in {0(auto),1,2,4}, ctas_per_sm in {0(auto),1,2,3,4}; returns 0 */
 int b200_qgemv_tune(int ksteps, int ctas_per_sm, int force_generic);
 

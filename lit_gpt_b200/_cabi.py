@@ -235,7 +235,7 @@ _CORE_SIGNATURES = {
                                 c_void_p]),
 }
 _CORE_SHARED = ("b200_abi_version", "b200_last_error", "b200_device_info", "b200_set_pdl", "b200_launch_count", "b200_rmsnorm", "b200_swiglu",
-                "b200_embedding", "b200_argmax", "b200_sample", "b200_attn_prefill", "b200_wait_error")
+                "b200_embedding", "b200_argmax", "b200_sample", "b200_attn_prefill", "b200_wait_error", "b200_wait_errors_take", "b200_wait_probe")
 
 _SIGNATURES = {
     "b200_abi_version": (c_int, []),
@@ -244,6 +244,8 @@ _SIGNATURES = {
     "b200_set_pdl": (c_int, [c_int]),
     "b200_launch_count": (c_int64, []),
     "b200_wait_error": (c_int, [c_void_p, ctypes.POINTER(ctypes.c_uint)]),
+    "b200_wait_errors_take": (ctypes.c_uint64, [ctypes.c_uint64]),
+    "b200_wait_probe": (c_int, [ctypes.c_uint64, c_void_p]),
     "b200_qgemv_tune": (c_int, [c_int, c_int, c_int]),
     "b200_quantize_4bit": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "b200_dequantize_4bit": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_int, c_void_p]),
@@ -363,6 +365,17 @@ def check(rc: int, what: str = "") -> None:
         if rc == 3:
             raise NotImplementedError(f"{what}: {msg}")
         raise B200Error(f"{what} failed (code {rc}): {msg}")
+
+
+def raise_wait_errors() -> None:
+    """Raise if a kernel of a loaded library gave up a bounded wait since the last call.  Each library has its own words, in host memory: no
+    launch and no synchronisation, so this belongs behind a point where the host has waited for results, and covers the launches before it."""
+    raised = 0
+    for lib in {id(lib): lib for lib in (_lib, _core) if lib is not None}.values():
+        raised |= lib.b200_wait_errors_take(2 ** 64 - 1)
+    if raised:
+        devices = ", ".join(str(d) for d in range(64) if raised >> d & 1)
+        raise B200Error(f"a kernel on device {devices} gave up a bounded wait on its own copies or matrix products; results since then are invalid")
 
 
 def ptr(t: torch.Tensor | None) -> int | None:

@@ -14,6 +14,7 @@ import torch
 
 import lit_gpt_b200.generate.base as generate_base
 from lit_gpt_b200 import GPT
+from lit_gpt_b200 import kernels as K
 
 
 @torch.inference_mode()
@@ -65,8 +66,11 @@ def generate(
         tokens.append(token)
         if stops:
             values.append(int(token))
+            K.raise_wait_errors()
             if stopped():
                 return
         if t - yield_i >= buffer_length:
             yield from tokens[yield_i:t]
             yield_i = t
+            K.raise_wait_errors()   # of the steps whose tokens the caller has read since
+    K.check_gemv_errors(device)

@@ -13,6 +13,7 @@
 // Output is written as (B, T, H * hs), the layout attn.proj consumes (model.py:653).
 #include "attn_tc05.cuh"
 #include "mma_tile.cuh"
+#include "tc05.cuh"
 
 namespace b200 {
 
@@ -534,6 +535,7 @@ extern "C" int b200_attn_prefill(const void* q, const void* k_cache, const void*
   B200_CHECK_ARG(n_head <= 65535 && batch <= 65535, "b200_attn_prefill: grid too large");
   cudaStream_t st = (cudaStream_t)stream;
   if (T >= kTc05MinRows) {
+    B200_CHECK_WAITS("b200_attn_prefill");
     const int64_t hs = head_size, plane = (int64_t)max_seq * hs;
     const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, (__nv_bfloat16*)y, hs * n_head * T, hs * T, hs,
                          n_groups * plane, plane, hs, n_groups * plane, plane, hs, hs * n_head * T, hs * n_head, nullptr, pos, pos_is_int64, 0, nullptr, 0, T, n_head,
@@ -562,6 +564,7 @@ extern "C" int b200_attn_prefill_ragged(const void* q, int64_t ldq, const void* 
                  (reinterpret_cast<uintptr_t>(y) & 3) == 0, "b200_attn_prefill_ragged: operands must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   if (max_q_len >= kTc05MinRows) {
+    B200_CHECK_WAITS("b200_attn_prefill_ragged");
     const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)y, 0, head_size, ldq, 0, head_size, ldk, 0, head_size,
                          ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), nullptr, 0, 0, nullptr, 0, max_q_len, n_head, n_head, 0, scale * kLog2e};
     B200_CUDA(launch_attn_tc05(A, head_size, n_seqs, st));
@@ -596,6 +599,7 @@ extern "C" int b200_attn_prefill_window_ex(const void* q, int64_t ldq, const voi
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(seqs)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(y) & 3) == 0, "b200_attn_prefill_window: operands must be 16-byte aligned");
   if (!r1 && gate_mode == 0 && max_q_len >= kTc05MinRows) {
+    B200_CHECK_WAITS("b200_attn_prefill_window");
     const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)y, 0, head_size, ldq, 0, head_size, ldk, 0, head_size,
                          ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), nullptr, 0, window, reinterpret_cast<const __nv_bfloat16*>(sink), 1, max_q_len, n_head, n_kv_head,
                          0, scale * kLog2e};

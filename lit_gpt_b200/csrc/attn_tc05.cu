@@ -416,7 +416,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
       }
     }
   }
-  if (!ok && err) *err = 1u;
+  if (!ok) *err = 1u;
   tc::fence_before();
   __syncthreads();
   if (warp == 12) {
@@ -441,7 +441,9 @@ cudaError_t launch_hs(const AttnTc05Args& a, int batch, cudaStream_t st) {
       !tensor_map_2d(&mv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.v, rows, cols, a.v_r * 2, 128))
     return cudaErrorInvalidValue;
   const dim3 grid((unsigned)((a.T + 2 * kAtBM - 1) / (2 * kAtBM)), (unsigned)a.n_head, (unsigned)batch);
-  return launch(attn_tc05_kernel<HS>, grid, dim3(kAtThreads), (size_t)smem, st, a, mk, mv, wait_error_word());
+  unsigned* const err = wait_error_word();
+  if (!err) return cudaErrorMemoryAllocation;
+  return launch(attn_tc05_kernel<HS>, grid, dim3(kAtThreads), (size_t)smem, st, a, mk, mv, err);
 }
 
 }  // namespace

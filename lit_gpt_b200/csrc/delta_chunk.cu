@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
     __syncthreads();   // S complete, this stage free
     if (tid == 0 && c + 2 < chunks) fetch(c + 2);
   }
-  if (!ok && A.err) *A.err = 1u;
+  if (!ok) *A.err = 1u;
   for (int i = tid; i < DK * NC; i += Y::kThreads) {
     const int n = i % NC, c = i / NC;
     if (c < krows * L && col0 + n < dv) slot[((int64_t)(c / L) * dv + col0 + n) * L + c % L] = c < dk ? st[n * PT + c] : 0.f;
@@ -450,6 +450,7 @@ size_t b200_delta_rule_workspace_bytes(int max_rows, int n_seqs, int heads, int 
 int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size_t workspace_bytes, b200_stream_t stream) {
   B200_CHECK_ARG(a && a->q && a->k && a->v && a->beta_in && a->decay_in && a->a_log && a->dt_bias && a->state && a->out && a->seqs && workspace,
                  "b200_delta_rule_chunked: null pointer");
+  B200_CHECK_WAITS("b200_delta_rule_chunked");
   B200_CHECK_ARG(a->n_seqs > 0 && a->n_seqs <= 65535 && a->heads > 0 && a->heads <= 65535 && a->kv_heads > 0 && a->heads % a->kv_heads == 0,
                  "b200_delta_rule_chunked: bad head counts");
   B200_CHECK_ARG(a->dk > 0 && a->dk <= 128 && a->dv > 0 && a->max_rows > 0, "b200_delta_rule_chunked: key size must be 1 .. 128, max_rows the longest sequence");
@@ -463,6 +464,7 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
   DcArgs A{a->q, a->k, a->v, a->ldq, a->ldk, a->ldv, a->beta_in, a->ld_beta, a->decay_in, a->ld_decay, a->a_log, a->dt_bias, a->state, a->state_slot_stride,
            a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv, 0, (int)fit, dc_dvb(a->dv),
            reinterpret_cast<float*>(workspace), item, wait_error_word()};
+  B200_CHECK_ARG(A.err, "b200_delta_rule_chunked: no error word");
   auto al = [](const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };
   const int vec = a->dk % 4 == 0 && al(a->q, a->ldq) && al(a->k, a->ldk);
   const int L = a->dk <= 64 ? 4 : 8;   // the stored layout of a state (delta.cu)

@@ -562,7 +562,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
       if (acc == 0) ph ^= 1u;
     }
   }
-  if (!ok && err) *err = 1u;
+  if (!ok) *err = 1u;
   tc::fence_before();
   if constexpr (PAIR) tc::cluster_sync();   // the other CTA's shared memory is read until its last product
   __syncthreads();
@@ -588,7 +588,9 @@ static cudaError_t launch_i8_gemm(const I8Params& p, cudaStream_t st) {
   const int mt = (int)((p.M + BN - 1) / BN), nt = (int)((p.N + BN - 1) / BN);
   const int64_t tiles = (int64_t)mt * nt, most = sm_count() / CTAS;
   const dim3 grid((unsigned)((tiles < most ? tiles : most) * CTAS));
-  return launch_cluster(int8_gemm_kernel<PAIR>, grid, dim3(kI8GemmThreads), CTAS, (size_t)kI8Smem, st, p, ma, mb, mt, nt, wait_error_word());
+  unsigned* const err = wait_error_word();
+  if (!err) return cudaErrorMemoryAllocation;
+  return launch_cluster(int8_gemm_kernel<PAIR>, grid, dim3(kI8GemmThreads), CTAS, (size_t)kI8Smem, st, p, ma, mb, mt, nt, err);
 }
 
 }  // namespace b200
@@ -631,6 +633,7 @@ size_t b200_linear_int8_workspace_bytes(int64_t M, int64_t K) {
 
 int b200_linear_int8(const b200_linear_int8_args* a, b200_stream_t stream) {
   B200_CHECK_ARG(a != nullptr, "b200_linear_int8: null args");
+  B200_CHECK_WAITS("b200_linear_int8");
   B200_CHECK_ARG(a->x && a->cb && a->scb && a->y && a->workspace, "b200_linear_int8: null x/cb/scb/y/workspace pointer");
   B200_CHECK_ARG(a->M > 0 && a->N > 0 && a->K > 0, "b200_linear_int8: M, N, K must be positive");
   B200_CHECK_ARG(a->workspace_bytes >= b200_linear_int8_workspace_bytes(a->M, a->K), "b200_linear_int8: workspace too small (%zu < %zu)",

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
       }
     }
   }
-  if (!ok && err) *err = 1u;
+  if (!ok) *err = 1u;
   tc::fence_before();
   if constexpr (CTAS == 2) tc::cluster_sync();   // the other CTA's shared memory is read until its last product
   __syncthreads();
@@ -431,12 +431,14 @@ static cudaError_t launch_gemm(GemmParams p, cudaStream_t st) {
   }
   alignas(64) CUtensorMap map;
   if (!tensor_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.x, p.M, p.K, p.K * 2, 128)) return cudaErrorInvalidValue;
+  unsigned* const err = wait_error_word();
+  if (!err) return cudaErrorMemoryAllocation;
   constexpr int BN = SWIGLU ? 128 : 128 * CTAS;
   p.n_tiles = (int)((p.N + BN - 1) / BN);
   p.m_tiles = (int)((p.M + 128 * CTAS * MT - 1) / (128 * CTAS * MT));
   const int64_t items = (int64_t)p.n_tiles * p.m_tiles * p.ksplit, units = sm_count() / CTAS;
   const cudaError_t e = launch_cluster(qgemm_tcgen05_kernel<CTAS, MT, INT4, SWIGLU>, dim3((unsigned)((items < units ? items : units) * CTAS)), dim3(kGThreads), CTAS,
-                                       (size_t)smem, st, p, map, wait_error_word());
+                                       (size_t)smem, st, p, map, err);
   if (e != cudaSuccess || p.ksplit == 1) return e;
   const int64_t MN = p.M * p.N;
   return launch(qgemm_splitk_reduce_kernel, dim3((unsigned)((MN / 8 + 255) / 256)), dim3(256), (size_t)0, st, (const float*)p.partial, p.bias, p.y, MN, p.N, p.ksplit);
@@ -485,6 +487,7 @@ size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
 }
 
 static int gemm_args(const b200_qgemm_args* a, GemmParams& p) {
+  B200_CHECK_WAITS("b200_qgemm");
   B200_CHECK_ARG(a != nullptr, "b200_qgemm: null args");
   B200_CHECK_ARG(a->packed && a->scale && a->x && a->y, "b200_qgemm: null packed/scale/x/y pointer");
   B200_CHECK_ARG(a->M > 0 && a->N > 0 && a->K > 0, "b200_qgemm: M, N, K must be positive");

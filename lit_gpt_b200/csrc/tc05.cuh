@@ -1,7 +1,9 @@
 // tcgen05 / TMA / mbarrier helpers shared by the kernels that keep their accumulators in tensor memory (int8.cu, attn_tc05.cu).
 //
 // Every wait is bounded: after about two seconds mbar_wait() gives up and returns false, the kernel raises the word wait_error_word()
-// hands out (host: b200_wait_error) and leaves through its ordinary teardown, so that a mistake costs one wrong result and not a hung GPU.
+// hands out and leaves through its ordinary teardown, so that a mistake costs one wrong result and not a hung GPU.  The host reports it: the
+// entry points of these kernels refuse the next call (B200_CHECK_WAITS), and the serving loops read the word (b200_wait_errors_take) wherever they
+// read a result back.
 // Before it leaves, the thread that issues copies waits for the last one into each of its stages, and the thread that issues products, when it
 // gave up, for those issued so far: neither may still write into memory that then belongs to another CTA.
 #pragma once
@@ -11,7 +13,16 @@
 
 namespace b200 {
 
-unsigned* wait_error_word();   // device address of the current device's error word (api.cu); null when it cannot be had
+unsigned* wait_error_word();         // the current device's error word (api.cu); null when it cannot be had
+bool take_wait_error(int device);    // true, once, after a kernel on `device` (-1: the current one) raised it
+
+#define B200_CHECK_WAITS(what)                                                                                                       \
+  do {                                                                                                                               \
+    if (b200::take_wait_error(-1)) {                                                                                                 \
+      b200::set_error(what ": a kernel launched earlier on this device gave up a bounded wait; outputs since then are invalid");     \
+      return B200_ERR_CUDA;                                                                                                          \
+    }                                                                                                                                \
+  } while (0)
 
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                       const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -54,14 +65,17 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
-static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
-  uint64_t t0, t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+// (64 tries take far less than 50 ms: where more went by, the GPU was held up, and the time does not count)
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) {
+  uint64_t last, t, spent = 0;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(last));
   for (;;) {
     for (int i = 0; i < 64; ++i)
       if (mbar_try(bar, parity)) return true;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (t - t0 > 2000000000ull) return false;
+    spent += t - last < 50000000ull ? t - last : 50000000ull;
+    last = t;
+    if (spent > limit_ns) return false;
   }
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_try(bar, parity) || mbar_try(bar, parity) || mbar_wait_slow(bar, parity); }

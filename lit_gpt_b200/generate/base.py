@@ -251,9 +251,9 @@ def generate(model: GPT, prompt: torch.Tensor, max_returned_tokens: int, *, temp
                     break
         if n_valid:
             tokens.append(dg.history[T + 1 : T + 1 + min(n_valid, done)].clone())
-        if getattr(model, "tp_world_size", 1) > 1:  # a peer that died mid-sequence shows up here, not as a hung GPU
-            K.check_gemv_errors(device)
-        return torch.cat(tokens)
+        out = torch.cat(tokens)
+        K.check_gemv_errors(device)  # a wait that gave up (a tensor-parallel peer that died mid-sequence, say) shows up here
+        return out
 
     for _ in range(2, max_returned_tokens - T + 1):
         token = next_token(model, input_pos, token.view(1, -1), temperature=temperature, top_k=top_k).clone()
@@ -261,7 +261,9 @@ def generate(model: GPT, prompt: torch.Tensor, max_returned_tokens: int, *, temp
         if token == eos_id:
             break
         input_pos = input_pos.add_(1)
-    return torch.cat(tokens)
+    out = torch.cat(tokens)
+    K.check_gemv_errors(device)
+    return out
 
 
 @torch.inference_mode()

@@ -39,6 +39,7 @@ class Session:
     def step(self, entries: Sequence[Tuple[Any, Sequence[int], Optional[Sequence[int]]]], end: Iterable[Any] = ()) -> Optional[torch.Tensor]:
         """entries: (request id, its next tokens, places among them whose logits are wanted or None for all).  Returns the
         wanted logits, fp32 (rows, vocab), in the order of the entries -- None when nothing is wanted."""
+        K.raise_wait_errors()   # of the steps whose logits the caller has read since
         model = self.model
         tokens: List[int] = []
         seqs: List[Tuple[int, int, int]] = []
@@ -88,6 +89,7 @@ def generate_batch(model: Any, prompts: Sequence[Sequence[int]], max_new_tokens:
         for r in range(logits.shape[0]):
             K.sample_(logits[r : r + 1], token, temperature, top_k, rng)
             picked.append(int(token))
+        K.raise_wait_errors()   # (the tokens were read back: the step is done)
         return picked
 
     live = list(range(len(prompts)))

@@ -353,13 +353,13 @@ def tp_gather(h: "C.TpHandoff", batch: int, n_per_rank: int, device: torch.devic
 
 def check_gemv_errors(device: torch.device) -> None:
     """Raise if a kernel on `device` gave up a bounded wait (a tensor-parallel peer that never delivered its packets, a
-    stream-K partner CTA, a stage of a tensor-memory kernel): synchronizes the current stream.  Called by generate() at
-    its sync points."""
+    stream-K partner CTA, a stage of a tensor-memory kernel of any loaded library): synchronizes the current stream.
+    generate() ends with it, on any number of GPUs; loops that read every step's token back call raise_wait_errors() there."""
+    if device.type != "cuda":
+        return
+    torch.cuda.current_stream(device).synchronize()
+    C.raise_wait_errors()
     code = ctypes.c_uint(0)
-    with torch.cuda.device(device):
-        C.check(C.load().b200_wait_error(C.stream_ptr(device), ctypes.byref(code)), "wait_error")
-    if code.value:
-        raise C.B200Error("a kernel gave up a bounded wait on its own copies or matrix products; the output of this step is invalid")
     key = ("qgemv_tiled", device.index if device.index is not None else torch.cuda.current_device())
     ws = _workspaces.get(key)
     if ws is None:
@@ -369,6 +369,11 @@ def check_gemv_errors(device: torch.device) -> None:
     if code.value:
         what = {1: "a stream-K partner CTA", 2: "a tensor-parallel peer"}.get(code.value, f"code {code.value}")
         raise C.B200Error(f"dequant-GEMV: {what} did not deliver within the bounded wait; the output of this step is invalid")
+
+
+def raise_wait_errors() -> None:
+    """``check_gemv_errors`` for the tensor-memory kernels alone and without a synchronisation: behind a point where the host has waited."""
+    C.raise_wait_errors()
 
 
 def qgemv_tiled_tune(depth: int = 0, ctas_per_sm: int = 0, l2_prefetch: bool = True) -> None:

@@ -30,6 +30,17 @@ def restore_default_dtype():
     torch.set_default_dtype(torch.float32)
 
 
+@pytest.fixture(autouse=True)
+def no_wait_gave_up(request):
+    """No kernel of a GPU test may have left by giving up a wait: its outputs would be unfinished."""
+    yield
+    if "gpu" in request.keywords and torch.cuda.is_available():
+        from lit_gpt_b200 import _cabi
+
+        torch.cuda.synchronize()
+        _cabi.raise_wait_errors()
+
+
 @pytest.fixture
 def golden():
     import numpy as np

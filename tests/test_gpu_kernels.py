@@ -948,3 +948,32 @@ def test_last_copies_are_waited_for(K):
         q, k, v = (_randw((1, 2, T, 128), i, std=1.0).cuda() for i in (2, 3, 4))
         K.attn_prefill(q, k, v, torch.arange(T, device="cuda"))
     K.check_gemv_errors(torch.device("cuda", 0))
+
+
+def test_a_wait_that_runs_out_is_reported(K):
+    """A wait of 20 ms that nothing ends: the context stays usable, the word is read once by the check, and an entry point whose kernels wait
+    refuses the next call when nobody asked before."""
+    from lit_gpt_b200 import _cabi as C
+
+    dev = torch.device("cuda", 0)
+    _, x, packed, scale, bs, _ = _gemv_case(K, 256, 256, 40, "nf4")
+    want = K.qgemm(x.cuda(), packed, scale, 256, 256, "nf4", bs)
+    K.check_gemv_errors(dev)
+    probe = lambda: C.check(C.load().b200_wait_probe(20_000_000, C.stream_ptr()), "probe")   # noqa: E731
+    probe()
+    with pytest.raises(C.B200Error, match="gave up a bounded wait"):
+        K.check_gemv_errors(dev)
+    K.check_gemv_errors(dev)
+    probe()
+    torch.cuda.synchronize()
+    with pytest.raises(C.B200Error, match="gave up a bounded wait"):
+        K.qgemm(x.cuda(), packed, scale, 256, 256, "nf4", bs)
+    assert torch.equal(K.qgemm(x.cuda(), packed, scale, 256, 256, "nf4", bs), want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        probe()
+    K.raise_wait_errors()
+    graph.replay()
+    torch.cuda.synchronize()
+    with pytest.raises(C.B200Error, match="device 0 gave up"):
+        K.raise_wait_errors()
