@@ -586,12 +586,15 @@ typedef struct b200_delta_rule_args {
   const int32_t* seqs; int n_seqs;
   int heads, kv_heads, dk, dv, channel_decay, dtype;
   int max_rows;   /* the longest sequence's rows in this step (a hint for the launch shape; 0: unknown, treated as 1) */
+  int64_t rows;   /* b200_delta_rule_chunked: the rows of all sequences together, or more */
 } b200_delta_rule_args;
 int64_t b200_delta_rule_state_floats(int dk, int dv);
 int b200_delta_rule(const b200_delta_rule_args* args, b200_stream_t stream);
 /* The same for prompts with keys of at most 128 numbers, 32 tokens at a time with matrix products instead of one by one (csrc/delta_chunk.cu).
- * max_rows must be the longest sequence's rows.  b200_delta_rule_workspace_bytes: scratch that lets every launch cover as much as pays, 0 when
- * the call is better served by b200_delta_rule; a smaller workspace (at least one chunk) works in more launches. */
+ * What is computed depends on `rows` alone (0: n_seqs sequences of max_rows each); more rows than that raise the error word.
+ * b200_delta_rule_workspace_bytes: scratch that lets every launch cover as much as pays for n_seqs sequences of at most max_rows rows, 0 when
+ * the call is better served by b200_delta_rule; for `rows` rows in all, ask for one sequence of rows + 31 (n_seqs - 1).  A smaller workspace
+ * (at least one chunk) works in more launches. */
 size_t b200_delta_rule_workspace_bytes(int max_rows, int n_seqs, int heads, int dk, int dv);
 int b200_delta_rule_chunked(const b200_delta_rule_args* args, void* workspace, size_t workspace_bytes, b200_stream_t stream);
 /* out[row, h, :] = dtype(o / sqrt(mean(o^2) + eps) * weight * gate(z) * out_scale) per head; gate 1 silu, 2 sigmoid; weight NULL: none */

@@ -33,9 +33,10 @@ struct DcArgs {
   float* out; int64_t ldo;
   const int4* seqs;
   int heads, kv_heads, dk, dv;
-  int chunk0, n_chunks;             // this launch's chunks of every sequence
+  int n_seqs;
+  int item0, n_items, most;         // this launch's chunks, counted through all sequences, of `most` in all
   int dvb;                          // blocks of eight value columns (an even number)
-  float* ws; int64_t item;          // per (sequence, chunk, head): W | K | Q, rows of DK + 4 | P (DK) | U [dvb][32][8] | O [dvb][32][8]
+  float* ws; int64_t item;          // per (chunk, head): W | K | Q, rows of DK + 4 | P (DK) | U [dvb][32][8] | O [dvb][32][8]
   unsigned* err;
 };
 
@@ -53,7 +54,38 @@ __device__ __forceinline__ float sum2(f2 v) { float a, b; un2(v, a, b); return a
 
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
-// One chunk of one head: grid (chunks, heads, sequences).  Tokens past the sequence's end count as k = q = v = 0, beta = 0, g = 1.
+// Chunks are counted through the sequences in their order, each with as many as its rows take.  Both functions are called by whole warps.
+__device__ __forceinline__ int dc_chunks(const int4& sq) { return sq.y > 0 ? (sq.y + kDcC - 1) / kDcC : 0; }
+// the sequence of chunk `at` and the chunk's number there; -1: there are not that many
+__device__ __forceinline__ int dc_find(const DcArgs& A, int at, int& chunk) {
+  const int lane = threadIdx.x & 31;
+  int before = 0;
+  for (int s0 = 0; s0 < A.n_seqs; s0 += 32) {
+    const int n = s0 + lane < A.n_seqs ? dc_chunks(A.seqs[s0 + lane]) : 0;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, before + incl > at);
+    if (past) {
+      const int w = __ffs(past) - 1;
+      chunk = at - before - __shfl_sync(0xffffffffu, incl - n, w);
+      return s0 + w;
+    }
+    before += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  return -1;
+}
+// how many chunks lie before sequence z
+__device__ __forceinline__ int dc_before(const DcArgs& A, int z) {
+  int n = 0;
+  for (int s = threadIdx.x & 31; s < z; s += 32) n += dc_chunks(A.seqs[s]);
+  return __reduce_add_sync(0xffffffffu, n);
+}
+
+// One chunk of one head: grid (chunks, heads).  Tokens past the sequence's end count as k = q = v = 0, beta = 0, g = 1.
 template <typename T, int DK, bool CHANNEL>
 __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_kernel(DcArgs A, int vec) {
   using I = DcItem<DK>;
@@ -70,13 +102,15 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_kernel(DcArgs A, in
   griddep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int h = blockIdx.y, hk = h / (A.heads / A.kv_heads);
-  const int4 sq = A.seqs[blockIdx.z];
-  const int t0 = (A.chunk0 + (int)blockIdx.x) * C;
-  if (t0 >= sq.y) return;
+  int chunk;
+  const int z = dc_find(A, A.item0 + (int)blockIdx.x, chunk);
+  if (z < 0) return;
+  const int4 sq = A.seqs[z];
+  const int t0 = chunk * C;
   const int nt = min(C, sq.y - t0);
   const int64_t row0 = (int64_t)sq.x + t0;
   const int dk = A.dk, dv = A.dv;
-  float* const item = A.ws + (((int64_t)blockIdx.z * A.n_chunks + blockIdx.x) * A.heads + h) * A.item;
+  float* const item = A.ws + ((int64_t)blockIdx.x * A.heads + h) * A.item;
 
   // ---- the chunk's keys, queries, decays and write strengths ----
   const float* const kp = A.k + row0 * A.ldk + (int64_t)hk * dk;
@@ -276,11 +310,12 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
   griddep_launch();
   griddep_wait();
   const int4 sq = A.seqs[blockIdx.z];
-  const int t_first = A.chunk0 * C;
-  if (t_first >= sq.y) return;
-  const int chunks = min(A.n_chunks, (sq.y - t_first + C - 1) / C);
+  const int before = dc_before(A, blockIdx.z), all = dc_chunks(sq);
+  const int c_first = max(0, A.item0 - before), chunks = min(all, A.item0 + A.n_items - before) - c_first, t_first = c_first * C;
+  if (tid == 0 && before + all > A.most) *A.err = 1u;   // more rows than the caller said
+  if (chunks <= 0 && (all > 0 || A.item0 > 0)) return;   // (a sequence without rows still starts its slot from zero)
   const int dk = A.dk, dv = A.dv;
-  const float* const items = A.ws + ((int64_t)blockIdx.z * A.n_chunks * A.heads + h) * A.item;
+  const float* const items = A.ws + ((int64_t)(before + c_first - A.item0) * A.heads + h) * A.item;
   const int64_t step = (int64_t)A.heads * A.item;
 
   auto fetch = [&](int c) {   // one thread
@@ -295,12 +330,12 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
     copy(dst + (I::kHead + Y::kSlice) * 4, src + I::kHead + (int64_t)(A.dvb + (col0 >> 3)) * C * 8, Y::kSlice * 4);
   };
   if (tid == 0) {
-    fetch(0);
+    if (chunks > 0) fetch(0);
     if (chunks > 1) fetch(1);
   }
   const int krows = (dk + L - 1) / L;
   float* const slot = A.state + (int64_t)sq.w * A.state_slot_stride + (int64_t)h * krows * L * dv;
-  const bool from_slot = sq.z > 0 || A.chunk0 > 0;
+  const bool from_slot = sq.z > 0 || c_first > 0;
   for (int i = tid; i < DK * NC; i += Y::kThreads) {
     const int n = i % NC, c = i / NC;
     st[n * PT + c] = from_slot && c < dk && col0 + n < dv ? slot[((int64_t)(c / L) * dv + col0 + n) * L + c % L] : 0.f;
@@ -392,7 +427,7 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
 }
 
 template <typename T, int DK, bool CHANNEL>
-cudaError_t chunk_launch(const DcArgs& A, int n_seqs, int vec, cudaStream_t st) {
+cudaError_t chunk_launch(const DcArgs& A, int vec, cudaStream_t st) {
   constexpr int C = kDcC;
   constexpr int smem = (2 * C * DK + (CHANNEL ? C * DK : C) + C + 8 * C * C + 4 * C * C) * 4;
   static PerDeviceOnce once;
@@ -401,11 +436,11 @@ cudaError_t chunk_launch(const DcArgs& A, int n_seqs, int vec, cudaStream_t st) 
     if (e != cudaSuccess) return e;
     once.done();
   }
-  return launch(delta_chunk_kernel<T, DK, CHANNEL>, dim3((unsigned)A.n_chunks, (unsigned)A.heads, (unsigned)n_seqs), dim3(kDcThreads), smem, st, A, vec);
+  return launch(delta_chunk_kernel<T, DK, CHANNEL>, dim3((unsigned)A.n_items, (unsigned)A.heads), dim3(kDcThreads), smem, st, A, vec);
 }
 
 template <int DK, int NC>
-cudaError_t carry_launch(const DcArgs& A, int n_seqs, int L, cudaStream_t st) {
+cudaError_t carry_launch(const DcArgs& A, int L, cudaStream_t st) {
   using Y = DcCarry<DK, NC>;
   static PerDeviceOnce once;
   if (once.need()) {
@@ -413,22 +448,22 @@ cudaError_t carry_launch(const DcArgs& A, int n_seqs, int L, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     once.done();
   }
-  return launch(delta_carry_kernel<DK, NC>, dim3((unsigned)((A.dv + NC - 1) / NC), (unsigned)A.heads, (unsigned)n_seqs), dim3(Y::kThreads), Y::kSmem, st, A, L);
+  return launch(delta_carry_kernel<DK, NC>, dim3((unsigned)((A.dv + NC - 1) / NC), (unsigned)A.heads, (unsigned)A.n_seqs), dim3(Y::kThreads), Y::kSmem, st, A, L);
 }
 
 template <typename T, int DK>
-cudaError_t segment_launch(const DcArgs& A, bool channel, int n_seqs, int vec, int L, cudaStream_t st) {
-  const cudaError_t e = channel ? chunk_launch<T, DK, true>(A, n_seqs, vec, st) : chunk_launch<T, DK, false>(A, n_seqs, vec, st);
+cudaError_t segment_launch(const DcArgs& A, bool channel, int vec, int L, cudaStream_t st) {
+  const cudaError_t e = channel ? chunk_launch<T, DK, true>(A, vec, st) : chunk_launch<T, DK, false>(A, vec, st);
   if (e != cudaSuccess) return e;
   // 16 columns per slice share the reads of W, Q and K best; with fewer slices than SMs, slices of 8 have the shorter chain
-  const int64_t wide = (int64_t)((A.dv + 15) / 16) * A.heads * n_seqs;
-  return wide * 4 >= (int64_t)sm_count() * 3 ? carry_launch<DK, 16>(A, n_seqs, L, st) : carry_launch<DK, 8>(A, n_seqs, L, st);
+  const int64_t wide = (int64_t)((A.dv + 15) / 16) * A.heads * A.n_seqs;
+  return wide * 4 >= (int64_t)sm_count() * 3 ? carry_launch<DK, 16>(A, L, st) : carry_launch<DK, 8>(A, L, st);
 }
 
 int dc_dvb(int dv) { return (dv + 15) / 16 * 2; }
 int64_t dc_item(int dk, int dv) { return (dk <= 64 ? (int64_t)DcItem<64>::kHead : (int64_t)DcItem<128>::kHead) + 2 * (int64_t)dc_dvb(dv) * kDcC * 8; }
 
-constexpr int64_t kDcMaxBytes = 256ll << 20;   // scratch of one segment of chunks
+constexpr int64_t kDcMaxBytes = 256ll << 20;   // scratch of one launch's chunks
 constexpr int kDcMinRows = 64;
 
 }  // namespace
@@ -453,16 +488,19 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
   B200_CHECK_WAITS("b200_delta_rule_chunked");
   B200_CHECK_ARG(a->n_seqs > 0 && a->n_seqs <= 65535 && a->heads > 0 && a->heads <= 65535 && a->kv_heads > 0 && a->heads % a->kv_heads == 0,
                  "b200_delta_rule_chunked: bad head counts");
-  B200_CHECK_ARG(a->dk > 0 && a->dk <= 128 && a->dv > 0 && a->max_rows > 0, "b200_delta_rule_chunked: key size must be 1 .. 128, max_rows the longest sequence");
+  B200_CHECK_ARG(a->dk > 0 && a->dk <= 128 && a->dv > 0 && a->rows >= 0 && (a->rows > 0 || a->max_rows > 0),
+                 "b200_delta_rule_chunked: key size must be 1 .. 128; the rows of all sequences (or the longest sequence's) are needed");
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(a->seqs) | reinterpret_cast<uintptr_t>(workspace)) & 15) == 0,
                  "b200_delta_rule_chunked: seqs and workspace must be 16-byte aligned");
   const int64_t item = dc_item(a->dk, a->dv);
-  int64_t fit = (int64_t)(workspace_bytes / (size_t)(item * 4)) / ((int64_t)a->n_seqs * a->heads);
+  int64_t fit = (int64_t)(workspace_bytes / (size_t)(item * 4)) / a->heads;   // chunks
   B200_CHECK_ARG(fit > 0, "b200_delta_rule_chunked: workspace too small (%zu bytes)", workspace_bytes);
-  const int total = (a->max_rows + kDcC - 1) / kDcC;
-  if (fit > total) fit = total;
+  // n sequences of `rows` rows in all have at most (rows + 31 n) / 32 chunks
+  const int64_t most = a->rows > 0 ? (a->rows + (int64_t)(kDcC - 1) * a->n_seqs) / kDcC : (int64_t)a->n_seqs * ((a->max_rows + kDcC - 1) / kDcC);
+  B200_CHECK_ARG(most <= 0x3fffffff, "b200_delta_rule_chunked: too many rows");
+  if (fit > most) fit = most;
   DcArgs A{a->q, a->k, a->v, a->ldq, a->ldk, a->ldv, a->beta_in, a->ld_beta, a->decay_in, a->ld_decay, a->a_log, a->dt_bias, a->state, a->state_slot_stride,
-           a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv, 0, (int)fit, dc_dvb(a->dv),
+           a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv, a->n_seqs, 0, (int)fit, (int)most, dc_dvb(a->dv),
            reinterpret_cast<float*>(workspace), item, wait_error_word()};
   B200_CHECK_ARG(A.err, "b200_delta_rule_chunked: no error word");
   auto al = [](const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };
@@ -470,11 +508,12 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
   const int L = a->dk <= 64 ? 4 : 8;   // the stored layout of a state (delta.cu)
   const bool ch = a->channel_decay != 0;
   cudaStream_t st = (cudaStream_t)stream;
-  for (A.chunk0 = 0; A.chunk0 < total; A.chunk0 += (int)fit) {
-    A.n_chunks = (int)(total - A.chunk0 < fit ? total - A.chunk0 : fit);
+  for (int64_t at = 0; at < most; at += fit) {
+    A.item0 = (int)at;
+    A.n_items = (int)(most - at < fit ? most - at : fit);
     B200_FLOAT_TYPES(a->dtype, T, {
-      if (a->dk <= 64) B200_CUDA((segment_launch<T, 64>(A, ch, a->n_seqs, vec, L, st)));
-      else B200_CUDA((segment_launch<T, 128>(A, ch, a->n_seqs, vec, L, st)));
+      if (a->dk <= 64) B200_CUDA((segment_launch<T, 64>(A, ch, vec, L, st)));
+      else B200_CUDA((segment_launch<T, 128>(A, ch, vec, L, st)));
     });
   }
   return B200_OK;

@@ -1069,7 +1069,7 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_in: torch
                channel_decay: bool, max_rows: int = 0) -> torch.Tensor:
     """Gated delta rule over the step's rows; state (slots, floats) fp32 is read (unless the sequence starts at 0) and written.
     q, k (n, kv_heads * dk), v (n, heads * dv) fp32; beta_in (n, heads), decay_in (n, heads [* dk]) raw projections; max_rows: the
-    longest sequence's rows in this step (picks the kernel and the launch shape; 0: unknown).  -> fp32 (n, heads * dv)"""
+    longest sequence's rows in this step (picks the kernel and the launch shape, not what is computed; 0: unknown).  -> fp32 (n, heads * dv)"""
     C.require_cuda(q, k, v, beta_in, decay_in, a_log, dt_bias, state, seqs)
     if not (q.dtype == k.dtype == v.dtype == state.dtype == torch.float32) or seqs.dtype != torch.int32 or not seqs.is_contiguous():
         raise C.B200Error("delta_rule: q, k, v and the state are fp32, seqs int32")
@@ -1085,12 +1085,18 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_in: torch
                            beta_in=beta_in.data_ptr(), ld_beta=beta_in.stride(0), decay_in=decay_in.data_ptr(), ld_decay=decay_in.stride(0),
                            a_log=a_log.data_ptr(), dt_bias=dt_bias.data_ptr(), state=state.data_ptr(), state_slot_stride=state.stride(0),
                            out=out.data_ptr(), ldo=out.stride(0), seqs=seqs.data_ptr(), n_seqs=seqs.shape[0], heads=heads, kv_heads=kv_heads,
-                           dk=dk, dv=dv, channel_decay=int(channel_decay), dtype=_code(beta_in), max_rows=int(max_rows))
+                           dk=dk, dv=dv, channel_decay=int(channel_decay), dtype=_code(beta_in), max_rows=int(max_rows), rows=q.shape[0])
     lib, n_seqs = C.load_core(), seqs.shape[0]
-    # a prompt goes 32 tokens at a time (max_rows has to be the longest sequence then: a value that cannot be is taken as unknown)
-    need = lib.b200_delta_rule_workspace_bytes(int(max_rows), n_seqs, heads, dk, dv) if DELTA_CHUNKED and max_rows * n_seqs >= q.shape[0] else 0
+    # a prompt goes 32 tokens at a time; max_rows says whether that pays, the rows there are how much scratch it takes
+    need = lib.b200_delta_rule_workspace_bytes(int(max_rows), n_seqs, heads, dk, dv) if DELTA_CHUNKED else 0
+    ws = None
     if need:
-        ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+        need = min(need, lib.b200_delta_rule_workspace_bytes(q.shape[0] + 31 * (n_seqs - 1), 1, heads, dk, dv) or need)
+        try:
+            ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+        except torch.OutOfMemoryError:   # token by token, which needs none
+            pass
+    if ws is not None:
         C.check(lib.b200_delta_rule_chunked(ctypes.byref(args), ws.data_ptr(), need, C.stream_ptr(q.device)), "delta_rule")
     else:
         C.check(lib.b200_delta_rule(ctypes.byref(args), C.stream_ptr(q.device)), "delta_rule")

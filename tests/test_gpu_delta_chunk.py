@@ -120,6 +120,50 @@ def test_delta_chunks_in_segments(K, chunks):
     assert torch.equal(out, want) and torch.equal(state, whole)
 
 
+@pytest.mark.parametrize("lens,hint", [((200, 10), 110), ((100, 1, 1), 64), ((70, 300, 5), 64), ((33, 0, 100, 64), 65)])
+def test_delta_chunks_compute_every_row_whatever_the_hint(K, lens, hint):
+    """max_rows picks the kernel; rows past it are computed all the same, and a sequence without rows starts its slot from zero as before."""
+    H, G, dk, dv = 4, 2, 64, 40
+    starts = [7 * (i % 2) for i in range(len(lens))]
+    data = _inputs(lens, starts, H, G, dk, dv, True, torch.float32, 11, 0)
+    dev = [t.contiguous().cuda() for t in data[:7]]
+    out = {}
+    for rows in (hint, max(lens), 0):   # 0: token by token
+        state = _stored(data[7], dk, 4).float().cuda()
+        out[rows] = K.delta_rule(*dev, state, data[8].cuda(), H, G, dk, dv, True, max_rows=rows), state
+    (a, sa), (b, sb), (c, sc) = out[hint], out[max(lens)], out[0]
+    assert torch.equal(a, b) and torch.equal(sa, sb)
+    assert (a - c).abs().max() <= 1e-4 * c.abs().max() and (sa - sc).abs().max() <= 1e-4 * sc.abs().max()
+
+
+def test_delta_chunk_scratch_follows_the_rows(K, monkeypatch):
+    """One prompt among many single rows takes scratch for the rows there are; without memory for it the call runs token by token."""
+    H, G, dk, dv, lens = 2, 2, 128, 32, (96,) + (1,) * 40
+    data = _inputs(lens, [3] * len(lens), H, G, dk, dv, False, torch.bfloat16, 3, 0)
+    dev, seqs = [t.contiguous().cuda() for t in data[:7]], data[8].cuda()
+    empty, asked = torch.empty, []
+
+    def run(limit):
+        def alloc(*a, **kw):
+            if kw.get("dtype") == torch.uint8:
+                asked.append(a[0])
+                if a[0] > limit:
+                    raise torch.OutOfMemoryError("scratch")
+            return empty(*a, **kw)
+
+        state = _stored(data[7], dk, 8).float().cuda()
+        monkeypatch.setattr(torch, "empty", alloc)
+        y = K.delta_rule(*dev, state, seqs, H, G, dk, dv, False, max_rows=96)
+        monkeypatch.undo()
+        return y, state
+
+    (a, sa), (b, sb) = run(1 << 40), run(0)
+    from lit_gpt_b200 import _cabi as C
+    chunk = C.load().b200_delta_rule_workspace_bytes(64, 1, H, dk, dv) // 2
+    assert asked[0] == (sum(lens) + 31 * len(lens)) // 32 * chunk
+    assert (a - b).abs().max() <= 1e-4 * b.abs().max() and (sa - sb).abs().max() <= 1e-4 * sb.abs().max()
+
+
 def test_delta_chunk_rule(K):
     """What stays with the token-by-token kernel: single rows, short portions, wide keys, unknown lengths."""
     from lit_gpt_b200 import _cabi as C
