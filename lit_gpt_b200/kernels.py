@@ -390,9 +390,11 @@ def qgemm(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, N: int, K:
     C.require_cuda(x, packed, scale, bias)
     x = _bf16c(x, "x")
     bias = _bf16c(bias, "bias")
+    if x.shape[-1] != K:
+        raise C.B200Error(f"qgemm: x has rows of {x.shape[-1]} numbers, the weights take {K}")
     M = x.numel() // K
-    if x.numel() != M * K:
-        raise C.B200Error("qgemm: x does not hold whole rows of length K")
+    if out is not None and (out.numel() != M * N or out.dtype != torch.bfloat16 or not out.is_contiguous()):
+        raise C.B200Error(f"qgemm: out must be {M} x {N} contiguous bfloat16 numbers")
     y = out if out is not None else torch.empty(tuple(x.shape[:-1]) + (N,), dtype=torch.bfloat16, device=x.device)
     need = C.load().b200_qgemm_workspace_bytes(M, N, K)   # fp32 partial sums of a one-tile prompt split over k ranges; 0 otherwise
     ws = _ws("qgemm", x.device, need) if need else None
@@ -413,9 +415,9 @@ def qgemm_swiglu(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, pac
     Raises NotImplementedError where ``qgemm_swiglu_supported`` is false."""
     C.require_cuda(x, packed, scale, packed2, scale2)
     x = _bf16c(x, "x")
+    if x.shape[-1] != K:
+        raise C.B200Error(f"qgemm_swiglu: x has rows of {x.shape[-1]} numbers, the weights take {K}")
     M = x.numel() // K
-    if x.numel() != M * K:
-        raise C.B200Error("qgemm_swiglu: x does not hold whole rows of length K")
     y = torch.empty(tuple(x.shape[:-1]) + (N,), dtype=torch.bfloat16, device=x.device)
     args = C.QGemmArgs(packed=packed.data_ptr(), scale=scale.data_ptr(), qtype=QTYPES[quant_type], blocksize=blocksize, M=M, N=N, K=K,
                        x=x.data_ptr(), y=y.data_ptr())

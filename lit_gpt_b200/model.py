@@ -657,7 +657,8 @@ class LLaMAMLP(nn.Module):
                 and f1.quant_type == f2.quant_type and f1.quant_type != "int8" and not torch.compiler.is_compiling()):
             # gate and up projections + SwiGLU in one pass over both weight matrices
             return self.proj(f1.gemv(x, other=f2))
-        if rows > 128 and x.is_cuda and x.dtype == torch.bfloat16 and not torch.compiler.is_compiling() and prefill_pair(f1, f2, rows):
+        if (rows > 128 and x.is_cuda and x.dtype == torch.bfloat16 and not torch.compiler.is_compiling() and prefill_pair(f1, f2, rows)
+                and x.size(-1) == f1.in_features):
             (pw, ps), (pw2, ps2) = f1.packed(), f2.packed()
             return self.proj(K.qgemm_swiglu(x, pw, ps, pw2, ps2, f1.out_features, f1.in_features, f1.quant_type, f1.blocksize))
         x_fc_1 = self.fc_1(x)

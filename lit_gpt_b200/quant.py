@@ -398,11 +398,19 @@ def prefill_linear(q: QLinear, x: torch.Tensor) -> torch.Tensor:
     return F.linear(x, w, q.bias)
 
 
+def _called_plainly(m: nn.Module) -> bool:
+    """True when calling `m` does nothing but run QLinear.forward: no override of it, no hook on the module or on all modules."""
+    every = torch.nn.modules.module
+    return (type(m).forward is QLinear.forward and type(m).__call__ is nn.Module.__call__ and "forward" not in m.__dict__
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or every._global_forward_hooks
+                     or every._global_forward_pre_hooks or every._global_backward_hooks or every._global_backward_pre_hooks))
+
+
 def prefill_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
     """True where the two projections of a gated MLP can be one launch with the product in its epilogue: plain 4-bit modules of one layout
     without a bias or a hook (a hook wants the projections' own outputs) whose reference layouts are resident, at sizes the library calls the shorter way."""
-    if not all(isinstance(m, QLinear) and type(m).forward is QLinear.forward and m.is_quantized and not m.released and m.quant_type != "int8"
-               and m.bias is None and not (m._forward_hooks or m._forward_pre_hooks) for m in (gate, up)):
+    if not all(isinstance(m, QLinear) and _called_plainly(m) and m.is_quantized and not m.released and m.quant_type != "int8" and m.bias is None
+               for m in (gate, up)):
         return False
     return (gate.quant_type == up.quant_type and gate.blocksize == up.blocksize and gate.in_features == up.in_features
             and gate.out_features == up.out_features
