@@ -396,8 +396,9 @@ def qgemm(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, N: int, K:
     if out is not None and (out.numel() != M * N or out.dtype != torch.bfloat16 or not out.is_contiguous()):
         raise C.B200Error(f"qgemm: out must be {M} x {N} contiguous bfloat16 numbers")
     y = out if out is not None else torch.empty(tuple(x.shape[:-1]) + (N,), dtype=torch.bfloat16, device=x.device)
-    need = C.load().b200_qgemm_workspace_bytes(M, N, K)   # fp32 partial sums of a one-tile prompt split over k ranges; 0 otherwise
-    ws = _ws("qgemm", x.device, need) if need else None
+    need = C.load().b200_qgemm_workspace_bytes(M, N, K)   # fp32 partial sums of a launch split over k ranges; 0 otherwise
+    # (from the allocator on every call: safe on any stream and inside a capture, whose graph then keeps it)
+    ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
     args = C.QGemmArgs(packed=packed.data_ptr(), scale=scale.data_ptr(), qtype=QTYPES[quant_type], blocksize=blocksize, M=M, N=N, K=K,
                        x=x.data_ptr(), bias=C.ptr(bias), y=y.data_ptr(), workspace=C.ptr(ws), workspace_bytes=0 if ws is None else ws.numel())
     C.check(C.load().b200_qgemm(ctypes.byref(args), C.stream_ptr(x.device)), "qgemm")

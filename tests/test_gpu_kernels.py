@@ -977,3 +977,34 @@ def test_a_wait_that_runs_out_is_reported(K):
     torch.cuda.synchronize()
     with pytest.raises(C.B200Error, match="device 0 gave up"):
         K.raise_wait_errors()
+
+
+@pytest.mark.parametrize("M,N,Kdim", [(300, 1280, 1280), (100, 768, 1024)])
+def test_qgemm_split_under_capture_and_on_streams(K, M, N, Kdim):
+    """A launch with k ranges captured without a call before it, replayed after calls that need more scratch, and run on two streams at once:
+    each has partial sums of its own."""
+    cases = []
+    for seed in (1, 2):
+        _, _, packed, scale, bs, _ = _gemv_case(K, N, Kdim, 1, "nf4", seed=seed)
+        cases.append((_randw((M, Kdim), seed + 5, std=1.0).cuda(), packed, scale))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = K.qgemm(*cases[0], N, Kdim, "nf4", 64)
+    want = [K.qgemm(*c, N, Kdim, "nf4", 64) for c in cases]
+    from lit_gpt_b200 import _cabi as C
+    assert C.load().b200_qgemm_workspace_bytes(M, N, Kdim) > 0
+    for rows in (400, 700, 1000):
+        K.qgemm(_randw((rows, Kdim), 3, std=1.0).cuda(), cases[0][1], cases[0][2], N, Kdim, "nf4", 64)
+    got.zero_()
+    graph.replay()
+    assert torch.equal(got, want[0])
+    streams = [torch.cuda.Stream() for _ in cases]
+    out = [[], []]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for c, s, o in zip(cases, streams, out):
+            with torch.cuda.stream(s):
+                o.append(K.qgemm(*c, N, Kdim, "nf4", 64))
+    torch.cuda.synchronize()
+    for o, w in zip(out, want):
+        assert all(torch.equal(y, w) for y in o)
