@@ -27,6 +27,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 // memory, barriers, tiles of twice the rows and keys: 8.8 against 5.1 us for 17 rows, 8.0 against 8.2 us for 128 -- and steps faster: 18.6 against
 // 31.5 us for 600 rows of 32 heads, 230 against 589 us for 4096.
 constexpr int kTc05MinRows = 128;
+// Its tensor maps want rows that do not overlap; anything else (one key row repeated by a stride of 0, say) stays with the tiles here.
+inline bool tc05_rows(int64_t ldk, int64_t ldv, int64_t cols) { return ldk >= cols && ldv >= cols; }
 
 // Where the operands live, in elements.  The cached layout of the GQA models is (B, H or G, rows, HS); a ragged batch packs the
 // query rows of all sequences into one (rows, H * HS) matrix and gives, per sequence, seqs[b] = {first query row, query rows,
@@ -563,7 +565,7 @@ extern "C" int b200_attn_prefill_ragged(const void* q, int64_t ldq, const void* 
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(seqs)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(y) & 3) == 0, "b200_attn_prefill_ragged: operands must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
-  if (max_q_len >= kTc05MinRows) {
+  if (max_q_len >= kTc05MinRows && tc05_rows(ldk, ldv, (int64_t)n_head * head_size)) {
     B200_CHECK_WAITS("b200_attn_prefill_ragged");
     const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)y, 0, head_size, ldq, 0, head_size, ldk, 0, head_size,
                          ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), nullptr, 0, 0, nullptr, 0, max_q_len, n_head, n_head, 0, scale * kLog2e};
@@ -598,7 +600,7 @@ extern "C" int b200_attn_prefill_window_ex(const void* q, int64_t ldq, const voi
   B200_CHECK_ARG(((ldq | ldk | ldv) & 7) == 0 && (ldy & 1) == 0, "b200_attn_prefill_window: leading dimensions must be multiples of 8 elements");
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(seqs)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(y) & 3) == 0, "b200_attn_prefill_window: operands must be 16-byte aligned");
-  if (!r1 && gate_mode == 0 && max_q_len >= kTc05MinRows) {
+  if (!r1 && gate_mode == 0 && max_q_len >= kTc05MinRows && tc05_rows(ldk, ldv, (int64_t)n_kv_head * head_size)) {
     B200_CHECK_WAITS("b200_attn_prefill_window");
     const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)y, 0, head_size, ldq, 0, head_size, ldk, 0, head_size,
                          ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), nullptr, 0, window, reinterpret_cast<const __nv_bfloat16*>(sink), 1, max_q_len, n_head, n_kv_head,

@@ -1008,3 +1008,37 @@ def test_qgemm_split_under_capture_and_on_streams(K, M, N, Kdim):
     torch.cuda.synchronize()
     for o, w in zip(out, want):
         assert all(torch.equal(y, w) for y in o)
+
+
+@pytest.mark.parametrize("hs,H", [(128, 2), (64, 3)])
+@pytest.mark.parametrize("repeat_keys", [False, True])
+def test_attn_ragged_tiles(K, hs, H, repeat_keys):
+    """Several sequences in one launch -- long portions, portions within a tile and single rows over longer contexts, the contexts' rows in another
+    order than the queries', rows that belong to nobody and are poisoned between them -- against each sequence alone in 64 bits.  With keys whose
+    rows are one row repeated by a stride of 0, too."""
+    new, start = (300, 1, 128, 1, 129, 40, 513), (0, 700, 255, 0, 127, 3, 640)
+    g = torch.Generator().manual_seed(hs)
+    order, at, ctx = (4, 0, 6, 2, 1, 5, 3), [0] * len(new), 5
+    for i in order:
+        at[i] = ctx
+        ctx += new[i] + start[i] + 3
+    n, ld = sum(new), 2 * H * hs + 16
+    q = torch.randn(n, H * hs, generator=g).bfloat16()
+    kv = torch.full((ctx, ld), float("nan")).bfloat16()
+    seqs, first = [], 0
+    for i, (m, s) in enumerate(zip(new, start)):
+        kv[at[i] : at[i] + m + s, : 2 * H * hs] = torch.randn(m + s, 2 * H * hs, generator=g).bfloat16()
+        seqs.append((first, m, s, at[i]))
+        first += m
+    dev = kv.cuda()
+    k, v = dev[:, : H * hs], dev[:, H * hs : 2 * H * hs]
+    one = torch.randn(1, H * hs, generator=g).bfloat16()
+    if repeat_keys:
+        k = one.cuda().expand(ctx, -1)
+    y = K.latent_prefill(q.cuda(), k, v, torch.tensor(seqs, dtype=torch.int32).cuda(), max(new), H, hs, hs, 0.2)
+    for f, m, s, a in seqs:
+        kk = one.expand(m + s, -1) if repeat_keys else kv[a : a + m + s, : H * hs]
+        lim = torch.arange(s, s + m)
+        ref = _attn_exact(q[f : f + m].view(m, H, hs), kk.reshape(m + s, H, hs), kv[a : a + m + s, H * hs : 2 * H * hs].reshape(m + s, H, hs), lim,
+                          torch.zeros_like(lim), 0.2)
+        _attn_close(y[f : f + m], ref)
