@@ -722,22 +722,36 @@ def test_qgemm_single_k_block(K):
 
 
 @pytest.mark.parametrize("qt", ["nf4", "fp4", "int4"])
-@pytest.mark.parametrize("M,N,Kdim", [(129, 9472, 256), (203, 11008, 4096), (257, 9472, 128), (513, 9480, 384), (1281, 5504, 512), (4096, 1408, 256)])
-def test_qgemm_swiglu_is_the_separate_launches(K, qt, M, N, Kdim):
-    """Both projections and their product in one launch: bit-equal to two GEMMs and the product wherever those run without k ranges
-    (the same sums in the same order, the same roundings), at rows and features on both sides of a tile."""
+@pytest.mark.parametrize("M,N,Kdim,ranges", [(129, 9472, 256, False), (257, 9472, 128, False), (513, 9480, 384, False), (1281, 5504, 512, False),
+                                             (4096, 1408, 256, False), (300, 5632, 2048, False), (1281, 2048, 2048, False), (203, 5632, 2048, True),
+                                             (129, 1024, 4096, True)])
+def test_qgemm_swiglu_is_the_separate_launches(K, qt, M, N, Kdim, ranges):
+    """Both projections and their product in one launch, at rows and features on both sides of a tile, with few and many k-blocks: bit-equal to two
+    GEMMs and the product where those run without k ranges (the same sums in the same order, the same roundings).  With k ranges the sums
+    differ in their last bits, so some of the bf16 roundings of either projection go the other way by one unit, 2^-8 of the number at most."""
     from lit_gpt_b200 import _cabi as C
     _, _, p1, s1, bs, _ = _gemv_case(K, N, Kdim, 1, qt, seed=M)
     _, _, p2, s2, _, _ = _gemv_case(K, N, Kdim, 1, qt, seed=N)
     x = _randw((M, Kdim), 5, std=3.0).cuda()
-    if not K.qgemm_swiglu_supported(M, N, Kdim, qt, bs):
-        with pytest.raises(NotImplementedError):
-            K.qgemm_swiglu(x, p1, s1, p2, s2, N, Kdim, qt, bs)
-        pytest.skip("the separate launches are the shorter way here")
-    assert C.load().b200_qgemm_workspace_bytes(M, N, Kdim) == 0
+    assert K.qgemm_swiglu_supported(M, N, Kdim, qt, bs)
+    assert (C.load().b200_qgemm_workspace_bytes(M, N, Kdim) > 0) == ranges
     y = K.qgemm_swiglu(x, p1, s1, p2, s2, N, Kdim, qt, bs)
     ref = K.swiglu(K.qgemm(x, p1, s1, N, Kdim, qt, bs), K.qgemm(x, p2, s2, N, Kdim, qt, bs))
-    assert torch.equal(y, ref)
+    if ranges:
+        assert (y.double() - ref.double()).norm() <= 2.0 ** -8 * ref.double().norm()
+    else:
+        assert torch.equal(y, ref)
+
+
+@pytest.mark.parametrize("qt", ["nf4", "fp4", "int4"])
+@pytest.mark.parametrize("M,N,Kdim", [(128, 11008, 4096), (513, 11008, 4096), (700, 5632, 4096)])
+def test_qgemm_swiglu_refuses_what_runs_apart(K, qt, M, N, Kdim):
+    bs = 128 if qt == "int4" else 64
+    assert not K.qgemm_swiglu_supported(M, N, Kdim, qt, bs)
+    x, w = torch.zeros(M, Kdim, dtype=torch.bfloat16, device="cuda"), torch.zeros(N * Kdim // 2, dtype=torch.uint8, device="cuda")
+    s = torch.zeros(N * Kdim // bs, dtype=torch.float32, device="cuda")
+    with pytest.raises(NotImplementedError):
+        K.qgemm_swiglu(x, w, s, w, s, N, Kdim, qt, bs)
 
 
 def test_mlp_prompt_pair_keeps_hooks(K):
