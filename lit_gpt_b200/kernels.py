@@ -426,9 +426,9 @@ def qgemm_swiglu(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, pac
     return y
 
 
-def qgemm_tune(mt3: bool = True) -> None:
+def qgemm_tune(wide: bool = True) -> None:
     """development switch: long prompts may use tiles of 512 tokens (default) or keep to 256"""
-    C.check(C.load().b200_qgemm_tune(1 if mt3 else 0), "qgemm_tune")
+    C.check(C.load().b200_qgemm_tune(1 if wide else 0), "qgemm_tune")
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, delta: Optional[torch.Tensor] = None,

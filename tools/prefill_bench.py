@@ -26,7 +26,7 @@ def main() -> None:
     ap.add_argument("--tokens", type=int, default=4096)
     ap.add_argument("--reps", type=int, default=5)
     ap.add_argument("--layers", type=int, default=None)
-    ap.add_argument("--mt3", type=int, default=1, help="0: GEMM tiles of 256 tokens instead of up to 512")
+    ap.add_argument("--wide", type=int, default=1, help="0: GEMM tiles of 256 tokens instead of up to 512")
     args = ap.parse_args()
 
     import bench
@@ -34,7 +34,7 @@ def main() -> None:
     from lit_gpt_b200 import kernels as K
     from lit_gpt_b200.fabric import Fabric
 
-    K.qgemm_tune(bool(args.mt3))
+    K.qgemm_tune(bool(args.wide))
     fabric = Fabric(devices=1, plugins=QuantPrecision(args.qt, torch.bfloat16))
     T = args.tokens
     model, cfg = bench.build_random_model(args.model, args.qt, T, 1, fabric, n_layer=args.layers)
