@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Headline benchmark: Llama-2-7B nf4 weight-only, batch-1 greedy decode tok/s (BASELINE.json configs[1]).
+"""Headline benchmark: Llama-2-7B nf4 weight-only, batch-1 greedy decode tok/s.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--workload NAME]
 
@@ -35,7 +35,7 @@ WORKLOADS = {
     "mistral-7b-int4-bs1": ("Mistral-7B-v0.1", "int4", 1, 16, 0),
     "llama2-70b-int4-bs1-ctx2048": ("Llama-2-70b-hf", "int4", 1, 16, 2032),
 }
-# algorithmic bytes per parameter (SURVEY §8d): nf4 / fp4 = 4 bits + one fp32 absmax per 64; int4 g128 = 4 bits + one fp16 scale and
+# algorithmic bytes per parameter: nf4 / fp4 = 4 bits + one fp32 absmax per 64; int4 g128 = 4 bits + one fp16 scale and
 # one 4-bit zero-point per 128 (0.51953).  The kernels stream the fused half2 {scale, zero} form of int4 (0.53125): reported as
 # `streamed_bytes_per_param`, not used for the roofline fraction.
 BPP = {"nf4": 0.5 + 4 / 64, "fp4": 0.5 + 4 / 64, "int4": 0.5 + 2.5 / 128}
@@ -51,7 +51,7 @@ def measured_peaks():
 
 
 class ClockSampler(threading.Thread):
-    """SM clock + throttle reasons sampled in-process through NVML every ~2 ms (B200_PROFILING.md clocks line); only the
+    """SM clock + throttle reasons sampled in-process through NVML every ~2 ms; only the
     samples taken between mark_start() and mark_end() -- the timed region -- are reported."""
 
     def __init__(self, device: "torch.device"):
@@ -156,7 +156,7 @@ def build_random_model(cfg_name: str, mode: str, max_seq: int, batch: int, fabri
 
 
 def step_bytes(full_cfg, mode: str, ctx: int, batch: int, tp: int, head_sharded: bool = False) -> dict:
-    """Algorithmic HBM bytes of one decode step per GPU (SURVEY §8d): packed weights + scales of every Linear once,
+    """Algorithmic HBM bytes of one decode step per GPU: packed weights + scales of every Linear once,
     plus the filled KV rows at n_query_groups heads in bf16.  lm_head is replicated under TP (generate/tp.py:77-80)."""
     c = full_cfg
     per_layer = c.n_embd * (c.n_head + 2 * c.n_query_groups) * c.head_size + c.n_embd * c.n_embd + 3 * c.n_embd * c.intermediate_size
@@ -339,7 +339,7 @@ def run_ours(args) -> None:
     def prefill_context():
         for blk in model.transformer.h:
             blk.attn.kv_cache.reset_parameters()
-        if ctx:  # synthetic N(0,1) K/V history (SURVEY §8d config 3), then the prompt after it
+        if ctx:  # synthetic N(0,1) K/V history, then the prompt after it
             gg = torch.Generator(device=dev).manual_seed(7)
             for blk in model.transformer.h:
                 blk.attn.kv_cache.k[:, :, :ctx].normal_(generator=gg)

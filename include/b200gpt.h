@@ -7,8 +7,8 @@
  *
  * Each function cites the reference interface it replaces (file:line into yuanyaaa/lit-gpt).  The reference's
  * own quantized arithmetic lives in bitsandbytes==0.41.0 (requirements-all.txt:3) behind
- * lightning.fabric.plugins.BitsandbytesPrecision (generate/base.py:129-134); see INTEGRATION.md for the
- * binding a maintainer would add.
+ * lightning.fabric.plugins.BitsandbytesPrecision (generate/base.py:129-134); a maintainer's
+ * binding is described with this project's documents.
  */
 #ifndef B200GPT_H
 #define B200GPT_H
@@ -27,7 +27,7 @@ typedef void* b200_stream_t; /* cudaStream_t */
 enum b200_status { B200_OK = 0, B200_ERR_INVALID = 1, B200_ERR_CUDA = 2, B200_ERR_UNSUPPORTED = 3 };
 enum b200_dtype { B200_BF16 = 0, B200_F16 = 1, B200_F32 = 2 };
 /* 4-bit weight formats.  NF4/FP4: bitsandbytes block-64 codebooks; INT4: this project's group-128 format
- * (the reference has no gptq/int4 code; see DESIGN.md §4.3). */
+ * (the reference has no gptq/int4 code). */
 enum b200_qtype { B200_Q_NF4 = 0, B200_Q_FP4 = 1, B200_Q_INT4 = 2 };
 /* GEMV epilogues */
 enum b200_epilogue { B200_EPI_STORE = 0, B200_EPI_RESIDUAL = 1, B200_EPI_SWIGLU = 2 };
@@ -128,7 +128,7 @@ int b200_untile_4bit(const void* tiled, int64_t N, int64_t K, int qtype, int blo
  * `prefetch`/`prefetch_bytes` (optional): a range the kernel asks the L2 to fetch (cp.async.bulk.prefetch.L2) -
  * the weights of the NEXT kernel in the decode graph - so HBM stays busy across the kernel boundary. */
 /* Tensor-parallel hand-off fused into the GEMV (replaces the all_reduce hook of generate/tp.py:73-74 on the decode path;
- * DESIGN.md §6).  PRODUCER = the row-parallel Linear (attn.proj, mlp.proj): its epilogue stores this rank's partial
+ * below).  PRODUCER = the row-parallel Linear (attn.proj, mlp.proj): its epilogue stores this rank's partial
  * into slot `rank` of EVERY rank's buffer over NVLink peer memory as self-validating 32-bit packets
  * `tag << 16 | bf16 bits` (one store per output element, no fence, no separate flag: the "LL" scheme).
  * CONSUMER = the next Linear (whose `delta` the all-reduced tensor would have been): its prologue polls the `world`
@@ -151,7 +151,7 @@ typedef struct b200_tp_handoff {
   void* recv_seq;         /* consumer: LOCAL sequence counter of the buffer read (bumped by the launch's last CTA) */
   void* recv_done;        /* consumer: local CTA counter */
 } b200_tp_handoff;
-/* All-gather over the same slots (SURVEY §8f-3: `lm_head` sharded by rows under tensor parallelism; the reference replicates it,
+/* All-gather over the same slots (`lm_head` sharded by rows under tensor parallelism; the reference replicates it,
  * generate/tp.py:77-80).  The sharded Linear's GEMV is launched as a PRODUCER (tp->send_seq / peer_y set, y may be NULL): rank r's
  * (batch, N / world) outputs land in slot r of every rank's gather buffer.  This call is the CONSUMER: it polls the `world` slots of
  * the local buffer (consumer fields of `h`), unpacks them into out (batch, world * n_per_rank) bf16 in rank order -- i.e. the
@@ -230,7 +230,7 @@ int b200_qgemv_tiled(const b200_qgemv_tiled_args* args, b200_stream_t stream);
 int b200_qgemv_tiled_tune(int depth, int ctas_per_sm, int l2_prefetch);
 /* diagnostics (no counterpart in the reference): the next `slots` b200_qgemv_tiled launches record eight per-CTA phase time
  * stamps (%globaltimer, ns) into buf[slots][160][8] (uint64, device memory, caller-owned, zeroed by the caller);
- * buf = NULL switches it off.  tools/trace_step.py turns them into the per-launch timeline quoted in DESIGN.md. */
+ * buf = NULL switches it off.  tools/trace_step.py turns them into the per-launch timeline. */
 int b200_qgemv_tiled_trace(void* buf, int slots);
 
 /* ---- RMSNorm (replaces lit_gpt/rmsnorm.py:19-25 and the residual add at lit_gpt/model.py:591) ------------
@@ -242,9 +242,9 @@ int b200_rmsnorm(const void* x, const void* delta, const void* weight, float eps
  *      view/permute/split, apply_rope 767-773, KVCache.forward 788-795, scaled_dot_product_attention 658-665)
  * qkv: (batch, (n_head + 2*n_groups) * head_size) bf16 in the reference's per-group interleaved order
  *      [q * q_per_kv, k, v] x n_groups (lit_gpt/model.py:621-628).
- * cos/sin: the model's own tables (max_seq, rope_n_elem), fp32 or bf16 (SURVEY F5: never recomputed in-kernel).
+ * cos/sin: the model's own tables (max_seq, rope_n_elem), fp32 or bf16 (never recomputed in-kernel).
  * pos: device int64/int32 scalar = position being written (input_pos); keys 0..pos are attended.
- * k_cache/v_cache: (batch, n_groups, max_seq, head_size) bf16, GQA-native (n_groups heads, SURVEY F6).
+ * k_cache/v_cache: (batch, n_groups, max_seq, head_size) bf16, GQA-native (n_groups heads).
  * out: (batch, n_head * head_size) bf16.  head_size in {64, 128}. */
 typedef struct b200_attn_decode_args {
   const void* qkv;

@@ -4,7 +4,7 @@ Same contract as the reference's ``chat.base.generate``: yields the new tokens o
 longest stop sequence so that a stop sequence is never emitted, and returns as soon as one matches.  On the fused quantized
 path every step is one replay of the captured decode graph (``generate.base.DecodeGraph``); the only host synchronisation is
 the read of the new token that a streaming caller needs anyway.  The prompt / UI / tokenizer parts of chat/base.py are out of
-scope (SURVEY §2).
+scope.
 """
 from __future__ import annotations
 

@@ -1,4 +1,4 @@
-"""Pre-quantized checkpoints (SURVEY §8f-2).
+"""Pre-quantized checkpoints.
 
 The reference re-quantizes from 16-bit weights on every launch and, under tensor parallelism, serialises the ranks while
 doing so (generate/tp.py:163-192; lit_gpt/utils.py:350-356 only knows plain ``weight`` / ``bias`` keys).  Here a model

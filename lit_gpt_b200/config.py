@@ -2,7 +2,7 @@
 ``from_name`` / ``from_json`` / ``from_checkpoint``, derived ``head_size`` / ``rope_n_elem`` /
 ``padded_vocab_size``) so a ``lit_config.json`` written by the reference loads unchanged.
 
-The registry below holds the model families on the hot path named by BASELINE.json (pythia for the plumbing config,
+The registry below holds the model families on the hot path (pythia for the plumbing config,
 Llama-2 / CodeLlama / Mistral / TinyLlama for the quantized decode configs); other families can be passed as kwargs
 or through ``lit_config.json``.
 """

@@ -1,9 +1,9 @@
-// Fused RoPE + KV-cache append + split-K flash-decode attention for T = 1 (DESIGN.md §5.3).
+// Fused RoPE + KV-cache append + split-K flash-decode attention for T = 1.
 //
 // Replaces, for one decode step, lit_gpt/model.py:624-653: the qkv view/permute/split (624-628), K/V expand
 // for GQA (633-635), apply_rope on q and k (641-644 -> 767-773), KVCache.forward index_copy_ (649 -> 788-795)
 // and F.scaled_dot_product_attention over the FULL max_seq cache with a boolean mask row (651 -> 658-665).
-// Here the cache is GQA-native (n_query_groups heads, SURVEY F6), only the filled positions 0..pos are read,
+// Here the cache is GQA-native (n_query_groups heads), only the filled positions 0..pos are read,
 // and the q_per_kv query heads of a group share each K/V row from registers.
 //
 // HBM-bound on the KV stream (bytes = 2 * groups * ctx * head_size * 2 B per layer): rows are read with

@@ -1,4 +1,4 @@
-// Peer-memory plumbing for the tensor-parallel hand-off (DESIGN.md §6): a symmetric buffer per rank, allocated here with
+// Peer-memory plumbing for the tensor-parallel hand-off: a symmetric buffer per rank, allocated here with
 // cudaMalloc (torch's caching allocator sub-allocates, and an IPC handle names a whole allocation), exported to the
 // other ranks of the node as a CUDA IPC handle and mapped by them.  Setup-time only: nothing here runs per token.
 // Replaces the NCCL all-reduce the reference issues from all_reduce_output (generate/tp.py:73-74) on the decode path;
@@ -10,7 +10,7 @@
 using namespace b200;
 
 namespace b200 {
-// Consumer side of an ALL-GATHER over the hand-off slots (lm_head sharded by rows, SURVEY §8f-3): slot r holds rank r's
+// Consumer side of an ALL-GATHER over the hand-off slots (lm_head sharded by rows): slot r holds rank r's
 // (batch, n_per_rank) outputs as self-validating packets `tag << 16 | bf16` written by that rank's GEMV epilogue; poll until the
 // tag matches, unpack into out (batch, world * n_per_rank) bf16; the last CTA bumps the buffer's sequence counter.
 __global__ void __launch_bounds__(256) tp_gather_kernel(const uint32_t* __restrict__ slots, int64_t slot_stride, int world, int batch,

@@ -1,4 +1,4 @@
-// Fused dequant-GEMV for batch 1..16 decode (the dominant kernel of the hot path; DESIGN.md §5.1).
+// Fused dequant-GEMV for batch 1..16 decode (the dominant kernel of the hot path).
 //
 // Replaces bnb.nn.Linear4bit.forward at lit_gpt/model.py:619,656,713,714,716,519 (reference: the
 // kgemm_4bit_inference_naive kernel for a single token, dequantize_4bit + cuBLAS otherwise).

@@ -1,4 +1,4 @@
-// Streaming fused dequant-GEMV over the TILED weight layout (csrc/tile.cu), batch 1..16 (DESIGN.md §5.1).
+// Streaming fused dequant-GEMV over the TILED weight layout (csrc/tile.cu), batch 1..16.
 //
 // Replaces bnb.nn.Linear4bit.forward at lit_gpt/model.py:619,656,713,714,716,519.
 //

@@ -2,7 +2,7 @@
 //   NF4 / FP4 block-wise 4-bit: restates bitsandbytes 0.41 kQuantizeBlockwise / kDequantizeBlockwise (the code the
 //   reference reaches through Params4bit.cuda(), generate/base.py:168, generate/tp.py:190); bit-exact to
 //   oracle/quant_ref.{py,c}.
-//   INT4 group-128: this project's own format (DESIGN.md §4.3), bit-exact to oracle/quant_ref.py::quantize_int4_g128.
+//   INT4 group-128: this project's own format, bit-exact to oracle/quant_ref.py::quantize_int4_g128.
 // These run once at load time; they are HBM-bound streaming kernels (one warp per quantisation block).
 #include "common.cuh"
 
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) dequantize_int4_kernel(const uint32_t* __
 }
 
 
-// ---- double quantisation of the absmax vector (bnb.nf4-dq / fp4-dq, SURVEY Q2): per 256 values, subtract the
+// ---- double quantisation of the absmax vector (bnb.nf4-dq / fp4-dq): per 256 values, subtract the
 // caller-given offset (mean), take the block absmax, map x / absmax2 to the nearest entry of the 256-entry
 // "dynamic" code with bitsandbytes' pivot search (kernels.cu dQuantize<0>), and write back the DEQUANTISED value
 // code[q] * absmax2 + offset, which is what every later dequantise / GEMV of a -dq layer uses.

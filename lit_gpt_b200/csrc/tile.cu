@@ -1,4 +1,4 @@
-// Kernel-side "tiled" weight layout for the streaming dequant-GEMV (DESIGN.md §4.4), and its inverse.
+// Kernel-side "tiled" weight layout for the streaming dequant-GEMV, and its inverse.
 //
 // The reference layout (bitsandbytes Params4bit: row-major packed nibbles + a separate absmax vector; this
 // project's int4: row-major qweight + {scale, zero} words) makes a warp that feeds mma.sync touch 8 different

@@ -82,7 +82,7 @@ def all_gather_output(world_size: int, module: torch.nn.Module, ins: Any, outs: 
 
 
 def shard_lm_head(fabric: Any, model: GPT) -> GPT:
-    """NOT in the reference (generate/tp.py:77-80 leaves `lm_head` replicated; SURVEY §8f-3 lists this as the next step): shard
+    """NOT in the reference (generate/tp.py:77-80 leaves `lm_head` replicated): shard
     `lm_head` by rows (vocabulary slices) so that each rank streams 1 / world of it.  Call after `tensor_parallel`, before the
     move to the GPU.  Decode: the slices are all-gathered over the peer-memory slots (b200_tp_gather) and every rank holds the full
     logits, bit-identical to the replicated Linear; prefill / module path: `all_gather` hook.  Skipped (model unchanged) when the

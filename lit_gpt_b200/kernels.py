@@ -90,7 +90,7 @@ def dynamic_map(device: torch.device) -> torch.Tensor:
 
 
 def double_quant_absmax(absmax: torch.Tensor, offset: Optional[float] = None):
-    """-> (q uint8 [n], absmax2 fp32 [ceil(n/256)], offset float, absmax_dequantised fp32 [n])  (SURVEY Q2)."""
+    """-> (q uint8 [n], absmax2 fp32 [ceil(n/256)], offset float, absmax_dequantised fp32 [n]) ."""
     C.require_cuda(absmax)
     absmax = absmax.contiguous().float()
     n = absmax.numel()

@@ -9,7 +9,7 @@ What differs is what runs underneath on a B200:
 * When every Linear is a quantized ``QLinear`` and the block is Llama-shaped, a decode step (T = 1) does not walk the
   module tree at all: ``GPT._fused_decode`` issues 5 kernels per block (norm folded into GEMV prologues, residual and
   SwiGLU into epilogues), all capturable in one CUDA graph.
-* Anything else (fp32 / CPU, e.g. BASELINE config 1) runs the reference formulation in plain torch, so results are
+* Anything else (fp32 / CPU, e.g. a pythia model on the CPU) runs the reference formulation in plain torch, so results are
   identical to the reference there.
 """
 from __future__ import annotations
@@ -451,7 +451,7 @@ class GPT(nn.Module):
         a0 = blocks[0].attn.attn if blocks else None
         # EXPERIMENT, off by default (B200_FUSE_ATTN_MAX_SEQ=1024 enables it): the attention step fused into the QKV GEMV's
         # kernel (b200_qgemv_tiled_args::attn).  Correct (tests/test_gpu_kernels.py::test_qgemv_tiled_fused_attention) and 32
-        # launches per token fewer, but measured SLOWER on B200 (632 vs 676 tok/s, DESIGN.md appendix): in-kernel the
+        # launches per token fewer, but measured SLOWER on B200 (632 vs 676 tok/s): in-kernel the
         # attention tail runs on one SM per head at the GEMV's register budget, 5.5 - 7.5 us against ~6 us for the stand-alone
         # cluster kernel INCLUDING its launch boundary
         fuse_attn = (not tp and B == 1 and a0 is not None and self.max_seq_length <= int(os.environ.get("B200_FUSE_ATTN_MAX_SEQ", "0"))
@@ -615,7 +615,7 @@ class CausalSelfAttention(nn.Module):
         probe = torch.empty(0, device=device, dtype=dtype)
         native = (probe.is_cuda and probe.dtype == torch.bfloat16 and c.head_size in FUSED_HEAD_SIZES
                   and c.rope_n_elem % 2 == 0 and (rope_cache_length is None or rope_cache_length == c.rope_n_elem))
-        if native:  # GQA-native: n_query_groups heads (the reference stores n_head, SURVEY F6)
+        if native:  # GQA-native: n_query_groups heads (the reference stores n_head)
             shape = (batch_size, c.n_query_groups, max_seq_length, c.head_size)
             return KVCache(shape, shape, device=device, dtype=dtype, gqa_native=True)
         heads = 1 if c.n_query_groups == 1 else c.n_head
@@ -672,7 +672,7 @@ class LLaMAMLP(nn.Module):
 
 
 class LLaMAMoE(nn.Module):
-    """Mixtral-style routing is outside the hot path (no BASELINE config uses it); kept so that
+    """Mixtral-style routing is outside the hot path (no benchmarked configuration uses it); kept so that
     ``config._mlp_class = "LLaMAMoE"`` resolves and fails with a clear message."""
 
     def __init__(self, config: Config) -> None:
@@ -683,7 +683,7 @@ class LLaMAMoE(nn.Module):
 def build_rope_cache(seq_len: int, n_elem: int, device: Optional[torch.device] = None, base: int = 10000,
                      condense_ratio: int = 1) -> Tuple[torch.Tensor, torch.Tensor]:
     """cos/sin tables (seq_len, n_elem).  Positions are an integer arange divided by a python int, i.e. they take
-    the DEFAULT float dtype exactly as the reference does (model.py:759; SURVEY F5) — the kernels consume these
+    the DEFAULT float dtype exactly as the reference does (model.py:759) — the kernels consume these
     tables and never recompute angles."""
     theta = 1.0 / (base ** (torch.arange(0, n_elem, 2, device=device).float() / n_elem))
     seq_idx = torch.arange(seq_len, device=device) / condense_ratio

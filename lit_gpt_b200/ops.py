@@ -1,4 +1,4 @@
-"""``torch.library`` custom ops over the C-ABI kernels (SURVEY §8b "Torch custom ops").
+"""``torch.library`` custom ops over the C-ABI kernels.
 
 The reference has no custom ops: its quantized Linear, RMSNorm and attention are compositions of ATen ops that
 ``torch.compile`` traces (tests/test_model.py:564-575 asserts zero graph breaks).  The replacements are opaque kernels,

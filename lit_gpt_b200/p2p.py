@@ -11,7 +11,7 @@ Buffer layout per rank:  [2 hand-off buffers][world slots][slot_bytes]  then, pe
 ``uint32 seq | .. | recv_done (+32)``.  A slot holds one 32-bit packet ``tag << 16 | bf16`` per element (the tag makes the
 packet self-validating: no fence and no separate arrival flag).  Consecutive hand-offs alternate between the two buffers
 (attention branch: 0, MLP branch: 1): a rank can only overwrite a peer's slot of buffer b after that peer has produced
-the next hand-off on the other buffer, i.e. after it has finished reading buffer b (DESIGN.md §6).
+the next hand-off on the other buffer, i.e. after it has finished reading buffer b.
 """
 from __future__ import annotations
 
@@ -39,7 +39,7 @@ class PeerComm:
         self.data_bytes = 2 * self.world * self.slot_bytes
         # two-stage exchange (b200_tp_handoff::reduced): every consumer CTA sums only its slice of the vector over the ranks and
         # republishes it in a local buffer that all CTAs then read.  OFF by default: bit-identical, but the extra dependent round
-        # trip costs more than the world x fewer L2 reads save (TP-8 Llama-2-7B 703 vs 851 tok/s, 70B 205 vs 214; DESIGN.md appendix).
+        # trip costs more than the world x fewer L2 reads save (TP-8 Llama-2-7B 703 vs 851 tok/s, 70B 205 vs 214).
         # B200_TP_TWO_STAGE_MIN=<world> switches it on from that many ranks.
         import os
 

@@ -55,9 +55,9 @@ class QLinear(nn.Module):
         self.in_features, self.out_features = in_features, out_features
         self.mode, self.compute_dtype = mode, compute_dtype
         self.quant_type = mode.split("-")[0]  # nf4 | fp4 | int4 | int8
-        self.threshold = 6.0  # int8 only: LLM.int8() outlier threshold (Linear8bitLt(threshold=6.0), SURVEY Q3)
+        self.threshold = 6.0  # int8 only: LLM.int8() outlier threshold (Linear8bitLt(threshold=6.0))
         self.SCB: Optional[torch.Tensor] = None  # int8 only: per-row absmax (bitsandbytes Int8Params.SCB); weight holds CB
-        self.double_quant = mode.endswith("-dq")  # compress_statistics=True: absmax itself 8-bit quantised (SURVEY Q2)
+        self.double_quant = mode.endswith("-dq")  # compress_statistics=True: absmax itself 8-bit quantised
         self.absmax: Optional[torch.Tensor] = None  # fp32 absmax the kernels read (for -dq: the dequantised statistics)
         self.blocksize = 128 if self.quant_type == "int4" else 64
         kw = dict(device=device, dtype=dtype)
@@ -95,7 +95,7 @@ class QLinear(nn.Module):
         """The per-block scale tensor the kernels consume (fp32 absmax, or packed half2 {scale, zero} for int4)."""
         return self.sz if self.quant_type == "int4" else self.absmax
 
-    # -- one resident copy of the weights (VERDICT r1 housekeeping): the tiled layout is a byte permutation of (weight, scale) ----
+    # -- one resident copy of the weights: the tiled layout is a byte permutation of (weight, scale) ----
     released = False
 
     def packed(self) -> tuple:
@@ -194,7 +194,7 @@ class QLinear(nn.Module):
                     self.fold = f
                     return
 
-    # -- pre-quantized checkpoints (SURVEY §8f-2): the packed tensors go to disk as they are, no re-quantisation on load --
+    # -- pre-quantized checkpoints: the packed tensors go to disk as they are, no re-quantisation on load --
     def export_packed(self) -> dict:
         """CPU copies of exactly what ``quantize_`` produced (packed codes + statistics), keyed for ``import_packed``."""
         if not self.is_quantized:
@@ -387,7 +387,7 @@ def prefill_linear(q: QLinear, x: torch.Tensor) -> torch.Tensor:
     """T > 16 rows: the tcgen05 / TMEM dequant-GEMM (csrc/qgemm.cu): weights are dequantised tile by tile in shared
     memory, the bf16 matrix never exists in HBM.  Shapes it does not cover (K not a multiple of the quantisation
     block, N % 8 != 0: toy configs only) take the reference's own formulation -- dequantize_4bit to bf16, then a
-    library GEMM (SURVEY Q1) -- with the dequantisation done by this library's kernel."""
+    library GEMM -- with the dequantisation done by this library's kernel."""
     if x.dtype == torch.bfloat16:
         try:
             pw, ps = q.packed()

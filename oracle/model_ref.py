@@ -3,7 +3,7 @@
 TEST INFRASTRUCTURE (see oracle/__init__.py) — never imported by the product.
 
 PINNED: ``tests/test_oracle_model.py`` checks every function here against golden vectors produced by the
-UNMODIFIED reference (``tests/golden/make_golden.py``) and, when /root/reference is present, against the
+UNMODIFIED reference (``tests/golden/make_golden.py``) and, when the reference is present, against the
 reference modules directly.  Each function cites the reference lines it restates.
 
 The weights are a plain ``dict[str, Tensor]`` with the reference's state-dict keys
@@ -76,7 +76,7 @@ def layernorm(x: Tensor, weight: Tensor, bias: Optional[Tensor], eps: float) -> 
 # -- lit_gpt/model.py:746-764 -----------------------------------------------------------------------
 def build_rope_cache(seq_len: int, n_elem: int, base: int = 10000, condense_ratio: int = 1,
                      pos_dtype: Optional[torch.dtype] = None) -> Tuple[Tensor, Tensor]:
-    """`pos_dtype` restates SURVEY F5: the reference divides an int64 arange by a python int, which yields
+    """`pos_dtype` restates a property of the reference: it divides an int64 arange by a python int, which yields
     the DEFAULT float dtype (bf16 under `--precision bf16-true`), so positions alias above 256."""
     theta = 1.0 / (base ** (torch.arange(0, n_elem, 2).float() / n_elem))
     seq_idx = torch.arange(seq_len).to(pos_dtype or torch.get_default_dtype()) / condense_ratio

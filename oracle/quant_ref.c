@@ -5,7 +5,7 @@
  *
  * PARITY UNPINNED: the arithmetic restated here lives in bitsandbytes==0.41.0 (reference
  * requirements-all.txt:3; call sites generate/base.py:129-134, generate/tp.py:127-134,
- * lit_gpt/lora.py:156-160), which is absent from /root/reference.  It follows the published kernels of
+ * lit_gpt/lora.py:156-160), which is absent from the reference.  It follows the published kernels of
  * that version: kQuantizeBlockwise / kDequantizeBlockwise / dQuantizeNF4 / dQuantizeFP4 /
  * dDequantizeFP4Tree (csrc/kernels.cu) and kgemm_4bit_inference_naive for the GEMV.  int4 group-128 is
  * this project's own format.  Cross-checked against oracle/quant_ref.py in tests/test_oracle_quant.py.
@@ -105,8 +105,8 @@ static inline float bf16_round(float f) {
 }
 
 /* y[b, n] = sum_k x[b, k] * bf16(code[q[n,k]] * absmax[(n*K+k)/bs])   (fp32 accumulate; y left in fp32).
- * This is "dequantize_4bit to the compute dtype, then F.linear" (the reference's batch>1 / prefill path,
- * SURVEY Q1) restated with a wide accumulator; it is also the timed CPU baseline for the GEMV. */
+ * This is "dequantize_4bit to the compute dtype, then F.linear" (the reference's batch>1 / prefill
+ * call) restated with a wide accumulator; it is also the timed CPU baseline for the GEMV. */
 void ref_gemv_4bit(const uint8_t* packed, const float* absmax, const float* x, float* y, int64_t N, int64_t K, int B,
                    int blocksize, int quant_type, int round_w_bf16) {
   const float* code = quant_type == 0 ? NF4_CODE : FP4_CODE;

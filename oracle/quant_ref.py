@@ -7,8 +7,8 @@ PARITY UNPINNED for every function in this file: the arithmetic of
 generate/base.py:105,129-134; generate/tp.py:104,127-134; lit_gpt/lora.py:156-160;
 lit_gpt/utils.py:85-87) lives in ``bitsandbytes==0.41.0``
 (requirements-all.txt:3), reached through ``lightning@ed367ca``
-(requirements.txt:2).  Neither is vendored under /root/reference nor installable
-here, and the reference's own tests hold no golden vectors for it (SURVEY §8c).
+(requirements.txt:2).  Neither is vendored by the reference nor installable
+here, and the reference's own tests hold no golden vectors for it.
 What follows restates the published algorithm of bitsandbytes 0.41.x
 (csrc/kernels.cu: kQuantizeBlockwise / kDequantizeBlockwise / dQuantizeNF4 /
 dQuantizeFP4 / dDequantizeFP4Tree / dQuantize<0>; bitsandbytes/functional.py:
@@ -245,7 +245,7 @@ def dequantize_absmax(q, absmax2, offset) -> np.ndarray:
 
 
 # ---------------------------------------------------------------------------------------------
-# int4 group-128 (this project's format; SURVEY F2: the reference has no gptq/int4 code)
+# int4 group-128 (this project's format: the reference has no gptq/int4 code)
 # ---------------------------------------------------------------------------------------------
 def _f16(x):
     return np.asarray(x, np.float16)

@@ -95,7 +95,7 @@ def main() -> None:
         out["gen_prompt"] = prompt.numpy()
         out["gen_tokens"] = toks.numpy()
         out["gen_logits"] = torch.stack(logits_log).numpy()
-        # batch-2 decode step at the model level (generate() is batch-1 only; SURVEY §8d config 3)
+        # batch-2 decode step at the model level (generate() is batch-1 only)
         model.set_kv_cache(batch_size=2)
         xb = torch.stack([x[0], x[0].flip(0)])
         out["b2_prefill_logits"] = model(xb, torch.arange(T)).numpy()

@@ -1,4 +1,4 @@
-"""The streaming generator of chat/base.py:24-68 (second caller of next_token, SURVEY §8f-1): the reference's own test vectors
+"""The streaming generator of chat/base.py:24-68 (second caller of next_token): the reference's own test vectors
 (tests/test_chat.py:16-51) for the stop-sequence / hold-back logic, run against lit_gpt_b200.chat.base.generate."""
 from itertools import repeat
 from unittest.mock import MagicMock

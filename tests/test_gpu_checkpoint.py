@@ -1,4 +1,4 @@
-"""Pre-quantized checkpoint round trip (lit_gpt_b200/checkpoint.py, SURVEY §8f-2): what is written is what sits in HBM, and a
+"""Pre-quantized checkpoint round trip (lit_gpt_b200/checkpoint.py): what is written is what sits in HBM, and a
 model loaded from it -- without running the quantizer -- is bit-identical to the one that was quantized from 16-bit weights."""
 import pytest
 import torch

@@ -1,4 +1,4 @@
-"""bnb.int8 (LLM.int8()) CUDA path against oracle/quant_ref.py:310-345 (SURVEY §8 Q3).
+"""bnb.int8 (LLM.int8()) CUDA path against oracle/quant_ref.py:310-345.
 
 Integer work (CB, SCB, CA, the int32 products, the rounding chain without outliers) is compared bit-exactly.  With
 outlier columns the fp32 side product is summed in ascending column order on the GPU and by a BLAS matmul in the

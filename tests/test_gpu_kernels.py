@@ -166,7 +166,7 @@ def test_qgemv_tiled_fused_attention(K, qt, H, Kdim, pos):
 @pytest.mark.parametrize("N,Kdim,B", [(5120, 13824, 16), (2048, 13824, 8), (1000, 5120, 16), (640, 8192, 16), (5120, 13824, 9), (96, 28672, 16)])
 def test_qgemv_tiled_k_windows(K, qt, N, Kdim, B):
     """Batch x K too large for the activation rows to sit in shared memory beside the ring (Llama-2-13B gptq.int4 at batch
-    16, BASELINE config 3): the kernel sweeps its tiles once per k-window.  Plain, norm + delta prologue with the residual
+    16): the kernel sweeps its tiles once per k-window.  Plain, norm + delta prologue with the residual
     epilogue, and the SwiGLU pair, against the oracle's dequantised weights."""
     w, x, packed, scale, bs, deq = _gemv_case(K, N, Kdim, B, qt, seed=N + B)
     tiled = K.tile_4bit(packed, scale, N, Kdim, qt, bs)
@@ -349,7 +349,7 @@ def test_qgemv_bias_and_errors(K):
 
 
 def test_qgemv_linearity_full_size(K):
-    """Size-independent property at the BASELINE shape (Llama-2-7B gate projection, 11008 x 4096):
+    """Size-independent property at the benchmark's shape (Llama-2-7B gate projection, 11008 x 4096):
     y(a*x1 + x2) tracks a*y(x1) + y(x2), and a one-hot x reads back a dequantised weight column exactly."""
     N, Kdim = 11008, 4096
     w = _randw((N, Kdim), 11)
@@ -631,7 +631,7 @@ def test_qgemv_tiled_bias_and_errors(K):
 
 
 def test_qgemv_tiled_onehot_reads_dequantised_column(K):
-    """Size-independent property at the BASELINE shape (Llama-2-7B gate projection 11008 x 4096)."""
+    """Size-independent property at the benchmark's shape (Llama-2-7B gate projection 11008 x 4096)."""
     N, Kdim = 11008, 4096
     w = _randw((N, Kdim), 11)
     packed, absmax = K.quantize_4bit(w.cuda(), "nf4")

@@ -1,8 +1,8 @@
 """End-to-end parity of the quantized CUDA path (GPT / generate through the public API) against the oracle:
 the reference's model restated in oracle/model_ref.py (pinned on reference goldens) with every Linear weight replaced
-by dequant(quant(W)) from oracle/quant_ref.py — exactly what `--quantize bnb.nf4` computes (SURVEY §8c).
+by dequant(quant(W)) from oracle/quant_ref.py — exactly what `--quantize bnb.nf4` computes.
 
-Tolerance (stated, as north_star asks): max-abs logit error of the CUDA path against the fp32 oracle must be
+Tolerance: max-abs logit error of the CUDA path against the fp32 oracle must be
 <= 2x the error of the reference formulation run in bf16 (oracle in bf16 on CPU) + 1e-3 * max|logit|; greedy tokens
 must agree wherever the oracle's top-1/top-2 margin exceeds that tolerance.
 """
@@ -131,7 +131,7 @@ def test_quantized_toy_against_oracle(golden, name, mode):
 
 @torch.inference_mode()
 def test_llama7b_width_two_layers_nf4():
-    """Llama-2-7B shapes (d=4096, 32 heads, I=11008, V=32000) at depth 2: every kernel at its BASELINE tile shapes."""
+    """Llama-2-7B shapes (d=4096, 32 heads, I=11008, V=32000) at depth 2: every kernel at the benchmark's tile shapes."""
     from lit_gpt_b200 import Config
 
     cfg = Config.from_name("Llama-2-7b-hf", n_layer=2)
@@ -154,7 +154,7 @@ def test_llama7b_width_two_layers_nf4():
 
 @torch.inference_mode()
 def test_mistral7b_width_two_layers_int4_gqa():
-    """Mistral-7B shapes (d = 4096, 32 heads / 8 KV groups, I = 14336, BASELINE config 4) at depth 2, gptq.int4: the grouped-
+    """Mistral-7B shapes (d = 4096, 32 heads / 8 KV groups, I = 14336) at depth 2, gptq.int4: the grouped-
     query decode kernel, the int4 streaming GEMV at K = 14336 and the prefill GEMM, end to end against the oracle."""
     from lit_gpt_b200 import Config
     from lit_gpt_b200.config import name_to_config
@@ -176,7 +176,7 @@ def test_mistral7b_width_two_layers_int4_gqa():
 @pytest.mark.parametrize("B", [4, 16])
 @torch.inference_mode()
 def test_llama13b_width_batched_decode_int4(B):
-    """Llama-2-13B shapes (d = 5120, I = 13824, BASELINE config 3) at depth 2, gptq.int4, batch 4 and 16: every row of the
+    """Llama-2-13B shapes (d = 5120, I = 13824) at depth 2, gptq.int4, batch 4 and 16: every row of the
     batched decode step (streaming GEMV: k-windows at batch 16) against the oracle run row by row."""
     from lit_gpt_b200 import Config
     from lit_gpt_b200.config import name_to_config
@@ -215,7 +215,7 @@ def test_llama13b_width_batched_decode_int4(B):
 
 @torch.inference_mode()
 def test_long_context_rollout_bf16_rope_tables(golden):
-    """A rollout past position 256 with the reference's bf16-default RoPE tables (SURVEY F5: build_rope_cache runs under the
+    """A rollout past position 256 with the reference's bf16-default RoPE tables (build_rope_cache runs under the
     bf16 default dtype in generate/base.py, so the tables themselves are bf16): the decode attention's split / cluster paths at
     a context of ~300 and the table handling, against the oracle using the same tables."""
     g = golden("llama_mha_hs128")
@@ -262,7 +262,7 @@ def test_chat_stream_matches_generate(golden):
 
 @torch.inference_mode()
 def test_batched_decode_matches_single(golden):
-    """batch 1/4/16 at the model level (generate() is batch-1; SURVEY §8d config 3): rows are independent."""
+    """batch 1/4/16 at the model level (generate() is batch-1): rows are independent."""
     g = golden("llama_mha_hs128")
     cfgd, kw = cfg_from_golden(g)
     rc = M.RefConfig.from_any(cfgd)
@@ -407,7 +407,7 @@ def _sequential_model(kw, p, mode, devices, max_seq):
 @pytest.mark.parametrize("devices", [1, 2])
 @torch.inference_mode()
 def test_sequential_placement_matches_single_device(golden, devices):
-    """generate/sequentially.py:31-97 (SURVEY §8f-4): blocks placed over `devices` GPUs by one process give the logits and the
+    """generate/sequentially.py:31-97: blocks placed over `devices` GPUs by one process give the logits and the
     greedy tokens of the same quantized model on one GPU, bit for bit (same kernels, the residual stream hops devices)."""
     if torch.cuda.device_count() < devices:
         pytest.skip(f"needs {devices} GPUs")

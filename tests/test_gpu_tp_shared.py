@@ -33,7 +33,7 @@ def test_tp2_tag_wraparound():
 
 
 def test_tp4_per_rank_mqa_int4():
-    # the Llama-2-70B pattern (SURVEY F7c): n_query_groups == world, every rank is left with ONE kv group (MQA per rank)
+    # the Llama-2-70B pattern: n_query_groups == world, every rank is left with ONE kv group (MQA per rank)
     _run(4, "int4", 8, 4, port=29643)
 
 
@@ -45,6 +45,6 @@ def test_tp8_row_shard_not_block_aligned():
 
 @pytest.mark.parametrize("world,mode", [(2, "nf4"), (4, "int4")])
 def test_tp_lm_head_sharded(world, mode):
-    # SURVEY §8f-3 (beyond generate/tp.py:77-80): lm_head sharded by rows, the vocabulary slices all-gathered over a third
+    # beyond generate/tp.py:77-80: lm_head sharded by rows, the vocabulary slices all-gathered over a third
     # peer-memory buffer (b200_tp_gather); prefill through the all_gather hook; full logits on every rank, against the oracle
     _run(world, mode, 8, 4, port=29645 + world, shard_head=True)

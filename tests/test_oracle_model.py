@@ -79,7 +79,7 @@ def test_units(golden):
     cos, sin = M.build_rope_cache(4096, 128, pos_dtype=torch.float32)
     torch.testing.assert_close(cos[rows], torch.from_numpy(u["rope_cos_f32"]))
     torch.testing.assert_close(sin[rows], torch.from_numpy(u["rope_sin_f32"]))
-    cosb, sinb = M.build_rope_cache(4096, 128, pos_dtype=torch.bfloat16)
+    cosb, sinb = M.build_rope_cache(4096, 128, pos_dtype=torch.bfloat16) 
     torch.testing.assert_close(cosb[rows], torch.from_numpy(u["rope_cos_bf16pos"]))
     assert len(torch.unique(cosb, dim=0)) == int(u["rope_bf16pos_distinct"]) == 769
     q = torch.from_numpy(u["rope_x"])
@@ -93,7 +93,7 @@ def test_units(golden):
     assert M.sample(torch.from_numpy(u["sample_logits"]), temperature=0.0).tolist() == u["sample_t0"].tolist() == [0]
 
 
-@pytest.mark.skipif(not reference_available(), reason="/root/reference not present (GPU box)")
+@pytest.mark.skipif(not reference_available(), reason="the reference is not present")
 @torch.inference_mode()
 def test_against_live_reference_bf16(golden):
     """bf16 rounding points of the restatement equal the reference's, op by op (bit-exact on CPU)."""

@@ -1,4 +1,4 @@
-"""generate/sequentially.py (SURVEY §8f-4): the reference's own test vectors for the layer-to-device map and `replace_device`
+"""generate/sequentially.py: the reference's own test vectors for the layer-to-device map and `replace_device`
 (tests/test_generate_sequentially.py:18-83), and the one-device placement on the CPU (:86-139)."""
 import itertools
 from re import escape

@@ -58,11 +58,11 @@ def test_tensor_parallel_llama():
             assert len(hooks) == 1 and hooks[0].func.__name__ == "all_reduce_output" and hooks[0].args == (8,)
     assert model.config.n_embd * 8 == config.n_embd
     assert model.config.n_head * 8 == config.n_head
-    assert model.config.n_query_groups * 8 == config.n_query_groups == 8  # TP-8 flips 70B to MQA per rank (SURVEY F7c)
+    assert model.config.n_query_groups * 8 == config.n_query_groups == 8  # TP-8 flips 70B to MQA per rank
     blk = model.transformer.h[0]
     assert tuple(blk.attn.attn.weight.shape) == (1280, 8192) and tuple(blk.attn.proj.weight.shape) == (8192, 1024)
     assert tuple(blk.mlp.fc_1.weight.shape) == (3584, 8192) and tuple(blk.mlp.proj.weight.shape) == (8192, 3584)
-    assert tuple(model.lm_head.weight.shape) == (32000, 8192)  # lm_head and wte are replicated (SURVEY F7b)
+    assert tuple(model.lm_head.weight.shape) == (32000, 8192)  # lm_head and wte are replicated
 
 
 _WORKER = r"""

@@ -93,7 +93,7 @@ def main() -> None:
     model = fabric._precision.convert_module(model)
     model = tensor_parallel(fabric, model)
     head_sharded = os.environ.get("B200_TP_SHARD_LM_HEAD", "0") == "1"
-    if head_sharded:   # SURVEY §8f-3: lm_head sharded by rows; the oracle is unchanged (whole rows per shard: same code words)
+    if head_sharded:   # lm_head sharded by rows; the oracle is unchanged (whole rows per shard: same code words)
         model = shard_lm_head(fabric, model)
         assert model.lm_head.out_features == cfg.padded_vocab_size // world
     with fabric.init_tensor():

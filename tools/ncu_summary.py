@@ -1,8 +1,8 @@
 #!/usr/bin/env python
-"""Summarise an Nsight Compute report (`--set full`) into the few numbers DESIGN.md argues with.
+"""Summarise an Nsight Compute report (`--set full`) into a few numbers.
 
-    python tools/ncu_summary.py gpurun_out/prof.ncu-rep > profiles/rNN_<kernel>_full.md
-    python tools/ncu_summary.py --launches gpurun_out/launches.csv > profiles/rNN_launches.md
+    python tools/ncu_summary.py prof.ncu-rep > <kernel>_full.md
+    python tools/ncu_summary.py --launches launches.csv > launches.md
 """
 import collections
 import csv

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Prefill throughput of the quantized model (SURVEY §8d config 4): one `model(x, arange(T))` call through the public
+"""Prefill throughput of the quantized model: one `model(x, arange(T))` call through the public
 GPT API — tcgen05 dequant-GEMM for every Linear, b200_rope_kv_append + b200_attn_prefill for the attention.
 
     python tools/prefill_bench.py [--model Mistral-7B-v0.1] [--qt int4] [--tokens 4096] [--reps 5]
