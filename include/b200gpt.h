@@ -592,9 +592,12 @@ int64_t b200_delta_rule_state_floats(int dk, int dv);
 int b200_delta_rule(const b200_delta_rule_args* args, b200_stream_t stream);
 /* The same for prompts with keys of at most 128 numbers, 32 tokens at a time with matrix products instead of one by one (csrc/delta_chunk.cu).
  * What is computed depends on `rows` alone (0: n_seqs sequences of max_rows each); more rows than that raise the error word.
- * b200_delta_rule_workspace_bytes: scratch that lets every launch cover as much as pays for n_seqs sequences of at most max_rows rows, 0 when
- * the call is better served by b200_delta_rule; for `rows` rows in all, ask for one sequence of rows + 31 (n_seqs - 1).  A smaller workspace
- * (at least one chunk) works in more launches. */
+ * Sequences of fewer than 64 rows beside longer ones still go one by one, in a launch of their own.
+ * b200_delta_rule_in_chunks: 1 where this is the shorter way for `rows` rows of n_seqs sequences, the longest of max_rows.
+ * b200_delta_rule_workspace_bytes: scratch that lets every launch cover as much as pays for n_seqs sequences of at most max_rows rows, 0 below 64
+ * rows; for `rows` rows in all, ask for one sequence of rows + 31 (k - 1), k = min(n_seqs, rows / 64).  A smaller workspace (at least one chunk)
+ * works in more launches. */
+int b200_delta_rule_in_chunks(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv, int channel_decay);
 size_t b200_delta_rule_workspace_bytes(int max_rows, int n_seqs, int heads, int dk, int dv);
 int b200_delta_rule_chunked(const b200_delta_rule_args* args, void* workspace, size_t workspace_bytes, b200_stream_t stream);
 /* out[row, h, :] = dtype(o / sqrt(mean(o^2) + eps) * weight * gate(z) * out_scale) per head; gate 1 silu, 2 sigmoid; weight NULL: none */

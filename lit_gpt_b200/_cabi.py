@@ -208,6 +208,7 @@ _CORE_SIGNATURES = {
     "b200_delta_rule_state_floats": (c_int64, [c_int, c_int]),
     "b200_delta_rule": (c_int, [ctypes.POINTER(DeltaRuleArgs), c_void_p]),
     "b200_delta_rule_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "b200_delta_rule_in_chunks": (c_int, [c_int64, c_int, c_int, c_int, c_int, c_int, c_int]),
     "b200_delta_rule_chunked": (c_int, [ctypes.POINTER(DeltaRuleArgs), c_void_p, c_size_t, c_void_p]),
     "b200_gated_rms_heads": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_float, c_float,
                                      c_int, c_void_p]),

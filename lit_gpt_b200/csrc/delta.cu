@@ -46,8 +46,9 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : lo
 
 // LPC lanes share one column of S, each holding KPL of its numbers (key i = r * LPC + lane); L is the group size of the stored
 // layout, which does not depend on how the kernel spreads a column over lanes.
-template <typename T, int LPC, int KPL, bool CHANNEL>
-__global__ void __launch_bounds__(kDrThreads) delta_rule_kernel(DrArgs A, int L) {
+// SHORT: sequences of `below` rows and more are somebody else's.
+template <typename T, int LPC, int KPL, bool CHANNEL, bool SHORT>
+__global__ void __launch_bounds__(kDrThreads) delta_rule_kernel(DrArgs A, int L, int below) {
   constexpr int kDrKPL = KPL;
   constexpr int DKP = KPL * LPC;               // padded key size
   constexpr int TT = kDrTile / DKP;            // tokens per staged tile
@@ -66,6 +67,9 @@ __global__ void __launch_bounds__(kDrThreads) delta_rule_kernel(DrArgs A, int L)
   const int h = blockIdx.y, hk = h / (A.heads / A.kv_heads);
   const int4 sq = A.seqs[blockIdx.z];
   const int first = sq.x, len = sq.y, pos0 = sq.z, slot = sq.w;
+  if constexpr (SHORT) {
+    if (len >= below) return;                  // those go in chunks (delta_chunk.cu)
+  }
   const int col = (int)blockIdx.x * COLS + cl;
   const bool col_ok = col < A.dv;
   const int dk = A.dk, dv = A.dv;
@@ -203,16 +207,16 @@ __global__ void __launch_bounds__(kDrThreads) delta_rule_kernel(DrArgs A, int L)
 }
 
 template <typename T, int LPC, int KPL>
-cudaError_t delta_launch(const DrArgs& A, bool channel, int n_seqs, cudaStream_t st) {
+cudaError_t delta_launch(const DrArgs& A, bool channel, int n_seqs, int below, cudaStream_t st) {
   constexpr int DKP = KPL * LPC, TT = kDrTile / DKP, COLS = kDrThreads / LPC;
   const dim3 grid((unsigned)((A.dv + COLS - 1) / COLS), (unsigned)A.heads, (unsigned)n_seqs);
   const int L = delta_lpc(A.dk);
-  if (channel) {
-    const size_t smem = (size_t)(3 * TT * DKP + TT * COLS + TT) * sizeof(float);
-    return launch(delta_rule_kernel<T, LPC, KPL, true>, grid, dim3(kDrThreads), smem, st, A, L);
+  const size_t smem = (size_t)((channel ? 3 * TT * DKP : 2 * TT * DKP + TT) + TT * COLS + TT) * sizeof(float);
+  auto go = [&](auto kernel) { return launch(kernel, grid, dim3(kDrThreads), smem, st, A, L, below); };
+  if constexpr (DKP <= 128) {   // (chunks take keys of at most 128 numbers)
+    if (below > 0) return channel ? go(delta_rule_kernel<T, LPC, KPL, true, true>) : go(delta_rule_kernel<T, LPC, KPL, false, true>);
   }
-  const size_t smem = (size_t)(2 * TT * DKP + TT + TT * COLS + TT) * sizeof(float);
-  return launch(delta_rule_kernel<T, LPC, KPL, false>, grid, dim3(kDrThreads), smem, st, A, L);
+  return channel ? go(delta_rule_kernel<T, LPC, KPL, true, false>) : go(delta_rule_kernel<T, LPC, KPL, false, false>);
 }
 
 // out[row, h, :] = T( o / sqrt(mean(o^2) + eps) * weight * gate(z[row, h, :]) ); one warp per (row, head)
@@ -276,6 +280,35 @@ __global__ void __launch_bounds__(128) gated_rms_wide_kernel(const float* __rest
 
 }  // namespace
 
+// Sequences of fewer than `below` rows (0: all), token by token (arguments checked by the callers)
+int delta_rule_walk(const b200_delta_rule_args* a, int below, b200_stream_t stream) {
+  const DrArgs A{a->q, a->k, a->v, a->ldq, a->ldk, a->ldv, a->beta_in, a->ld_beta, a->decay_in, a->ld_decay, a->a_log, a->dt_bias,
+                 a->state, a->state_slot_stride, a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv};
+  const bool ch = a->channel_decay != 0;
+  cudaStream_t st = (cudaStream_t)stream;
+  // Two ways to spread a column over lanes.  Few lanes with 16 numbers each: three reduction rounds per token and whole
+  // 128-byte lines of state per warp -- best for single tokens and for the per-head decay.  A prompt with per-channel decays
+  // carries a third staged array and the softplus / exponential of every decay: there a column on 16 or 32 lanes with 4 or 8
+  // numbers each (four times the warps) measured faster (0.66 against 0.85 us per token at 8 heads of 128 x 128).
+  // (that is with 64 to 128 CTAs of the narrow split; once those alone fill the GPU, more warps only add reduction rounds)
+  const int64_t narrow_ctas = (int64_t)((a->dv + kDrThreads / delta_lpc(a->dk) - 1) / (kDrThreads / delta_lpc(a->dk))) * a->heads * a->n_seqs;
+  const bool wide = ch && a->max_rows > 1 && a->dk > 32 && a->dk <= 256 && narrow_ctas < (int64_t)sm_count() * 3 / 2;
+  B200_FLOAT_TYPES(a->dtype, T, {
+    if (wide) {
+      if (a->dk <= 64) B200_CUDA((delta_launch<T, 16, 4>(A, ch, a->n_seqs, below, st)));
+      else if (a->dk <= 128) B200_CUDA((delta_launch<T, 32, 4>(A, ch, a->n_seqs, below, st)));
+      else B200_CUDA((delta_launch<T, 32, 8>(A, ch, a->n_seqs, below, st)));
+    } else {
+      const int lpc = delta_lpc(a->dk);
+      if (lpc == 4) B200_CUDA((delta_launch<T, 4, 16>(A, ch, a->n_seqs, below, st)));
+      else if (lpc == 8) B200_CUDA((delta_launch<T, 8, 16>(A, ch, a->n_seqs, below, st)));
+      else if (lpc == 16) B200_CUDA((delta_launch<T, 16, 16>(A, ch, a->n_seqs, below, st)));
+      else B200_CUDA((delta_launch<T, 32, 16>(A, ch, a->n_seqs, below, st)));
+    }
+  });
+  return B200_OK;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -291,31 +324,7 @@ int b200_delta_rule(const b200_delta_rule_args* a, b200_stream_t stream) {
                  "b200_delta_rule: bad head counts");
   B200_CHECK_ARG(a->dk > 0 && a->dk <= 512 && a->dv > 0, "b200_delta_rule: key size must be 1 .. 512");
   B200_CHECK_ARG((reinterpret_cast<uintptr_t>(a->seqs) & 15) == 0, "b200_delta_rule: seqs must be 16-byte aligned");
-  const DrArgs A{a->q, a->k, a->v, a->ldq, a->ldk, a->ldv, a->beta_in, a->ld_beta, a->decay_in, a->ld_decay, a->a_log, a->dt_bias,
-                 a->state, a->state_slot_stride, a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv};
-  const bool ch = a->channel_decay != 0;
-  cudaStream_t st = (cudaStream_t)stream;
-  // Two ways to spread a column over lanes.  Few lanes with 16 numbers each: three reduction rounds per token and whole
-  // 128-byte lines of state per warp -- best for single tokens and for the per-head decay.  A prompt with per-channel decays
-  // carries a third staged array and the softplus / exponential of every decay: there a column on 16 or 32 lanes with 4 or 8
-  // numbers each (four times the warps) measured faster (0.66 against 0.85 us per token at 8 heads of 128 x 128).
-  // (that is with 64 to 128 CTAs of the narrow split; once those alone fill the GPU, more warps only add reduction rounds)
-  const int64_t narrow_ctas = (int64_t)((a->dv + kDrThreads / delta_lpc(a->dk) - 1) / (kDrThreads / delta_lpc(a->dk))) * a->heads * a->n_seqs;
-  const bool wide = ch && a->max_rows > 1 && a->dk > 32 && a->dk <= 256 && narrow_ctas < (int64_t)sm_count() * 3 / 2;
-  B200_FLOAT_TYPES(a->dtype, T, {
-    if (wide) {
-      if (a->dk <= 64) B200_CUDA((delta_launch<T, 16, 4>(A, ch, a->n_seqs, st)));
-      else if (a->dk <= 128) B200_CUDA((delta_launch<T, 32, 4>(A, ch, a->n_seqs, st)));
-      else B200_CUDA((delta_launch<T, 32, 8>(A, ch, a->n_seqs, st)));
-    } else {
-      const int lpc = delta_lpc(a->dk);
-      if (lpc == 4) B200_CUDA((delta_launch<T, 4, 16>(A, ch, a->n_seqs, st)));
-      else if (lpc == 8) B200_CUDA((delta_launch<T, 8, 16>(A, ch, a->n_seqs, st)));
-      else if (lpc == 16) B200_CUDA((delta_launch<T, 16, 16>(A, ch, a->n_seqs, st)));
-      else B200_CUDA((delta_launch<T, 32, 16>(A, ch, a->n_seqs, st)));
-    }
-  });
-  return B200_OK;
+  return delta_rule_walk(a, 0, stream);
 }
 
 int b200_gated_rms_heads(const float* o, int64_t ldo, const void* z, int64_t ldz, const void* weight, void* out, int64_t ld_out, int64_t rows,

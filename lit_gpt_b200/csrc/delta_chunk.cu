@@ -22,6 +22,7 @@ namespace {
 
 constexpr int kDcC = 32;            // tokens per chunk
 constexpr int kDcThreads = 128;
+constexpr int kDcMinRows = 64;
 
 struct DcArgs {
   const float* q; const float* k; const float* v;
@@ -33,7 +34,7 @@ struct DcArgs {
   float* out; int64_t ldo;
   const int4* seqs;
   int heads, kv_heads, dk, dv;
-  int n_seqs;
+  int n_seqs, longs;                // sequences, and how many of them can have chunks
   int item0, n_items, most;         // this launch's chunks, counted through all sequences, of `most` in all
   int dvb;                          // blocks of eight value columns (an even number)
   float* ws; int64_t item;          // per (chunk, head): W | K | Q, rows of DK + 4 | P (DK) | U [dvb][32][8] | O [dvb][32][8]
@@ -54,8 +55,9 @@ __device__ __forceinline__ float sum2(f2 v) { float a, b; un2(v, a, b); return a
 
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
-// Chunks are counted through the sequences in their order, each with as many as its rows take.  Both functions are called by whole warps.
-__device__ __forceinline__ int dc_chunks(const int4& sq) { return sq.y > 0 ? (sq.y + kDcC - 1) / kDcC : 0; }
+// Chunks are counted through the sequences in their order, each with as many as its rows take; sequences of fewer than kDcMinRows have none and go
+// token by token.  The functions below are called by whole warps.
+__device__ __forceinline__ int dc_chunks(const int4& sq) { return sq.y >= kDcMinRows ? (sq.y + kDcC - 1) / kDcC : 0; }
 // the sequence of chunk `at` and the chunk's number there; -1: there are not that many
 __device__ __forceinline__ int dc_find(const DcArgs& A, int at, int& chunk) {
   const int lane = threadIdx.x & 31;
@@ -78,11 +80,22 @@ __device__ __forceinline__ int dc_find(const DcArgs& A, int at, int& chunk) {
   }
   return -1;
 }
-// how many chunks lie before sequence z
-__device__ __forceinline__ int dc_before(const DcArgs& A, int z) {
-  int n = 0;
-  for (int s = threadIdx.x & 31; s < z; s += 32) n += dc_chunks(A.seqs[s]);
-  return __reduce_add_sync(0xffffffffu, n);
+// the z-th of the sequences that have chunks, and how many chunks lie before its own; -1: there are not that many
+__device__ __forceinline__ int dc_nth(const DcArgs& A, int z, int& before) {
+  const int lane = threadIdx.x & 31;
+  before = 0;
+  for (int s0 = 0; s0 < A.n_seqs; s0 += 32) {
+    const int n = s0 + lane < A.n_seqs ? dc_chunks(A.seqs[s0 + lane]) : 0;
+    const unsigned have = __ballot_sync(0xffffffffu, n > 0);
+    if (z < __popc(have)) {
+      const int w = (int)__fns(have, 0, z + 1);
+      before += __reduce_add_sync(0xffffffffu, lane < w ? n : 0);
+      return s0 + w;
+    }
+    z -= __popc(have);
+    before += __reduce_add_sync(0xffffffffu, n);
+  }
+  return -1;
 }
 
 // One chunk of one head: grid (chunks, heads).  Tokens past the sequence's end count as k = q = v = 0, beta = 0, g = 1.
@@ -277,7 +290,7 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_kernel(DcArgs A, in
   }
 }
 
-// The state through the chunks, in order: grid (slices of NC value columns, heads, sequences), 16 NC threads.  Chunk c + 1 is on its way into
+// The state through the chunks, in order: grid (slices of NC value columns, heads, sequences that can have chunks), 16 NC threads.  Chunk c + 1 is on its way into
 // the second stage (bulk copies) while chunk c is worked on; the slice of S lies in shared memory by column, so that four keys' numbers are
 // one access for either factor of W S and Q S.
 template <int DK, int NC>
@@ -309,11 +322,14 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
   }
   griddep_launch();
   griddep_wait();
-  const int4 sq = A.seqs[blockIdx.z];
-  const int before = dc_before(A, blockIdx.z), all = dc_chunks(sq);
+  int before;
+  const int z = dc_nth(A, blockIdx.z, before);
+  if (z < 0) return;
+  const int4 sq = A.seqs[z];
+  const int all = dc_chunks(sq);
   const int c_first = max(0, A.item0 - before), chunks = min(all, A.item0 + A.n_items - before) - c_first, t_first = c_first * C;
   if (tid == 0 && before + all > A.most) *A.err = 1u;   // more rows than the caller said
-  if (chunks <= 0 && (all > 0 || A.item0 > 0)) return;   // (a sequence without rows still starts its slot from zero)
+  if (chunks <= 0) return;
   const int dk = A.dk, dv = A.dv;
   const float* const items = A.ws + ((int64_t)(before + c_first - A.item0) * A.heads + h) * A.item;
   const int64_t step = (int64_t)A.heads * A.item;
@@ -330,7 +346,7 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
     copy(dst + (I::kHead + Y::kSlice) * 4, src + I::kHead + (int64_t)(A.dvb + (col0 >> 3)) * C * 8, Y::kSlice * 4);
   };
   if (tid == 0) {
-    if (chunks > 0) fetch(0);
+    fetch(0);
     if (chunks > 1) fetch(1);
   }
   const int krows = (dk + L - 1) / L;
@@ -448,7 +464,7 @@ cudaError_t carry_launch(const DcArgs& A, int L, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     once.done();
   }
-  return launch(delta_carry_kernel<DK, NC>, dim3((unsigned)((A.dv + NC - 1) / NC), (unsigned)A.heads, (unsigned)A.n_seqs), dim3(Y::kThreads), Y::kSmem, st, A, L);
+  return launch(delta_carry_kernel<DK, NC>, dim3((unsigned)((A.dv + NC - 1) / NC), (unsigned)A.heads, (unsigned)A.longs), dim3(Y::kThreads), Y::kSmem, st, A, L);
 }
 
 template <typename T, int DK>
@@ -456,7 +472,7 @@ cudaError_t segment_launch(const DcArgs& A, bool channel, int vec, int L, cudaSt
   const cudaError_t e = channel ? chunk_launch<T, DK, true>(A, vec, st) : chunk_launch<T, DK, false>(A, vec, st);
   if (e != cudaSuccess) return e;
   // 16 columns per slice share the reads of W, Q and K best; with fewer slices than SMs, slices of 8 have the shorter chain
-  const int64_t wide = (int64_t)((A.dv + 15) / 16) * A.heads * A.n_seqs;
+  const int64_t wide = (int64_t)((A.dv + 15) / 16) * A.heads * A.longs;
   return wide * 4 >= (int64_t)sm_count() * 3 ? carry_launch<DK, 16>(A, L, st) : carry_launch<DK, 8>(A, L, st);
 }
 
@@ -464,15 +480,44 @@ int dc_dvb(int dv) { return (dv + 15) / 16 * 2; }
 int64_t dc_item(int dk, int dv) { return (dk <= 64 ? (int64_t)DcItem<64>::kHead : (int64_t)DcItem<128>::kHead) + 2 * (int64_t)dc_dvb(dv) * kDcC * 8; }
 
 constexpr int64_t kDcMaxBytes = 256ll << 20;   // scratch of one launch's chunks
-constexpr int kDcMinRows = 64;
 
 }  // namespace
+
+int delta_rule_walk(const b200_delta_rule_args* a, int below, b200_stream_t stream);   // delta.cu
 
 }  // namespace b200
 
 using namespace b200;
 
 extern "C" {
+
+int b200_delta_rule_in_chunks(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv, int channel_decay) {
+  if (max_rows < kDcMinRows || rows < max_rows || n_seqs <= 0 || heads <= 0 || dk <= 0 || dk > 128 || dv <= 0) return 0;
+  // us of either way, fitted to launches of 4 to 256 heads (times sequences of the longest one's length) of 128 x 128: a walk's token takes what its
+  // chain of reductions takes until the heads fill the GPU, a chunk's as long as the carry's chain, and both the same work beyond; the short sequences'
+  // walk comes on top of the chunks and runs half beside the long one's.  Measured, walk / chunks, 16 heads, 64, 128, 512 rows alone: decays per channel
+  // 54 / 43, 104 / 49, 404 / 82; per head 28 / 31, 50 / 35, 181 / 69.  Beside 32 single rows: 76 / 104, 91 / 109, 316 / 159; 56 / 75, 66 / 80, 217 / 118.
+  // 16 sequences of 64, of 256 rows: 207 / 245, 822 / 682; 145 / 202, 528 / 539.
+  const double n = max_rows, same = (double)rows / max_rows < n_seqs ? (double)rows / max_rows : n_seqs, one = heads * (dk * (double)dv / 16384.0), load = one * same;
+  const int64_t shorts = n_seqs - (rows + max_rows - 1) / max_rows;
+  auto most = [](double a, double b) { return a > b ? a : b; };
+  double walk, chunks, few;
+  if (channel_decay) {
+    const bool wide = (int64_t)heads * n_seqs * ((dv + 15) / 16) < sm_count() * 3 / 2;   // (delta_rule_walk's choice)
+    walk = 5.0 + n * most(0.35, wide ? 0.17 + 0.038 * load : most(0.36 + 0.01 * load, 0.0126 * load));
+    chunks = 28.0 + (n + 24.0) * most(0.1, 0.0114 * load);
+    few = 0.13 * one;
+  } else {
+    walk = 5.0 + n * most(most(0.35, 0.25 + 0.0062 * load), 0.0088 * load);
+    chunks = 20.0 + (n + 24.0) * most(0.085, 0.009 * load);
+    few = 0.09 * one;
+  }
+  if (shorts > 0) {
+    walk += 0.5 * few * shorts;
+    chunks += few * shorts;
+  }
+  return chunks < walk;
+}
 
 size_t b200_delta_rule_workspace_bytes(int max_rows, int n_seqs, int heads, int dk, int dv) {
   if (max_rows < kDcMinRows || n_seqs <= 0 || heads <= 0 || dk <= 0 || dk > 128 || dv <= 0) return 0;
@@ -495,12 +540,22 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
   const int64_t item = dc_item(a->dk, a->dv);
   int64_t fit = (int64_t)(workspace_bytes / (size_t)(item * 4)) / a->heads;   // chunks
   B200_CHECK_ARG(fit > 0, "b200_delta_rule_chunked: workspace too small (%zu bytes)", workspace_bytes);
-  // n sequences of `rows` rows in all have at most (rows + 31 n) / 32 chunks
-  const int64_t most = a->rows > 0 ? (a->rows + (int64_t)(kDcC - 1) * a->n_seqs) / kDcC : (int64_t)a->n_seqs * ((a->max_rows + kDcC - 1) / kDcC);
+  // n sequences of `rows` rows in all have at most (rows + 31 n) / 32 chunks, and n of them kDcMinRows rows each at least
+  const int64_t longs = a->rows > 0 && a->rows / kDcMinRows < a->n_seqs ? a->rows / kDcMinRows : a->n_seqs;
+  const int64_t most = a->rows > 0 ? (longs > 0 ? (a->rows + (kDcC - 1) * longs) / kDcC : 0) : longs * ((a->max_rows + kDcC - 1) / kDcC);
   B200_CHECK_ARG(most <= 0x3fffffff, "b200_delta_rule_chunked: too many rows");
   if (fit > most) fit = most;
+  // In a step of several sequences the short ones -- single rows beside a prompt -- keep the walk: a row alone would cost a whole chunk and a link of
+  // the carry.  One prompt of 1024 rows beside 32 single rows, 16 heads of 128 x 128 with decays per channel: 250 us; 494 with chunks for all, 679 with
+  // the walk for all.
+  if (a->n_seqs > 1 || most == 0) {
+    b200_delta_rule_args few = *a;
+    if (few.max_rows >= kDcMinRows) few.max_rows = kDcMinRows - 1;
+    const int rc = delta_rule_walk(&few, kDcMinRows, stream);
+    if (rc != B200_OK || most == 0) return rc;
+  }
   DcArgs A{a->q, a->k, a->v, a->ldq, a->ldk, a->ldv, a->beta_in, a->ld_beta, a->decay_in, a->ld_decay, a->a_log, a->dt_bias, a->state, a->state_slot_stride,
-           a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv, a->n_seqs, 0, (int)fit, (int)most, dc_dvb(a->dv),
+           a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv, a->n_seqs, (int)longs, 0, (int)fit, (int)most, dc_dvb(a->dv),
            reinterpret_cast<float*>(workspace), item, wait_error_word()};
   B200_CHECK_ARG(A.err, "b200_delta_rule_chunked: no error word");
   auto al = [](const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };

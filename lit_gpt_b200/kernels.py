@@ -1064,7 +1064,7 @@ def delta_rule_state_floats(dk: int, dv: int) -> int:
     return int(C.load_core().b200_delta_rule_state_floats(dk, dv))
 
 
-DELTA_CHUNKED = True   # tests switch it off to run prompts token by token
+DELTA_CHUNKED: Optional[bool] = None   # None: where that is the shorter way; tests set True (wherever it runs) or False (token by token)
 
 
 def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_in: torch.Tensor, decay_in: torch.Tensor, a_log: torch.Tensor,
@@ -1091,12 +1091,16 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_in: torch
                            dk=dk, dv=dv, channel_decay=int(channel_decay), dtype=_code(beta_in), max_rows=int(max_rows), rows=q.shape[0])
     lib, n_seqs = C.load_core(), seqs.shape[0]
     # a prompt goes 32 tokens at a time; max_rows says whether that pays, the rows there are how much scratch it takes
-    need = lib.b200_delta_rule_workspace_bytes(int(max_rows), n_seqs, heads, dk, dv) if DELTA_CHUNKED else 0
-    ws = None
-    if need:
-        need = min(need, lib.b200_delta_rule_workspace_bytes(q.shape[0] + 31 * (n_seqs - 1), 1, heads, dk, dv) or need)
+    n, ws = q.shape[0], None
+    chunks = DELTA_CHUNKED
+    if chunks is None:
+        chunks = lib.b200_delta_rule_in_chunks(n, int(max_rows), n_seqs, heads, dk, dv, int(channel_decay)) != 0
+    elif chunks:
+        chunks = lib.b200_delta_rule_workspace_bytes(int(max_rows), n_seqs, heads, dk, dv) != 0
+    if chunks:
+        need = lib.b200_delta_rule_workspace_bytes(max(64, n + 31 * (min(n_seqs, n // 64) - 1)), 1, heads, dk, dv)
         try:
-            ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+            ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
         except torch.OutOfMemoryError:   # token by token, which needs none
             pass
     if ws is not None:

@@ -121,8 +121,9 @@ def test_delta_chunks_in_segments(K, chunks):
 
 
 @pytest.mark.parametrize("lens,hint", [((200, 10), 110), ((100, 1, 1), 64), ((70, 300, 5), 64), ((33, 0, 100, 64), 65)])
-def test_delta_chunks_compute_every_row_whatever_the_hint(K, lens, hint):
+def test_delta_chunks_compute_every_row_whatever_the_hint(K, monkeypatch, lens, hint):
     """max_rows picks the kernel; rows past it are computed all the same, and a sequence without rows starts its slot from zero as before."""
+    monkeypatch.setattr(K, "DELTA_CHUNKED", True)
     H, G, dk, dv = 4, 2, 64, 40
     starts = [7 * (i % 2) for i in range(len(lens))]
     data = _inputs(lens, starts, H, G, dk, dv, True, torch.float32, 11, 0)
@@ -157,11 +158,27 @@ def test_delta_chunk_scratch_follows_the_rows(K, monkeypatch):
         monkeypatch.undo()
         return y, state
 
-    (a, sa), (b, sb) = run(1 << 40), run(0)
+    monkeypatch.setattr(K, "DELTA_CHUNKED", True)
+    a, sa = run(1 << 40)
+    monkeypatch.setattr(K, "DELTA_CHUNKED", True)
+    b, sb = run(0)
     from lit_gpt_b200 import _cabi as C
     chunk = C.load().b200_delta_rule_workspace_bytes(64, 1, H, dk, dv) // 2
-    assert asked[0] == (sum(lens) + 31 * len(lens)) // 32 * chunk
+    assert asked[0] == (sum(lens) + 31 * 2) // 32 * chunk   # two sequences of 64 rows at most, whatever their number
     assert (a - b).abs().max() <= 1e-4 * b.abs().max() and (sa - sb).abs().max() <= 1e-4 * sb.abs().max()
+
+
+def test_delta_chunks_or_tokens(K):
+    """What a step's rows decide: a prompt alone or beside single rows, many long sequences that fill the GPU token by token, short prompts, wide keys."""
+    from lit_gpt_b200 import _cabi as C
+
+    pays = C.load().b200_delta_rule_in_chunks
+    for channel in (0, 1):
+        for heads in (4, 16, 32):
+            assert pays(512, 512, 1, heads, 128, 128, channel) and pays(1024 + 32, 1024, 33, heads, 128, 128, channel)
+            assert not pays(63, 63, 1, heads, 128, 128, channel) and not pays(4096, 4096, 1, heads, 129, 128, channel)
+        assert not pays(64 + 32, 64, 33, 16, 128, 128, channel) and not pays(64 * 64, 64, 64, 16, 128, 128, channel)
+    assert pays(64, 64, 1, 16, 128, 128, 1) and not pays(64, 64, 1, 16, 128, 128, 0) and not pays(10, 100, 1, 16, 128, 128, 1)
 
 
 def test_delta_chunk_rule(K):
