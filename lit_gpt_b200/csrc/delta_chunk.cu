@@ -471,9 +471,9 @@ template <typename T, int DK>
 cudaError_t segment_launch(const DcArgs& A, bool channel, int vec, int L, cudaStream_t st) {
   const cudaError_t e = channel ? chunk_launch<T, DK, true>(A, vec, st) : chunk_launch<T, DK, false>(A, vec, st);
   if (e != cudaSuccess) return e;
-  // 16 columns per slice share the reads of W, Q and K best; with fewer slices than SMs, slices of 8 have the shorter chain
-  const int64_t wide = (int64_t)((A.dv + 15) / 16) * A.heads * A.longs;
-  return wide * 4 >= (int64_t)sm_count() * 3 ? carry_launch<DK, 16>(A, L, st) : carry_launch<DK, 8>(A, L, st);
+  // Slices of 8 columns: the shorter chain.  Slices of 16, which read W, Q and K half as often, are 2 - 60 % slower at every number of heads (512
+  // rows, decays per channel, us with 8 and 16: 4 heads of 128 x 128 67 and 82, 16 heads 83 and 86, 32 heads 181 and 191; 16 heads of 64 x 128 62 and 94).
+  return carry_launch<DK, 8>(A, L, st);
 }
 
 int dc_dvb(int dv) { return (dv + 15) / 16 * 2; }
