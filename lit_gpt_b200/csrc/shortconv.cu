@@ -309,9 +309,12 @@ int b200_short_conv(const void* in, int64_t ld_in, const b200_conv_group* groups
   }
   const int per = kCvThreads / 32;
   B200_CHECK_ARG((P.total_heads + per - 1) / per <= 65535, "b200_short_conv: too many heads");
-  // Rows per warp: enough of them to spare the re-reads once the warps outnumber what the SMs hold at a time (about 32 each), else one
-  const int64_t warps = rows * P.total_heads;
-  const int rpw = warps >= (int64_t)sm_count() * 32 * 8 ? 8 : (warps >= (int64_t)sm_count() * 32 * 4 ? 4 : 1);
+  // Rows per warp, by (row, head) pairs per SM: more rows spare re-reads and set-up, fewer fill the SMs.  us with 1, 4 and 8 rows a warp, 40 heads of
+  // 128 rotated and normed / 48 heads of 128 with silu and unit norm / 12 heads of 64, four taps: 128 rows (35, 42, 10 pairs per SM) 11.4, 12.4, 18.0 /
+  // 11.2, 11.1, 16.3 / 6.4, 9.1, 12.4; 300 rows (81, 97, 24) 18.4, 13.5, 19.0 / 20.2, 17.1, 16.9 / 6.3, 8.9, 12.4; 1024 rows (277, 332, 83)
+  // 47, 30, 34 / 53, 34, 31 / 10.9, 9.7, 13.0; 4096 rows (1107, 1328, 332) 194, 117, 104 / 236, 150, 137 / 27, 20, 19.
+  const int64_t per_sm = rows * P.total_heads / sm_count();
+  const int rpw = per_sm >= 320 ? 8 : (per_sm >= 64 ? 4 : 1);
   const dim3 grid((unsigned)((rows + rpw - 1) / rpw), (unsigned)((P.total_heads + per - 1) / per));
   // pairs of neighbouring channels are read with one access when every head starts on an even channel of even-pitched, aligned rows
   const size_t esz = dtype == B200_F32 ? 4 : 2;

@@ -792,7 +792,7 @@ def test_short_conv_row_groups(dtype, taps, dim, heads, rows):
 
     tail = tail0.clone()
     whole = run(inp, tail, seqs)
-    part = 18944 // heads // 2   # half the fewest rows that are grouped: a long sequence alone runs in parts, its tail carried
+    part = 18944 // heads // 2   # fewer rows than are grouped: a long sequence alone runs in parts, its tail carried
     for first, n, start, slot in seqs:
         t1, got = tail0[slot : slot + 1].clone(), []
         for o in range(0, n, part):
