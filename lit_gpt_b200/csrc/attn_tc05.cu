@@ -1,6 +1,7 @@
 // Causal attention of a prompt's rows over a key-value cache or packed rows, head sizes 64 and 128, on the 5th-generation tensor cores.
 //
 // One CTA = 256 query rows of one head as two tiles of 128, key tiles of 128, one tile's softmax beside the other's products:
+//   (small launches: 128 rows per CTA, the second tile empty)
 //   * warps 0-3 and 4-7: the softmax of query tile 0 and 1, one row per thread.  S (128 columns of tensor memory) is read into registers, the
 //     probabilities go back over it as bf16, the left operand of P V, in two halves so that P V starts on the first.  Half of S is
 //     kept in registers from the maximum to the exponentials, the other half read again: 128 registers a thread are all that 16 warps have;
@@ -9,8 +10,10 @@
 //     16 each, S of a tile's next step right behind its P V;
 //   * warp 13 brings the keys, warp 14 the values, two stages each, 128-byte-swizzled: whole tiles by TMA, a tile that ends past the last visible
 //     key row by row with cp.async, zeros behind it -- what lies there may be anything, or not be memory at all.  The softmax warps bring Q.
+// A masked key has weight 0, and 0 times an infinite or NaN value is NaN: a value that is not finite reaches the rows before its own, within its
+// tile of 128 keys and 128 query rows.
 // Softmax in fp32 with the exact running maximum, so that the largest probability is 1 and loses nothing to its rounding; probabilities are
-// summed as rounded.  (Moving the maximum only when it grew by 2^8 saves a tenth of the time and raises the error against 64 bits by half.)
+// summed as rounded, as they multiply V (the sum of the unrounded ones makes the error against 64 bits 0.1 to 0.4 % larger).  (Moving the maximum only when it grew by 2^8 saves a tenth of the time and raises the error against 64 bits by half.)
 //
 // Bound: the chain of one tile -- 128 exponentials a row on the special-function units (16 a clock and SM), then its two products, 1270 clocks
 // where shared memory feeds them -- of which the other tile's fills the gaps.  32 heads of 128 over 8 key-value heads, 4096 rows: 230 us, 598
@@ -95,7 +98,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   __shared__ int s_max[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int h = blockIdx.y, b = blockIdx.z, grp = h / (A.n_head / A.n_groups);
-  const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * kAtBM;   // late rows, which see most keys, are scheduled first
+  const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * A.span;   // late rows, which see most keys, are scheduled first
   const uint32_t smem = (tc::smem_u32(at_smem) + 1023u) & ~1023u;
   const uint32_t sq_ = smem, sk_ = smem + 2 * C::kBytes, sv_ = smem + 4 * C::kBytes;
   const uint32_t bars = tc::smem_u32(s_bars);
@@ -136,7 +139,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   int lim = -1;
   if (warp < 8) {
     const int r = r0 + tid;
-    if (r < T) {
+    if (r < T && tid < A.span) {
       const int64_t p = A.seqs ? (int64_t)pos0 + r : (A.pos64 ? reinterpret_cast<const int64_t*>(A.pos)[r] : (int64_t)reinterpret_cast<const int32_t*>(A.pos)[r]);
       lim = (int)(p < 0 ? 0 : (p >= max_seq ? max_seq - 1 : p));
     }
@@ -287,7 +290,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   } else {
     // ================================ softmax: a row per thread ================================
     const int t = warp >> 2, r = r0 + tid;
-    copy_tile<HS, 128>(sq_ + t * C::kBytes, A.q + (int64_t)b * A.q_b + (int64_t)h * A.q_h + qrow0 * A.q_r, A.q_r, r0 + t * kAtBM, T, tid & 127);
+    copy_tile<HS, 128>(sq_ + t * C::kBytes, A.q + (int64_t)b * A.q_b + (int64_t)h * A.q_h + qrow0 * A.q_r, A.q_r, r0 + t * kAtBM, min(T, r0 + A.span), tid & 127);
     asm volatile("cp.async.wait_all;" ::: "memory");
     tc::fence_smem_async();
     __syncwarp();
@@ -426,7 +429,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
 }
 
 template <int HS>
-cudaError_t launch_hs(const AttnTc05Args& a, int batch, cudaStream_t st) {
+cudaError_t launch_hs(AttnTc05Args a, int batch, cudaStream_t st) {
   constexpr int smem = AtTile<HS>::kSmem;
   static PerDeviceOnce once;
   if (once.need()) {
@@ -440,7 +443,12 @@ cudaError_t launch_hs(const AttnTc05Args& a, int batch, cudaStream_t st) {
   if (!tensor_map_2d(&mk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.k, rows, cols, a.k_r * 2, 128) ||
       !tensor_map_2d(&mv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.v, rows, cols, a.v_r * 2, 128))
     return cudaErrorInvalidValue;
-  const dim3 grid((unsigned)((a.T + 2 * kAtBM - 1) / (2 * kAtBM)), (unsigned)a.n_head, (unsigned)batch);
+  // One tile of rows per CTA while twice the CTAs are no more than the SMs: two tiles take turns on one SM's special-function units, and the second
+  // one's longer key range would be all that is left of the launch.  32 heads of 128, 160 / 256 / 400 rows from position 0, us with two tiles and with
+  // one: 12.6, 10.8 / 13.2, 11.3 / 17.9, 16.0; from position 4000 80.6, 70.6 / 84.9, 72.6 / 86.7, 77.4.
+  const int64_t pairs = (int64_t)((a.T + 2 * kAtBM - 1) / (2 * kAtBM)) * a.n_head * batch;
+  a.span = pairs * 2 <= sm_count() ? kAtBM : 2 * kAtBM;
+  const dim3 grid((unsigned)((a.T + a.span - 1) / a.span), (unsigned)a.n_head, (unsigned)batch);
   unsigned* const err = wait_error_word();
   if (!err) return cudaErrorMemoryAllocation;
   return launch(attn_tc05_kernel<HS>, grid, dim3(kAtThreads), (size_t)smem, st, a, mk, mv, err);

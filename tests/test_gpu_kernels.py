@@ -868,7 +868,8 @@ def _attn_close(y, ref):
 
 
 @pytest.mark.parametrize("T,start,tail", [(128, 0, 0), (129, 0, 7), (255, 130, 0), (256, 128, 128), (257, 0, 1), (300, 1, 200), (640, 0, 0), (130, 1000, 3)])
-@pytest.mark.parametrize("B,H,G,hs,pos_dtype", [(1, 4, 4, 128, torch.int64), (2, 8, 2, 64, torch.int32)])
+@pytest.mark.parametrize("B,H,G,hs,pos_dtype", [(1, 4, 4, 128, torch.int64), (2, 8, 2, 64, torch.int32),   # one tile of rows per CTA
+                                                (1, 76, 4, 128, torch.int64), (2, 38, 2, 64, torch.int32)])  # two: CTAs enough for the SMs
 def test_attn_prefill_tiles(K, T, start, tail, B, H, G, hs, pos_dtype):
     """Rows and keys on either side of the tiles of the prompt kernel; whatever lies behind the last position must not be seen."""
     g = torch.Generator().manual_seed(T + start)
@@ -895,7 +896,7 @@ def test_attn_prefill_tiles_sharp_rows_and_any_positions(K):
 
 
 @pytest.mark.parametrize("window", [0, 1, 127, 128, 129, 300])
-@pytest.mark.parametrize("hs,H,G", [(128, 4, 2), (64, 3, 3)])
+@pytest.mark.parametrize("hs,H,G", [(128, 4, 2), (64, 3, 3), (128, 40, 2), (64, 38, 38)])
 def test_attn_window_tiles(K, window, hs, H, G):
     """Packed ragged prompts with a window and a sink: windows ending on either side of a key tile, a sequence of one row, rows between heads
     of other columns; the next sequence's rows are poisoned in turn."""
@@ -1024,7 +1025,7 @@ def test_qgemm_split_under_capture_and_on_streams(K, M, N, Kdim):
         assert all(torch.equal(y, w) for y in o)
 
 
-@pytest.mark.parametrize("hs,H", [(128, 2), (64, 3)])
+@pytest.mark.parametrize("hs,H", [(128, 2), (64, 3), (128, 5), (64, 6)])
 @pytest.mark.parametrize("repeat_keys", [False, True])
 def test_attn_ragged_tiles(K, hs, H, repeat_keys):
     """Several sequences in one launch -- long portions, portions within a tile and single rows over longer contexts, the contexts' rows in another
