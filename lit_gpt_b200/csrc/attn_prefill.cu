@@ -23,12 +23,22 @@ constexpr int kPfBM = 128;   // query rows per CTA
 constexpr int kPfBN = 64;    // keys per tile
 constexpr int kPfThreads = 256;
 constexpr float kLog2e = 1.4426950408889634f;
-// Plain causal (windowed, with a sink) prompts from this many rows on go to the tcgen05 kernel (attn_tc05.cu).  It starts slower -- tensor
-// memory, barriers, tiles of twice the rows and keys: 8.8 against 5.1 us for 17 rows, 8.0 against 8.2 us for 128 -- and steps faster: 18.6 against
-// 31.5 us for 600 rows of 32 heads, 230 against 589 us for 4096.
+// Plain causal (windowed, with a sink) prompts from this many rows on go to the tcgen05 kernel (attn_tc05.cu).  It starts slower -- tensor memory,
+// barriers, tiles of 128 keys -- and steps faster.  32 heads of 128, us of the tiles here and of that kernel: from position 0 100 rows 9.2, 10.4; 128 rows
+// 9.4, 9.0; 160 rows 9.3, 10.8; 200 rows 12.9, 11.2; 600 rows 32.6, 20.0; 4096 rows 589, 230; from position 1000 128 rows 42.6, 25.4; 160 rows 42.7, 27.1.  (Where
+// a portion starts is known on the device only: the 1.5 us that 129 to 190 rows from position 0 lose are the price of the 15 that later portions win.)
 constexpr int kTc05MinRows = 128;
 // Its tensor maps want rows that do not overlap; anything else (one key row repeated by a stride of 0, say) stays with the tiles here.
 inline bool tc05_rows(int64_t ldk, int64_t ldv, int64_t cols) { return ldk >= cols && ldv >= cols; }
+// A ragged step whose sequences are mostly short (single rows beside a prompt) has one nearly empty CTA of that kernel per head and sequence, and one that
+// only leaves per head, sequence and further tile of the longest one: it pays with contexts long enough.  32 single rows beside a prompt, us here and
+// there: 32 heads of 128 over 300 keys each beside 160 rows 82, 88, beside 512 97, 108; over 2000 keys 356, 249 and 376, 271; 16 heads of 64 over 300
+// keys 34, 42 and 41, 50; over 2000 151, 125 and 156, 130.  Lines through both ends cross at these lengths.
+inline bool tc05_mixed(int64_t rows, int64_t kv_rows, int n_seqs, int max_q_len, int head_size) {
+  if (rows <= 0 || rows >= (int64_t)kTc05MinRows * n_seqs) return true;   // whole prompts (or not told)
+  const int64_t more = (max_q_len - 1) / 256;
+  return kv_rows >= n_seqs * (head_size == 128 ? 400 + 100 * more : 550 + 370 * more);
+}
 
 // Where the operands live, in elements.  The cached layout of the GQA models is (B, H or G, rows, HS); a ragged batch packs the
 // query rows of all sequences into one (rows, H * HS) matrix and gives, per sequence, seqs[b] = {first query row, query rows,
@@ -558,6 +568,12 @@ extern "C" int b200_attn_prefill(const void* q, const void* k_cache, const void*
 extern "C" int b200_attn_prefill_ragged(const void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv, const int32_t* seqs,
                                         int n_seqs, int max_q_len, void* y, int64_t ldy, int n_head, int head_size, float scale,
                                         b200_stream_t stream) {
+  return b200_attn_prefill_ragged_ex(q, ldq, k, ldk, v, ldv, seqs, n_seqs, max_q_len, y, ldy, n_head, head_size, scale, 0, 0, stream);
+}
+
+extern "C" int b200_attn_prefill_ragged_ex(const void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv, const int32_t* seqs,
+                                           int n_seqs, int max_q_len, void* y, int64_t ldy, int n_head, int head_size, float scale,
+                                           int64_t rows, int64_t kv_rows, b200_stream_t stream) {
   B200_CHECK_ARG(q && k && v && seqs && y, "b200_attn_prefill_ragged: null pointer");
   B200_CHECK_ARG(n_seqs > 0 && n_seqs <= 65535 && max_q_len > 0 && n_head > 0 && n_head <= 65535, "b200_attn_prefill_ragged: bad shape");
   B200_CHECK_ARG(head_size == 64 || head_size == 128, "b200_attn_prefill_ragged: head_size must be 64 or 128 (got %d)", head_size);
@@ -565,7 +581,7 @@ extern "C" int b200_attn_prefill_ragged(const void* q, int64_t ldq, const void* 
   B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(seqs)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(y) & 3) == 0, "b200_attn_prefill_ragged: operands must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
-  if (max_q_len >= kTc05MinRows && tc05_rows(ldk, ldv, (int64_t)n_head * head_size)) {
+  if (max_q_len >= kTc05MinRows && tc05_rows(ldk, ldv, (int64_t)n_head * head_size) && tc05_mixed(rows, kv_rows, n_seqs, max_q_len, head_size)) {
     B200_CHECK_WAITS("b200_attn_prefill_ragged");
     const AttnTc05Args A{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)y, 0, head_size, ldq, 0, head_size, ldk, 0, head_size,
                          ldv, 0, ldy, reinterpret_cast<const int4*>(seqs), nullptr, 0, 0, nullptr, 0, max_q_len, n_head, n_head, 0, scale * kLog2e};

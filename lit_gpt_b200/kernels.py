@@ -737,9 +737,9 @@ def latent_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, seqs: torc
     if (plain and q.dtype == torch.bfloat16 and dk == dv and dk in (64, 128) and not (q.stride(0) | k.stride(0) | v.stride(0)) & 7
             and not (q.data_ptr() | k.data_ptr() | v.data_ptr() | seqs.data_ptr()) & 15 and LATENT_PREFILL_MMA):
         # tensor-core tiles of the GQA models' prefill kernel, over the packed operands
-        C.check(C.load_core().b200_attn_prefill_ragged(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), seqs.data_ptr(),
-                                                       seqs.shape[0], max_q_len, out.data_ptr(), out.stride(0), n_head, dk, float(scale),
-                                                       C.stream_ptr(q.device)), "attn_prefill_ragged")
+        C.check(C.load_core().b200_attn_prefill_ragged_ex(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), seqs.data_ptr(),
+                                                          seqs.shape[0], max_q_len, out.data_ptr(), out.stride(0), n_head, dk, float(scale), q.shape[0],
+                                                          k.shape[0], C.stream_ptr(q.device)), "attn_prefill_ragged")
         return out
     gm = _gate_mode(gate, n_head, dv)
     if (k_shared is not None and q.dtype == torch.bfloat16 and LATENT_PREFILL_MMA and dv in (64, 128) and dk - k_shared.shape[-1] == dv

@@ -1057,3 +1057,22 @@ def test_attn_ragged_tiles(K, hs, H, repeat_keys):
         ref = _attn_exact(q[f : f + m].view(m, H, hs), kk.reshape(m + s, H, hs), kv[a : a + m + s, H * hs : 2 * H * hs].reshape(m + s, H, hs), lim,
                           torch.zeros_like(lim), 0.2)
         _attn_close(y[f : f + m], ref)
+
+
+@pytest.mark.parametrize("hs", [128, 64])
+@pytest.mark.parametrize("ctx", [20, 2000])
+def test_attn_ragged_single_rows_beside_a_prompt(K, hs, ctx):
+    """A prompt of 300 rows and twelve single rows over short and over long contexts: whichever tiles the step takes, the same attention."""
+    H, new, start = 2, (300,) + (1,) * 12, (0,) + tuple(ctx + i for i in range(12))
+    g = torch.Generator().manual_seed(ctx)
+    n, m = sum(new), sum(new) + sum(start)
+    q, k, v = (torch.randn(r, H * hs, generator=g).bfloat16() for r in (n, m, m))
+    seqs, first, at = [], 0, 0
+    for a, s in zip(new, start):
+        seqs.append((first, a, s, at))
+        first, at = first + a, at + a + s
+    y = K.latent_prefill(q.cuda(), k.cuda(), v.cuda(), torch.tensor(seqs, dtype=torch.int32).cuda(), 300, H, hs, hs, 0.2)
+    for f, a, s, c in seqs:
+        lim = torch.arange(s, s + a)
+        ref = _attn_exact(q[f : f + a].view(a, H, hs), k[c : c + a + s].view(a + s, H, hs), v[c : c + a + s].view(a + s, H, hs), lim, torch.zeros_like(lim), 0.2)
+        _attn_close(y[f : f + a], ref)
