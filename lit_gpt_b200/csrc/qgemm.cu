@@ -9,12 +9,13 @@
 //     the tensor core's K-major 128-byte-swizzled layout.  Even and odd k-blocks belong to eight warps each: a warp has two blocks' time
 //     for its loads, look-ups and the proxy fence, and 32 codes a thread to overlap;
 //   * warp 16 fetches the activation tiles (128 tokens x 64 k per CTA and sub-tile) by TMA, rows past M zero-filled by the hardware;
-//   * warp 17 of the pair's first CTA issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, 256 x 256 x 16) into TENSOR MEMORY; tcgen05.commit
+//   * warp 17 (of the pair's first CTA) issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, 256 x 256 x 16) into TENSOR MEMORY; tcgen05.commit
 //     hands each stage back to both CTAs;
-//   * across the pair every hand-over has cluster scope: warp 17 of the second CTA passes its CTA's dequantised tiles on to the first CTA's
-//     barrier, and each CTA's warp 16 passes a stage's return on to its dequantising warps.  Those wait and arrive on barriers of their own
-//     CTA only -- a release or an acquire at cluster scope waits for all that a thread has under way, and their weight loads always are
-//     (700 to 1500 clocks a k-block);
+//   * across the pair every hand-over has cluster scope.  A dequantising warp of the second CTA announces its rows with 16 bytes of them, a bulk
+//     copy to the first CTA whose arrival there is the release (it is started after the writes, so it follows them), and each CTA's warp 16 passes a
+//     stage's return on to the dequantising warps.  Those wait on barriers of their own CTA only.  (An arrival with release at cluster scope takes 1400
+//     clocks, whichever thread makes it: the SM's weight loads under way hold it up.  4096 -> 11008 at 203 rows, nf4: 49.7 us; with one thread that
+//     passes the second CTA's tiles on with such arrivals 69.4, with two in turn 50.8; 14336 -> 4096 at 4096 rows, int4: 366, 437, 360.)
 //   * the sixteen warps read the accumulators with tcgen05.ld, add the bias, round to bf16 and store rows of y.
 // SWIGLU: the pair's first CTA dequantises 128 rows of the gate projection and the second the same rows of the up projection, so that a
 // thread holds both halves of its outputs and stores silu(gate) * up, with the roundings of the separate launches.
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   constexpr int BN = 128 * CTAS, BM = BN;           // features per tile, tokens per sub-tile
   __shared__ __align__(8) uint64_t s_bars[3 * C::kStages + 3];
   __shared__ uint32_t s_tmem;
+  __shared__ uint4 s_token[CTAS == 2 ? C::kStages : 1][8];   // where the bytes of the other CTA's warps land
   __shared__ float s_code[16 * 32];                 // fp32 code book, one copy per lane (conflict-free look-ups)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = CTAS == 2 ? tc::cluster_rank() : 0u;
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   const uint32_t room = CTAS == 2 ? idle + 8 : empty;   // where the dequantising warps learn that a stage is theirs
   if (tid == 0) {
     for (int s = 0; s < C::kStages; ++s) {
-      tc::mbar_init(full + 8 * s, rank == 0 ? 8 + CTAS : 8);   // half of the dequantising warps; in the first CTA the copies and the other CTA's tile
+      tc::mbar_init(full + 8 * s, 9);   // half of the dequantising warps and the copies
       tc::mbar_init(empty + 8 * s, 1);
       if (CTAS == 2) tc::mbar_init(room + 8 * s, 1);
     }
@@ -198,7 +200,10 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
         }
         tc::fence_smem_async();                       // generic-proxy writes -> visible to the tensor core
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(full + 8 * s);
+        if (lane == 0) {
+          if (CTAS == 2 && rank == 1) tc::copy_to_cta(tc::at_rank(tc::smem_u32(&s_token[s][warp & 7]), 0), dst + sw128(wr, wh * 4), 16, tc::at_rank(full + 8 * s, 0));
+          else tc::mbar_arrive(full + 8 * s);
+        }
       }
       q += t.nkb;
       // ---- accumulators -> y (or partial sums): warp w has rows 32 (w % 4) .. + 31 and a quarter of the columns ----
@@ -283,7 +288,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
           ok = wait(empty + 8 * s, ((uint32_t)(q / C::kStages) & 1u) ^ 1u);
           if (!ok) break;
           if (CTAS == 2) tc::mbar_arrive(room + 8 * s);
-          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * t.mts * kTileBytes);
+          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * t.mts * kTileBytes + (CTAS - 1) * 8 * 16);
           const uint32_t st = tiles + s * C::kStage, bar = CTAS == 2 ? tc::at_rank(full + 8 * s, 0) : full + 8 * s;
           for (int mt = 0; mt < t.mts; ++mt) {
             const int row = (int)(t.m0 + mt * BM + rank * 128), col = (t.kb0 + l) * kBK;
@@ -329,17 +334,6 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
       if constexpr (CTAS == 2) tc::commit_pair(idle);
       else tc::commit(idle);
       tc::mbar_wait(idle, 0);
-    }
-  } else if (lane == 0 && CTAS == 2) {
-    // ============================ THE SECOND CTA'S TILES, PASSED ON TO THE FIRST ================================
-    for (int i = first; i < total && ok; i += step) {
-      const int nkb = item(i).nkb;
-      for (int l = 0; l < nkb; ++l, ++q) {
-        const int s = q % C::kStages;
-        ok = tc::mbar_wait(full + 8 * s, (uint32_t)(q / C::kStages) & 1u);
-        if (!ok) break;
-        tc::mbar_arrive_at(tc::at_rank(full + 8 * s, 0));
-      }
     }
   }
   if (!ok) *err = 1u;

@@ -147,6 +147,11 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t slot) {   // one warp o
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "n"(COLS) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
+// bytes (a multiple of 16) of this CTA's shared memory into another CTA's, counted on a barrier there
+__device__ __forceinline__ void copy_to_cta(uint32_t cluster_dst, uint32_t src, uint32_t bytes, uint32_t cluster_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(cluster_dst), "r"(src), "r"(bytes), "r"(cluster_bar) : "memory");
+}
 template <int COLS>
 __device__ __forceinline__ void tmem_free_pair(uint32_t tmem) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(COLS) : "memory");
