@@ -2,7 +2,7 @@
 //
 // Replaces, for T > 16 rows, bnb.nn.Linear4bit.forward's "dequantize_4bit of the WHOLE weight to bf16, then F.linear"
 // (call sites lit_gpt/model.py:519,619,656,713,714,716): the bf16 weight is never materialised in HBM.
-// Persistent over output tiles of 256 features x 256 MT tokens, a CTA PAIR each (cta_group::2; up to 128 tokens: one CTA on 128 x 128),
+// Persistent over output tiles of 256 features x 256 MT tokens, a CTA PAIR each (cta_group::2; up to 128 tokens: one CTA on 128 x 128; up to 256 of small matrices: one on 128 x 256),
 // walking K in blocks of 64.  Per CTA:
 //   * warps 0-15 rebuild the bf16 values of 128 features from the packed 4-bit weights and their absmax / {scale, zero} with exactly the
 //     dequantise kernel's arithmetic (bf16_rn(code_fp32 * absmax_fp32), resp. bf16_rn(scale * (q - zero))) and write them into shared memory in
@@ -22,7 +22,7 @@
 // Bound: with MT = 2 the tensor pipe and the shared memory that feeds it (a CTA alone on 128 x 128 reads 128 bytes a clock of it for the
 // products alone, the pair 64); one dequantised tile serves 512 tokens.  What was before -- a CTA on 128 features x 384 tokens, one thread that
 // loaded the activations between its own dequantising, every warp in every k-block -- spent 1750 clocks a k-block whatever the tokens.
-// 4096 tokens, 4096 -> 14336: int4 516 -> 390 us, nf4 591 -> 410; 14336 -> 4096: int4 532 -> 334 (1440 TFLOP/s), nf4 631 -> 356.
+// 4096 tokens, 4096 -> 14336: int4 516 -> 406 us, nf4 591 -> 414; 14336 -> 4096: int4 532 -> 358 (1340 TFLOP/s), nf4 631 -> 368.
 #include "tc05.cuh"
 
 namespace b200 {
@@ -379,16 +379,20 @@ struct GemmPlan {
   int ctas, mt, ksplit;
 };
 
-// Tile and k ranges by the time of the last SM to finish, in clocks as measured over launches of one round: a k-block takes about 1500 with two
-// sub-tiles of 256 tokens, 1130 with one (the dequantisation, which a second sub-tile shares), 950 for a CTA alone on 128 tokens; a tile
-// costs 6000 more to start and to store, partial sums of k ranges 13000 and a clock per 1860 bytes.  k ranges are for launches that leave
-// SMs idle -- two at least where half of them would be: at least four k-blocks per range, at most 16 ranges and 64 MB of partial sums, and
-// no more than fill the SMs once.
+// Tile and k ranges by the time of the last SM to finish, in clocks as measured over launches of one round.  A k-block takes about 1500 with two
+// sub-tiles of 256 tokens, 1130 with one (the dequantisation, which a second sub-tile shares), 1380 for a CTA alone on two sub-tiles of 128, 950 on
+// one; a launch 14400 with pairs (7.6 us from the launch before it to its last store besides its k-blocks, of which a cluster's start is the most) and
+// 8400 without; a further round of tiles 6000; k ranges 4000, 500 for each and a clock per 1200 bytes of partial sums.  k ranges are for
+// launches that leave SMs idle -- two at least where half of them would be: at least four k-blocks per range, at most 16 ranges and 64 MB of partial
+// sums, and no more than fill the SMs once.
+// 129 to 256 rows, us of a CTA alone on 256 tokens and of a pair, both in four k ranges, nf4 / int4, at 203 rows: 2048 x 2048 17.4, 18.9 / 15.8, 16.7; 4096 x
+// 4096 26.1, 26.7 / 23.3, 23.1; 11008 -> 4096 46.1, 43.2 / 40.7, 36.2.
+static int64_t gemm_start(const GemmPlan& g) { return g.ctas == 1 ? 2400 : 8400; }
 static int64_t gemm_clocks(int64_t M, int64_t N, int64_t K, const GemmPlan& g) {
   const int64_t nkb = K / kBK, units = sm_count() / g.ctas, s = g.ksplit;
   const int64_t tiles = ((N + 128 * g.ctas - 1) / (128 * g.ctas)) * ((M + 128 * g.ctas * g.mt - 1) / (128 * g.ctas * g.mt));
-  const int64_t per = g.ctas == 1 ? 950 : g.mt == 1 ? 1130 : 1500;
-  return ((tiles * s + units - 1) / units) * (((nkb + s - 1) / s) * per + 6000) + (s > 1 ? 13000 + s * M * N * 4 / 1860 : 0);
+  const int64_t per = g.ctas == 1 ? (g.mt == 1 ? 950 : 1380) : (g.mt == 1 ? 1130 : 1500);
+  return ((tiles * s + units - 1) / units) * (((nkb + s - 1) / s) * per + 6000) + gemm_start(g) + (s > 1 ? 4000 + 500 * s + s * M * N * 4 / 1200 : 0);
 }
 
 static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool split_ok) {
@@ -396,10 +400,11 @@ static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool split_ok) {
   const int64_t sms = sm_count();
   GemmPlan best{1, 1, 1};
   int64_t best_t = -1;
-  for (int kind = 0; kind < 3; ++kind) {
-    const int ctas = kind ? 2 : 1, mt = kind == 2 ? 2 : 1;
-    if (kind == 0 ? M > 128 : M <= 128) continue;            // a pair's second half would be padding; a CTA alone would dequantise twice
-    if (kind == 2 && (M <= 256 || !g_gemm_wide.load())) continue;
+  for (int kind = 0; kind < 4; ++kind) {
+    const int ctas = kind < 2 ? 1 : 2, mt = kind & 1 ? 2 : 1;
+    if (kind == 0 ? M > 128 : M <= 128) continue;            // a second half would be padding; a CTA alone on 128 tokens would dequantise twice
+    if (kind == 1 && M > 256) continue;
+    if (kind == 3 && (M <= 256 || !g_gemm_wide.load())) continue;
     const int64_t units = sms / ctas, tiles = ((N + 128 * ctas - 1) / (128 * ctas)) * ((M + 128 * ctas * mt - 1) / (128 * ctas * mt));
     int64_t most = split_ok ? units / tiles : 1;
     if (most > nkb / 4) most = nkb / 4;
@@ -440,22 +445,23 @@ static cudaError_t launch_gemm(GemmParams p, cudaStream_t st) {
 
 template <bool INT4>
 static cudaError_t launch_plan(const GemmParams& p, const GemmPlan& g, cudaStream_t st) {
-  if (g.ctas == 1) return launch_gemm<1, 1, INT4>(p, st);
+  if (g.ctas == 1) return g.mt == 2 ? launch_gemm<1, 2, INT4>(p, st) : launch_gemm<1, 1, INT4>(p, st);
   return g.mt == 2 ? launch_gemm<2, 2, INT4>(p, st) : launch_gemm<2, 1, INT4>(p, st);
 }
 
 // Sub-tiles of a gate / up pair in one launch, by gemm_plan's clocks; 0 where two launches and the product are the shorter way.  The product
 // costs 4000 to start and a clock per 550 elements; half of that counts, and a twentieth has to be won, since the second of two launches starts
 // on the SMs that the first one's last round leaves idle: what pays is a round of tiles saved, or small matrices.  us, two launches and the
-// product against one, nf4 / int4: 4096 -> 14336 at 4096 rows 1014 -> 904 / 981 -> 917, at 2048 538 -> 462 / 517 -> 449; 4096 -> 11008 at 1000 rows
-// 257 -> 193 / 247 -> 192; 2048 -> 5632 at 203 rows 62 -> 40 / 55 -> 30.  Left apart: 4096 -> 11008 at 203 rows 98 against 105 / 107 against 98, at 4096
-// 757 against 712 / 685 against 667; 5120 -> 13824 at 2048 515 against 515 / 494 against 527.
+// product against one, nf4 / int4: 4096 -> 14336 at 4096 rows 1017 -> 928 / 999 -> 918, at 2048 538 -> 467 / 545 -> 514; 4096 -> 11008 at 1000 rows
+// 256 -> 197 / 253 -> 196; 2048 -> 5632 at 203 rows 62 -> 38 / 50 -> 30.  Left apart: 4096 -> 11008 at 203 rows 98 against 105 / 107 against 98, 5120 -> 13824
+// at 2048 515 against 515 / 494 against 527 -- and, as the price of one line for both types, 4096 -> 11008 at 4096, where one launch would win
+// 3 to 6 % (757 against 712 / 685 against 667).
 static int swiglu_tiles(int64_t M, int64_t N, int64_t K) {
   if (M <= 128) return 0;
   const int64_t units = sm_count() / 2, n = (N + 127) / 128, nkb = K / kBK;
   const GemmPlan one = gemm_plan(M, N, K, true);
-  int64_t apart = gemm_clocks(M, N, K, one);
-  if (one.mt == 2 && (M - 1) % 512 < 256) apart -= 370 * (nkb / one.ksplit);   // the last tiles have one sub-tile
+  int64_t apart = gemm_clocks(M, N, K, one) - gemm_start(one);   // (the second launch's start is hidden as well)
+  if (one.ctas == 2 && one.mt == 2 && (M - 1) % 512 < 256) apart -= 370 * (nkb / one.ksplit);   // the last tiles have one sub-tile
   const int64_t worth = (2 * apart + 2000 + M * N / 1100) / 20 * 19;
   int64_t best = 0, best_t = worth;
   for (int mt = 1; mt <= (M > 256 && g_gemm_wide.load() ? 2 : 1); ++mt) {
