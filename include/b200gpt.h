@@ -340,7 +340,7 @@ typedef struct b200_qgemm_args {
 size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200_qgemm(const b200_qgemm_args* args, b200_stream_t stream);
 /* y = silu(gate) * up of two projections of the same x (bf16 each, silu to bf16, product to bf16: the roundings of two b200_qgemm and
- * b200_swiglu), `args` holding the gate and packed2 / scale2 the up projection in the same layout; no bias.  supported: 1 where one launch is
+ * b200_swiglu, and their bits where those run without k ranges), `args` holding the gate and packed2 / scale2 the up projection in the same layout; no bias.  supported: 1 where one launch is
  * the shorter way (nothing is launched); elsewhere the call returns B200_ERR_UNSUPPORTED. */
 int b200_qgemm_swiglu_supported(int64_t M, int64_t N, int64_t K, int qtype, int blocksize);
 int b200_qgemm_swiglu(const b200_qgemm_args* args, const void* packed2, const void* scale2, b200_stream_t stream);

@@ -412,7 +412,8 @@ def qgemm_swiglu_supported(M: int, N: int, K: int, quant_type: str = "nf4", bloc
 
 def qgemm_swiglu(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, packed2: torch.Tensor, scale2: torch.Tensor, N: int, K: int,
                  quant_type: str = "nf4", blocksize: int = 64) -> torch.Tensor:
-    """silu(x . dequant(W)^T) * (x . dequant(W2)^T), bf16-rounded where two ``qgemm`` and ``swiglu`` round, in one launch.
+    """silu(x . dequant(W)^T) * (x . dequant(W2)^T), bf16-rounded where two ``qgemm`` and ``swiglu`` round, in one launch.  The same
+    bits as theirs where they sum k in one range; otherwise (few tiles) their sums differ in the last bits before those roundings.
     Raises NotImplementedError where ``qgemm_swiglu_supported`` is false."""
     C.require_cuda(x, packed, scale, packed2, scale2)
     x = _bf16c(x, "x")
