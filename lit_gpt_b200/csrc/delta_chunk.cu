@@ -34,7 +34,7 @@ struct DcArgs {
   float* out; int64_t ldo;
   const int4* seqs;
   int heads, kv_heads, dk, dv;
-  int n_seqs, longs;                // sequences, and how many of them can have chunks
+  int n_seqs, longs, min_rows;      // sequences, how many of them can have chunks, and from how many rows on they have
   int item0, n_items, most;         // this launch's chunks, counted through all sequences, of `most` in all
   int dvb;                          // blocks of eight value columns (an even number)
   float* ws; int64_t item;          // per (chunk, head): W | K | Q, rows of DK + 4 | P (DK) | U [dvb][32][8] | O [dvb][32][8]
@@ -55,15 +55,16 @@ __device__ __forceinline__ float sum2(f2 v) { float a, b; un2(v, a, b); return a
 
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
-// Chunks are counted through the sequences in their order, each with as many as its rows take; sequences of fewer than kDcMinRows have none and go
-// token by token.  The functions below are called by whole warps.
-__device__ __forceinline__ int dc_chunks(const int4& sq) { return sq.y >= kDcMinRows ? (sq.y + kDcC - 1) / kDcC : 0; }
+// Chunks are counted through the sequences in their order, each with as many as its rows take; among several sequences, those of fewer than
+// kDcMinRows have none and go token by token.  (A single one always has a chunk, which without rows keeps or clears the slot's state as the walk
+// would.)  The functions below are called by whole warps.
+__device__ __forceinline__ int dc_chunks(const DcArgs& A, const int4& sq) { return sq.y >= A.min_rows ? (max(sq.y, 1) + kDcC - 1) / kDcC : 0; }
 // the sequence of chunk `at` and the chunk's number there; -1: there are not that many
 __device__ __forceinline__ int dc_find(const DcArgs& A, int at, int& chunk) {
   const int lane = threadIdx.x & 31;
   int before = 0;
   for (int s0 = 0; s0 < A.n_seqs; s0 += 32) {
-    const int n = s0 + lane < A.n_seqs ? dc_chunks(A.seqs[s0 + lane]) : 0;
+    const int n = s0 + lane < A.n_seqs ? dc_chunks(A, A.seqs[s0 + lane]) : 0;
     int incl = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -85,7 +86,7 @@ __device__ __forceinline__ int dc_nth(const DcArgs& A, int z, int& before) {
   const int lane = threadIdx.x & 31;
   before = 0;
   for (int s0 = 0; s0 < A.n_seqs; s0 += 32) {
-    const int n = s0 + lane < A.n_seqs ? dc_chunks(A.seqs[s0 + lane]) : 0;
+    const int n = s0 + lane < A.n_seqs ? dc_chunks(A, A.seqs[s0 + lane]) : 0;
     const unsigned have = __ballot_sync(0xffffffffu, n > 0);
     if (z < __popc(have)) {
       const int w = (int)__fns(have, 0, z + 1);
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
   const int z = dc_nth(A, blockIdx.z, before);
   if (z < 0) return;
   const int4 sq = A.seqs[z];
-  const int all = dc_chunks(sq);
+  const int all = dc_chunks(A, sq);
   const int c_first = max(0, A.item0 - before), chunks = min(all, A.item0 + A.n_items - before) - c_first, t_first = c_first * C;
   if (tid == 0 && before + all > A.most) *A.err = 1u;   // more rows than the caller said
   if (chunks <= 0) return;
@@ -555,7 +556,7 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
     if (rc != B200_OK || most == 0) return rc;
   }
   DcArgs A{a->q, a->k, a->v, a->ldq, a->ldk, a->ldv, a->beta_in, a->ld_beta, a->decay_in, a->ld_decay, a->a_log, a->dt_bias, a->state, a->state_slot_stride,
-           a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv, a->n_seqs, (int)longs, 0, (int)fit, (int)most, dc_dvb(a->dv),
+           a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->kv_heads, a->dk, a->dv, a->n_seqs, (int)longs, a->n_seqs > 1 ? kDcMinRows : 0, 0, (int)fit, (int)most, dc_dvb(a->dv),
            reinterpret_cast<float*>(workspace), item, wait_error_word()};
   B200_CHECK_ARG(A.err, "b200_delta_rule_chunked: no error word");
   auto al = [](const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };

@@ -137,6 +137,23 @@ def test_delta_chunks_compute_every_row_whatever_the_hint(K, monkeypatch, lens, 
     assert (a - c).abs().max() <= 1e-4 * c.abs().max() and (sa - sc).abs().max() <= 1e-4 * sc.abs().max()
 
 
+@pytest.mark.parametrize("rows", [40, 1, 0])
+@pytest.mark.parametrize("start", [0, 9])
+def test_delta_chunks_of_a_short_sequence_in_a_long_buffer(K, monkeypatch, rows, start):
+    """One sequence whose rows are fewer than the buffer's and than the hint says: its rows and its state, as token by token."""
+    H, G, dk, dv = 2, 1, 64, 24
+    data = _inputs((100,), (start,), H, G, dk, dv, True, torch.float32, 2, 0)
+    dev, seqs = [t.contiguous().cuda() for t in data[:7]], torch.tensor([[0, rows, start, 1]], dtype=torch.int32).cuda()
+    out = []
+    for chunked in (True, False):
+        monkeypatch.setattr(K, "DELTA_CHUNKED", chunked)
+        state = _stored(data[7], dk, 4).float().cuda()
+        out.append((K.delta_rule(*dev, state, seqs, H, G, dk, dv, True, max_rows=100)[:rows], state))
+    (a, sa), (b, sb) = out
+    assert rows == 0 or (a - b).abs().max() <= 1e-4 * b.abs().max()
+    assert (sa - sb).abs().max() <= 1e-4 * sb.abs().max()
+
+
 def test_delta_chunk_scratch_follows_the_rows(K, monkeypatch):
     """One prompt among many single rows takes scratch for the rows there are; without memory for it the call runs token by token."""
     H, G, dk, dv, lens = 2, 2, 128, 32, (96,) + (1,) * 40
