@@ -7,8 +7,7 @@
 // earlier steps left in its state slot.  Whether a tap lies before the sequence start, in the tail or in the step is decided
 // by its POSITION alone, so a slot that another sequence used before needs no clearing.
 //
-// The channels form up to three groups of heads (e.g. queries, keys, values); one warp owns one (row, head) and applies
-// after the convolution, in fp32:
+// The channels form up to three groups of heads (e.g. queries, keys, values); the lanes of a head apply after the convolution, in fp32:
 //   act  : none | silu
 //   post : none
 //        | rotate + norm : rotary positions on the first rot_dims dimensions, interleaved pairs (2i, 2i + 1) turned by the
@@ -237,6 +236,215 @@ __global__ void __launch_bounds__(kCvThreads) short_conv_kernel(const T* __restr
   }
 }
 
+// x / (1 + exp(-x)) by the approximate reciprocal and one correction of the quotient by its remainder (Markstein): as close as the division, without
+// its branches.  Beyond 80 the quotient is x or below 1e-32 and the remainder could overflow: left as it is (infinities and NaN as by the division).
+__device__ __forceinline__ float silu_cv(float x) {
+  const float y = 1.0f + expf(-x), r = __fdividef(1.0f, y), q = x * r;
+  return fabsf(x) < 80.0f ? fmaf(fmaf(-q, y, x), r, q) : q;
+}
+// 1 / sqrt(x): the approximation and one Newton step
+__device__ __forceinline__ float rsqrt_cv(float x) {
+  const float r = rsqrtf(x), h = 0.5f * x * r;
+  return x > 1e-30f && x < 1e30f ? fmaf(r, fmaf(-h, r, 0.5f), r) : r;
+}
+
+// Four neighbouring channels of a row as they lie in memory
+template <typename T>
+struct CvRaw;
+template <>
+struct CvRaw<__nv_bfloat16> {
+  uint2 w;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { w = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void zero() { w = make_uint2(0, 0); }
+  __device__ __forceinline__ void floats(float (&f)[8], int at) const { f[at] = bf16lo(w.x); f[at + 1] = bf16hi(w.x); f[at + 2] = bf16lo(w.y); f[at + 3] = bf16hi(w.y); }
+};
+template <>
+struct CvRaw<float> {
+  float4 w;
+  __device__ __forceinline__ void load(const float* p) { w = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void zero() { w = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ void floats(float (&f)[8], int at) const { f[at] = w.x; f[at + 1] = w.y; f[at + 2] = w.z; f[at + 3] = w.w; }
+};
+__device__ __forceinline__ void store4(float* p, const float (&f)[8], int at) { *reinterpret_cast<float4*>(p) = make_float4(f[at], f[at + 1], f[at + 2], f[at + 3]); }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&f)[8], int at) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(f[at], f[at + 1]), pack_bf16(f[at + 2], f[at + 3]));
+}
+
+constexpr int kCv8Taps = 4;
+struct Cv8Blocks {   // per group: heads of a CTA (a power of two, the other lanes take further strips of rows), first CTA along y
+  int heads[kCvMaxGroups], first[kCvMaxGroups];
+};
+
+// Four taps, heads of a multiple of eight channels on 16-byte boundaries: a lane has two times four channels of its head, LPR lanes a head, R neighbouring
+// rows a lane.  All rows that R outputs read are fetched before the first is used, and the R chains of activation, norm and store run side by
+// side; the cosines and sines of a CTA's rows are computed once for all its heads.
+// Bound: the rows' way from L2 (R + 3 rows for R outputs), then the activation's instructions.  us against two channels a lane, each row's activation,
+// norm and store before the next row's, rows of 24 heads of 128 rotated and normed / 48 heads with silu and unit norm, four taps: bf16 300 rows 12.4 -> 6.3
+// / 16.3 -> 8.3, 2048 rows 31.2 -> 15.1 / 59.6 -> 29.8; fp32 2048 rows 24.9 -> 20.6 / 45.6 -> 39.2.  Eight neighbouring channels a lane: 17.3 / 31.7 and
+// fp32 26.5 / 44.9 (half of every 32-byte sector per access).  R = 8: 23.4 / 41.1 (registers).
+template <typename T, int LPR, int R>
+__global__ void __launch_bounds__(kCvThreads, 4) short_conv8_kernel(const T* __restrict__ in, int64_t ld_in, CvParams P, Cv8Blocks B, const T* __restrict__ tail,
+                                                                    int64_t tail_slot_stride, int tail_cols, const int4* __restrict__ seqs,
+                                                                    const int* __restrict__ row_seq, int64_t rows) {
+  constexpr int UNITS = kCvThreads / LPR, H = kCv8Taps - 1;
+  __shared__ float2 s_turn[UNITS * R * LPR * 4];   // [row of the CTA][pair of channels]: cosine and sine
+  griddep_launch();
+  griddep_wait();
+  const int tid = threadIdx.x, unit = tid / LPR, sub = tid % LPR;
+  int gi = 0;
+  while (gi + 1 < P.n_groups && (int)blockIdx.y >= B.first[gi + 1]) ++gi;
+  const CvGroup& G = P.g[gi];
+  const int hb = B.heads[gi], strips = UNITS / hb;
+  const int hh = ((int)blockIdx.y - B.first[gi]) * hb + unit % hb;
+  const int64_t cta0 = (int64_t)blockIdx.x * (strips * R), row0 = cta0 + (unit / hb) * R;
+  if (cta0 >= rows) return;
+  const int dim = G.dim, d[2] = {4 * sub, 4 * (LPR + sub)};
+  const bool has[2] = {d[0] < dim, d[1] < dim};
+  const int c = G.col0 + hh * dim;
+
+  CvRaw<T> win[R + H][2];   // rows row0 - 3 .. row0 + R - 1 of the step
+#pragma unroll
+  for (int i = 0; i < R + H; ++i) {
+    const int64_t row = row0 + i - H;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      if (has[p] && row >= 0 && row < rows) win[i][p].load(in + row * ld_in + c + d[p]);
+      else win[i][p].zero();
+    }
+  }
+  float w[8][kCv8Taps];
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const T* wt = reinterpret_cast<const T*>(G.w) + ((int64_t)hh * dim + d[p]) * kCv8Taps;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (has[p]) load8(wt + 8 * i, f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { w[4 * p + 2 * i][j] = f[j]; w[4 * p + 2 * i + 1][j] = f[4 + j]; }
+    }
+  }
+  int4 sq[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) sq[r] = row0 + r < rows ? seqs[row_seq[row0 + r]] : make_int4(0, 0, 0, 0);
+  const int half = G.rot_dims >> 1;
+  if (G.post == 1) {
+    for (int i = tid; i < strips * R * half; i += kCvThreads) {
+      const int r = i / half, p = i - r * half;
+      const int64_t row = cta0 + r;
+      if (row >= rows) break;
+      const int4 s = seqs[row_seq[row]];
+      // the angle in double, reduced to [-pi, pi] before the fp32 sine and cosine: exact to fp32 at any position
+      double a = (double)(s.z + (int)(row - s.x)) * G.inv_freq[p];
+      a -= 6.283185307179586476925286766559 * rint(a * 0.15915494309189533576888376337251);
+      float sn, cs;
+      sincosf((float)a, &sn, &cs);
+      s_turn[r * (LPR * 4) + p] = make_float2(cs * G.rot_mscale, sn * G.rot_mscale);
+    }
+    __syncthreads();
+  }
+
+  float val[R][8], ss[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int at = (int)(row0 + r - sq[r].x);   // row within the step's part of its sequence
+    float u[kCv8Taps][8];
+#pragma unroll
+    for (int j = 0; j < kCv8Taps; ++j)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) win[r + j][p].floats(u[j], 4 * p);
+    if (at < H && row0 + r < rows) {   // some taps lie before the step: in the tail, or before the sequence's first token
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        const int back = H - j;
+        if (back <= at) continue;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          CvRaw<T> t;
+          if (has[p] && back <= sq[r].z + at) t.load(tail + (int64_t)sq[r].w * tail_slot_stride + (int64_t)(H - (back - at)) * tail_cols + c + d[p]);
+          else t.zero();
+          t.floats(u[j], 4 * p);
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float a = 0.f;
+#pragma unroll
+      for (int j = 0; j < kCv8Taps; ++j) a = fmaf(w[e][j], u[j][e], a);
+      val[r][e] = a;
+    }
+    if (G.act == 1) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) val[r][e] = silu_cv(val[r][e]);
+    }
+    if (G.post == 1) {
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const int dim0 = d[e >> 2] + (e & 3);
+        if (dim0 + 1 < G.rot_dims) {
+          const float2 t = s_turn[((unit / hb) * R + r) * (LPR * 4) + (dim0 >> 1)];
+          const float x = val[r][e], y = val[r][e + 1];
+          val[r][e] = x * t.x - y * t.y;
+          val[r][e + 1] = y * t.x + x * t.y;
+        }
+      }
+    }
+    ss[r] = 0.f;
+    if (G.post != 0) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss[r] = fmaf(val[r][e], val[r][e], ss[r]);   // lanes past dim hold zeros
+    }
+  }
+  if (G.post != 0) {
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < R; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (row0 + r >= rows) continue;
+    float mul = G.post_scale;
+    if (G.post == 1) mul *= rsqrt_cv(ss[r] / (float)dim + G.eps);
+    else if (G.post == 2) mul *= rsqrt_cv(ss[r] + G.eps);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) val[r][e] *= mul;
+    const int64_t o = (row0 + r) * G.ld_out + (int64_t)hh * dim;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      if (!has[p]) continue;
+      if (G.out_f32) store4(reinterpret_cast<float*>(G.out) + o + d[p], val[r], 4 * p);
+      else store4(reinterpret_cast<T*>(G.out) + o + d[p], val[r], 4 * p);
+    }
+  }
+}
+
+// Four rows a lane from about eight CTAs per SM on, else one.  us with one and four, bf16, 24 heads of 128: 300 rows 6.3, 6.9, 1024 rows 12.5, 10.8; 24 heads
+// of 64: 1024 rows 7.5, 8.1, 2048 rows 11.9, 11.0.
+bool conv8_four(int64_t rows, int heads, int lanes_per_head) { return rows * heads >= (int64_t)sm_count() * (kCvThreads / lanes_per_head) * 8; }
+
+template <typename T, int LPR>
+cudaError_t short_conv8_launch(cudaStream_t st, const T* in, int64_t ld_in, const CvParams& P, const T* tail, int64_t tail_slot_stride, int tail_cols,
+                               const int4* seqs, const int* row_seq, int64_t rows) {
+  constexpr int UNITS = kCvThreads / LPR;
+  Cv8Blocks B{};
+  int y = 0, strips = 1;
+  for (int g = 0; g < P.n_groups; ++g) {
+    int hb = UNITS;
+    while (P.g[g].heads % hb) hb >>= 1;
+    B.heads[g] = hb;
+    B.first[g] = y;
+    y += P.g[g].heads / hb;
+    strips = g == 0 || UNITS / hb < strips ? UNITS / hb : strips;
+  }
+  const bool four = conv8_four(rows, P.total_heads, LPR);
+  const int per = strips * (four ? 4 : 1);
+  const dim3 grid((unsigned)((rows + per - 1) / per), (unsigned)y);
+  return four ? launch(short_conv8_kernel<T, LPR, 4>, grid, dim3(kCvThreads), 0, st, in, ld_in, P, B, tail, tail_slot_stride, tail_cols, seqs, row_seq, rows)
+              : launch(short_conv8_kernel<T, LPR, 1>, grid, dim3(kCvThreads), 0, st, in, ld_in, P, B, tail, tail_slot_stride, tail_cols, seqs, row_seq, rows);
+}
+
 template <typename T, int NIT>
 cudaError_t short_conv_launch(int taps, dim3 grid, cudaStream_t st, const T* in, int64_t ld_in, const CvParams& P, const T* tail,
                               int64_t tail_slot_stride, int tail_cols, const int4* seqs, const int* row_seq, int64_t rows, int rows_per_warp, int pairs) {
@@ -330,8 +538,25 @@ int b200_short_conv(const void* in, int64_t ld_in, const b200_conv_group* groups
   }
   if (pairs && w16) pairs |= 2;   // even channels times four taps: every pair's taps start on a 16-byte boundary
   if (out2) pairs |= 4;
+  // Four taps, eight channels a lane where every head's channels lie on 16-byte boundaries; fp32 only with four rows a lane: with one, 64 rows of 24 heads
+  // take 6.5 us against 5.4.
+  const int64_t e16 = 16 / (int64_t)esz;
+  bool vec8 = taps == kCv8Taps && max_dim <= 256 && P.total_heads <= 65535 && ld_in % e16 == 0 && tail_cols % e16 == 0 && tail_slot_stride % e16 == 0 && w16 &&
+              ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(tail)) & 15) == 0;
+  vec8 = vec8 && (dtype != B200_F32 || conv8_four(rows, P.total_heads, max_dim <= 64 ? 8 : (max_dim <= 128 ? 16 : 32)));
+  for (int i = 0; i < n_groups; ++i)
+    vec8 = vec8 && groups[i].dim % 8 == 0 && groups[i].col0 % e16 == 0 && reinterpret_cast<uintptr_t>(groups[i].out) % 16 == 0 &&
+           groups[i].ld_out % (groups[i].out_f32 ? 4 : e16) == 0;
   cudaStream_t st = (cudaStream_t)stream;
   const int4* sq = reinterpret_cast<const int4*>(seqs);
+  if (vec8) {
+    B200_FLOAT_TYPES(dtype, T, {
+      if (max_dim <= 64) B200_CUDA((short_conv8_launch<T, 8>(st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows)));
+      else if (max_dim <= 128) B200_CUDA((short_conv8_launch<T, 16>(st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows)));
+      else B200_CUDA((short_conv8_launch<T, 32>(st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows)));
+    });
+    return B200_OK;
+  }
   B200_FLOAT_TYPES(dtype, T, {
     if (max_dim <= 64) B200_CUDA((short_conv_launch<T, 1>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows, rpw, pairs)));
     else if (max_dim <= 128) B200_CUDA((short_conv_launch<T, 2>(taps, grid, st, (const T*)in, ld_in, P, (const T*)tail, tail_slot_stride, tail_cols, sq, row_seq, rows, rpw, pairs)));
