@@ -8,20 +8,23 @@
 // so everything but S0 is computed for all chunks side by side (delta_chunk_kernel), and what is left to do in order per chunk is three
 // small products on a slice of S0's columns (delta_carry_kernel; the columns never mix).
 //
-// All of it is fp32.  The decays enter as running products, as in the token-by-token walk: no logarithm or quotient is taken, so any decay
-// in [0, 1] is safe.  W, U come from the forward substitution in token order.
+// All numbers are fp32 and products of them are formed on the tensor cores as three products of tf32 halves (tf32x3.cuh).  The decays enter as running
+// products, as in the token-by-token walk: no logarithm or quotient is taken, so any decay in [0, 1] is safe.
+// Error of the read-out and of the state against 64 bits, relative, mean over ten shapes of 64 to 2048 tokens: 2.52e-7 and 2.28e-7; with the products as
+// fp32 multiply-adds 2.60e-7 and 2.62e-7, token by token 2.37e-7 and 2.33e-7.
 //
-// Bound: the carry's chain of chunks, three products and as many barriers each, and the per-chunk work, which fills the GPU.  The walk of
-// delta.cu costs 0.4 us (one decay per head) to 0.65 us (per channel) a token whatever the width: a layer of 16 heads of 128 x 128 with
-// decays per channel takes 1413 us for 2048 tokens with it and 467 us with this one.
+// Bound: the chain of chunks (1.6 us each at sixteen columns a CTA, a third of it tensor pipe, the rest latency between its two products and three
+// barriers), then the per-chunk work (two CTAs an SM; issue slots).  16 heads of 128 x 128 with decays per channel, 2048 tokens: 343 -> 202 us (chunks
+// 155 -> 90, chain 180 -> 108) against all of it in fp32 multiply-adds read from shared memory, 1640 token by token.
 #include "tc05.cuh"
+#include "tf32x3.cuh"
 
 namespace b200 {
 
 namespace {
 
 constexpr int kDcC = 32;            // tokens per chunk
-constexpr int kDcThreads = 128;
+constexpr int kDcChunkThreads = 256;
 constexpr int kDcMinRows = 64;
 
 struct DcArgs {
@@ -36,18 +39,17 @@ struct DcArgs {
   int heads, kv_heads, dk, dv;
   int n_seqs, longs, min_rows;      // sequences, how many of them can have chunks, and from how many rows on they have
   int item0, n_items, most;         // this launch's chunks, counted through all sequences, of `most` in all
-  int dvb;                          // blocks of eight value columns (an even number)
-  float* ws; int64_t item;          // per (chunk, head): W | K | Q, rows of DK + 4 | P (DK) | U [dvb][32][8] | O [dvb][32][8]
+  int dvb;                          // blocks of eight value columns (a multiple of four)
+  float* ws; int64_t item;          // per (chunk, head): W | Q (32 rows of DK) | K by key (DK rows of 32) | P (DK) | U [dvb][32][8] | O [dvb][32][8]
   unsigned* err;
 };
 
 template <int DK>
 struct DcItem {
-  static constexpr int kPitch = DK + 4, kMat = kDcC * kPitch, kHead = 3 * kMat + DK;   // floats; rows four floats apart in their banks
+  static constexpr int kMat = kDcC * DK, kHead = 3 * kMat + DK;   // floats
 };
 
 typedef unsigned long long f2;   // two packed floats
-__device__ __forceinline__ f2 pk2(float a, float b) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ void un2(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
@@ -100,21 +102,49 @@ __device__ __forceinline__ int dc_nth(const DcArgs& A, int z, int& before) {
 }
 
 // One chunk of one head: grid (chunks, heads).  Tokens past the sequence's end count as k = q = v = 0, beta = 0, g = 1.
+//
+// The tokens form four blocks of eight.  Per channel, a decay from token j of an earlier block to token i is the product of the one from j to the end of
+// its block, those of the blocks between, and the one from the start of i's block to i: the pairs of different blocks are then matrix products of scaled
+// rows (16 rows of a tile: eight k, eight q), and only the pairs within a block walk the decays one by one.  With one decay per head all pairs are matrix
+// products of the plain rows and the decay a factor of the result.  T = (1 + beta A)^-1 by forward substitution; W = T (beta P k), U = T (beta v), and
+// B W, B U as (B T) times the same.
+template <int DK>
+struct DcChunk {
+  static constexpr int NW = DK / 16;                     // warps with channels (sixteen each) in A and B
+  static constexpr int kPart = 1280;                     // floats of a warp's share of A and B
+  static constexpr int kPK = DK + 2, kPV = 130;          // pitches of the right-hand sides: the four tokens of a quarter warp on different banks
+  static constexpr int kRhs = kDcC * (kPK + kPV);
+  static constexpr int kScratch = NW * kPart > kRhs ? NW * kPart : kRhs;
+  static constexpr int kFloats = 3 * kDcC * DK + kScratch + 4 * kDcC * kDcC + 4 * DK + 3 * kDcC;
+  static constexpr int kSmem = kFloats * 4;
+};
+
+template <int DK>
+__device__ __forceinline__ int dc_at(int row, int c) { return row * DK + ((((c >> 2) ^ (row >> 3) ^ ((row & 1) << 2)) << 2) | (c & 3)); }
+__device__ __forceinline__ int dc_at32(int row, int c) { return row * kDcC + (x3::unit_row(row, c >> 2) << 2) + (c & 3); }
+
 template <typename T, int DK, bool CHANNEL>
-__global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_kernel(DcArgs A, int vec) {
+__global__ void __launch_bounds__(kDcChunkThreads, 2) delta_chunk_kernel(DcArgs A, int vec, int vec_v) {
   using I = DcItem<DK>;
-  constexpr int C = kDcC, CPW = DK / 4;                 // channels per warp
+  using Y = DcChunk<DK>;
+  constexpr int C = kDcC, NT = kDcChunkThreads;
   extern __shared__ __align__(128) float dc_smem[];
-  float* const ks = dc_smem;                            // [C][DK]
-  float* const qs = ks + C * DK;                        // [C][DK]
-  float* const gs = qs + C * DK;                        // [C][DK] (per channel) or [C]
-  float* const bs = gs + (CHANNEL ? C * DK : C);        // [C]
-  float* const part = bs + C;                           // [4 warps][A, B][C][C]
-  float2* const a2 = reinterpret_cast<float2*>(part + 8 * C * C);   // [C][C]  -beta_i A_ij, twice
-  float2* const b2 = a2 + C * C;                                    // [C][C]  B_ij, twice
+  float* const ks = dc_smem;                            // [C][DK] k; then k P within the block
+  float* const qs = ks + C * DK;                        // [C][DK] q; then q P within the block; then q P
+  float* const gs = qs + C * DK;                        // [C][DK] g; then k times the decay to its block's end   (per head: [C][C] decays R)
+  float* const part = gs + C * DK;                      // [NW][kPart] shares of A and B; then the right-hand sides
+  float* const pk = part;                               // [C][kPK]  beta P k
+  float* const vb = part + C * Y::kPK;                  // [C][kPV]  beta v
+  float* const am = part + Y::kScratch;                 // [C][C]    -beta_i A_ij
+  float* const bm = am + C * C;                         // [C][C]    B_ij
+  float* const tm = bm + C * C;                         // [2 C][C]  T, then B T
+  float* const dd = tm + 2 * C * C;                     // [4][DK]   decays of whole blocks
+  float* const bs = dd + 4 * DK;                        // [C] beta
+  float* const gh = bs + C;                             // [C] g per head
+  float* const ph = gh + C;                             // [C] P per head
   griddep_launch();
   griddep_wait();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
   const int h = blockIdx.y, hk = h / (A.heads / A.kv_heads);
   int chunk;
   const int z = dc_find(A, A.item0 + (int)blockIdx.x, chunk);
@@ -125,200 +155,395 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_kernel(DcArgs A, in
   const int64_t row0 = (int64_t)sq.x + t0;
   const int dk = A.dk, dv = A.dv;
   float* const item = A.ws + ((int64_t)blockIdx.x * A.heads + h) * A.item;
+  bool odd = false;                                     // a number that is not finite
+  auto seen = [&](float x) { odd = odd || !(fabsf(x) <= 3.4028234e38f); };
 
-  // ---- the chunk's keys, queries, decays and write strengths ----
+  // ---- the chunk's keys, queries, decays, values and write strengths: every load is on its way before the first number is used ----
   const float* const kp = A.k + row0 * A.ldk + (int64_t)hk * dk;
   const float* const qp = A.q + row0 * A.ldq + (int64_t)hk * dk;
-#pragma unroll 4
-  for (int i = tid * 4; i < C * DK; i += kDcThreads * 4) {
-    const int t = i / DK, c = i % DK;
-    float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), qv = kv;
-    if (t < nt && c < dk) {
-      if (vec) {
-        kv = *reinterpret_cast<const float4*>(kp + (int64_t)t * A.ldk + c);
-        qv = *reinterpret_cast<const float4*>(qp + (int64_t)t * A.ldq + c);
-      } else {
-        float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (c + e < dk) { a[e] = kp[(int64_t)t * A.ldk + c + e]; b[e] = qp[(int64_t)t * A.ldq + c + e]; }
-        kv = make_float4(a[0], a[1], a[2], a[3]);
-        qv = make_float4(b[0], b[1], b[2], b[3]);
-      }
-    }
-    *reinterpret_cast<float4*>(ks + i) = kv;
-    *reinterpret_cast<float4*>(qs + i) = qv;
-  }
-  const float neg_a = -expf(load_as_float(reinterpret_cast<const T*>(A.a_log), h));
+  const float* const vp = A.v + row0 * A.ldv + (int64_t)h * dv;
   const T* const bias = reinterpret_cast<const T*>(A.dt_bias);
   const T* const dec = reinterpret_cast<const T*>(A.decay_in);
+  constexpr int KN = C * DK / (NT * 4);
+  float4 kv[KN], qv[KN];
+#pragma unroll
+  for (int n = 0; n < KN; ++n) {
+    const int i = tid * 4 + n * NT * 4, t = i / DK, c = i % DK;
+    kv[n] = qv[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < nt && c < dk) {
+      const float *const a = kp + (int64_t)t * A.ldk + c, *const b = qp + (int64_t)t * A.ldq + c;
+      if (vec) {
+        kv[n] = *reinterpret_cast<const float4*>(a);
+        qv[n] = *reinterpret_cast<const float4*>(b);
+      } else {
+        kv[n] = make_float4(a[0], c + 1 < dk ? a[1] : 0.f, c + 2 < dk ? a[2] : 0.f, c + 3 < dk ? a[3] : 0.f);
+        qv[n] = make_float4(b[0], c + 1 < dk ? b[1] : 0.f, c + 2 < dk ? b[2] : 0.f, c + 3 < dk ? b[3] : 0.f);
+      }
+    }
+  }
+  constexpr int STEP = NT / DK, GN = CHANNEL ? C / STEP : 1;   // decays per channel: a thread's channel stays the same
+  const int gc = tid % DK, gt = tid / DK;
+  float x[GN], bc = 0.f;
   if constexpr (CHANNEL) {
-#pragma unroll 4
-    for (int i = tid; i < C * DK; i += kDcThreads) {
-      const int t = i / DK, c = i % DK;
-      float g = 1.f;
-      if (t < nt && c < dk) g = expf(neg_a * dc_softplus(load_as_float(dec, (row0 + t) * A.ld_decay + (int64_t)h * dk + c) + load_as_float(bias, (int64_t)h * dk + c)));
-      gs[i] = g;
+    if (gc < dk) bc = load_as_float(bias, (int64_t)h * dk + gc);
+#pragma unroll
+    for (int n = 0; n < GN; ++n) {
+      const int t = gt + n * STEP;
+      x[n] = t < nt && gc < dk ? load_as_float(dec, (row0 + t) * A.ld_decay + (int64_t)h * dk + gc) : 0.f;
+    }
+  }
+  auto values = [&](int c0, float4 (&v)[4]) {           // columns c0 .. c0 + 127: four of a row per access
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int t = warp + 8 * n, c = c0 + lane * 4;
+      v[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < nt && c < dv) {
+        const float* p = vp + (int64_t)t * A.ldv + c;
+        if (vec_v) v[n] = *reinterpret_cast<const float4*>(p);
+        else v[n] = make_float4(p[0], c + 1 < dv ? p[1] : 0.f, c + 2 < dv ? p[2] : 0.f, c + 3 < dv ? p[3] : 0.f);
+      }
+    }
+  };
+  auto put_values = [&](const float4 (&v)[4]) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int t = warp + 8 * n;
+      const float b = bs[t];
+      float* const d = vb + t * Y::kPV + lane * 4;
+      *reinterpret_cast<float2*>(d) = make_float2(b * v[n].x, b * v[n].y);
+      *reinterpret_cast<float2*>(d + 2) = make_float2(b * v[n].z, b * v[n].w);
+    }
+  };
+  float4 v0[4];
+  values(0, v0);
+  const float neg_a = -expf(load_as_float(reinterpret_cast<const T*>(A.a_log), h));
+  if constexpr (CHANNEL) {
+#pragma unroll
+    for (int n = 0; n < GN; ++n) {
+      const int t = gt + n * STEP;
+      const float g = t < nt && gc < dk ? expf(neg_a * dc_softplus(x[n] + bc)) : 1.f;
+      seen(g);
+      gs[dc_at<DK>(t, gc)] = g;
     }
   } else if (tid < C) {
-    gs[tid] = tid < nt ? expf(neg_a * dc_softplus(load_as_float(dec, (row0 + tid) * A.ld_decay + h) + load_as_float(bias, h))) : 1.f;
+    const float g = tid < nt ? expf(neg_a * dc_softplus(load_as_float(dec, (row0 + tid) * A.ld_decay + h) + load_as_float(bias, h))) : 1.f;
+    seen(g);
+    gh[tid] = g;
   }
-  if (tid < C) bs[tid] = tid < nt ? 1.0f / (1.0f + expf(-load_as_float(reinterpret_cast<const T*>(A.beta_in), (row0 + tid) * A.ld_beta + h))) : 0.f;
+  if (tid < C) {
+    const float b = tid < nt ? 1.0f / (1.0f + expf(-load_as_float(reinterpret_cast<const T*>(A.beta_in), (row0 + tid) * A.ld_beta + h))) : 0.f;
+    seen(b);
+    bs[tid] = b;
+  }
+#pragma unroll
+  for (int n = 0; n < KN; ++n) {
+    const int i = tid * 4 + n * NT * 4, t = i / DK, c = i % DK;
+    seen(kv[n].x + kv[n].y + kv[n].z + kv[n].w);
+    seen(qv[n].x + qv[n].y + qv[n].z + qv[n].w);
+    *reinterpret_cast<float4*>(ks + dc_at<DK>(t, c)) = kv[n];
+    *reinterpret_cast<float4*>(qs + dc_at<DK>(t, c)) = qv[n];
+  }
+#pragma unroll
+  for (int n = 0; n < 4; ++n) seen(v0[n].x + v0[n].y + v0[n].z + v0[n].w);
   __syncthreads();
 
-  // ---- A and B: lane j carries R_ij k_j in this warp's channels from token to token ----
-  {
-    f2 r[CPW / 2];
-    float rs = 0.f;
+  // ---- A and B, a warp's sixteen channels ----
+  if (warp < Y::NW) {
+    float* const mine = part + warp * Y::kPart;
+    if constexpr (CHANNEL) {
+      // pairs within a block: lane j carries R_ij k_j from token to token.  [block][A, B][i][j]
+      const int b = lane >> 3, jl = lane & 7;
+      f2 r[8];
 #pragma unroll
-    for (int p = 0; p < CPW / 2; ++p) r[p] = 0ull;
-    if constexpr (!CHANNEL) {
-#pragma unroll
-      for (int p = 0; p < CPW / 2; ++p) r[p] = *reinterpret_cast<const f2*>(ks + lane * DK + warp * CPW + 2 * p);
-    }
+      for (int p = 0; p < 8; ++p) r[p] = 0ull;
 #pragma unroll 1
-    for (int i = 0; i < C; ++i) {
-      const int at = i * DK + warp * CPW;
-      f2 a = 0ull, b = 0ull, a_ = 0ull, b_ = 0ull;
+      for (int il = 0; il < 8; ++il) {
+        f2 a = 0ull, c = 0ull, a_ = 0ull, c_ = 0ull;
 #pragma unroll
-      for (int p = 0; p < CPW / 2; p += 2) {
-        const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(ks + at + 2 * p), qq = *reinterpret_cast<const ulonglong2*>(qs + at + 2 * p);
-        if constexpr (CHANNEL) {
-          const ulonglong2 gg = *reinterpret_cast<const ulonglong2*>(gs + at + 2 * p);
-          r[p] = lane == i ? kk.x : mul2(r[p], gg.x);
-          r[p + 1] = lane == i ? kk.y : mul2(r[p + 1], gg.y);
+        for (int e = 0; e < 4; ++e) {
+          const int at = dc_at<DK>(8 * b + il, warp * 16 + 4 * e);
+          const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(ks + at), qq = *reinterpret_cast<const ulonglong2*>(qs + at),
+                           gg = *reinterpret_cast<const ulonglong2*>(gs + at);
+          r[2 * e] = jl == il ? kk.x : mul2(r[2 * e], gg.x);
+          r[2 * e + 1] = jl == il ? kk.y : mul2(r[2 * e + 1], gg.y);
+          a = fma2(kk.x, r[2 * e], a);
+          c = fma2(qq.x, r[2 * e], c);
+          a_ = fma2(kk.y, r[2 * e + 1], a_);
+          c_ = fma2(qq.y, r[2 * e + 1], c_);
         }
-        a = fma2(kk.x, r[p], a);
-        b = fma2(qq.x, r[p], b);
-        a_ = fma2(kk.y, r[p + 1], a_);
-        b_ = fma2(qq.y, r[p + 1], b_);
+        mine[b * 128 + il * 8 + jl] = sum2(a) + sum2(a_);
+        mine[b * 128 + 64 + il * 8 + jl] = sum2(c) + sum2(c_);
       }
-      float sa = sum2(a) + sum2(a_), sb = sum2(b) + sum2(b_);
-      if constexpr (!CHANNEL) {
-        rs = lane == i ? 1.f : rs * gs[i];
-        sa *= rs;
-        sb *= rs;
-      }
-      part[(warp * 2 * C + i) * C + lane] = sa;
-      part[(warp * 2 * C + C + i) * C + lane] = sb;
     }
-    // K: what the write of token j leaves at the chunk's end
-    float* const kh = item + I::kMat + lane * I::kPitch + warp * CPW;
+  }
+  if constexpr (CHANNEL) {
+    __syncthreads();
+    for (int n = tid; n < 4 * DK; n += NT) {
+      const int c = n % DK, b = n / DK;
+      float k[8], g[8];
 #pragma unroll
-    for (int p = 0; p < CPW / 2; p += 2) {
-      const f2 m = CHANNEL ? 0ull : pk2(rs, rs);
-      *reinterpret_cast<ulonglong2*>(kh + 2 * p) = CHANNEL ? make_ulonglong2(r[p], r[p + 1]) : make_ulonglong2(mul2(r[p], m), mul2(r[p + 1], m));
+      for (int e = 0; e < 8; ++e) { k[e] = ks[dc_at<DK>(8 * b + e, c)]; g[e] = gs[dc_at<DK>(8 * b + e, c)]; }
+      float cum = 1.f, rest = 1.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        cum *= g[e];
+        ks[dc_at<DK>(8 * b + e, c)] = k[e] * cum;
+        qs[dc_at<DK>(8 * b + e, c)] *= cum;
+      }
+#pragma unroll
+      for (int e = 7; e >= 0; --e) {
+        gs[dc_at<DK>(8 * b + e, c)] = k[e] * rest;
+        rest *= g[e];
+      }
+      dd[b * DK + c] = cum;
+    }
+    __syncthreads();
+  } else if (warp == 7) {   // decays per head: R_ij, P_i
+    float r = 0.f, p = 1.f;
+    for (int i = 0; i < C; ++i) {
+      const float g = gh[i];
+      p *= g;
+      r = lane == i ? 1.f : r * g;
+      gs[i * C + lane] = r;
+      if (lane == i) ph[i] = p;
+    }
+  }
+  if (warp < Y::NW) {
+    // pairs of different blocks (per head: of all blocks up to the row's own): rows g8 of a tile are k, rows g8 + 8 are q
+    float* const mine = part + warp * Y::kPart + (CHANNEL ? 512 : 0);
+    const int c = warp * 16 + 4 * t4;
+    const float* const rhs = CHANNEL ? gs : ks;
+    int tile = 0;
+#pragma unroll
+    for (int bi = CHANNEL ? 1 : 0; bi < 4; ++bi) {
+      x3::Split<8> a;
+      a.set4(0, *reinterpret_cast<const float4*>(ks + dc_at<DK>(8 * bi + g8, c)));
+      a.set4(4, *reinterpret_cast<const float4*>(qs + dc_at<DK>(8 * bi + g8, c)));
+#pragma unroll
+      for (int bj = 0; bj < (CHANNEL ? bi : bi + 1); ++bj, ++tile) {
+        float4 r = *reinterpret_cast<const float4*>(rhs + dc_at<DK>(8 * bj + g8, c));
+        if constexpr (CHANNEL) {
+#pragma unroll
+          for (int m = bj + 1; m < bi; ++m) {
+            const float4 f = *reinterpret_cast<const float4*>(dd + m * DK + c);
+            r.x *= f.x; r.y *= f.y; r.z *= f.z; r.w *= f.w;
+          }
+        }
+        x3::Split<4> b;
+        b.set4(0, r);
+        float d[4];
+        x3::mma16(d, a, b);
+        *reinterpret_cast<float2*>(mine + tile * 128 + g8 * 8 + 2 * t4) = make_float2(d[0], d[1]);
+        *reinterpret_cast<float2*>(mine + tile * 128 + 64 + g8 * 8 + 2 * t4) = make_float2(d[2], d[3]);
+      }
     }
   }
   __syncthreads();
-  for (int i = tid; i < C * C; i += kDcThreads) {
-    const int t = i / C, j = i % C;
+#pragma unroll 1
+  for (int n = tid; n < C * C; n += NT) {
+    const int t = n / C, j = n % C, bi = t >> 3, bj = j >> 3;
     float sa = 0.f, sb = 0.f;
+    if (j <= t) {
+      const int tile = CHANNEL ? (bi == bj ? bi : 4 + bi * (bi - 1) / 2 + bj) : bi * (bi + 1) / 2 + bj;
+      const float* const p = part + tile * 128 + (t & 7) * 8 + (j & 7);
 #pragma unroll
-    for (int w = 0; w < 4; ++w) { sa += part[w * 2 * C * C + i]; sb += part[(w * 2 + 1) * C * C + i]; }
-    const float a = j < t ? -bs[t] * sa : 0.f, b = j <= t ? sb : 0.f;
-    a2[i] = make_float2(a, a);
-    b2[i] = make_float2(b, b);
-  }
-  // ---- decays from the chunk's start: k becomes beta P k (the right-hand side of W), q becomes P q ----
-  for (int c = tid; c < DK; c += kDcThreads) {
-    float cum = 1.f;
-#pragma unroll 4
-    for (int i = 0; i < C; ++i) {
-      cum *= CHANNEL ? gs[i * DK + c] : gs[i];
-      ks[i * DK + c] *= bs[i] * cum;
-      qs[i * DK + c] *= cum;
+      for (int w = 0; w < Y::NW; ++w) { sa += p[w * Y::kPart]; sb += p[w * Y::kPart + 64]; }
+      if constexpr (!CHANNEL) { const float r = gs[t * C + j]; sa *= r; sb *= r; }
     }
-    item[3 * I::kMat + c] = cum;
+    am[n] = j < t ? -bs[t] * sa : 0.f;
+    bm[dc_at32(t, j)] = sb;
+  }
+  odd = __syncthreads_or(odd) != 0;
+
+  // ---- T in one warp; the right-hand sides, K and P in the others ----
+  put_values(v0);
+  if (warp == 0) {
+    float x[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      float s = lane == i ? 1.f : 0.f, s_ = 0.f;
+#pragma unroll
+      for (int l = 0; l < i; l += 4) {
+        const float4 m = *reinterpret_cast<const float4*>(am + i * C + l);
+        if (l < i) s = fmaf(m.x, x[l], s);
+        if (l + 1 < i) s_ = fmaf(m.y, x[l + 1], s_);
+        if (l + 2 < i) s = fmaf(m.z, x[l + 2], s);
+        if (l + 3 < i) s_ = fmaf(m.w, x[l + 3], s_);
+      }
+      x[i] = lane <= i ? s + s_ : 0.f;
+      tm[dc_at32(i, lane)] = x[i];
+    }
+  } else {
+    for (int n = tid - 32; n < 4 * DK; n += NT - 32) {
+      const int c = n % DK, b = n / DK;
+      float before = 1.f, after = 1.f;
+      if constexpr (CHANNEL) {
+        for (int m = 0; m < b; ++m) before *= dd[m * DK + c];
+        for (int m = b + 1; m < 4; ++m) after *= dd[m * DK + c];
+      }
+      float kl[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = 8 * b + e, at = dc_at<DK>(i, c);
+        if constexpr (!CHANNEL) { before = ph[i]; after = gs[(C - 1) * C + i]; }
+        const float kv = ks[at];
+        kl[e] = (CHANNEL ? gs[at] : kv) * after;
+        pk[i * Y::kPK + c] = kv * before * bs[i];
+        qs[at] *= before;
+      }
+      float* const kt = item + 2 * I::kMat + c * C;
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        *reinterpret_cast<float4*>(kt + (x3::unit_row(c, 2 * b + u) << 2)) = make_float4(kl[4 * u], kl[4 * u + 1], kl[4 * u + 2], kl[4 * u + 3]);
+      if (b == 3) item[3 * I::kMat + c] = CHANNEL ? before * dd[3 * DK + c] : ph[C - 1];
+    }
   }
   __syncthreads();
 
-  // ---- forward substitution, two columns per thread: the columns of W, then those of U ----
+  // ---- B T: a tile of sixteen rows and eight columns per warp ----
+  auto dot = [&](const float* m, int i, const float* x, int pitch) {   // sum over j <= i of m_ij x_j, in order: nothing of a later token enters
+    float s = 0.f;
+    for (int j = 0; j <= i; ++j) s = fmaf(m[dc_at32(i, j)], x[j * pitch], s);
+    return s;
+  };
+  if (odd) {
+    for (int n = tid; n < C * C; n += NT) {
+      const int i = n / C, j = n % C;
+      float s = 0.f;
+      for (int l = j; l <= i; ++l) s = fmaf(bm[dc_at32(i, l)], tm[dc_at32(l, j)], s);
+      tm[dc_at32(C + i, j)] = s;
+    }
+  } else {
+    const int mt = warp & 1, col = (warp >> 1) * 8 + g8;
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int kk = 0; kk <= mt; ++kk) {
+      x3::Split<8> a;
+      x3::Split<4> b;
+      a.set4(0, *reinterpret_cast<const float4*>(bm + dc_at32(16 * mt + g8, 16 * kk + 4 * t4)));
+      a.set4(4, *reinterpret_cast<const float4*>(bm + dc_at32(16 * mt + g8 + 8, 16 * kk + 4 * t4)));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) b.set(e, tm[dc_at32(16 * kk + 4 * t4 + e, col)]);
+      float s[4];
+      x3::mma16(s, a, b);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d[e] += s[e];
+    }
+    const int c = (warp >> 1) * 8 + 2 * t4, row = C + 16 * mt + g8;
+    *reinterpret_cast<float2*>(tm + dc_at32(row, c)) = make_float2(d[0], d[1]);
+    *reinterpret_cast<float2*>(tm + dc_at32(row + 8, c)) = make_float2(d[2], d[3]);
+  }
+  __syncthreads();
+
+  // ---- [T; B T] times the right-hand sides: W, U and, from B T, Q = P q - B W and O ----
   float* const uo = item + I::kHead;
   const int64_t o_off = (int64_t)A.dvb * C * 8;
-  const int pairs = DK / 2 + A.dvb * 4;
-  for (int p = tid; p < pairs; p += kDcThreads) {
-    const bool is_w = p < DK / 2;
-    const int vc = 2 * (p - DK / 2);
-    f2 x[C];
-    if (is_w) {
-#pragma unroll
-      for (int i = 0; i < C; ++i) x[i] = *reinterpret_cast<const f2*>(ks + i * DK + 2 * p);
+  auto keys_at = [](int row, int c) { return row * DK + (x3::unit_row(row, c >> 2) << 2) + (c & 3); };
+  for (int c0 = 0;; c0 += 128) {                        // blocks of 128 value columns; the key columns go with the first
+    const int vn = min(128, A.dvb * 8 - c0), first = c0 == 0 ? 0 : DK, cols = DK + vn;
+    if (odd) {
+      for (int n = first * C + tid; n < cols * C; n += NT) {
+        const int i = n % C, c = n / C;
+        const float* const x = c < DK ? pk + c : vb + c - DK;
+        const int pitch = c < DK ? Y::kPK : Y::kPV;
+        const float t = dot(tm, i, x, pitch), y = dot(tm + C * C, i, x, pitch);
+        if (c < DK) {
+          item[keys_at(i, c)] = t;
+          item[I::kMat + keys_at(i, c)] = qs[dc_at<DK>(i, c)] - y;
+        } else {
+          float* const d = uo + ((c0 + c - DK) >> 3) * (C * 8) + i * 8 + ((c - DK) & 7);
+          d[0] = t;
+          d[o_off] = y;
+        }
+      }
     } else {
-      const float* vp = A.v + row0 * A.ldv + (int64_t)h * dv + vc;
+      for (int p = first / 16 + warp; p < cols / 16; p += NT / 32) {   // sixteen columns at a time
+        const bool keys = p * 16 < DK;
+        const float* const src = keys ? pk + p * 16 : vb + p * 16 - DK;
+        const int pitch = keys ? Y::kPK : Y::kPV;
+        x3::Split<4> b[2][2];
 #pragma unroll
-      for (int i = 0; i < C; ++i) {
-        const float b = bs[i];
-        x[i] = pk2(i < nt && vc < dv ? b * vp[(int64_t)i * A.ldv] : 0.f, i < nt && vc + 1 < dv ? b * vp[(int64_t)i * A.ldv + 1] : 0.f);
+        for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) b[kk][n].set(e, src[(16 * kk + 4 * t4 + e) * pitch + 8 * n + g8]);
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) {
+          float d[2][4];
+#pragma unroll
+          for (int kk = 0; kk <= (mt & 1); ++kk) {
+            x3::Split<8> a;
+            a.set4(0, *reinterpret_cast<const float4*>(tm + dc_at32(16 * mt + g8, 16 * kk + 4 * t4)));
+            a.set4(4, *reinterpret_cast<const float4*>(tm + dc_at32(16 * mt + g8 + 8, 16 * kk + 4 * t4)));
+            float s[2][4];
+            x3::mma16<2>(s, {&a, &a}, {&b[kk][0], &b[kk][1]});
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) d[n][e] = kk == 0 ? s[n][e] : d[n][e] + s[n][e];
+          }
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const int i = 16 * (mt & 1) + g8 + 8 * r, c = p * 16 + 8 * n + 2 * t4;
+              float2 y = make_float2(d[n][2 * r], d[n][2 * r + 1]);
+              if (keys) {
+                if (mt >= 2) {
+                  const float2 x = *reinterpret_cast<const float2*>(qs + dc_at<DK>(i, c));
+                  y = make_float2(x.x - y.x, x.y - y.y);
+                }
+                *reinterpret_cast<float2*>(item + (mt >= 2 ? I::kMat : 0) + keys_at(i, c)) = y;
+              } else {
+                *reinterpret_cast<float2*>(uo + (mt >= 2 ? o_off : 0) + ((c0 + c - DK) >> 3) * (C * 8) + i * 8 + 2 * t4) = y;
+              }
+            }
+        }
       }
     }
+    if (c0 + 128 >= A.dvb * 8) break;
+    values(c0 + 128, v0);
 #pragma unroll
-    for (int i = 1; i < C; ++i) {
-#pragma unroll
-      for (int j = 0; j + 1 < i; j += 2) {
-        const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(a2 + i * C + j);
-        x[i] = fma2(m.x, x[j], x[i]);
-        x[i] = fma2(m.y, x[j + 1], x[i]);
-      }
-      if (i & 1) x[i] = fma2(*reinterpret_cast<const f2*>(a2 + i * C + i - 1), x[i - 1], x[i]);
-    }
-    float* const dst = is_w ? item + 2 * p : uo + (int64_t)(vc >> 3) * C * 8 + (vc & 7);
-    const int pitch = is_w ? I::kPitch : 8;
-#pragma unroll
-    for (int i = 0; i < C; ++i) *reinterpret_cast<f2*>(dst + i * pitch) = x[i];
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      f2 y = 0ull, z = 0ull;
-#pragma unroll
-      for (int j = 0; j < i; j += 2) {   // pairs (j, j + 1); the last pair of an odd row ends with B_ii
-        const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(b2 + i * C + j);
-        y = fma2(m.x, x[j], y);
-        z = fma2(m.y, x[j + 1], z);
-      }
-      if (!(i & 1)) y = fma2(*reinterpret_cast<const f2*>(b2 + i * C + i), x[i], y);
-      float y0, y1, z0, z1;
-      un2(y, y0, y1);
-      un2(z, z0, z1);
-      y0 += z0;
-      y1 += z1;
-      if (is_w) {
-        const float2 qh = *reinterpret_cast<const float2*>(qs + i * DK + 2 * p);
-        *reinterpret_cast<float2*>(dst + 2 * I::kMat + i * pitch) = make_float2(qh.x - y0, qh.y - y1);
-      } else {
-        *reinterpret_cast<float2*>(dst + o_off + i * pitch) = make_float2(y0, y1);
-      }
-    }
+    for (int n = 0; n < 4; ++n) seen(v0[n].x + v0[n].y + v0[n].z + v0[n].w);
+    odd = __syncthreads_or(odd) != 0;                   // (this block's columns have been read, too)
+    put_values(v0);
+    __syncthreads();
   }
 }
 
-// The state through the chunks, in order: grid (slices of NC value columns, heads, sequences that can have chunks), 16 NC threads.  Chunk c + 1 is on its way into
-// the second stage (bulk copies) while chunk c is worked on; the slice of S lies in shared memory by column, so that four keys' numbers are
-// one access for either factor of W S and Q S.
-template <int DK, int NC>
+// The state through the chunks, in order: grid (slices of NC = 8 NT G value columns, heads, sequences that can have chunks).  The next chunks are on their
+// way (bulk copies) while one is worked on.  G groups of eight warps have 8 NT columns each and go their own way through the same chunks, so that one
+// group's products fill the other's waits.  The slice of S lies in registers as the accumulators of K^T u, sixteen keys a warp, and for W S and Q S in
+// shared memory by column as hi and lo; those two are tiles of sixteen tokens, half of the keys per warp.
+template <int DK, int NT, int G>
 struct DcCarry {
   using I = DcItem<DK>;
-  static constexpr int kThreads = 16 * NC;
-  static constexpr int kSlice = kDcC * NC;                         // floats of U (of O) per chunk and slice
+  static constexpr int NC = 8 * NT, kThreads = 256 * G, kStages = 3;
+  static constexpr int kSlice = kDcC * NC * G;                     // floats of U (of O) per chunk and slice
   static constexpr int kStage = I::kHead + 2 * kSlice;             // floats
-  static constexpr int kFloats = 2 * kStage + NC * I::kPitch + 8 * (kThreads / 2) + 2 * kDcC * NC;
+  static constexpr int kGroup = 2 * NC * DK + 2 * kDcC * NC + 4 * NT * 128;
+  static constexpr int kFloats = kStages * kStage + G * kGroup;
   static constexpr int kSmem = kFloats * 4;
 };
 
-template <int DK, int NC>
-__global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
+template <int DK, int NT, int G>
+__global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L, int vec_o) {
   using I = DcItem<DK>;
-  using Y = DcCarry<DK, NC>;
-  constexpr int C = kDcC, PT = I::kPitch, TILES = Y::kThreads / 2, CG = NC / 4;
+  using Y = DcCarry<DK, NT, G>;
+  constexpr int C = kDcC, NC = Y::NC, STAGES = Y::kStages, KK = DK / 16;   // KK: tiles of sixteen keys
   extern __shared__ __align__(128) float dc_smem[];
-  float* const st = dc_smem + 2 * Y::kStage;            // S by column: [NC][DK + 4]
-  float* const red = st + NC * PT;                      // [2][TILES] float4: the second half's sums
-  float2* const u2 = reinterpret_cast<float2*>(red + 8 * TILES);   // [C][NC] u, twice
-  __shared__ __align__(8) uint64_t s_full[2];
-  const int tid = threadIdx.x, h = blockIdx.y, col0 = (int)blockIdx.x * NC;
+  __shared__ __align__(8) uint64_t s_full[STAGES];
+  __shared__ unsigned s_done[STAGES];                   // groups that are done with the stage, ever
+  __shared__ int s_gave_up;
+  const int tid = threadIdx.x & 255, group = threadIdx.x >> 8, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, h = blockIdx.y;
+  const int col0 = ((int)blockIdx.x * G + group) * NC;
+  float* const st = dc_smem + STAGES * Y::kStage + group * Y::kGroup;   // S by column, as hi and lo: 2 x [NC][DK]
+  float* const ut = st + 2 * NC * DK;                   // u by column: 2 x [NC][C]
+  float* const red = ut + 2 * C * NC;                   // [4][NT][32] float4: the second half's sums
   const uint32_t full = tc::smem_u32(s_full);
-  if (tid == 0) {
-    tc::mbar_init(full, 1);
-    tc::mbar_init(full + 8, 1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) { tc::mbar_init(full + 8 * i, 1); s_done[i] = 0u; }
+    s_gave_up = 0;
     tc::mbar_init_fence();
   }
   griddep_launch();
@@ -329,155 +554,218 @@ __global__ void __launch_bounds__(16 * NC) delta_carry_kernel(DcArgs A, int L) {
   const int4 sq = A.seqs[z];
   const int all = dc_chunks(A, sq);
   const int c_first = max(0, A.item0 - before), chunks = min(all, A.item0 + A.n_items - before) - c_first, t_first = c_first * C;
-  if (tid == 0 && before + all > A.most) *A.err = 1u;   // more rows than the caller said
+  if (threadIdx.x == 0 && before + all > A.most) *A.err = 1u;   // more rows than the caller said
   if (chunks <= 0) return;
   const int dk = A.dk, dv = A.dv;
   const float* const items = A.ws + ((int64_t)(before + c_first - A.item0) * A.heads + h) * A.item;
   const int64_t step = (int64_t)A.heads * A.item;
+  const int block0 = (int)blockIdx.x * G * NT;          // of eight columns
 
   auto fetch = [&](int c) {   // one thread
     const float* src = items + c * step;
-    const uint32_t bar = full + 8 * (c & 1), dst = tc::smem_u32(dc_smem + (c & 1) * Y::kStage);
+    const uint32_t bar = full + 8 * (c % STAGES), dst = tc::smem_u32(dc_smem + (c % STAGES) * Y::kStage);
     tc::mbar_expect_tx(bar, Y::kStage * 4);
     auto copy = [&](uint32_t to, const float* from, uint32_t bytes) {
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to), "l"(from), "r"(bytes), "r"(bar) : "memory");
     };
     copy(dst, src, I::kHead * 4);
-    copy(dst + I::kHead * 4, src + I::kHead + (int64_t)(col0 >> 3) * C * 8, Y::kSlice * 4);
-    copy(dst + (I::kHead + Y::kSlice) * 4, src + I::kHead + (int64_t)(A.dvb + (col0 >> 3)) * C * 8, Y::kSlice * 4);
+    copy(dst + I::kHead * 4, src + I::kHead + (int64_t)block0 * C * 8, Y::kSlice * 4);
+    copy(dst + (I::kHead + Y::kSlice) * 4, src + I::kHead + (int64_t)(A.dvb + block0) * C * 8, Y::kSlice * 4);
   };
-  if (tid == 0) {
-    fetch(0);
-    if (chunks > 1) fetch(1);
+  auto group_sync = [&] { asm volatile("bar.sync %0, 256;" ::"r"(group + 1) : "memory"); };
+  if (threadIdx.x == 0) {
+    for (int c = 0; c < STAGES && c < chunks; ++c) fetch(c);
   }
   const int krows = (dk + L - 1) / L;
   float* const slot = A.state + (int64_t)sq.w * A.state_slot_stride + (int64_t)h * krows * L * dv;
   const bool from_slot = sq.z > 0 || c_first > 0;
-  for (int i = tid; i < DK * NC; i += Y::kThreads) {
+  auto at = [](int n, int c) { return n * DK + (x3::unit_col(n, c >> 2) << 2) + (c & 3); };
+  auto put = [](float* p, int plane, int i, float x) {
+    x3::Split<1> v;
+    v.set(0, x);
+    p[i] = __uint_as_float(v.hi[0]);
+    p[plane + i] = __uint_as_float(v.lo[0]);
+  };
+  for (int i = tid; i < DK * NC; i += 256) {
     const int n = i % NC, c = i / NC;
-    st[n * PT + c] = from_slot && c < dk && col0 + n < dv ? slot[((int64_t)(c / L) * dv + col0 + n) * L + c % L] : 0.f;
+    put(st, NC * DK, at(n, c), from_slot && c < dk && col0 + n < dv ? slot[((int64_t)(c / L) * dv + col0 + n) * L + c % L] : 0.f);
   }
-  // W S and Q S: a thread has row `rp` of both, columns cg + CG {0 .. 3}, half of the keys
-  const int half = tid / TILES, tile = tid % TILES, cg = tile % CG, rp = tile / CG;
-  // K^T u: four keys, two columns
-  const int kc = (tid % (DK / 4)) * 4, n0 = (tid / (DK / 4)) * 2;
-  constexpr int NSTEP = Y::kThreads / (DK / 4) * 2;    // columns covered at a time
-  bool ok = true;
   __syncthreads();
+  const bool mine = warp < KK;
+  const int key = 16 * warp + g;                        // K^T u: keys key, key + 8
+  const int mt = warp & 3, kh = warp >> 2, row = 16 * (mt & 1) + g;   // W S, Q S: tokens row, row + 8 of W (mt < 2) or Q, keys of half kh
+  float S[NT][4];                                       // columns 8 n + 2 t4, + 1
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = at(8 * n + 2 * t4 + (e & 1), key + 8 * (e >> 1));
+      S[n][e] = mine ? st[i] + st[NC * DK + i] : 0.f;
+    }
+  bool ok = true;
   for (int c = 0; c < chunks; ++c) {
-    const float* const sg = dc_smem + (c & 1) * Y::kStage;
-    ok = __syncthreads_and(tc::mbar_wait(full + 8 * (c & 1), (uint32_t)(c >> 1) & 1u)) != 0;
-    if (!ok) {   // given up: let the copies of this and the next chunk land before leaving
-      if (tid == 0) {
-        tc::mbar_wait(full + 8 * (c & 1), (uint32_t)(c >> 1) & 1u);
-        if (c + 1 < chunks) tc::mbar_wait(full + 8 * ((c + 1) & 1), (uint32_t)((c + 1) >> 1) & 1u);
-      }
-      break;
-    }
-    {
-      f2 w[4], o[4];
+    const float* const sg = dc_smem + (c % STAGES) * Y::kStage;
+    if (!tc::mbar_wait(full + 8 * (c % STAGES), (uint32_t)(c / STAGES) & 1u)) *(volatile int*)&s_gave_up = 1;
+    float acc[NT][4];
+    const float* const wr = sg + (mt >> 1) * I::kMat + row * DK;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) w[e] = o[e] = 0ull;
-      const float* const wr = sg + rp * PT + half * (DK / 2);
-      const float* const qr = wr + 2 * I::kMat;
-      const float* const sc = st + cg * PT + half * (DK / 2);
-#pragma unroll 4
-      for (int k = 0; k < DK / 2; k += 4) {
-        const ulonglong2 w4 = *reinterpret_cast<const ulonglong2*>(wr + k), q4 = *reinterpret_cast<const ulonglong2*>(qr + k);
+    for (int k0 = 0; k0 < KK / 2; k0 += 2) {            // two tiles of keys at a time
+      x3::Split<8> a[2];
+      x3::Split<4> b[2 * NT];
+      const x3::Split<8>* pa[2 * NT];
+      const x3::Split<4>* pb[2 * NT];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int u = 4 * (kh * (KK / 2) + k0 + k) + t4;
+        a[k].set4(0, *reinterpret_cast<const float4*>(wr + (x3::unit_row(row, u) << 2)));
+        a[k].set4(4, *reinterpret_cast<const float4*>(wr + 8 * DK + (x3::unit_row(row, u) << 2)));
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          const float* const p = st + (8 * n + g) * DK + (x3::unit_col(g, u) << 2);
+          b[k * NT + n].load4(0, p, p + NC * DK);
+          pa[k * NT + n] = &a[k];
+          pb[k * NT + n] = &b[k * NT + n];
+        }
+      }
+      float s[2 * NT][4];
+      x3::mma16<2 * NT>(s, pa, pb);
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const ulonglong2 s4 = *reinterpret_cast<const ulonglong2*>(sc + e * CG * PT + k);
-          w[e] = fma2(w4.x, s4.x, w[e]);
-          o[e] = fma2(q4.x, s4.x, o[e]);
-          w[e] = fma2(w4.y, s4.y, w[e]);
-          o[e] = fma2(q4.y, s4.y, o[e]);
+          const float x = s[n][e] + s[NT + n][e];
+          acc[n][e] = k0 == 0 ? x : acc[n][e] + x;
         }
-      }
-      const float4 sw = make_float4(sum2(w[0]), sum2(w[1]), sum2(w[2]), sum2(w[3])), so = make_float4(sum2(o[0]), sum2(o[1]), sum2(o[2]), sum2(o[3]));
-      float4* const rd = reinterpret_cast<float4*>(red);
-      if (half == 1) {
-        rd[tile] = sw;
-        rd[TILES + tile] = so;
-      }
-      __syncthreads();
-      if (half == 0) {
-        const float4 a = rd[tile], b = rd[TILES + tile];
-        const float uw[4] = {sw.x + a.x, sw.y + a.y, sw.z + a.z, sw.w + a.w}, oq[4] = {so.x + b.x, so.y + b.y, so.z + b.z, so.w + b.w};
-        const int t = t_first + c * C + rp;
-        float* const orow = A.out + ((int64_t)sq.x + t) * A.ldo + (int64_t)h * dv;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int n = cg + e * CG, at = I::kHead + (n >> 3) * C * 8 + rp * 8 + (n & 7);
-          const float u = sg[at] - uw[e];
-          u2[rp * NC + n] = make_float2(u, u);
-          if (t < sq.y && col0 + n < dv) orow[col0 + n] = sg[at + Y::kSlice] + oq[e];
-        }
-      }
-      __syncthreads();
     }
-    {
-      const float* const kr = sg + I::kMat + kc;
-      const ulonglong2 p4 = *reinterpret_cast<const ulonglong2*>(sg + 3 * I::kMat + kc);
+    float4* const rd = reinterpret_cast<float4*>(red) + mt * NT * 32 + lane;
+    if (kh == 1) {
 #pragma unroll
-      for (int n = n0; n < NC; n += NSTEP) {
-        float* const s0 = st + n * PT + kc;
-        ulonglong2 a = *reinterpret_cast<const ulonglong2*>(s0), b = *reinterpret_cast<const ulonglong2*>(s0 + PT);
-        a.x = mul2(a.x, p4.x); a.y = mul2(a.y, p4.y); b.x = mul2(b.x, p4.x); b.y = mul2(b.y, p4.y);
-#pragma unroll 8
-        for (int j = 0; j < C; ++j) {
-          const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kr + j * PT), uu = *reinterpret_cast<const ulonglong2*>(u2 + j * NC + n);
-          a.x = fma2(k4.x, uu.x, a.x); a.y = fma2(k4.y, uu.x, a.y);
-          b.x = fma2(k4.x, uu.y, b.x); b.y = fma2(k4.y, uu.y, b.y);
+      for (int n = 0; n < NT; ++n) rd[n * 32] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+    }
+    group_sync();
+    if (*(volatile int*)&s_gave_up) { ok = false; break; }
+    if (kh == 0) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const float4 x = rd[n * 32];
+        const float y[4] = {acc[n][0] + x.x, acc[n][1] + x.y, acc[n][2] + x.z, acc[n][3] + x.w};
+        const float* const uo = sg + I::kHead + (mt >= 2 ? Y::kSlice : 0) + (group * NT + n) * C * 8 + 2 * t4;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int tok = row + 8 * r;
+          const float2 f = *reinterpret_cast<const float2*>(uo + tok * 8);
+          if (mt < 2) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) put(ut, C * NC, (8 * n + 2 * t4 + e) * C + (x3::unit_col(2 * t4 + e, tok >> 2) << 2) + (tok & 3), (e ? f.y : f.x) - y[2 * r + e]);
+          } else {
+            const int t = t_first + c * C + tok, col = col0 + 8 * n + 2 * t4;
+            float* const o = A.out + ((int64_t)sq.x + t) * A.ldo + (int64_t)h * dv + col;
+            if (t < sq.y) {
+              if (vec_o && col < dv) *reinterpret_cast<float2*>(o) = make_float2(f.x + y[2 * r], f.y + y[2 * r + 1]);
+              else {
+                if (col < dv) o[0] = f.x + y[2 * r];
+                if (col + 1 < dv) o[1] = f.y + y[2 * r + 1];
+              }
+            }
+          }
         }
-        *reinterpret_cast<ulonglong2*>(s0) = a;
-        *reinterpret_cast<ulonglong2*>(s0 + PT) = b;
       }
     }
-    __syncthreads();   // S complete, this stage free
-    if (tid == 0 && c + 2 < chunks) fetch(c + 2);
+    x3::Split<8> a[2];
+    if (mine) {                                         // (what does not depend on u, ahead of the barrier)
+      const float* const kt = sg + 2 * I::kMat + key * C;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        a[k].set4(0, *reinterpret_cast<const float4*>(kt + (x3::unit_row(key, 4 * k + t4) << 2)));
+        a[k].set4(4, *reinterpret_cast<const float4*>(kt + 8 * C + (x3::unit_row(key, 4 * k + t4) << 2)));
+      }
+      const float p0 = sg[3 * I::kMat + key], p1 = sg[3 * I::kMat + key + 8];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) { S[n][0] *= p0; S[n][1] *= p0; S[n][2] *= p1; S[n][3] *= p1; }
+    }
+    group_sync();
+    if (mine) {
+      x3::Split<4> b[2 * NT];
+      const x3::Split<8>* pa[2 * NT];
+      const x3::Split<4>* pb[2 * NT];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          const float* const p = ut + (8 * n + g) * C + (x3::unit_col(g, 4 * k + t4) << 2);
+          b[k * NT + n].load4(0, p, p + C * NC);
+          pa[k * NT + n] = &a[k];
+          pb[k * NT + n] = &b[k * NT + n];
+        }
+      float s[2 * NT][4];
+      x3::mma16<2 * NT>(s, pa, pb);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[n][e] += s[n][e] + s[NT + n][e];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) put(st, NC * DK, at(8 * n + 2 * t4 + (e & 1), key + 8 * (e >> 1)), S[n][e]);
+      }
+    }
+    group_sync();   // S complete, this group done with the stage
+    if (tid == 0 && c + STAGES < chunks) {   // the last group to be done sends for the next chunk
+      __threadfence_block();
+      if (atomicAdd(&s_done[c % STAGES], 1u) % G == G - 1) {
+        __threadfence_block();
+        fetch(c + STAGES);
+      }
+    }
   }
-  if (!ok) *A.err = 1u;
-  for (int i = tid; i < DK * NC; i += Y::kThreads) {
+  if (!ok) {   // given up: the copies under way land before the CTA leaves
+    if (tid == 0) {
+      *A.err = 1u;
+      for (int e = 0; e < chunks && e < STAGES; ++e) tc::mbar_wait(full + 8 * e, *(volatile unsigned*)&s_done[e] / G & 1u);   // (sent once and once per G counts)
+    }
+  }
+  for (int i = tid; i < DK * NC; i += 256) {
     const int n = i % NC, c = i / NC;
-    if (c < krows * L && col0 + n < dv) slot[((int64_t)(c / L) * dv + col0 + n) * L + c % L] = c < dk ? st[n * PT + c] : 0.f;
+    if (c < krows * L && col0 + n < dv) slot[((int64_t)(c / L) * dv + col0 + n) * L + c % L] = c < dk ? st[at(n, c)] + st[NC * DK + at(n, c)] : 0.f;
   }
 }
 
 template <typename T, int DK, bool CHANNEL>
-cudaError_t chunk_launch(const DcArgs& A, int vec, cudaStream_t st) {
-  constexpr int C = kDcC;
-  constexpr int smem = (2 * C * DK + (CHANNEL ? C * DK : C) + C + 8 * C * C + 4 * C * C) * 4;
+cudaError_t chunk_launch(const DcArgs& A, int vec, int vec_v, cudaStream_t st) {
+  constexpr int smem = DcChunk<DK>::kSmem;
   static PerDeviceOnce once;
   if (once.need()) {
     const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<T, DK, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     once.done();
   }
-  return launch(delta_chunk_kernel<T, DK, CHANNEL>, dim3((unsigned)A.n_items, (unsigned)A.heads), dim3(kDcThreads), smem, st, A, vec);
+  return launch(delta_chunk_kernel<T, DK, CHANNEL>, dim3((unsigned)A.n_items, (unsigned)A.heads), dim3(kDcChunkThreads), smem, st, A, vec, vec_v);
 }
 
-template <int DK, int NC>
-cudaError_t carry_launch(const DcArgs& A, int L, cudaStream_t st) {
-  using Y = DcCarry<DK, NC>;
+template <int DK, int NT, int G>
+cudaError_t carry_launch(const DcArgs& A, int L, int vec_o, cudaStream_t st) {
+  using Y = DcCarry<DK, NT, G>;
   static PerDeviceOnce once;
   if (once.need()) {
-    const cudaError_t e = cudaFuncSetAttribute(delta_carry_kernel<DK, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, Y::kSmem);
+    const cudaError_t e = cudaFuncSetAttribute(delta_carry_kernel<DK, NT, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, Y::kSmem);
     if (e != cudaSuccess) return e;
     once.done();
   }
-  return launch(delta_carry_kernel<DK, NC>, dim3((unsigned)((A.dv + NC - 1) / NC), (unsigned)A.heads, (unsigned)A.longs), dim3(Y::kThreads), Y::kSmem, st, A, L);
+  constexpr int cols = Y::NC * G;
+  return launch(delta_carry_kernel<DK, NT, G>, dim3((unsigned)((A.dv + cols - 1) / cols), (unsigned)A.heads, (unsigned)A.longs), dim3(Y::kThreads), Y::kSmem, st, A, L, vec_o);
 }
 
 template <typename T, int DK>
-cudaError_t segment_launch(const DcArgs& A, bool channel, int vec, int L, cudaStream_t st) {
-  const cudaError_t e = channel ? chunk_launch<T, DK, true>(A, vec, st) : chunk_launch<T, DK, false>(A, vec, st);
+cudaError_t segment_launch(const DcArgs& A, bool channel, int vec, int vec_v, int vec_o, int L, cudaStream_t st) {
+  const cudaError_t e = channel ? chunk_launch<T, DK, true>(A, vec, vec_v, st) : chunk_launch<T, DK, false>(A, vec, vec_v, st);
   if (e != cudaSuccess) return e;
-  // Slices of 8 columns: the shorter chain.  Slices of 16, which read W, Q and K half as often, are 2 - 60 % slower at every number of heads (512
-  // rows, decays per channel, us with 8 and 16: 4 heads of 128 x 128 67 and 82, 16 heads 83 and 86, 32 heads 181 and 191; 16 heads of 64 x 128 62 and 94).
-  return carry_launch<DK, 8>(A, L, st);
+  // The fewest columns a CTA with which all CTAs run at once, one an SM.  us of both kernels, 512 tokens with decays per channel, 8, 16 (one or two column
+  // tiles in one group) and 32 (two groups) columns a CTA: 8 heads 44, 55, 71; 16 heads 65, 57, 73; 32 heads 128, 112, 98.
+  const int64_t walks = (int64_t)A.heads * A.longs;
+  if (walks * ((A.dv + 7) / 8) <= sm_count()) return carry_launch<DK, 1, 1>(A, L, vec_o, st);
+  if (walks * ((A.dv + 15) / 16) <= sm_count()) return carry_launch<DK, 2, 1>(A, L, vec_o, st);
+  return carry_launch<DK, 2, 2>(A, L, vec_o, st);
 }
 
-int dc_dvb(int dv) { return (dv + 15) / 16 * 2; }
+int dc_dvb(int dv) { return (dv + 31) / 32 * 4; }
 int64_t dc_item(int dk, int dv) { return (dk <= 64 ? (int64_t)DcItem<64>::kHead : (int64_t)DcItem<128>::kHead) + 2 * (int64_t)dc_dvb(dv) * kDcC * 8; }
 
 constexpr int64_t kDcMaxBytes = 256ll << 20;   // scratch of one launch's chunks
@@ -497,8 +785,8 @@ int b200_delta_rule_in_chunks(int64_t rows, int max_rows, int n_seqs, int heads,
   // us of either way, fitted to launches of 4 to 256 heads (times sequences of the longest one's length) of 128 x 128: a walk's token takes what its
   // chain of reductions takes until the heads fill the GPU, a chunk's as long as the carry's chain, and both the same work beyond; the short sequences'
   // walk comes on top of the chunks and runs half beside the long one's.  Measured, walk / chunks, 16 heads, 64, 128, 512 rows alone: decays per channel
-  // 54 / 43, 104 / 49, 404 / 82; per head 28 / 31, 50 / 35, 181 / 69.  Beside 32 single rows: 76 / 104, 91 / 109, 316 / 159; 56 / 75, 66 / 80, 217 / 118.
-  // 16 sequences of 64, of 256 rows: 207 / 245, 822 / 682; 145 / 202, 528 / 539.
+  // 56 / 29, 108 / 33, 422 / 55; per head 29 / 24, 53 / 28, 194 / 50.  Beside 32 single rows: 75 / 95, 90 / 100, 312 / 138; 55 / 72, 65 / 76, 216 / 114.
+  // 16 sequences of 64, of 256 rows: 206 / 121, 818 / 344; 144 / 107, 526 / 300.
   const double n = max_rows, same = (double)rows / max_rows < n_seqs ? (double)rows / max_rows : n_seqs, one = heads * (dk * (double)dv / 16384.0), load = one * same;
   const int64_t shorts = n_seqs - (rows + max_rows - 1) / max_rows;
   auto most = [](double a, double b) { return a > b ? a : b; };
@@ -506,18 +794,19 @@ int b200_delta_rule_in_chunks(int64_t rows, int max_rows, int n_seqs, int heads,
   if (channel_decay) {
     const bool wide = (int64_t)heads * n_seqs * ((dv + 15) / 16) < sm_count() * 3 / 2;   // (delta_rule_walk's choice)
     walk = 5.0 + n * most(0.35, wide ? 0.17 + 0.038 * load : most(0.36 + 0.01 * load, 0.0126 * load));
-    chunks = 28.0 + (n + 24.0) * most(0.1, 0.0114 * load);
+    chunks = 22.0 + (n + 24.0) * most(0.022, 0.0053 * load);
     few = 0.13 * one;
   } else {
-    walk = 5.0 + n * most(most(0.35, 0.25 + 0.0062 * load), 0.0088 * load);
-    chunks = 20.0 + (n + 24.0) * most(0.085, 0.009 * load);
+    walk = 5.0 + n * most(0.25 + 0.0062 * load, 0.0088 * load);
+    chunks = 20.0 + (n + 24.0) * most(0.02, 0.0047 * load);
     few = 0.09 * one;
   }
   if (shorts > 0) {
-    walk += 0.5 * few * shorts;
+    walk += 0.3 * few * shorts;
     chunks += few * shorts;
   }
-  return chunks < walk;
+  // Two chunks at most in any sequence: little but starts to save, and scratch for every row to be had for it; the walk stays unless it takes 1.7 times as long.
+  return (max_rows <= 2 * kDcC ? 1.7 : 1.0) * chunks < walk;
 }
 
 size_t b200_delta_rule_workspace_bytes(int max_rows, int n_seqs, int heads, int dk, int dv) {
@@ -561,6 +850,7 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
   B200_CHECK_ARG(A.err, "b200_delta_rule_chunked: no error word");
   auto al = [](const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };
   const int vec = a->dk % 4 == 0 && al(a->q, a->ldq) && al(a->k, a->ldk);
+  const int vec_v = a->dv % 4 == 0 && al(a->v, a->ldv), vec_o = a->dv % 2 == 0 && a->ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 7) == 0;
   const int L = a->dk <= 64 ? 4 : 8;   // the stored layout of a state (delta.cu)
   const bool ch = a->channel_decay != 0;
   cudaStream_t st = (cudaStream_t)stream;
@@ -568,8 +858,8 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
     A.item0 = (int)at;
     A.n_items = (int)(most - at < fit ? most - at : fit);
     B200_FLOAT_TYPES(a->dtype, T, {
-      if (a->dk <= 64) B200_CUDA((segment_launch<T, 64>(A, ch, vec, L, st)));
-      else B200_CUDA((segment_launch<T, 128>(A, ch, vec, L, st)));
+      if (a->dk <= 64) B200_CUDA((segment_launch<T, 64>(A, ch, vec, vec_v, vec_o, L, st)));
+      else B200_CUDA((segment_launch<T, 128>(A, ch, vec, vec_v, vec_o, L, st)));
     });
   }
   return B200_OK;
