@@ -91,16 +91,16 @@ __global__ void __launch_bounds__(128) int8_outlier_flags_kernel(const __half* _
   }
 }
 
-// ordered compaction of the flagged columns (ascending k: the fp32 side product is summed in this order)
-__global__ void __launch_bounds__(1024) int8_compact_kernel(const int* __restrict__ flags, int64_t K, int* __restrict__ idx,
-                                                            int* __restrict__ count) {
-  __shared__ int s_sum[32];
-  griddep_launch();
-  griddep_wait();
+// ordered compaction of the flagged columns (ascending k: the fp32 side product is summed in this order), by one CTA of 256 threads
+__device__ __forceinline__ void int8_compact(const int* __restrict__ flags, int64_t K, int* __restrict__ idx, int* __restrict__ count) {
+  __shared__ int s_sum[8];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int64_t per = (K + 1023) / 1024, beg = t * per < K ? t * per : K, end = beg + per < K ? beg + per : K;
+  const int64_t per = (K / 4 + 255) / 256, beg = t * per < K / 4 ? t * per : K / 4, end = beg + per < K / 4 ? beg + per : K / 4;   // fours of columns
   int c = 0;
-  for (int64_t k = beg; k < end; ++k) c += flags[k];
+  for (int64_t i = beg; i < end; ++i) {
+    const int4 f = reinterpret_cast<const int4*>(flags)[i];
+    c += f.x + f.y + f.z + f.w;
+  }
   int incl = c;   // inclusive scan over the warp, then over the warps' sums
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -112,22 +112,34 @@ __global__ void __launch_bounds__(1024) int8_compact_kernel(const int* __restric
   int before = 0;
   for (int w = 0; w < warp; ++w) before += s_sum[w];
   int pos = before + incl - c;
-  for (int64_t k = beg; k < end; ++k) {
-    if (flags[k]) idx[pos++] = (int)k;
+  if (c) {
+    for (int64_t i = beg; i < end; ++i) {
+      const int4 f = reinterpret_cast<const int4*>(flags)[i];
+      const int k = (int)(4 * i);
+      if (f.x) idx[pos++] = k;
+      if (f.y) idx[pos++] = k + 1;
+      if (f.z) idx[pos++] = k + 2;
+      if (f.w) idx[pos++] = k + 3;
+    }
   }
-  if (t == 1023) *count = before + incl;
+  if (t == 255) *count = before + incl;
 }
 
 // one CTA per activation row: SCA = absmax over the non-outlier columns, CA = rint(x * 127 / SCA) (0 in outlier columns)
 // (K is a multiple of 64 and the rows start on 16-byte boundaries: eight columns per access, the first 8192 kept in registers between
-// the maximum and the rounding)
+// the maximum and the rounding); the first CTA makes the list of outlier columns beside them (a launch of its own between the flags and the rows took 4 us of
+// a call's 62)
 __global__ void __launch_bounds__(256) int8_rowquant_kernel(const __half* __restrict__ x, int64_t K, const int* __restrict__ flags,
-                                                            int8_t* __restrict__ ca, float* __restrict__ sca) {
+                                                            int8_t* __restrict__ ca, float* __restrict__ sca, int* __restrict__ idx, int* __restrict__ count) {
   __shared__ float s_max[8];
   constexpr int KEEP = 4;
   griddep_launch();
   griddep_wait();
-  const int64_t m = blockIdx.x;
+  if (blockIdx.x == 0) {
+    int8_compact(flags, K, idx, count);
+    return;
+  }
+  const int64_t m = (int64_t)blockIdx.x - 1;
   const __half* row = x + m * K;
   const int nv = (int)(K >> 3);
   auto load = [&](int i, float (&f)[8]) {   // eight columns, outliers as 0
@@ -287,23 +299,24 @@ __global__ void __launch_bounds__(kI8Threads) int8_gemv_kernel(const I8Params p)
 
 // ---- prefill: M > 16 ----------------------------------------------------------------------------------------------
 // Persistent over output tiles, neighbouring CTAs on the same weight rows.  One thread loads 128-byte-wide boxes of both operands by TMA into a
-// ring of stages, one issues tcgen05.mma kind::i8 (K = 32) into one of two tensor-memory accumulators, and eight epilogue warps scale, round
+// ring of stages, one issues tcgen05.mma kind::i8 (K = 32) into one of two tensor-memory accumulators, and sixteen epilogue warps scale, round
 // and store the other: the epilogue (a division, three roundings and the outlier columns per output) hides behind the next tile's products.
-//   PAIR = true: a CTA pair on 256 rows x 256 features, each CTA holding 128 rows of either operand.  Shared memory is the limit of the
-//   int8 pipe -- a CTA alone on 128 x 128 moves 128 bytes in and 128 bytes out of it per clock at full rate, twice what it carries, the pair
-//   half as much.  777 x 4096 -> 11008 with its three preparing kernels, six outlier columns: 780 us with fragments read from L2, 100 us with
-//   128 x 128 tiles, 71 us with pairs (4096 rows -> 12288: 338 and 229 us, 1.8 POP/s; without outlier columns 2.1).
+//   PAIR = true: a CTA pair on 256 rows x up to 256 features (i8_features), each CTA holding 128 rows of the activations and half of the features.  The
+//   copies are the limit of the int8 pipe: an SM takes 48.7 bytes a clock of 128-byte boxes from L2 (measured with copies alone), the pair's products at
+//   full rate 64, a CTA alone on 128 x 128 twice that.  777 x 4096 -> 11008 with its preparing kernels, six outlier columns: 780 us with fragments read
+//   from L2, 100 us with 128 x 128 tiles, 66.6 us with pairs of 256 features and eight epilogue warps, 62.7 with sixteen and 224 features (4096 rows ->
+//   12288: 338, 220 and 221 us, 1.9 POP/s).
 //   PAIR = false: one CTA on 128 x 128, for up to 128 rows, where the second half of a pair's rows would be padding.
-constexpr int kI8EpiWarps = 8, kI8GemmThreads = (kI8EpiWarps + 2) * 32;
+constexpr int kI8EpiWarps = 16, kI8GemmThreads = (kI8EpiWarps + 2) * 32;
 constexpr int kI8KB = 128;                       // int8 columns per stage: one 128-byte swizzle row
 constexpr int kI8Stages = 6, kI8Stage = 256 * kI8KB, kI8Smem = kI8Stages * kI8Stage + 1024;   // 128 rows of either operand
 static_assert(kI8Smem >= tc::kPairMinSmem, "one CTA of a pair per SM");
 
 // kind::i8: D = int32, A = B = signed 8 bit, both K-major
 template <bool PAIR>
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-  constexpr uint32_t kM = PAIR ? 256 : 128, kN = PAIR ? 256 : 128;
-  constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((kN >> 3) << 17) | ((kM >> 4) << 24);
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, int n, uint32_t accumulate) {
+  constexpr uint32_t kM = PAIR ? 256 : 128;
+  const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((kM >> 4) << 24);
   if constexpr (PAIR)
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -327,13 +340,13 @@ __device__ __forceinline__ float2 round_f16x2(float a, float b) { return __half2
 
 template <bool PAIR>
 __global__ void __launch_bounds__(kI8GemmThreads, 1)
-int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int m_tiles, int n_tiles, unsigned* err) {
-  constexpr int CTAS = PAIR ? 2 : 1, BN = 128 * CTAS;
+int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int m_tiles, int n_tiles, int bn, unsigned* err) {
+  constexpr int CTAS = PAIR ? 2 : 1, BM = 128 * CTAS, BN = BM;   // bn: features of a tile, a multiple of 32 up to BN
   extern __shared__ __align__(1024) uint8_t i8_smem[];
   __shared__ __align__(8) uint64_t s_bars[2 * kI8Stages + 5];
   __shared__ uint32_t s_tmem;
   __shared__ __align__(16) float s_feat[10][BN];               // per feature of the tile: weight scale, bias, weight in the first eight outlier columns
-  __shared__ __align__(16) float s_more[kI8EpiWarps][8][32];   // per epilogue warp: the weights of 32 features in the next eight
+  __shared__ __align__(16) float s_more[kI8EpiWarps][8][16];   // per epilogue warp: the weights of 16 features in the next eight
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = PAIR ? tc::cluster_rank() : 0u;
   const uint32_t tiles = (tc::smem_u32(i8_smem) + 1023u) & ~1023u;
@@ -368,12 +381,12 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
       int s = 0;
       uint32_t ph = 1;
       for (int t = first; t < total && ok; t += step) {
-        const int m0 = (t % m_tiles) * BN + (int)rank * 128, n0 = (t / m_tiles) * BN + (int)rank * 128;
+        const int m0 = (t % m_tiles) * BM + (int)rank * 128, n0 = (t / m_tiles) * bn + (int)rank * (bn / CTAS);
         for (int kb = 0; kb < nkb; ++kb) {
           ok = PAIR ? tc::mbar_wait_cluster(empty + 8 * s, ph) : tc::mbar_wait(empty + 8 * s, ph);
           if (!ok) break;
           const uint32_t st = tiles + s * kI8Stage;
-          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * kI8Stage);
+          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, (BM + bn) * kI8KB);
           if constexpr (PAIR) {
             const uint32_t bar = tc::at_rank(full + 8 * s, 0);
             tc::tma_load_2d_pair(st, &map_a, kb * kI8KB, m0, bar);
@@ -406,7 +419,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
           const uint32_t st = tiles + s * kI8Stage;
           const uint64_t da = tc::desc_sw128(st), db = tc::desc_sw128(st + 128 * kI8KB);
 #pragma unroll
-          for (int k = 0; k < kI8KB / 32; ++k) umma_i8<PAIR>(tmem + acc * BN, da + 2 * k, db + 2 * k, (kb | k) != 0);
+          for (int k = 0; k < kI8KB / 32; ++k) umma_i8<PAIR>(tmem + acc * BN, da + 2 * k, db + 2 * k, bn, (kb | k) != 0);
           if constexpr (PAIR) tc::commit_pair(empty + 8 * s);
           else tc::commit(empty + 8 * s);
           if (++s == kI8Stages) { s = 0; ph ^= 1u; }
@@ -425,7 +438,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
       }
     }
   } else {
-    // ---- epilogue: warp w holds rows 32 (w % 4) .. + 31 and half of the columns ----
+    // ---- epilogue: warp w holds rows 32 (w % 4) .. + 31 and every fourth sixteen of the columns ----
     int acc = 0;
     uint32_t ph = 0;
     const int no = *p.count;
@@ -433,10 +446,9 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
     int k0[8];   // the first eight outlier columns
 #pragma unroll
     for (int j = 0; j < 8; ++j) k0[j] = j < no ? p.idx[j] : 0;
-    float(&more)[8][32] = s_more[warp];
+    float(&more)[8][16] = s_more[warp];
     for (int t = first; t < total; t += step) {
-      const int64_t m = (int64_t)(t % m_tiles) * BN + rank * 128 + (warp & 3) * 32 + lane, n0 = (int64_t)(t / m_tiles) * BN;
-      const int half = (warp >> 2) * (BN / 2);
+      const int64_t mw = (int64_t)(t % m_tiles) * BM + rank * 128 + (warp & 3) * 32, m = mw + lane, n0 = (int64_t)(t / m_tiles) * bn;
       const bool mok = m < p.M;
       const float sca = mok ? p.sca[m] : 0.f;
       const __half* const xr = p.x + (mok ? m : 0) * p.K;
@@ -445,8 +457,8 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
       for (int j = 0; j < 8; ++j) x0[j] = j < no ? __half2float(xr[k0[j]]) : 0.f;
       // the tile's features, one per thread, while its products are still running (a gather per 32 columns in the loop below cost more than
       // the products: 72 us of 266 at 4096 rows with six outlier columns)
-      asm volatile("bar.sync 1, 256;" ::: "memory");   // the last tile's readers are done
-      if (tid < BN) {
+      asm volatile("bar.sync 1, %0;" ::"n"(kI8EpiWarps * 32) : "memory");   // the last tile's readers are done
+      if (tid < bn) {
         const int64_t n = n0 + tid;
         const bool nok = n < p.N;
         const float scb = nok ? p.scb[n] : 0.f, ws = __fdiv_rn(scb, 127.0f);
@@ -460,17 +472,18 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
         for (int j = 0; j < 8; ++j)
           if (j < no) s_feat[2 + j][tid] = round_f16(__fmul_rn(w[j], ws));
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(kI8EpiWarps * 32) : "memory");
       ok = ok && __all_sync(0xffffffffu, PAIR ? tc::mbar_wait_cluster(acc_full + 8 * acc, ph) : tc::mbar_wait(acc_full + 8 * acc, ph));
       tc::fence_after();
+      const int c_end = mw < p.M && ok ? bn : 0;   // (a warp whose rows are all past the last one has nothing to do)
 #pragma unroll 1
-      for (int c0 = half; c0 < half + BN / 2 && ok; c0 += 32) {
-        uint32_t v[32];
-        tc::ld32(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * BN + c0));
+      for (int c0 = (warp >> 2) * 16; c0 < c_end; c0 += 64) {
+        uint32_t v[16];
+        tc::ld16(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * BN + c0));
         tc::wait_ld(v);
-        float out[32];
+        float out[16];
 #pragma unroll
-        for (int e = 0; e < 32; e += 2) {
+        for (int e = 0; e < 16; e += 2) {
           const float2 sc = *reinterpret_cast<const float2*>(&s_feat[0][c0 + e]);
           const float2 o = round_f16x2(__fmul_rn((float)(int)v[e], i8_scale(__fmul_rn(sca, sc.x))), __fmul_rn((float)(int)v[e + 1], i8_scale(__fmul_rn(sca, sc.y))));
           out[e] = o.x;
@@ -478,7 +491,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
         }
         if (p.bias) {
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
+          for (int e = 0; e < 16; e += 2) {
             const float2 b = *reinterpret_cast<const float2*>(&s_feat[1][c0 + e]);
             const float2 o = round_f16x2(out[e] + b.x, out[e + 1] + b.y);
             out[e] = o.x;
@@ -486,15 +499,15 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
           }
         }
         if (no > 0) {
-          float sub[32];
+          float sub[16];
 #pragma unroll
-          for (int e = 0; e < 32; ++e) sub[e] = 0.f;
+          for (int e = 0; e < 16; ++e) sub[e] = 0.f;
           auto add = [&](int j0, const float (&xv)[8], const float* rows, int ld) {   // ascending columns
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               if (j0 + j < no) {
 #pragma unroll
-                for (int e = 0; e < 32; e += 4) {
+                for (int e = 0; e < 16; e += 4) {
                   const float4 w = *reinterpret_cast<const float4*>(rows + j * ld + e);
                   sub[e] = fmaf(xv[j], w.x, sub[e]);
                   sub[e + 1] = fmaf(xv[j], w.y, sub[e + 1]);
@@ -506,9 +519,10 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
           };
           add(0, x0, &s_feat[2][c0], BN);
           for (int j0 = 8; j0 < no; j0 += 8) {
-            const int64_t n = n0 + c0 + lane;
+            const int f = lane & 15;
+            const int64_t n = n0 + c0 + f;
             const bool nok = n < p.N;
-            const float ws = __fdiv_rn(s_feat[0][c0 + lane], 127.0f);
+            const float ws = __fdiv_rn(s_feat[0][c0 + f], 127.0f);
             const int8_t* const cb = p.cb + (nok ? n : 0) * p.K;
             float xv[8], w[8];
 #pragma unroll
@@ -518,13 +532,15 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
               w[j] = j0 + j < no ? (float)cb[k] : 0.f;
             }
             __syncwarp();
+            if (lane < 16) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) more[j][lane] = round_f16(__fmul_rn(w[j], ws));
+              for (int j = 0; j < 8; ++j) more[j][lane] = round_f16(__fmul_rn(w[j], ws));
+            }
             __syncwarp();
-            add(j0, xv, &more[0][0], 32);
+            add(j0, xv, &more[0][0], 16);
           }
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
+          for (int e = 0; e < 16; e += 2) {
             const float2 r = round_f16x2(sub[e], sub[e + 1]);
             out[e] += r.x;      // rounded by the store
             out[e + 1] += r.y;
@@ -534,7 +550,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
           __half* const yr = p.y + m * p.N + n0 + c0;
           if (vec) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
+            for (int e = 0; e < 16; e += 8) {
               if (n0 + c0 + e < p.N) {
                 uint32_t o[4];
 #pragma unroll
@@ -547,7 +563,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
             }
           } else {
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
+            for (int e = 0; e < 16; ++e)
               if (n0 + c0 + e < p.N) yr[e] = __float2half_rn(out[e]);
           }
         }
@@ -573,6 +589,20 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
   }
 }
 
+// Features of a pair's tile: a round of tiles takes about 235 + bn for each k-block, so that fewer features pay where they cost no further round.  us of the
+// whole call at 256, 224, 192, 160, 128, 64 features, six outlier columns: 4096 -> 11008 at 777 rows (3, 3, 4, 4, 5, 10 rounds) 64.5, 62.7, 69.9, 67.8, 72.4, 111;
+// 4096 -> 12288 at 512 rows (2, 2, 2, 3, 3, 6) 51.7, 50.1, 47.8, 58.1, 54.4, 79.6; 4096 -> 4096 at 200 rows (all 1) 32.3, 31.6, 29.8, 29.2, 27.9, 26.6.
+// A CTA alone (up to 128 rows) keeps 128: with 64 it is 2 us shorter at 4096 features and 4 to 9 longer from 6144 on.
+static int i8_features(int64_t N, int64_t row_tiles, int64_t pairs) {
+  int best = 256;
+  int64_t best_t = -1;
+  for (int bn = 256; bn >= 64; bn -= 32) {
+    const int64_t t = (row_tiles * ((N + bn - 1) / bn) + pairs - 1) / pairs * (235 + bn);
+    if (best_t < 0 || t < best_t) { best_t = t; best = bn; }
+  }
+  return best;
+}
+
 template <bool PAIR>
 static cudaError_t launch_i8_gemm(const I8Params& p, cudaStream_t st) {
   static PerDeviceOnce once;
@@ -581,16 +611,17 @@ static cudaError_t launch_i8_gemm(const I8Params& p, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     once.done();
   }
+  constexpr int CTAS = PAIR ? 2 : 1, BM = 128 * CTAS;
+  const int64_t most = sm_count() / CTAS;
+  const int mt = (int)((p.M + BM - 1) / BM), bn = PAIR ? i8_features(p.N, mt, most) : BM, nt = (int)((p.N + bn - 1) / bn);
+  const int64_t tiles = (int64_t)mt * nt;
   alignas(64) CUtensorMap ma, mb;
-  if (!tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.ca, p.M, p.K, p.K, 128) || !tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.cb, p.N, p.K, p.K, 128))
+  if (!tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.ca, p.M, p.K, p.K, 128) || !tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.cb, p.N, p.K, p.K, bn / CTAS))
     return cudaErrorInvalidValue;
-  constexpr int CTAS = PAIR ? 2 : 1, BN = 128 * CTAS;
-  const int mt = (int)((p.M + BN - 1) / BN), nt = (int)((p.N + BN - 1) / BN);
-  const int64_t tiles = (int64_t)mt * nt, most = sm_count() / CTAS;
   const dim3 grid((unsigned)((tiles < most ? tiles : most) * CTAS));
   unsigned* const err = wait_error_word();
   if (!err) return cudaErrorMemoryAllocation;
-  return launch_cluster(int8_gemm_kernel<PAIR>, grid, dim3(kI8GemmThreads), CTAS, (size_t)kI8Smem, st, p, ma, mb, mt, nt, err);
+  return launch_cluster(int8_gemm_kernel<PAIR>, grid, dim3(kI8GemmThreads), CTAS, (size_t)kI8Smem, st, p, ma, mb, mt, nt, bn, err);
 }
 
 }  // namespace b200
@@ -657,8 +688,7 @@ int b200_linear_int8(const b200_linear_int8_args* a, b200_stream_t stream) {
   const dim3 fg((unsigned)((a->K / 8 + 127) / 128), (unsigned)((a->M + block_rows - 1) / block_rows));
   cudaError_t e = fg.y > 1 ? cudaMemsetAsync(flags, 0, (size_t)a->K * sizeof(int), st) : cudaSuccess;
   if (e == cudaSuccess) e = launch(int8_outlier_flags_kernel, fg, dim3(128), 0, st, x, a->M, a->K, a->threshold, block_rows, flags);
-  if (e == cudaSuccess) e = launch(int8_compact_kernel, dim3(1), dim3(1024), 0, st, (const int*)flags, a->K, idx, count);
-  if (e == cudaSuccess) e = launch(int8_rowquant_kernel, dim3((unsigned)a->M), dim3(256), 0, st, x, a->K, (const int*)flags, ca, sca);
+  if (e == cudaSuccess) e = launch(int8_rowquant_kernel, dim3((unsigned)a->M + 1), dim3(256), 0, st, x, a->K, (const int*)flags, ca, sca, idx, count);
   I8Params p{};
   p.cb = reinterpret_cast<const int8_t*>(a->cb);
   p.scb = reinterpret_cast<const float*>(a->scb);
