@@ -2,12 +2,16 @@
 //
 // Replaces, for T > 16 rows, bnb.nn.Linear4bit.forward's "dequantize_4bit of the WHOLE weight to bf16, then F.linear"
 // (call sites lit_gpt/model.py:519,619,656,713,714,716): the bf16 weight is never materialised in HBM.
-// Persistent over output tiles of 256 features x 256 MT tokens, a CTA PAIR each (cta_group::2; up to 128 tokens: one CTA on 128 x 128; up to 256 of small matrices: one on 128 x 256),
-// walking K in blocks of 64.  Per CTA:
-//   * warps 0-15 rebuild the bf16 values of 128 features from the packed 4-bit weights and their absmax / {scale, zero} with exactly the
+// Persistent over output tiles of up to 256 features x 256 MT tokens, a CTA PAIR each (cta_group::2; up to 128 tokens: one CTA on up to 128 x 128; up to 256 of
+// small matrices: one on 128 x 256), walking K in blocks of 64.  Per CTA:
+//   * warp 18 fetches packed weights, two k-blocks of the CTA's features at a time, into buffers of their own by TMA, ahead of the stages.  (Read by the
+//     dequantising warps themselves, sixteen rows of 32 bytes an access, they took 128 of the 810 shared-memory and L1 cycles of a k-block: nf4, 64 rows
+//     x 11008 -> 4096 33 -> 27 us, 4096 -> 12288 at 613 rows 93 -> 88; int4, which has cycles to spare, 1 % longer.)
+//   * warps 0-15 rebuild the bf16 values of up to 128 features from the packed 4-bit weights and their absmax / {scale, zero} with exactly the
 //     dequantise kernel's arithmetic (bf16_rn(code_fp32 * absmax_fp32), resp. bf16_rn(scale * (q - zero))) and write them into shared memory in
 //     the tensor core's K-major 128-byte-swizzled layout.  Even and odd k-blocks belong to eight warps each: a warp has two blocks' time
-//     for its loads, look-ups and the proxy fence, and 32 codes a thread to overlap;
+//     for its look-ups and the proxy fence, and 32 codes a thread to overlap.  (Three groups of eight take the same time to a tenth of a us: what bounds
+//     them is throughput.);
 //   * warp 16 fetches the activation tiles (128 tokens x 64 k per CTA and sub-tile) by TMA, rows past M zero-filled by the hardware;
 //   * warp 17 (of the pair's first CTA) issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, 256 x 256 x 16) into TENSOR MEMORY; tcgen05.commit
 //     hands each stage back to both CTAs;
@@ -19,10 +23,8 @@
 //   * the sixteen warps read the accumulators with tcgen05.ld, add the bias, round to bf16 and store rows of y.
 // SWIGLU: the pair's first CTA dequantises 128 rows of the gate projection and the second the same rows of the up projection, so that a
 // thread holds both halves of its outputs and stores silu(gate) * up, with the roundings of the separate launches.
-// Bound: with MT = 2 the tensor pipe and the shared memory that feeds it (a CTA alone on 128 x 128 reads 128 bytes a clock of it for the
-// products alone, the pair 64); one dequantised tile serves 512 tokens.  What was before -- a CTA on 128 features x 384 tokens, one thread that
-// loaded the activations between its own dequantising, every warp in every k-block -- spent 1750 clocks a k-block whatever the tokens.
-// 4096 tokens, 4096 -> 14336: int4 516 -> 406 us, nf4 591 -> 414; 14336 -> 4096: int4 532 -> 358 (1340 TFLOP/s), nf4 631 -> 368.
+// Bound: long prompts by power (1.3 GHz and 80 % tensor pipe at 4096 tokens, 4096 -> 14336, int4: 1106 clk a k-block of 512 tokens, 1024 of them products);
+// one sub-tile by the look-ups and stores of a tile's features (606 clk a k-block without, at 256 features int4 about 800 and nf4 950).
 #include "tc05.cuh"
 
 namespace b200 {
@@ -40,9 +42,10 @@ struct GemmParams {
   int ksplit;                 // > 1 (too few tiles for the SMs): an item owns a range of k-blocks and writes fp32 partial sums
   float* partial;             // (ksplit, M, N) fp32, summed in range order by qgemm_splitk_reduce_kernel
   int n_tiles, m_tiles;
+  int bn;                     // features per tile: a multiple of 16 (of 32 for a gate / up pair) up to 128 per CTA
 };
 
-constexpr int kGDequant = 512, kGThreads = kGDequant + 64;   // 16 dequantising warps, the copies' and the products'
+constexpr int kGGroups = 2, kGDequantWarps = 8 * kGGroups, kGThreads = (kGDequantWarps + 3) * 32;   // groups of dequantising warps, the activations', the products' and the weights' warp
 constexpr int kBK = 64;
 constexpr int kTileBytes = 128 * kBK * 2;   // one 128-row x 64-k bf16 operand tile = 16 KB
 
@@ -50,9 +53,9 @@ constexpr int kTileBytes = 128 * kBK * 2;   // one 128-row x 64-k bf16 operand t
 __device__ __forceinline__ uint32_t sw128(int r, int c) { return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4)); }
 
 template <int CTAS>
-__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
-  // D = f32, A = B = bf16, both K-major, N = M = 128 per CTA of the group
-  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 * CTAS >> 3) << 17) | ((uint32_t)(128 * CTAS >> 4) << 24);
+__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, int n, uint32_t accumulate) {
+  // D = f32, A = B = bf16, both K-major, M = 128 per CTA of the group
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 * CTAS >> 4) << 24);
   if constexpr (CTAS == 2)
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
@@ -63,18 +66,21 @@ __device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, ui
 
 template <int MT>
 struct GemmTile {
-  static constexpr int kStages = MT == 2 ? 4 : 6;          // an even number: a stage belongs to one half of the dequantising warps
+  static constexpr int kStages = MT == 2 ? 4 : 6;
   static constexpr int kStage = (MT + 1) * kTileBytes;     // MT activation tiles + 1 weight tile
-  static constexpr int kSmem = kStages * kStage + 1024;
+  static constexpr int kPairs = 3, kPair = 128 * 64;       // buffers of packed weights: two k-blocks of 128 features each
+  static constexpr int kSmem = kStages * kStage + kPairs * kPair + 1024;
   static_assert(kSmem >= tc::kPairMinSmem, "one CTA of a pair per SM");
 };
 
 template <int CTAS, int MT, bool INT4, bool SWIGLU>
-__global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_x, unsigned* err) {
+__global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                     const __grid_constant__ CUtensorMap map_w2, unsigned* err) {
   using C = GemmTile<MT>;
   extern __shared__ __align__(1024) uint8_t g_smem[];
-  constexpr int BN = 128 * CTAS, BM = BN;           // features per tile, tokens per sub-tile
-  __shared__ __align__(8) uint64_t s_bars[3 * C::kStages + 3];
+  constexpr int BM = 128 * CTAS, BN = BM;           // tokens per sub-tile; columns of an accumulator
+  const int bn = p.bn, half = bn / CTAS, busy = (half + 15) / 16;   // features of a tile, of a CTA; dequantising warps of a group that have some
+  __shared__ __align__(8) uint64_t s_bars[3 * C::kStages + 3 + 2 * C::kPairs];
   __shared__ uint32_t s_tmem;
   __shared__ uint4 s_token[CTAS == 2 ? C::kStages : 1][8];   // where the bytes of the other CTA's warps land
   __shared__ float s_code[16 * 32];                 // fp32 code book, one copy per lane (conflict-free look-ups)
@@ -83,23 +89,26 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   const uint32_t tiles = (tc::smem_u32(g_smem) + 1023u) & ~1023u;
   const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]), acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_free = acc_full + 8, idle = acc_full + 16;
   const uint32_t room = CTAS == 2 ? idle + 8 : empty;   // where the dequantising warps learn that a stage is theirs
+  const uint32_t packed = tiles + C::kStages * C::kStage, w_full = tc::smem_u32(&s_bars[3 * C::kStages + 3]), w_empty = w_full + 8 * C::kPairs;
   if (tid == 0) {
     for (int s = 0; s < C::kStages; ++s) {
-      tc::mbar_init(full + 8 * s, 9);   // half of the dequantising warps and the copies
+      tc::mbar_init(full + 8 * s, 1 + busy);   // a group of dequantising warps and the copies
       tc::mbar_init(empty + 8 * s, 1);
       if (CTAS == 2) tc::mbar_init(room + 8 * s, 1);
     }
     tc::mbar_init(acc_full, 1);
-    tc::mbar_init(acc_free, 16 * CTAS);
+    tc::mbar_init(acc_free, kGDequantWarps * CTAS);
     tc::mbar_init(idle, 1);
+    for (int i = 0; i < C::kPairs; ++i) { tc::mbar_init(w_full + 8 * i, 1); tc::mbar_init(w_empty + 8 * i, kGGroups * busy); }
     tc::mbar_init_fence();
     tc::prefetch_map(&map_x);
+    tc::prefetch_map(SWIGLU && rank ? &map_w2 : &map_w);
   }
   if (!INT4)
     for (int i = tid; i < 16 * 32; i += kGThreads) s_code[i] = code_value(p.qtype, i >> 5);
   griddep_launch();
   griddep_wait();
-  if (warp == 17) {
+  if (warp == kGDequantWarps + 1) {
     if constexpr (CTAS == 2) tc::tmem_alloc_pair<BN * MT>(tc::smem_u32(&s_tmem));
     else tc::tmem_alloc<BN * MT>(tc::smem_u32(&s_tmem));
   }
@@ -116,7 +125,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     const int z = i / (p.n_tiles * p.m_tiles), r = i - z * (p.n_tiles * p.m_tiles), m = r / p.n_tiles;
     t.z = z;
     t.m0 = (int64_t)m * (BM * MT);
-    t.n0 = (int64_t)(r - m * p.n_tiles) * (SWIGLU ? 128 : BN);
+    t.n0 = (int64_t)(r - m * p.n_tiles) * (SWIGLU ? half : bn);
     t.kb0 = (int)(((int64_t)nkb_all * z) / p.ksplit);
     t.nkb = (int)(((int64_t)nkb_all * (z + 1)) / p.ksplit) - t.kb0;
     t.mts = MT == 1 || p.M - t.m0 <= BM ? 1 : MT;     // sub-tiles with tokens in them
@@ -129,56 +138,61 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     return CTAS == 2 ? tc::mbar_wait_cluster(bar, parity) : tc::mbar_wait(bar, parity);
   };
 
-  if (warp < 16) {
+  if (warp < kGDequantWarps) {
     // =========================================== DEQUANTISE, THEN STORE =========================================
     constexpr int LAG = 2;
-    const int g = warp >> 3, tg = tid & 255, wr = tg >> 1, wh = tg & 1;   // half of the warps, feature, half of the k-block
+    const int g = warp >> 3, at = ((warp & 7) - 2 * g) & 7, wr = at * 16 + (lane & 15), wh = lane >> 4;   // group of warps, place in it, feature, half of
+    // the k-block (a tile of fewer features leaves the last places idle: two warps on, so that the groups' idle ones belong to different schedulers)
     uint32_t acc_ph = 0;
+    int pairs = 0;                                    // buffers of weights so far
     for (int i = first; i < total && ok; i += step) {
       const Item t = item(i);
-      const int64_t wn = t.n0 + (SWIGLU ? 0 : rank * 128) + wr;
-      const bool wvalid = wn < p.N;
-      const uint8_t* wp = (SWIGLU && rank ? p.packed2 : p.packed) + (wvalid ? wn : 0) * (p.K >> 1) + (int64_t)t.kb0 * 32 + wh * 16;
-      const uint32_t* sp = (SWIGLU && rank ? p.scale2 : p.scale) + (wvalid ? wn : 0) * (INT4 ? (p.K >> 7) : (p.K >> 6));
-      const int l0 = (q + g) & 1;                     // this half's first k-block of the item
-      uint4 qn[LAG];
+      const int64_t wn = t.n0 + (SWIGLU ? 0 : (int)rank * half) + wr;   // (rows of a warp past the CTA's features are written and not read)
+      const uint32_t* sp = (SWIGLU && rank ? p.scale2 : p.scale) + (wn < p.N ? wn : 0) * (INT4 ? (p.K >> 7) : (p.K >> 6));
+      const int l0 = (g + kGGroups - q % kGGroups) % kGGroups;   // this group's first k-block of the item
       uint32_t sn[LAG];
 #pragma unroll
       for (int e = 0; e < LAG; ++e) {
-        const int l = l0 + 2 * e;
-        qn[e] = make_uint4(0u, 0u, 0u, 0u);
-        sn[e] = 0u;
-        if (l < t.nkb) { qn[e] = ldg_stream_v4(wp + (int64_t)l * 32); sn[e] = sp[INT4 ? ((t.kb0 + l) >> 1) : (t.kb0 + l)]; }
+        const int l = l0 + kGGroups * e;
+        sn[e] = l < t.nkb ? sp[INT4 ? ((t.kb0 + l) >> 1) : (t.kb0 + l)] : 0u;
       }
-      for (int l = l0; l < t.nkb; l += 2) {
+      for (int l = at < busy ? l0 : t.nkb; l < t.nkb; l += kGGroups) {
         const int s = (q + l) % C::kStages;
         const uint32_t ph = (uint32_t)((q + l) / C::kStages) & 1u;
-        const uint4 w = qn[0];
         const uint32_t sc = sn[0];
 #pragma unroll
-        for (int e = 0; e + 1 < LAG; ++e) { qn[e] = qn[e + 1]; sn[e] = sn[e + 1]; }
-        const int ln = l + 2 * LAG;
-        if (ln < t.nkb) { qn[LAG - 1] = ldg_stream_v4(wp + (int64_t)ln * 32); sn[LAG - 1] = sp[INT4 ? ((t.kb0 + ln) >> 1) : (t.kb0 + ln)]; }
-        const uint32_t qw[4] = {w.x, w.y, w.z, w.w};
+        for (int e = 0; e + 1 < LAG; ++e) sn[e] = sn[e + 1];
+        const int ln = l + kGGroups * LAG;
+        if (ln < t.nkb) sn[LAG - 1] = sp[INT4 ? ((t.kb0 + ln) >> 1) : (t.kb0 + ln)];
+        const int pair = pairs + (l >> 1), buf = pair % C::kPairs;
         const uint32_t dst = tiles + s * C::kStage + MT * kTileBytes;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(w_full + 8 * buf, (uint32_t)(pair / C::kPairs) & 1u));
+        if (!ok) break;
+        uint32_t qw[4];
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(qw[0]), "=r"(qw[1]), "=r"(qw[2]), "=r"(qw[3])
+                     : "r"(packed + buf * C::kPair + wr * 64 + ((((l & 1) * 2 + wh) ^ ((wr >> 1) & 3)) << 4)));
         ok = __all_sync(0xffffffffu, tc::mbar_wait(room + 8 * s, CTAS == 2 ? ph : ph ^ 1u));
         if (!ok) break;
         if (INT4) {
-          // bf16_rn(scale * (q - zero)) with three instructions per code: the nibble is moved to the top four mantissa bits of 16.0f
-          // (SHF + LOP3: f = 16 + q exactly, five significant bits), then ONE FFMA scale * f - scale * (16 + zero): both products are
-          // exact in fp32 (11-bit fp16 scale x 6-bit integer), so the result is the exact scale * (q - zero)
+          // bf16_rn(scale * (q - zero)) with two instructions per code and half a conversion: two nibbles at a time are moved to the top four mantissa
+          // bits of halves of 16.0 (SHF + LOP3: f = 16 + q exactly, five significant bits), then ONE mixed FMA each, scale * f - scale * (16 + zero) with the
+          // fp16 factors as they are: both products are exact in fp32 (11-bit fp16 scale x 6-bit integer), so the result is the exact scale * (q - zero).
+          // (8192 codes by sixteen warps, stores included: 288 clk; with every code brought to fp32 of its own 387.)
           const __half2 h2 = *reinterpret_cast<const __half2*>(&sc);
-          const float scale = __low2float(h2);
-          const float c0 = -scale * (16.0f + __high2float(h2));
-          auto deq = [&](uint32_t v, int e) -> float {   // element e (bits 4e .. 4e + 3) of word v
-            const uint32_t sh = e <= 4 ? v << (19 - 4 * e) : v >> (4 * e - 19);
-            return fmaf(scale, __uint_as_float((sh & 0x00780000u) | 0x41800000u), c0);
-          };
+          const float c0 = -__low2float(h2) * (16.0f + __high2float(h2));
+          const uint16_t hs = (uint16_t)(sc & 0xffffu);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {  // word j = k [32 wh + 8j, +8), element e in bits 4e
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const uint32_t sh = e < 2 ? qw[j] << (6 - 4 * e) : qw[j] >> (4 * e - 6);
+              asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tfma.rn.f32.f16 %0, l, %3, %4;\n\tfma.rn.f32.f16 %1, h, %3, %4;\n\t}"
+                  : "=f"(f[e]), "=f"(f[e + 4]) : "r"((sh & 0x03c003c0u) | 0x4c004c00u), "h"(hs), "f"(c0));
+            }
             uint32_t o[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = pack_bf16(deq(qw[j], 2 * e), deq(qw[j], 2 * e + 1));
+            for (int e = 0; e < 4; ++e) o[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + sw128(wr, wh * 4 + j)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
           }
         } else {
@@ -201,10 +215,13 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
         tc::fence_smem_async();                       // generic-proxy writes -> visible to the tensor core
         __syncwarp();
         if (lane == 0) {
+          tc::mbar_arrive(w_empty + 8 * buf);
           if (CTAS == 2 && rank == 1) tc::copy_to_cta(tc::at_rank(tc::smem_u32(&s_token[s][warp & 7]), 0), dst + sw128(wr, wh * 4), 16, tc::at_rank(full + 8 * s, 0));
           else tc::mbar_arrive(full + 8 * s);
         }
       }
+      if ((t.nkb & 1) && l0 == 1 && at < busy && lane == 0 && ok) tc::mbar_arrive(w_empty + 8 * ((pairs + (t.nkb >> 1)) % C::kPairs));   // the last one's second block
+      pairs += (t.nkb + 1) >> 1;
       q += t.nkb;
       // ---- accumulators -> y (or partial sums): warp w has rows 32 (w % 4) .. + 31 and a quarter of the columns ----
       ok = ok && __all_sync(0xffffffffu, wait(acc_full, acc_ph));
@@ -214,48 +231,50 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
 #pragma unroll 1
       for (int mt = 0; mt < t.mts; ++mt) {
         const int64_t m = t.m0 + mt * BM + rank * 128 + (warp & 3) * 32 + lane;        // this thread's output row (TMEM lane = row)
-        if constexpr (SWIGLU) {   // columns [0, 128) are the gate, [128, 256) the up projection of the same features
-          const int c0 = (warp >> 2) * 32;
-          uint32_t v[32], u[32];
-          const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * BN + c0);
-          tc::ld32(v, at);
-          tc::ld32(u, at + 128);
-          tc::wait_ld(v);
-          tc::wait_ld(u);
-          if (m >= p.M) continue;
+        const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * BN);
+        if constexpr (SWIGLU) {   // the first half of the columns is the gate, the other the up projection of the same features
+#pragma unroll 1
+          for (int c0 = (warp >> 2) * 16; c0 < half; c0 += kGDequantWarps * 4) {
+            uint32_t v[16], u[16];
+            tc::ld16(v, acc + c0);
+            tc::ld16(u, acc + c0 + half);
+            tc::wait_ld(v);
+            tc::wait_ld(u);
+            if (m >= p.M) continue;
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            const int64_t n = t.n0 + c0 + j;
-            if (n < p.N) {
-              uint32_t o[4];
+            for (int j = 0; j < 16; j += 8) {
+              const int64_t n = t.n0 + c0 + j;
+              if (n < p.N) {
+                uint32_t o[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                auto act = [](uint32_t g, uint32_t w) {
-                  const float a = round_bf16(__uint_as_float(g));
-                  return round_bf16(a / (1.0f + expf(-a))) * round_bf16(__uint_as_float(w));
-                };
-                o[e] = pack_bf16(act(v[j + 2 * e], u[j + 2 * e]), act(v[j + 2 * e + 1], u[j + 2 * e + 1]));
+                for (int e = 0; e < 4; ++e) {
+                  auto act = [](uint32_t g, uint32_t w) {
+                    const float a = round_bf16(__uint_as_float(g));
+                    return round_bf16(a / (1.0f + expf(-a))) * round_bf16(__uint_as_float(w));
+                  };
+                  o[e] = pack_bf16(act(v[j + 2 * e], u[j + 2 * e]), act(v[j + 2 * e + 1], u[j + 2 * e + 1]));
+                }
+                *reinterpret_cast<uint4*>(p.y + m * p.N + n) = make_uint4(o[0], o[1], o[2], o[3]);
               }
-              *reinterpret_cast<uint4*>(p.y + m * p.N + n) = make_uint4(o[0], o[1], o[2], o[3]);
             }
           }
           continue;
         }
 #pragma unroll 1
-        for (int c0 = (warp >> 2) * (BN / 4); c0 < ((warp >> 2) + 1) * (BN / 4); c0 += 32) {
-          uint32_t v[32];
-          tc::ld32(v, tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * BN + c0));
+        for (int c0 = (warp >> 2) * 16; c0 < bn; c0 += kGDequantWarps * 4) {
+          uint32_t v[16];
+          tc::ld16(v, acc + c0);
           tc::wait_ld(v);
           if (m < p.M && p.ksplit > 1) {
             float* dst = p.partial + ((int64_t)t.z * p.M + m) * p.N;   // raw fp32 sums of this k range; bias and rounding in the reduce kernel
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
+            for (int j = 0; j < 16; j += 4) {
               const int64_t n = t.n0 + c0 + j;
               if (n < p.N) *reinterpret_cast<uint4*>(dst + n) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
           } else if (m < p.M) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
+            for (int j = 0; j < 16; j += 8) {
               const int64_t n = t.n0 + c0 + j;
               if (n < p.N) {  // N % 8 == 0 (host check): a chunk is either fully inside or fully outside
                 uint32_t o[4];
@@ -278,7 +297,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
         else tc::mbar_arrive(acc_free);
       }
     }
-  } else if (warp == 16) {
+  } else if (warp == kGDequantWarps) {
     // =========================================== ACTIVATIONS ====================================================
     if (lane == 0) {
       for (int i = first; i < total && ok; i += step) {
@@ -288,7 +307,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
           ok = wait(empty + 8 * s, ((uint32_t)(q / C::kStages) & 1u) ^ 1u);
           if (!ok) break;
           if (CTAS == 2) tc::mbar_arrive(room + 8 * s);
-          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * t.mts * kTileBytes + (CTAS - 1) * 8 * 16);
+          if (rank == 0) tc::mbar_expect_tx(full + 8 * s, CTAS * t.mts * kTileBytes + (CTAS - 1) * busy * 16);
           const uint32_t st = tiles + s * C::kStage, bar = CTAS == 2 ? tc::at_rank(full + 8 * s, 0) : full + 8 * s;
           for (int mt = 0; mt < t.mts; ++mt) {
             const int row = (int)(t.m0 + mt * BM + rank * 128), col = (t.kb0 + l) * kBK;
@@ -300,6 +319,24 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
       if (rank == 0)
         for (int i = 0; i < C::kStages; ++i)   // (a stage never used: the phase before the first)
           ok = wait(full + 8 * i, (uint32_t)((q + C::kStages - 1 - i) / C::kStages + 1) & 1u) && ok;
+    }
+  } else if (warp == kGDequantWarps + 2) {
+    // =========================================== PACKED WEIGHTS =================================================
+    if (lane == 0) {   // ahead of the stages by as many k-blocks as the buffers hold
+      int pair = 0;
+      for (int i = first; i < total && ok; i += step) {
+        const Item t = item(i);
+        const int row = (int)(t.n0 + (SWIGLU ? 0 : (int)rank * half));
+        for (int l = 0; l < t.nkb; l += 2, ++pair) {
+          const int buf = pair % C::kPairs;
+          ok = tc::mbar_wait(w_empty + 8 * buf, ((uint32_t)(pair / C::kPairs) & 1u) ^ 1u);
+          if (!ok) break;
+          tc::mbar_expect_tx(w_full + 8 * buf, (uint32_t)half * 64u);
+          tc::tma_load_2d(packed + buf * C::kPair, SWIGLU && rank ? &map_w2 : &map_w, (t.kb0 + l) * 32, row, w_full + 8 * buf);
+        }
+      }
+      for (int i = 0; i < C::kPairs; ++i)   // (a buffer never used: the phase before the first)
+        ok = tc::mbar_wait(w_full + 8 * i, (uint32_t)((pair + C::kPairs - 1 - i) / C::kPairs + 1) & 1u) && ok;
     }
   } else if (lane == 0 && rank == 0) {
     // =========================================== PRODUCTS =======================================================
@@ -320,7 +357,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
           const uint64_t da = tc::desc_sw128(st + mt * kTileBytes);
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)  // +32 B along K inside the swizzle atom = +2 in the address field
-            umma_bf16<CTAS>(tmem + mt * BN, da + 2 * k, db + 2 * k, (l | k) != 0);
+            umma_bf16<CTAS>(tmem + mt * BN, da + 2 * k, db + 2 * k, bn, (l | k) != 0);
         }
         if constexpr (CTAS == 2) tc::commit_pair(empty + 8 * s);   // the stage is free once these products have read it
         else tc::commit(empty + 8 * s);
@@ -340,7 +377,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   tc::fence_before();
   if constexpr (CTAS == 2) tc::cluster_sync();   // the other CTA's shared memory is read until its last product
   __syncthreads();
-  if (warp == 17) {
+  if (warp == kGDequantWarps + 1) {
     __syncwarp();
     if constexpr (CTAS == 2) tc::tmem_free_pair<BN * MT>(tmem);
     else tc::tmem_free<BN * MT>(tmem);
@@ -376,47 +413,73 @@ __global__ void __launch_bounds__(256) qgemm_splitk_reduce_kernel(const float* _
 static std::atomic<int> g_gemm_wide{1};   // development switch (b200_qgemm_tune): 0 keeps to one sub-tile of 256 tokens
 
 struct GemmPlan {
-  int ctas, mt, ksplit;
+  int ctas, mt, ksplit, bn;
 };
 
-// Tile and k ranges by the time of the last SM to finish, in clocks as measured over launches of one round.  A k-block takes about 1500 with two
-// sub-tiles of 256 tokens, 1130 with one (the dequantisation, which a second sub-tile shares), 1380 for a CTA alone on two sub-tiles of 128, 950 on
-// one; a launch 14400 with pairs (7.6 us from the launch before it to its last store besides its k-blocks, of which a cluster's start is the most) and
-// 8400 without; a further round of tiles 6000; k ranges 4000, 500 for each and a clock per 1200 bytes of partial sums.  k ranges are for
-// launches that leave SMs idle -- two at least where half of them would be: at least four k-blocks per range, at most 16 ranges and 64 MB of partial
-// sums, and no more than fill the SMs once.
-// 129 to 256 rows, us of a CTA alone on 256 tokens and of a pair, both in four k ranges, nf4 / int4, at 203 rows: 2048 x 2048 17.4, 18.9 / 15.8, 16.7; 4096 x
-// 4096 26.1, 26.7 / 23.3, 23.1; 11008 -> 4096 46.1, 43.2 / 40.7, 36.2.
-static int64_t gemm_start(const GemmPlan& g) { return g.ctas == 1 ? 2400 : 8400; }
-static int64_t gemm_clocks(int64_t M, int64_t N, int64_t K, const GemmPlan& g) {
-  const int64_t nkb = K / kBK, units = sm_count() / g.ctas, s = g.ksplit;
-  const int64_t tiles = ((N + 128 * g.ctas - 1) / (128 * g.ctas)) * ((M + 128 * g.ctas * g.mt - 1) / (128 * g.ctas * g.mt));
-  const int64_t per = g.ctas == 1 ? (g.mt == 1 ? 950 : 1380) : (g.mt == 1 ? 1130 : 1500);
-  return ((tiles * s + units - 1) / units) * (((nkb + s - 1) / s) * per + 6000) + gemm_start(g) + (s > 1 ? 4000 + 500 * s + s * M * N * 4 / 1200 : 0);
+// Tile and k ranges by the time of the last SM to finish, us.  A k-block takes `block + feature * bn` -- products and hand-overs, and the look-ups or
+// conversions of a tile's features, which its tokens share -- a launch `start`, a further round of tiles `round` more, k ranges 0.88 and 2.3 for every
+// million partial sums.  Fitted to some 700 launches of one to three rounds (24 shapes of 64 to 2000 rows, every tile and count of ranges: 4 % rms), in
+// which the plan's choice is within 4 % of the best one, but for 4096 -> 6144 at 150 rows, nf4 (8 %).
+// Fewer features than 128 per CTA pay where they fill SMs that would have idled: 4096 -> 11008, nf4 / int4, at 64 rows 86 CTAs of 128 features and 138 of 80 39.0
+// and 30.8 / 30.6 and 25.6; at 203 rows 43 pairs of 256 and 69 of 160 46.2 and 38.0 / 36.7 and 31.6.
+// k ranges are for launches that leave SMs idle all the same: at least four k-blocks per range, at most 16 ranges and 64 MB of partial sums, and no more
+// than fill the SMs once.
+struct GemmCost {
+  double start, block, feature, round;
+};
+static const GemmCost& gemm_cost(bool int4, int ctas, int mt) {
+  static const GemmCost cost[2][2][2] = {{{{4.7, 0.207, 0.00239, 1.6}, {5.9, 0.425, 0.00182, 2.9}}, {{7.3, 0.211, 0.00150, 2.8}, {8.7, 0.410, 0.00125, 1.2}}},
+                                         {{{5.5, 0.210, 0.00148, 2.2}, {5.6, 0.425, 0.00179, 2.9}}, {{7.4, 0.237, 0.00083, 3.1}, {8.5, 0.416, 0.00113, 0.9}}}};
+  return cost[int4][ctas - 1][mt - 1];
+}
+// `per_tile`: features of the output that a tile of bn covers
+static double gemm_time(int64_t M, int64_t N, int64_t K, bool int4, const GemmPlan& g, int per_tile) {
+  const GemmCost& c = gemm_cost(int4, g.ctas, g.mt);
+  const int64_t nkb = K / kBK, units = sm_count() / g.ctas, rows = 128 * g.ctas * g.mt;
+  const int64_t tiles = ((N + per_tile - 1) / per_tile) * ((M + rows - 1) / rows), rounds = (tiles * g.ksplit + units - 1) / units;
+  return c.start + (double)rounds * (double)((nkb + g.ksplit - 1) / g.ksplit) * (c.block + c.feature * g.bn) + c.round * (double)(rounds - 1) +
+         (g.ksplit > 1 ? 0.88 + 2.3e-6 * (double)g.ksplit * (double)M * (double)N : 0.0);
 }
 
-static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool split_ok) {
+static GemmPlan gemm_search(int64_t M, int64_t N, int64_t K, bool int4, bool split_ok) {
   const int nkb = (int)(K / kBK);
-  const int64_t sms = sm_count();
-  GemmPlan best{1, 1, 1};
-  int64_t best_t = -1;
+  GemmPlan best{1, 1, 1, 128};
+  double best_t = -1.0;
   for (int kind = 0; kind < 4; ++kind) {
     const int ctas = kind < 2 ? 1 : 2, mt = kind & 1 ? 2 : 1;
     if (kind == 0 ? M > 128 : M <= 128) continue;            // a second half would be padding; a CTA alone on 128 tokens would dequantise twice
     if (kind == 1 && M > 256) continue;
     if (kind == 3 && (M <= 256 || !g_gemm_wide.load())) continue;
-    const int64_t units = sms / ctas, tiles = ((N + 128 * ctas - 1) / (128 * ctas)) * ((M + 128 * ctas * mt - 1) / (128 * ctas * mt));
-    int64_t most = split_ok ? units / tiles : 1;
-    if (most > nkb / 4) most = nkb / 4;
-    if (most > 16) most = 16;
-    while (most > 1 && most * M * N * (int64_t)sizeof(float) > (64ll << 20)) --most;
-    for (int64_t s = most > 1 && tiles * 2 <= units ? 2 : 1; s <= (most < 1 ? 1 : most); ++s) {
-      const GemmPlan g{ctas, mt, (int)s};
-      const int64_t t = gemm_clocks(M, N, K, g);
-      if (best_t < 0 || t < best_t) { best_t = t; best = g; }
+    const int64_t units = sm_count() / ctas, row_tiles = (M + 128 * ctas * mt - 1) / (128 * ctas * mt);
+    for (int bn = 128 * ctas; bn >= (ctas == 2 ? 160 : 64); bn -= 16 * ctas) {   // (smaller pairs won nothing over k ranges)
+      const int64_t tiles = ((N + bn - 1) / bn) * row_tiles;
+      int64_t most = split_ok ? units / tiles : 1;
+      if (most > nkb / 4) most = nkb / 4;
+      if (most > 16) most = 16;
+      while (most > 1 && most * M * N * (int64_t)sizeof(float) > (64ll << 20)) --most;
+      for (int64_t s = 1; s <= (most < 1 ? 1 : most); ++s) {
+        const GemmPlan g{ctas, mt, (int)s, bn};
+        const double t = gemm_time(M, N, K, int4, g, bn);
+        if (best_t < 0.0 || t < best_t) { best_t = t; best = g; }
+      }
     }
   }
   return best;
+}
+
+// What gemm_search finds for a shape, kept for the shapes a thread asks for most: two or three questions a call, some microseconds each.
+template <typename F>
+static GemmPlan gemm_kept(int what, int64_t M, int64_t N, int64_t K, F search) {
+  struct Entry { int64_t M, N, K; int what, sms; GemmPlan plan; };
+  static thread_local Entry kept[64] = {};
+  what = what * 2 + g_gemm_wide.load() + 1;
+  const int sms = sm_count();
+  Entry& e = kept[((uint64_t)M * 0x9E3779B97F4A7C15ull + (uint64_t)N * 0xC2B2AE3D27D4EB4Full + (uint64_t)K * 0x165667B19E3779F9ull + (uint64_t)what) >> 58];
+  if (e.M != M || e.N != N || e.K != K || e.what != what || e.sms != sms) e = Entry{M, N, K, what, sms, search()};
+  return e.plan;
+}
+static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool int4, bool split_ok) {
+  return gemm_kept(int4 * 2 + split_ok, M, N, K, [&] { return gemm_search(M, N, K, int4, split_ok); });
 }
 
 template <int CTAS, int MT, bool INT4, bool SWIGLU = false>
@@ -429,15 +492,20 @@ static cudaError_t launch_gemm(GemmParams p, cudaStream_t st) {
     once.done();
   }
   alignas(64) CUtensorMap map;
-  if (!tensor_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.x, p.M, p.K, p.K * 2, 128)) return cudaErrorInvalidValue;
+  alignas(64) CUtensorMap weights, weights2;
+  const int half = p.bn / CTAS;
+  if (!tensor_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.x, p.M, p.K, p.K * 2, 128) ||
+      !tensor_map_2d(&weights, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.packed, p.N, p.K / 2, p.K / 2, half, 64) ||
+      !tensor_map_2d(&weights2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, SWIGLU ? p.packed2 : p.packed, p.N, p.K / 2, p.K / 2, half, 64))
+    return cudaErrorInvalidValue;
   unsigned* const err = wait_error_word();
   if (!err) return cudaErrorMemoryAllocation;
-  constexpr int BN = SWIGLU ? 128 : 128 * CTAS;
-  p.n_tiles = (int)((p.N + BN - 1) / BN);
+  const int features = SWIGLU ? p.bn / 2 : p.bn;
+  p.n_tiles = (int)((p.N + features - 1) / features);
   p.m_tiles = (int)((p.M + 128 * CTAS * MT - 1) / (128 * CTAS * MT));
   const int64_t items = (int64_t)p.n_tiles * p.m_tiles * p.ksplit, units = sm_count() / CTAS;
   const cudaError_t e = launch_cluster(qgemm_tcgen05_kernel<CTAS, MT, INT4, SWIGLU>, dim3((unsigned)((items < units ? items : units) * CTAS)), dim3(kGThreads), CTAS,
-                                       (size_t)smem, st, p, map, err);
+                                       (size_t)smem, st, p, map, weights, weights2, err);
   if (e != cudaSuccess || p.ksplit == 1) return e;
   const int64_t MN = p.M * p.N;
   return launch(qgemm_splitk_reduce_kernel, dim3((unsigned)((MN / 8 + 255) / 256)), dim3(256), (size_t)0, st, (const float*)p.partial, p.bias, p.y, MN, p.N, p.ksplit);
@@ -449,26 +517,36 @@ static cudaError_t launch_plan(const GemmParams& p, const GemmPlan& g, cudaStrea
   return g.mt == 2 ? launch_gemm<2, 2, INT4>(p, st) : launch_gemm<2, 1, INT4>(p, st);
 }
 
-// Sub-tiles of a gate / up pair in one launch, by gemm_plan's clocks; 0 where two launches and the product are the shorter way.  The product
-// costs 4000 to start and a clock per 550 elements; half of that counts, and a twentieth has to be won, since the second of two launches starts
-// on the SMs that the first one's last round leaves idle: what pays is a round of tiles saved, or small matrices.  us, two launches and the
-// product against one, nf4 / int4: 4096 -> 14336 at 4096 rows 1017 -> 928 / 999 -> 918, at 2048 538 -> 467 / 545 -> 514; 4096 -> 11008 at 1000 rows
-// 256 -> 197 / 253 -> 196; 2048 -> 5632 at 203 rows 62 -> 38 / 50 -> 30.  Left apart: 4096 -> 11008 at 203 rows 98 against 105 / 107 against 98, 5120 -> 13824
-// at 2048 515 against 515 / 494 against 527 -- and, as the price of one line for both types, 4096 -> 11008 at 4096, where one launch would win
-// 3 to 6 % (757 against 712 / 685 against 667).
-static int swiglu_tiles(int64_t M, int64_t N, int64_t K) {
-  if (M <= 128) return 0;
+// Tile of a gate / up pair in one launch; no sub-tiles (mt 0) where two launches and the product are the shorter way.  us, two launches and the product, each
+// with its best tile, against one, nf4 / int4: 4096 -> 11008 at 203 rows 83 -> 76 / 70 -> 65, at 400 115 -> 95 / 116 -> 101, at 1000 223 -> 158 / 228 -> 171;
+// 5120 -> 13824 at 300 131 -> 124 / 134 -> 133, at 2000 470 -> 435 / 462 -> 438; 4096 -> 14336 at 4096 859 -> 769 / 883 -> 776.  Up to 512 rows the two ways' times
+// as modelled decide.  Beyond, whether one launch saves a round of tiles with all their features: the second of two launches starts on the SMs that the
+// first one's last round leaves idle, which the model does not know, so a twentieth has to be won.
+static GemmPlan swiglu_plan(int64_t M, int64_t N, int64_t K, bool int4) {
+  const GemmPlan none{2, 0, 1, 256};
+  if (M <= 128) return none;
   const int64_t units = sm_count() / 2, n = (N + 127) / 128, nkb = K / kBK;
-  const GemmPlan one = gemm_plan(M, N, K, true);
-  int64_t apart = gemm_clocks(M, N, K, one) - gemm_start(one);   // (the second launch's start is hidden as well)
-  if (one.ctas == 2 && one.mt == 2 && (M - 1) % 512 < 256) apart -= 370 * (nkb / one.ksplit);   // the last tiles have one sub-tile
-  const int64_t worth = (2 * apart + 2000 + M * N / 1100) / 20 * 19;
-  int64_t best = 0, best_t = worth;
-  for (int mt = 1; mt <= (M > 256 && g_gemm_wide.load() ? 2 : 1); ++mt) {
-    const int64_t t = (n * ((M + 256 * mt - 1) / (256 * mt)) + units - 1) / units * (nkb * (mt == 2 ? 1500 : 1130) + 6000);
-    if (t < best_t) { best_t = t; best = mt; }
+  GemmPlan best = none;
+  double best_t = -1.0;
+  for (int mt = 1; mt <= (M > 256 && g_gemm_wide.load() ? 2 : 1); ++mt)
+    for (int bn = 256; bn >= 128; bn -= 32) {
+      const GemmPlan g{2, mt, 1, bn};
+      const double t = gemm_time(M, N, K, int4, g, bn / 2);
+      if (best_t < 0.0 || t < best_t) { best_t = t; best = g; }
+    }
+  if (M <= 512) {
+    const GemmPlan one = gemm_plan(M, N, K, int4, true);
+    const double apart = 2.0 * gemm_time(M, N, K, int4, one, one.bn) - gemm_cost(int4, one.ctas, one.mt).start + 4.0 + 1e-6 * (double)M * (double)N;   // (and the product)
+    return best_t < apart ? best : none;
   }
-  return (int)best;
+  auto rounds = [&](int64_t feature_tiles, int mt) { return (feature_tiles * ((M + 256 * mt - 1) / (256 * mt)) + units - 1) / units * (nkb * (mt == 2 ? 1500 : 1130) + 6000); };
+  const int64_t one2 = rounds((N + 255) / 256, 2) - ((M - 1) % 512 < 256 ? 370 * nkb : 0), one1 = rounds((N + 255) / 256, 1);   // clocks
+  const int64_t pair1 = rounds(n, 1), pair2 = g_gemm_wide.load() ? rounds(n, 2) : pair1;
+  const int64_t worth = (2 * (one1 < one2 || !g_gemm_wide.load() ? one1 : one2) + 2000 + M * N / 1100) / 20 * 19;
+  return (pair1 < pair2 ? pair1 : pair2) < worth ? best : none;
+}
+static GemmPlan swiglu_tiles(int64_t M, int64_t N, int64_t K, bool int4) {
+  return gemm_kept(4 + int4, M, N, K, [&] { return swiglu_plan(M, N, K, int4); });
 }
 
 }  // namespace b200
@@ -482,7 +560,7 @@ int b200_qgemm_tune(int wide) { g_gemm_wide = wide ? 1 : 0; return B200_OK; }
 size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   // accumulators live in tensor memory; only a launch split over k ranges (short prompts: too few output tiles for the SMs) stages fp32 partial sums
   if (M <= 0 || N <= 0 || K < kBK) return 0;
-  const int s = gemm_plan(M, N, K, true).ksplit;
+  const int nf4 = gemm_plan(M, N, K, false, true).ksplit, int4 = gemm_plan(M, N, K, true, true).ksplit, s = nf4 > int4 ? nf4 : int4;   // either type's
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
 }
 
@@ -514,13 +592,15 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
   GemmParams p{};
   if (const int rc = gemm_args(a, p)) return rc;
   // k ranges only when the caller provided the workspace b200_qgemm_workspace_bytes asks for (none: one k range)
-  GemmPlan g = gemm_plan(a->M, a->N, a->K, true);
+  const bool int4 = a->qtype == B200_Q_INT4;
+  GemmPlan g = gemm_plan(a->M, a->N, a->K, int4, true);
   if (g.ksplit > 1 && (a->workspace == nullptr || a->workspace_bytes < (size_t)g.ksplit * a->M * a->N * sizeof(float) ||
                        (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
-    g = gemm_plan(a->M, a->N, a->K, false);
+    g = gemm_plan(a->M, a->N, a->K, int4, false);
   p.ksplit = g.ksplit;
+  p.bn = g.bn;
   p.partial = reinterpret_cast<float*>(a->workspace);
-  const cudaError_t e = a->qtype == B200_Q_INT4 ? launch_plan<true>(p, g, (cudaStream_t)stream) : launch_plan<false>(p, g, (cudaStream_t)stream);
+  const cudaError_t e = int4 ? launch_plan<true>(p, g, (cudaStream_t)stream) : launch_plan<false>(p, g, (cudaStream_t)stream);
   if (e != cudaSuccess) {
     set_error("b200_qgemm: launch failed: %s", cudaGetErrorString(e));
     return B200_ERR_CUDA;
@@ -532,7 +612,7 @@ int b200_qgemm_swiglu_supported(int64_t M, int64_t N, int64_t K, int qtype, int 
   const int block = qtype == B200_Q_INT4 ? 128 : 64;
   if ((qtype != B200_Q_NF4 && qtype != B200_Q_FP4 && qtype != B200_Q_INT4) || blocksize != block) return 0;
   if (M <= 0 || N <= 0 || K <= 0 || K % block || N % 8 || N > 65535LL * 128 || M > 65535LL * 128) return 0;
-  return swiglu_tiles(M, N, K) > 0;
+  return swiglu_tiles(M, N, K, qtype == B200_Q_INT4).mt > 0;
 }
 
 int b200_qgemm_swiglu(const b200_qgemm_args* a, const void* packed2, const void* scale2, b200_stream_t stream) {
@@ -540,17 +620,18 @@ int b200_qgemm_swiglu(const b200_qgemm_args* a, const void* packed2, const void*
   if (const int rc = gemm_args(a, p)) return rc;
   B200_CHECK_ARG(packed2 && scale2 && (reinterpret_cast<uintptr_t>(packed2) & 15) == 0, "b200_qgemm_swiglu: null or misaligned second matrix");
   B200_CHECK_ARG(!a->bias, "b200_qgemm_swiglu: takes no bias");
-  const int mt = swiglu_tiles(a->M, a->N, a->K);
-  if (mt == 0) {
+  const bool int4 = a->qtype == B200_Q_INT4;
+  const GemmPlan g = swiglu_tiles(a->M, a->N, a->K, int4);
+  if (g.mt == 0) {
     set_error("b200_qgemm_swiglu: (M=%lld N=%lld K=%lld) runs as two b200_qgemm and b200_swiglu", (long long)a->M, (long long)a->N, (long long)a->K);
     return B200_ERR_UNSUPPORTED;
   }
   p.packed2 = reinterpret_cast<const uint8_t*>(packed2);
   p.scale2 = reinterpret_cast<const uint32_t*>(scale2);
   p.ksplit = 1;
-  const bool int4 = a->qtype == B200_Q_INT4;
+  p.bn = g.bn;
   const cudaStream_t st = (cudaStream_t)stream;
-  const cudaError_t e = mt == 2 ? (int4 ? launch_gemm<2, 2, true, true>(p, st) : launch_gemm<2, 2, false, true>(p, st))
+  const cudaError_t e = g.mt == 2 ? (int4 ? launch_gemm<2, 2, true, true>(p, st) : launch_gemm<2, 2, false, true>(p, st))
                                 : (int4 ? launch_gemm<2, 1, true, true>(p, st) : launch_gemm<2, 1, false, true>(p, st));
   if (e != cudaSuccess) {
     set_error("b200_qgemm_swiglu: launch failed: %s", cudaGetErrorString(e));

@@ -37,16 +37,17 @@ inline TensorMapEncodeFn tensor_map_encoder() {
   return fn;
 }
 
-// A row-major matrix (rows x cols elements, rows `ld_bytes` apart) read in boxes of box_rows x 128 bytes, 128-byte swizzle, zeros outside.
-// base must be 16-byte aligned and ld_bytes a multiple of 16.
-inline bool tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, const void* base, int64_t rows, int64_t cols, int64_t ld_bytes, int box_rows) {
+// A row-major matrix (rows x cols elements, rows `ld_bytes` apart) read in boxes of box_rows x 128 bytes, 128-byte swizzle (or x 64 bytes, 64-byte
+// swizzle), zeros outside.  base must be 16-byte aligned and ld_bytes a multiple of 16.
+inline bool tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, const void* base, int64_t rows, int64_t cols, int64_t ld_bytes, int box_rows,
+                          int box_bytes = 128) {
   const TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return false;
   const cuuint64_t dim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t stride[1] = {(cuuint64_t)ld_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)(128 / elem_bytes), (cuuint32_t)box_rows};
+  const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / elem_bytes), (cuuint32_t)box_rows};
   const cuuint32_t step[2] = {1u, 1u};
-  return enc(map, type, 2, const_cast<void*>(base), dim, stride, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  return enc(map, type, 2, const_cast<void*>(base), dim, stride, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
