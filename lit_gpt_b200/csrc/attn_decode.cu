@@ -182,10 +182,10 @@ int b200_attn_decode(const b200_attn_decode_args* a, b200_stream_t stream) {
   int nsplit = a->num_splits;
   if (nsplit <= 0) {
     const int ctas = a->batch * a->n_groups * head_chunks;
-    // measured (tools/attn_bench.py --splits): the kernels are bound by dependent round trips, so short key ranges per
-    // CTA win until the merge grows; about 3 CTAs per SM for the scalar kernel, 1 for the tensor-core one
-    nsplit = ((gqa ? 1 : 3) * sm_count() + ctas - 1) / ctas;
-    const int by_len = gqa ? (a->max_seq + 255) / 256 : (a->max_seq + 31) / 32;   // gqa: two 32-key tiles per warp at least
+    // measured (tools/attn_bench.py --splits): the scalar kernel is bound by dependent round trips, so short key ranges per
+    // CTA win until the merge grows, at about 3 CTAs per SM; the tensor-core one has one CTA an SM and a rule of its own
+    nsplit = gqa ? attn_decode_gqa_splits(ctas, a->max_seq, (int64_t)ctas * a->max_seq * a->head_size * 4) : (3 * sm_count() + ctas - 1) / ctas;
+    const int by_len = (a->max_seq + 31) / 32;
     if (nsplit > by_len) nsplit = by_len;
     // many sequences x heads over a long cache (13B, batch 16, 2048 positions: 640 CTAs of 1 MB each): three key ranges per (sequence,
     // head) still pay -- 136 -> 120 us per layer, 4.9 -> 5.6 TB/s (tools/attn_bench.py --splits) -- the last wave is shorter

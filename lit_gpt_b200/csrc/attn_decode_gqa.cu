@@ -325,25 +325,67 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
 
 bool attn_decode_gqa_supported(int head_size, int qpk) { return head_size == kGqHS && qpk >= 2 && qpk <= kGqRows; }
 
+static cudaLaunchConfig_t gqa_cluster_config(int splits, dim3 grid, cudaStream_t st, cudaLaunchAttribute (&attr)[2]) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = (size_t)kGqSmem;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// clusters of `splits` CTAs (one CTA an SM, a cluster within a group of SMs) that run at once; asked of the runtime once per device
+static int gqa_clusters(int splits) {
+  static std::atomic<int> kept[64][9] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / (splits * 2);
+  int n = kept[dev][splits].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = gqa_cluster_config(splits, dim3((unsigned)splits, 1, 1), nullptr, attr);
+    if (cudaFuncSetAttribute(attn_decode_gqa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, attn_decode_gqa_kernel<true>, &cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = sm_count() / (splits * 2);
+    }
+    kept[dev][splits].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// Key ranges per (sequence, group): whatever runs in ONE round of CTAs, by what a CTA takes for its keys (6.3 ns each, all of them together at 6.2 TB/s) and the
+// merge (1.8 to 2.7 us in a cluster, 4 through the workspace).  A second round costs as much as the first: eight sequences, 8 groups of 4 heads,
+// 3000 positions in 1, 2, 3, 4 ranges (64, 128, 192, 256 CTAs) 24.8, 22.3, 30.7, 28.6 us; 1000 positions 11.3, 12.2, 19.6, 18.6; two sequences, 3900 positions in 4, 6, 8, 10
+// ranges (16 clusters of 8 do not fit at once) 13.7, 12.9, 21.0, 19.7; one sequence, 3000 positions in 4, 8, 16, 19 11.6, 9.2, 10.0, 10.0.
+int attn_decode_gqa_splits(int pairs, int max_seq, int64_t bytes) {
+  const int by_len = (max_seq + 255) / 256;   // two 32-key tiles per warp at least
+  int best = 1;
+  double best_t = -1.0;
+  for (int ns = 1; ns <= by_len && ns <= 64; ++ns) {
+    if (ns > 1 && (ns <= 8 ? gqa_clusters(ns) < pairs : (int64_t)pairs * ns > sm_count())) continue;
+    const double keys = 6.3e-3 * max_seq / ns * (double)((int64_t)pairs * ns > sm_count() ? ((int64_t)pairs * ns + sm_count() - 1) / sm_count() : 1), all = (double)bytes / 6.2e6;
+    const double t = (keys > all ? keys : all) + (ns == 1 ? 0.0 : ns <= 8 ? 1.6 + 0.13 * ns : 3.5 + 0.05 * ns);
+    if (best_t < 0.0 || t < best_t) { best_t = t; best = ns; }
+  }
+  return best;
+}
+
 cudaError_t launch_attn_decode_gqa(const AttnParams& p, dim3 grid, cudaStream_t st) {
   const bool cluster = grid.x >= 2 && grid.x <= 8;
   auto kernel = cluster ? attn_decode_gqa_kernel<true> : attn_decode_gqa_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem);
   if (e != cudaSuccess) return e;
   if (!cluster) return launch(kernel, grid, dim3(128), (size_t)kGqSmem, st, p);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = (size_t)kGqSmem;
-  cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = grid.x;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
+  cudaLaunchConfig_t cfg = gqa_cluster_config((int)grid.x, grid, st, attr);
   cfg.numAttrs = g_pdl.load(std::memory_order_relaxed) ? 2 : 1;
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaLaunchKernelEx(&cfg, kernel, p);
