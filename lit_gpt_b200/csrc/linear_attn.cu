@@ -17,6 +17,7 @@
 //   1. walk every piece from S = 0 without read-out: its own contribution D and the product P of its decays;
 //   2. scan_kernel: the state at the start of every piece, S <- P S + D from piece to piece, and the sequence's final state;
 //   3. walk every piece from its starting state with read-out.
+// With decays per channel and enough rows and heads the pieces are not walked but worked on by matrix products (linear_chunk.cuh).
 // No logarithm or quotient of decays is taken, so any decay in [0, 1] is safe.  A sequence that starts at position 0 starts from
 // S = 0 whatever its slot holds.  The state is stored [head][dk][dv].
 #include "common.cuh"
@@ -44,6 +45,7 @@ struct LaArgs {
   float* ws_state;                  // [seq][piece][head][dk][dv]
   float* ws_prod;                   // [seq][piece][head][dk]
   int vec_k, vec_z, vec_v, vec_s;   // 16-byte accesses possible on q and k / z / v / the state
+  int pair_o;                       // 8-byte ones on the read-out (and the states)
 };
 
 typedef unsigned long long f2;   // two packed floats
@@ -352,25 +354,43 @@ cudaError_t walk_launch(const LaArgs& A, int n_seqs, cudaStream_t st) {
   return launch(walk_kernel<T, TQ, LK, KPL, CHANNEL, MODE>, grid, dim3(kLaThreads), smem, st, A);
 }
 
-template <typename T, typename TQ, int LK, int KPL, bool CHANNEL>
-cudaError_t scan_launch(const LaArgs& A, int n_seqs, cudaStream_t st) {
-  if (A.n_pieces <= 1) return walk_launch<T, TQ, LK, KPL, CHANNEL, 0>(A, n_seqs, st);
-  cudaError_t e = walk_launch<T, TQ, LK, KPL, CHANNEL, 1>(A, n_seqs, st);
-  if (e != cudaSuccess) return e;
+cudaError_t states_launch(const LaArgs& A, int n_seqs, cudaStream_t st) {
   const bool v4 = A.vec_s && A.dv % 4 == 0;
   const int64_t per = (int64_t)A.dk * A.dv / (v4 ? 4 : 1);
   const dim3 grid((unsigned)((per + 255) / 256), (unsigned)A.heads, (unsigned)n_seqs);
-  e = v4 ? launch(scan_kernel<4>, grid, dim3(256), 0, st, A) : launch(scan_kernel<1>, grid, dim3(256), 0, st, A);
+  return v4 ? launch(scan_kernel<4>, grid, dim3(256), 0, st, A) : launch(scan_kernel<1>, grid, dim3(256), 0, st, A);
+}
+
+}  // namespace
+
+}  // namespace b200
+
+#include "linear_chunk.cuh"
+
+namespace b200 {
+
+namespace {
+
+// qp: pieces on the tensor cores (per-channel decays)
+template <typename T, typename TQ, int LK, int KPL, bool CHANNEL>
+cudaError_t scan_launch(const LaArgs& A, int n_seqs, float* qp, cudaStream_t st) {
+  if constexpr (CHANNEL && LK * KPL <= 128) {
+    if (qp) return piece_launch<T, LK * KPL <= 64 ? 64 : 128>(A, n_seqs, qp, st);
+  }
+  if (A.n_pieces <= 1) return walk_launch<T, TQ, LK, KPL, CHANNEL, 0>(A, n_seqs, st);
+  cudaError_t e = walk_launch<T, TQ, LK, KPL, CHANNEL, 1>(A, n_seqs, st);
+  if (e != cudaSuccess) return e;
+  e = states_launch(A, n_seqs, st);
   if (e != cudaSuccess) return e;
   return walk_launch<T, TQ, LK, KPL, CHANNEL, 2>(A, n_seqs, st);
 }
 
 // qk_f32: queries and keys are fp32 whatever T is (with fixed decays)
 template <typename T, int LK, int KPL>
-cudaError_t pick_launch(const LaArgs& A, int n_seqs, bool channel, bool qk_f32, cudaStream_t st) {
-  if (channel) return scan_launch<T, T, LK, KPL, true>(A, n_seqs, st);
-  if (qk_f32) return scan_launch<T, float, LK, KPL, false>(A, n_seqs, st);
-  return scan_launch<T, T, LK, KPL, false>(A, n_seqs, st);
+cudaError_t pick_launch(const LaArgs& A, int n_seqs, bool channel, bool qk_f32, float* qp, cudaStream_t st) {
+  if (channel) return scan_launch<T, T, LK, KPL, true>(A, n_seqs, qp, st);
+  if (qk_f32) return scan_launch<T, float, LK, KPL, false>(A, n_seqs, nullptr, st);
+  return scan_launch<T, T, LK, KPL, false>(A, n_seqs, nullptr, st);
 }
 
 int la_cols(int dk) { return kLaThreads / (dk <= 64 ? 8 : dk <= 128 ? 16 : 32) * kLaNC; }
@@ -384,6 +404,27 @@ int la_piece(int64_t rows, int max_rows, int heads, int dk, int dv) {
   const int64_t want = (rows * blocks + (int64_t)sm_count() * 12 - 1) / ((int64_t)sm_count() * 12);
   int64_t p = (want + 15) / 16 * 16;
   return (int)(p < 32 ? 32 : p);
+}
+
+// floats of the walk's pieces: states and decays
+size_t la_walk_floats(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv) {
+  const int p = la_piece(rows, max_rows, heads, dk, dv);
+  const int64_t pieces = (max_rows + p - 1) / p;
+  return pieces <= 1 ? 0 : (size_t)n_seqs * pieces * heads * dk * (dv + 1);
+}
+// Pieces of kLcC tokens on the tensor cores, for decays per channel (0: not for this shape): states and decays, and the rows' queries from their piece's start
+size_t la_chunk_floats(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv) {
+  if (g_la_piece > 0 || dk > 128 || max_rows < 2 * kLcC) return 0;
+  // Where they are the shorter way (us, walk and pieces, bf16).  128 x 128 per head: 8 heads of 768 rows 58 / 63, of 1024 66 / 64, of 2048 118 / 71,
+  // of 8192 393 / 264; 64 heads of 130 rows 69 / 67, of 256 113 / 70.  64 x 64: 4 heads of 700 rows 29 / 31, of 1024 33 / 29, of 2048 43 / 39.
+  // A CTA's time does not fall with what it leaves empty of its tile, the walk's does: 96 x 96, 8 heads of 2048 rows 98 / 71, but 64 x 64, 8 heads of
+  // 4096 rows (two waves of CTAs) 72 / 76 and 32 x 32, 8 heads of 2048 rows 35 / 41.
+  const int64_t work = rows * heads * dk * dv, tile = (int64_t)(dk <= 64 ? 64 : 128) * ((dv + 127) / 128 * 128);
+  if (work < (dk <= 64 ? 1 << 24 : 1 << 27) || 2 * (int64_t)dk * dv < tile) return 0;
+  if (4 * (int64_t)dk * dv < 3 * tile && (rows + kLcC - 1) / kLcC * heads * ((dv + 127) / 128) > 2 * sm_count()) return 0;
+  const int64_t pieces = (max_rows + kLcC - 1) / kLcC;
+  if ((int64_t)n_seqs * pieces > 65535) return 0;
+  return (((size_t)n_seqs * pieces * heads * dk * (dv + 1) + 3) & ~(size_t)3) + (size_t)rows * heads * dk;
 }
 
 }  // namespace
@@ -401,9 +442,8 @@ int b200_linear_attn_tune(int piece) {
 }
 
 size_t b200_linear_attn_workspace_bytes(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv) {
-  const int p = la_piece(rows, max_rows, heads, dk, dv);
-  const int64_t pieces = (max_rows + p - 1) / p;
-  return pieces <= 1 ? 0 : (size_t)n_seqs * pieces * heads * dk * (dv + 1) * sizeof(float);
+  const size_t walk = la_walk_floats(rows, max_rows, n_seqs, heads, dk, dv), chunks = la_chunk_floats(rows, max_rows, n_seqs, heads, dk, dv);
+  return (walk > chunks ? walk : chunks) * sizeof(float);
 }
 
 int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
@@ -414,10 +454,12 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
   B200_CHECK_ARG(a->dk > 0 && a->dk <= 512 && a->dv > 0, "b200_linear_attn: key size must be 1 .. 512");
   B200_CHECK_ARG(a->state_slot_stride >= (int64_t)a->heads * a->dk * a->dv, "b200_linear_attn: the state slots are too small");
   B200_CHECK_ARG((reinterpret_cast<uintptr_t>(a->seqs) & 15) == 0, "b200_linear_attn: seqs must be 16-byte aligned");
-  const int piece = la_piece(a->rows, a->max_rows, a->heads, a->dk, a->dv);
+  const size_t chunk_floats = a->decay_in ? la_chunk_floats(a->rows, a->max_rows, a->n_seqs, a->heads, a->dk, a->dv) : 0;
+  const bool chunks = chunk_floats && a->workspace && a->workspace_bytes >= chunk_floats * sizeof(float) && (reinterpret_cast<uintptr_t>(a->workspace) & 15) == 0;
+  const int piece = chunks ? kLcC : la_piece(a->rows, a->max_rows, a->heads, a->dk, a->dv);
   const int n_pieces = (a->max_rows + piece - 1) / piece;
   B200_CHECK_ARG((int64_t)a->n_seqs * n_pieces <= 65535, "b200_linear_attn: too many pieces");
-  const size_t need = b200_linear_attn_workspace_bytes(a->rows, a->max_rows, a->n_seqs, a->heads, a->dk, a->dv);
+  const size_t need = chunks ? 0 : la_walk_floats(a->rows, a->max_rows, a->n_seqs, a->heads, a->dk, a->dv) * sizeof(float);
   B200_CHECK_ARG(need == 0 || (a->workspace && a->workspace_bytes >= need), "b200_linear_attn: workspace too small (%zu of %zu bytes)", a->workspace_bytes, need);
   B200_CHECK_ARG(!a->qk_f32 || a->head_decay, "b200_linear_attn: fp32 queries and keys go with fixed decays");
   const size_t esz = a->dtype == B200_F32 ? 4 : 2, qsz = a->qk_f32 ? 4 : esz;
@@ -428,11 +470,13 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
            a->head_decay, a->state, a->state_slot_stride, a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->dk, a->dv, piece, n_pieces,
            ws, ws ? ws + states : nullptr,
            al(a->q, a->ldq * qsz) && al(a->k, a->ldk * qsz) && a->dk % 8 == 0, a->decay_in && al(a->decay_in, a->ld_decay * 4) && a->dk % 8 == 0,
-           al(a->v, a->ldv * esz) && a->dv % 8 == 0, al(a->state, a->state_slot_stride * 4) && al(ws, 0) && a->dv % 4 == 0};
+           al(a->v, a->ldv * esz) && a->dv % 8 == 0, al(a->state, a->state_slot_stride * 4) && al(ws, 0) && a->dv % 4 == 0,
+           a->dv % 2 == 0 && a->ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 7) == 0};
+  float* const qp = chunks ? ws + (chunk_floats - (size_t)a->rows * a->heads * a->dk) : nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   const bool ch = a->decay_in != nullptr;
   B200_FLOAT_TYPES(a->dtype, T, {
-    if (ch && n_pieces > 1) {
+    if (ch && n_pieces > 1 && !chunks) {
       int64_t blocks = (a->rows * a->heads * a->dk + 255) / 256;
       const int64_t cap = (int64_t)sm_count() * 16;
       if (blocks > cap) blocks = cap;
@@ -441,11 +485,11 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
       A.z_ready = 1;
     }
     const bool qf = a->qk_f32 != 0;
-    if (a->dk <= 32) B200_CUDA((pick_launch<T, 8, 4>(A, a->n_seqs, ch, qf, st)));
-    else if (a->dk <= 64) B200_CUDA((pick_launch<T, 8, 8>(A, a->n_seqs, ch, qf, st)));
-    else if (a->dk <= 128) B200_CUDA((pick_launch<T, 16, 8>(A, a->n_seqs, ch, qf, st)));
-    else if (a->dk <= 256) B200_CUDA((pick_launch<T, 32, 8>(A, a->n_seqs, ch, qf, st)));
-    else B200_CUDA((pick_launch<T, 32, 16>(A, a->n_seqs, ch, qf, st)));
+    if (a->dk <= 32) B200_CUDA((pick_launch<T, 8, 4>(A, a->n_seqs, ch, qf, qp, st)));
+    else if (a->dk <= 64) B200_CUDA((pick_launch<T, 8, 8>(A, a->n_seqs, ch, qf, qp, st)));
+    else if (a->dk <= 128) B200_CUDA((pick_launch<T, 16, 8>(A, a->n_seqs, ch, qf, qp, st)));
+    else if (a->dk <= 256) B200_CUDA((pick_launch<T, 32, 8>(A, a->n_seqs, ch, qf, qp, st)));
+    else B200_CUDA((pick_launch<T, 32, 16>(A, a->n_seqs, ch, qf, qp, st)));
   });
   return B200_OK;
 }
