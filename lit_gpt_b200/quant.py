@@ -344,7 +344,11 @@ class QLinear(nn.Module):
         # K = 8192 does not: that call is a small prefill and takes the GEMM); shapes without a tiled layout (toy
         # configs) keep the reference-layout GEMV
         if rows <= GEMV_MAX_ROWS and (self.tiled is None or self.streams(rows)):
-            y = self.gemv(x, bias=self.bias)
+            bias = self.bias
+            if self.tiled is not None and (self.fold == 1 or bias is None):
+                y = K.qgemv_tiled_rows(x, self.tiled, self.out_features, self.in_features, self.quant_type, self.blocksize, bias, self.fold)
+            else:
+                y = self.gemv(x, bias=bias)
         else:
             y = prefill_linear(self, x)
         return y if in_dtype == torch.bfloat16 else y.to(in_dtype)
