@@ -77,10 +77,13 @@ __global__ void __launch_bounds__(128) rope_kv_append_kernel(const __nv_bfloat16
 
 // The same for heads and rotated parts of whole 16-element units whose pointers allow 16-byte accesses.  One CTA per token: a thread keeps
 // one unit -- eight elements and the eight they are turned with -- and walks the heads, so its cosines and sines are read once per token.
-// Bound: bytes (the projection read, q and the cache rows written).  The kernel above, with an element per thread and two barriers per head,
-// takes 116 us for 4096 tokens of 32 + 8 + 8 heads of 128 (100 MB: 15 us at the copy rate).
+// Bound: bytes (the projection read, q and the cache rows written), and how many loads are under way: those of a thread's first heads are issued
+// before the position and the tables that depend on it have arrived.  4096 tokens, 32 + 32 + 32 heads of 128 (201 MB: 31 us at the copy rate): 60 -> 53 us,
+// fp32 tables 50 -> 43; 32 + 8 + 8 heads 41 -> 34 and 32 -> 30 (the kernel above, with an element per thread and two barriers per head, 116).
+// Two heads at a time with bf16 tables, three with fp32 ones, whose turns take fewer registers: three with bf16 tables 51 us, but 13.1 instead
+// of 11.8 for 613 tokens of 40 + 40 + 40 heads; two with fp32 ones 51.
 template <typename PosT, bool TB>
-__global__ void __launch_bounds__(256) rope_kv_append_vec_kernel(const __nv_bfloat16* __restrict__ qkv, const void* __restrict__ cos,
+__global__ void __launch_bounds__(256, 3) rope_kv_append_vec_kernel(const __nv_bfloat16* __restrict__ qkv, const void* __restrict__ cos,
                                                                  const void* __restrict__ sin, int table_presel, int rope_n,
                                                                  const PosT* __restrict__ pos, __nv_bfloat16* __restrict__ kc,
                                                                  __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ q_out, int T,
@@ -90,11 +93,25 @@ __global__ void __launch_bounds__(256) rope_kv_append_vec_kernel(const __nv_bflo
   const int t = blockIdx.x, b = blockIdx.y, units = hs >> 4, lanes = 256 / units;
   const int u = (int)threadIdx.x % units, hl = (int)threadIdx.x / units;
   if (hl >= lanes) return;
-  int64_t ps = (int64_t)pos[t];
-  ps = ps < 0 ? 0 : (ps >= max_seq ? max_seq - 1 : ps);
+  constexpr int R = TB ? 2 : 3;   // heads of a thread whose loads are under way together
+  const int64_t p0 = (int64_t)pos[t];
   const int half = rope_n >> 1, rope_units = rope_n >> 4;
   const bool turns = u < rope_units;
   const int d0 = turns ? u * 8 : rope_n + (u - rope_units) * 16, d1 = turns ? d0 + half : d0 + 8;   // this unit's two runs of eight
+  const int qpk = n_head / n_groups, heads = n_groups * (qpk + 2);
+  const __nv_bfloat16* row = qkv + ((int64_t)b * T + t) * heads * hs;
+  uint4 a[R], c[R];
+  auto fetch = [&](int first) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int hh = first + r * lanes;
+      if (hh >= heads) break;
+      a[r] = *reinterpret_cast<const uint4*>(row + (int64_t)hh * hs + d0);
+      c[r] = *reinterpret_cast<const uint4*>(row + (int64_t)hh * hs + d1);
+    }
+  };
+  fetch(hl);
+  const int64_t ps = p0 < 0 ? 0 : (p0 >= max_seq ? max_seq - 1 : p0);
   float c0[8], c1[8], s0[8], s1[8];
   if (turns) {
     const int64_t at = (table_presel ? (int64_t)t : ps) * rope_n;
@@ -104,34 +121,36 @@ __global__ void __launch_bounds__(256) rope_kv_append_vec_kernel(const __nv_bflo
     };
     get(cos, d0, c0); get(cos, d1, c1); get(sin, d0, s0); get(sin, d1, s1);
   }
-  const int qpk = n_head / n_groups, heads = n_groups * (qpk + 2);
-  const __nv_bfloat16* row = qkv + ((int64_t)b * T + t) * heads * hs;
   auto turn = [](float x, float c, float r, float s) -> float {   // rope_elem's rounding points (the last one is the store's)
     if (TB) return __fadd_rn(round_bf16(__fmul_rn(x, c)), round_bf16(__fmul_rn(r, s)));
     return __fadd_rn(__fmul_rn(x, c), __fmul_rn(r, s));
   };
-#pragma unroll 2
-  for (int hh = hl; hh < heads; hh += lanes) {
-    const int g = hh / (qpk + 2), h = hh - g * (qpk + 2);
-    const __nv_bfloat16* src = row + (int64_t)hh * hs;
-    __nv_bfloat16* dst = h < qpk ? q_out + (((int64_t)b * n_head + g * qpk + h) * T + t) * hs
-                                 : (h == qpk ? kc : vc) + (((int64_t)b * n_groups + g) * max_seq + ps) * hs;
-    const uint4 a = *reinterpret_cast<const uint4*>(src + d0), c = *reinterpret_cast<const uint4*>(src + d1);
-    if (!turns || h == qpk + 1) {
-      *reinterpret_cast<uint4*>(dst + d0) = a;
-      *reinterpret_cast<uint4*>(dst + d1) = c;
-      continue;
-    }
-    const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wc[4] = {c.x, c.y, c.z, c.w};
-    float y0[8], y1[8];
+#pragma unroll 1
+  for (int first = hl; first < heads; first += R * lanes) {
+    if (first != hl) fetch(first);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float x0 = i & 1 ? bf16hi(wa[i >> 1]) : bf16lo(wa[i >> 1]), x1 = i & 1 ? bf16hi(wc[i >> 1]) : bf16lo(wc[i >> 1]);
-      y0[i] = turn(x0, c0[i], -x1, s0[i]);
-      y1[i] = turn(x1, c1[i], x0, s1[i]);
+    for (int r = 0; r < R; ++r) {
+      const int hh = first + r * lanes;
+      if (hh >= heads) break;
+      const int g = hh / (qpk + 2), h = hh - g * (qpk + 2);
+      __nv_bfloat16* dst = h < qpk ? q_out + (((int64_t)b * n_head + g * qpk + h) * T + t) * hs
+                                   : (h == qpk ? kc : vc) + (((int64_t)b * n_groups + g) * max_seq + ps) * hs;
+      if (!turns || h == qpk + 1) {
+        *reinterpret_cast<uint4*>(dst + d0) = a[r];
+        *reinterpret_cast<uint4*>(dst + d1) = c[r];
+        continue;
+      }
+      const uint32_t wa[4] = {a[r].x, a[r].y, a[r].z, a[r].w}, wc[4] = {c[r].x, c[r].y, c[r].z, c[r].w};
+      float y0[8], y1[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float x0 = i & 1 ? bf16hi(wa[i >> 1]) : bf16lo(wa[i >> 1]), x1 = i & 1 ? bf16hi(wc[i >> 1]) : bf16lo(wc[i >> 1]);
+        y0[i] = turn(x0, c0[i], -x1, s0[i]);
+        y1[i] = turn(x1, c1[i], x0, s1[i]);
+      }
+      store8(dst + d0, y0);
+      store8(dst + d1, y1);
     }
-    store8(dst + d0, y0);
-    store8(dst + d1, y1);
   }
 }
 
