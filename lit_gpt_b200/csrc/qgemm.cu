@@ -68,7 +68,10 @@ template <int MT>
 struct GemmTile {
   static constexpr int kStages = MT == 2 ? 4 : 6;
   static constexpr int kStage = (MT + 1) * kTileBytes;     // MT activation tiles + 1 weight tile
-  static constexpr int kPairs = 3, kPair = 128 * 64;       // buffers of packed weights: two k-blocks of 128 features each
+  // Buffers of packed weights: two k-blocks of 128 features each.  Every warp that gives one back has waited for that very pair, so that its arrival cannot
+  // be counted into the phase of the pair before it in the buffer, whatever the numbers of stages and buffers (the stages alone would let one group of warps run
+  // five blocks ahead of the other).
+  static constexpr int kPairs = 3, kPair = 128 * 64;
   static constexpr int kSmem = kStages * kStage + kPairs * kPair + 1024;
   static_assert(kSmem >= tc::kPairMinSmem, "one CTA of a pair per SM");
 };
@@ -220,7 +223,11 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
           else tc::mbar_arrive(full + 8 * s);
         }
       }
-      if ((t.nkb & 1) && l0 == 1 && at < busy && lane == 0 && ok) tc::mbar_arrive(w_empty + 8 * ((pairs + (t.nkb >> 1)) % C::kPairs));   // the last one's second block
+      if ((t.nkb & 1) && l0 == 1 && at < busy && ok) {   // the last pair's second block, which does not exist: its buffer is given back like any other, once it has been filled
+        const int pair = pairs + (t.nkb >> 1), buf = pair % C::kPairs;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(w_full + 8 * buf, (uint32_t)(pair / C::kPairs) & 1u));
+        if (ok && lane == 0) tc::mbar_arrive(w_empty + 8 * buf);
+      }
       pairs += (t.nkb + 1) >> 1;
       q += t.nkb;
       // ---- accumulators -> y (or partial sums): warp w has rows 32 (w % 4) .. + 31 and a quarter of the columns ----
