@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   extern __shared__ __align__(128) float dc_smem[];
   __shared__ __align__(8) uint64_t s_full[STAGES];
   __shared__ unsigned s_done[STAGES];                   // groups that are done with the stage, ever
-  __shared__ int s_gave_up;
+  __shared__ int s_gave_up[G];                          // a wait of this group gave up: its warps decide by one word of their own, between two of their barriers
   const int tid = threadIdx.x & 255, group = threadIdx.x >> 8, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, h = blockIdx.y;
   const int col0 = ((int)blockIdx.x * G + group) * NC;
   float* const st = dc_smem + STAGES * Y::kStage + group * Y::kGroup;   // S by column, as hi and lo: 2 x [NC][DK]
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   const uint32_t full = tc::smem_u32(s_full);
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) { tc::mbar_init(full + 8 * i, 1); s_done[i] = 0u; }
-    s_gave_up = 0;
+    for (int i = 0; i < G; ++i) s_gave_up[i] = 0;
     tc::mbar_init_fence();
   }
   griddep_launch();
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   bool ok = true;
   for (int c = 0; c < chunks; ++c) {
     const float* const sg = dc_smem + (c % STAGES) * Y::kStage;
-    if (!tc::mbar_wait(full + 8 * (c % STAGES), (uint32_t)(c / STAGES) & 1u)) *(volatile int*)&s_gave_up = 1;
+    if (!tc::mbar_wait(full + 8 * (c % STAGES), (uint32_t)(c / STAGES) & 1u)) *(volatile int*)&s_gave_up[group] = 1;
     float acc[NT][4];
     const float* const wr = sg + (mt >> 1) * I::kMat + row * DK;
 #pragma unroll
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
       for (int n = 0; n < NT; ++n) rd[n * 32] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
     }
     group_sync();
-    if (*(volatile int*)&s_gave_up) { ok = false; break; }
+    if (*(volatile int*)&s_gave_up[group]) { ok = false; break; }
     if (kh == 0) {
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
