@@ -666,7 +666,8 @@ typedef struct b200_linear_attn_args {
   void* workspace; size_t workspace_bytes;
   int qk_f32;
 } b200_linear_attn_args;
-size_t b200_linear_attn_workspace_bytes(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv);
+size_t b200_linear_attn_workspace_bytes(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv);   /* enough for either kind of decays */
+size_t b200_linear_attn_workspace_bytes_ex(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv, int channel_decay);
 int b200_linear_attn(const b200_linear_attn_args* args, b200_stream_t stream);
 /* test and tuning knob: tokens per piece of a prompt (0: chosen by size); returns the previous setting */
 int b200_linear_attn_tune(int piece);

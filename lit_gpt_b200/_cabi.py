@@ -220,6 +220,7 @@ _CORE_SIGNATURES = {
     "b200_ring_store_keep": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int64,
                                      c_int, c_void_p]),
     "b200_linear_attn_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int, c_int]),
+    "b200_linear_attn_workspace_bytes_ex": (c_size_t, [c_int64, c_int, c_int, c_int, c_int, c_int, c_int]),
     "b200_linear_attn": (c_int, [ctypes.POINTER(LinearAttnArgs), c_void_p]),
     "b200_linear_attn_tune": (c_int, [c_int]),
     "b200_token_gate": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),

@@ -16,6 +16,7 @@
 // Bound: the chain of chunks (1.6 us each at sixteen columns a CTA, a third of it tensor pipe, the rest latency between its two products and three
 // barriers), then the per-chunk work (two CTAs an SM; issue slots).  16 heads of 128 x 128 with decays per channel, 2048 tokens: 343 -> 202 us (chunks
 // 155 -> 90, chain 180 -> 108) against all of it in fp32 multiply-adds read from shared memory, 1640 token by token.
+#include "seq_pieces.cuh"
 #include "tc05.cuh"
 #include "tf32x3.cuh"
 
@@ -57,50 +58,8 @@ __device__ __forceinline__ float sum2(f2 v) { float a, b; un2(v, a, b); return a
 
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
-// Chunks are counted through the sequences in their order, each with as many as its rows take; among several sequences, those of fewer than
-// kDcMinRows have none and go token by token.  (A single one always has a chunk, which without rows keeps or clears the slot's state as the walk
-// would.)  The functions below are called by whole warps.
-__device__ __forceinline__ int dc_chunks(const DcArgs& A, const int4& sq) { return sq.y >= A.min_rows ? (max(sq.y, 1) + kDcC - 1) / kDcC : 0; }
-// the sequence of chunk `at` and the chunk's number there; -1: there are not that many
-__device__ __forceinline__ int dc_find(const DcArgs& A, int at, int& chunk) {
-  const int lane = threadIdx.x & 31;
-  int before = 0;
-  for (int s0 = 0; s0 < A.n_seqs; s0 += 32) {
-    const int n = s0 + lane < A.n_seqs ? dc_chunks(A, A.seqs[s0 + lane]) : 0;
-    int incl = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const unsigned past = __ballot_sync(0xffffffffu, before + incl > at);
-    if (past) {
-      const int w = __ffs(past) - 1;
-      chunk = at - before - __shfl_sync(0xffffffffu, incl - n, w);
-      return s0 + w;
-    }
-    before += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  return -1;
-}
-// the z-th of the sequences that have chunks, and how many chunks lie before its own; -1: there are not that many
-__device__ __forceinline__ int dc_nth(const DcArgs& A, int z, int& before) {
-  const int lane = threadIdx.x & 31;
-  before = 0;
-  for (int s0 = 0; s0 < A.n_seqs; s0 += 32) {
-    const int n = s0 + lane < A.n_seqs ? dc_chunks(A, A.seqs[s0 + lane]) : 0;
-    const unsigned have = __ballot_sync(0xffffffffu, n > 0);
-    if (z < __popc(have)) {
-      const int w = (int)__fns(have, 0, z + 1);
-      before += __reduce_add_sync(0xffffffffu, lane < w ? n : 0);
-      return s0 + w;
-    }
-    z -= __popc(have);
-    before += __reduce_add_sync(0xffffffffu, n);
-  }
-  return -1;
-}
-
+// Chunks are counted through the sequences (seq_pieces.cuh); among several sequences, those of fewer than kDcMinRows have none and go token by token.
+// (A single one always has a chunk, which without rows keeps or clears the slot's state as the walk would.)
 // One chunk of one head: grid (chunks, heads).  Tokens past the sequence's end count as k = q = v = 0, beta = 0, g = 1.
 //
 // The tokens form four blocks of eight.  Per channel, a decay from token j of an earlier block to token i is the product of the one from j to the end of
@@ -147,7 +106,7 @@ __global__ void __launch_bounds__(kDcChunkThreads, 2) delta_chunk_kernel(DcArgs 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
   const int h = blockIdx.y, hk = h / (A.heads / A.kv_heads);
   int chunk;
-  const int z = dc_find(A, A.item0 + (int)blockIdx.x, chunk);
+  const int z = seq_of_piece(A.seqs, A.n_seqs, A.min_rows, C, A.item0 + (int)blockIdx.x, chunk);
   if (z < 0) return;
   const int4 sq = A.seqs[z];
   const int t0 = chunk * C;
@@ -549,10 +508,10 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   griddep_launch();
   griddep_wait();
   int before;
-  const int z = dc_nth(A, blockIdx.z, before);
+  const int z = seq_with_pieces(A.seqs, A.n_seqs, A.min_rows, C, blockIdx.z, before);
   if (z < 0) return;
   const int4 sq = A.seqs[z];
-  const int all = dc_chunks(A, sq);
+  const int all = seq_pieces(sq, A.min_rows, C);
   const int c_first = max(0, A.item0 - before), chunks = min(all, A.item0 + A.n_items - before) - c_first, t_first = c_first * C;
   if (threadIdx.x == 0 && before + all > A.most) *A.err = 1u;   // more rows than the caller said
   if (chunks <= 0) return;

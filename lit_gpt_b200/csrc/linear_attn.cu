@@ -21,6 +21,7 @@
 // No logarithm or quotient of decays is taken, so any decay in [0, 1] is safe.  A sequence that starts at position 0 starts from
 // S = 0 whatever its slot holds.  The state is stored [head][dk][dv].
 #include "common.cuh"
+#include "seq_pieces.cuh"
 
 namespace b200 {
 
@@ -42,10 +43,12 @@ struct LaArgs {
   const int4* seqs;
   int heads, dk, dv;
   int piece, n_pieces;              // tokens per piece, pieces per sequence in the workspace
-  float* ws_state;                  // [seq][piece][head][dk][dv]
+  float* ws_state;                  // [seq][piece][head][dk][dv], on the tensor cores [piece][head][dk][dv]
   float* ws_prod;                   // [seq][piece][head][dk]
   int vec_k, vec_z, vec_v, vec_s;   // 16-byte accesses possible on q and k / z / v / the state
   int pair_o;                       // 8-byte ones on the read-out (and the states)
+  // pieces on the tensor cores, counted through the sequences: how many there are sequences, from how many rows on they have pieces, how many can, and this launch's pieces
+  int n_seqs, least, longs, item0, n_items;
 };
 
 typedef unsigned long long f2;   // two packed floats
@@ -292,13 +295,23 @@ template <int V>
 __global__ void __launch_bounds__(256) scan_kernel(LaArgs A) {
   griddep_launch();
   griddep_wait();
-  const int4 sq = A.seqs[blockIdx.z];
-  const int n = (sq.y + A.piece - 1) / A.piece, h = blockIdx.y;
+  int z = blockIdx.z, first = 0;
+  int64_t at = (int64_t)z * A.n_pieces;               // the workspace's piece to begin with
+  if (A.n_items > 0) {
+    int before;
+    z = seq_with_pieces(A.seqs, A.n_seqs, A.least, A.piece, z, before);
+    if (z < 0) return;
+    first = max(0, A.item0 - before);
+    at = before + first - A.item0;
+  }
+  const int4 sq = A.seqs[z];
+  const int n = A.n_items > 0 ? (int)min((int64_t)seq_pieces(sq, A.least, A.piece) - first, A.n_items - at) : (sq.y + A.piece - 1) / A.piece, h = blockIdx.y;
+  if (A.n_items > 0 && n <= 0) return;                // (none of this launch's)
   const int64_t e = ((int64_t)blockIdx.x * 256 + threadIdx.x) * V, per = (int64_t)A.dk * A.dv;
   if (e >= per) return;
   const int i = (int)(e / A.dv);
   float* const slot = A.state + (int64_t)sq.w * A.slot_stride + h * per + e;
-  const int64_t w0 = (int64_t)blockIdx.z * A.n_pieces * A.heads + h;
+  const int64_t w0 = at * A.heads + h;
   float* const ws = A.ws_state + w0 * per + e;
   const float* const pr = A.ws_prod + w0 * A.dk + i;
   const int64_t wst = (int64_t)A.heads * per, pst = (int64_t)A.heads * A.dk;
@@ -313,7 +326,7 @@ __global__ void __launch_bounds__(256) scan_kernel(LaArgs A) {
     if constexpr (V == 4) *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
     else *p = f[0];
   };
-  if (sq.z > 0) ld(slot, S);
+  if (sq.z > 0 || first > 0) ld(slot, S);
   constexpr int U = 8;
   for (int c0 = 0; c0 < n; c0 += U) {
     float D[U][V], P[U];
@@ -375,7 +388,7 @@ namespace {
 template <typename T, typename TQ, int LK, int KPL, bool CHANNEL>
 cudaError_t scan_launch(const LaArgs& A, int n_seqs, float* qp, cudaStream_t st) {
   if constexpr (CHANNEL && LK * KPL <= 128) {
-    if (qp) return piece_launch<T, LK * KPL <= 64 ? 64 : 128>(A, n_seqs, qp, st);
+    if (qp) return piece_launch<T, LK * KPL <= 64 ? 64 : 128>(A, qp, st);
   }
   if (A.n_pieces <= 1) return walk_launch<T, TQ, LK, KPL, CHANNEL, 0>(A, n_seqs, st);
   cudaError_t e = walk_launch<T, TQ, LK, KPL, CHANNEL, 1>(A, n_seqs, st);
@@ -412,19 +425,34 @@ size_t la_walk_floats(int64_t rows, int max_rows, int n_seqs, int heads, int dk,
   const int64_t pieces = (max_rows + p - 1) / p;
   return pieces <= 1 ? 0 : (size_t)n_seqs * pieces * heads * dk * (dv + 1);
 }
-// Pieces of kLcC tokens on the tensor cores, for decays per channel (0: not for this shape): states and decays, and the rows' queries from their piece's start
-size_t la_chunk_floats(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv) {
-  if (g_la_piece > 0 || dk > 128 || max_rows < 2 * kLcC) return 0;
+// Pieces of kLcC tokens on the tensor cores, for decays per channel
+struct LaChunks {
+  int least = 1, longs = 0;   // rows from which on a sequence has pieces, sequences that can have that many
+  int64_t most = 0, fit = 0;  // pieces there can be, pieces of one launch (0: not for this shape)
+  size_t floats = 0;          // states and decays, and the rows' queries from their piece's start
+};
+constexpr int64_t kLcMaxBytes = 256ll << 20;   // scratch of one launch's pieces: long prompts go in several, the state passed on in its slot
+LaChunks la_chunks(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv) {
+  LaChunks c;
+  if (g_la_piece > 0 || dk > 128 || max_rows < 2 * kLcC || n_seqs > 65535) return c;
   // Where they are the shorter way (us, walk and pieces, bf16).  128 x 128 per head: 8 heads of 768 rows 58 / 63, of 1024 66 / 64, of 2048 118 / 71,
   // of 8192 393 / 264; 64 heads of 130 rows 69 / 67, of 256 113 / 70.  64 x 64: 4 heads of 700 rows 29 / 31, of 1024 33 / 29, of 2048 43 / 39.
   // A CTA's time does not fall with what it leaves empty of its tile, the walk's does: 96 x 96, 8 heads of 2048 rows 98 / 71, but 64 x 64, 8 heads of
   // 4096 rows (two waves of CTAs) 72 / 76 and 32 x 32, 8 heads of 2048 rows 35 / 41.
   const int64_t work = rows * heads * dk * dv, tile = (int64_t)(dk <= 64 ? 64 : 128) * ((dv + 127) / 128 * 128);
-  if (work < (dk <= 64 ? 1 << 24 : 1 << 27) || 2 * (int64_t)dk * dv < tile) return 0;
-  if (4 * (int64_t)dk * dv < 3 * tile && (rows + kLcC - 1) / kLcC * heads * ((dv + 127) / 128) > 2 * sm_count()) return 0;
-  const int64_t pieces = (max_rows + kLcC - 1) / kLcC;
-  if ((int64_t)n_seqs * pieces > 65535) return 0;
-  return (((size_t)n_seqs * pieces * heads * dk * (dv + 1) + 3) & ~(size_t)3) + (size_t)rows * heads * dk;
+  if (work < (dk <= 64 ? 1 << 24 : 1 << 27) || 2 * (int64_t)dk * dv < tile) return c;
+  if (4 * (int64_t)dk * dv < 3 * tile && (rows + kLcC - 1) / kLcC * heads * ((dv + 127) / 128) > 2 * sm_count()) return c;
+  // n sequences of `rows` rows in all have at most (rows + 63 n) / 64 pieces
+  c.longs = (int)(rows / c.least < n_seqs ? rows / c.least : n_seqs);
+  c.most = (rows + (int64_t)(kLcC - 1) * c.longs) / kLcC;
+  const int64_t per = (int64_t)heads * dk * (dv + 1 + kLcC);
+  c.fit = kLcMaxBytes / 4 / per;
+  if (c.fit > c.most) c.fit = c.most;
+  if (c.fit > 65535) c.fit = 65535;
+  c.floats = (((size_t)c.fit * heads * dk * (dv + 1) + 3) & ~(size_t)3) + (size_t)c.fit * kLcC * heads * dk;
+  if (c.most > 0x3fffffff) c.fit = 0;
+  if (c.fit == 0) c.floats = 0;
+  return c;
 }
 
 }  // namespace
@@ -442,8 +470,13 @@ int b200_linear_attn_tune(int piece) {
 }
 
 size_t b200_linear_attn_workspace_bytes(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv) {
-  const size_t walk = la_walk_floats(rows, max_rows, n_seqs, heads, dk, dv), chunks = la_chunk_floats(rows, max_rows, n_seqs, heads, dk, dv);
-  return (walk > chunks ? walk : chunks) * sizeof(float);
+  const size_t walk = b200_linear_attn_workspace_bytes_ex(rows, max_rows, n_seqs, heads, dk, dv, 0), channel = b200_linear_attn_workspace_bytes_ex(rows, max_rows, n_seqs, heads, dk, dv, 1);
+  return walk > channel ? walk : channel;
+}
+
+size_t b200_linear_attn_workspace_bytes_ex(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv, int channel_decay) {
+  const size_t chunks = channel_decay ? la_chunks(rows, max_rows, n_seqs, heads, dk, dv).floats : 0;
+  return (chunks ? chunks : la_walk_floats(rows, max_rows, n_seqs, heads, dk, dv)) * sizeof(float);
 }
 
 int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
@@ -454,10 +487,10 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
   B200_CHECK_ARG(a->dk > 0 && a->dk <= 512 && a->dv > 0, "b200_linear_attn: key size must be 1 .. 512");
   B200_CHECK_ARG(a->state_slot_stride >= (int64_t)a->heads * a->dk * a->dv, "b200_linear_attn: the state slots are too small");
   B200_CHECK_ARG((reinterpret_cast<uintptr_t>(a->seqs) & 15) == 0, "b200_linear_attn: seqs must be 16-byte aligned");
-  const size_t chunk_floats = a->decay_in ? la_chunk_floats(a->rows, a->max_rows, a->n_seqs, a->heads, a->dk, a->dv) : 0;
-  const bool chunks = chunk_floats && a->workspace && a->workspace_bytes >= chunk_floats * sizeof(float) && (reinterpret_cast<uintptr_t>(a->workspace) & 15) == 0;
+  const LaChunks lc = a->decay_in ? la_chunks(a->rows, a->max_rows, a->n_seqs, a->heads, a->dk, a->dv) : LaChunks{};
+  const bool chunks = lc.fit > 0 && a->workspace && a->workspace_bytes >= lc.floats * sizeof(float) && (reinterpret_cast<uintptr_t>(a->workspace) & 15) == 0;
   const int piece = chunks ? kLcC : la_piece(a->rows, a->max_rows, a->heads, a->dk, a->dv);
-  const int n_pieces = (a->max_rows + piece - 1) / piece;
+  const int n_pieces = chunks ? 0 : (a->max_rows + piece - 1) / piece;
   B200_CHECK_ARG((int64_t)a->n_seqs * n_pieces <= 65535, "b200_linear_attn: too many pieces");
   const size_t need = chunks ? 0 : la_walk_floats(a->rows, a->max_rows, a->n_seqs, a->heads, a->dk, a->dv) * sizeof(float);
   B200_CHECK_ARG(need == 0 || (a->workspace && a->workspace_bytes >= need), "b200_linear_attn: workspace too small (%zu of %zu bytes)", a->workspace_bytes, need);
@@ -465,14 +498,14 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
   const size_t esz = a->dtype == B200_F32 ? 4 : 2, qsz = a->qk_f32 ? 4 : esz;
   auto al = [](const void* p, int64_t bytes) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)bytes) & 15) == 0; };
   float* const ws = (float*)a->workspace;
-  const int64_t states = (int64_t)a->n_seqs * n_pieces * a->heads * a->dk * a->dv;
+  const int64_t states = (chunks ? lc.fit : (int64_t)a->n_seqs * n_pieces) * a->heads * a->dk * a->dv;
   LaArgs A{a->q, a->k, a->v, a->ldq, a->ldk, a->ldv, a->act, a->q_scale, a->decay_in, a->ld_decay, a->decay_bias, a->decay_in ? 1.0f / a->tau : 0.f, 0,
            a->head_decay, a->state, a->state_slot_stride, a->out, a->ldo, reinterpret_cast<const int4*>(a->seqs), a->heads, a->dk, a->dv, piece, n_pieces,
            ws, ws ? ws + states : nullptr,
            al(a->q, a->ldq * qsz) && al(a->k, a->ldk * qsz) && a->dk % 8 == 0, a->decay_in && al(a->decay_in, a->ld_decay * 4) && a->dk % 8 == 0,
            al(a->v, a->ldv * esz) && a->dv % 8 == 0, al(a->state, a->state_slot_stride * 4) && al(ws, 0) && a->dv % 4 == 0,
-           a->dv % 2 == 0 && a->ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 7) == 0};
-  float* const qp = chunks ? ws + (chunk_floats - (size_t)a->rows * a->heads * a->dk) : nullptr;
+           a->dv % 2 == 0 && a->ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 7) == 0, a->n_seqs, lc.least, lc.longs, 0, 0};
+  float* const qp = chunks ? ws + (lc.floats - (size_t)lc.fit * kLcC * a->heads * a->dk) : nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   const bool ch = a->decay_in != nullptr;
   B200_FLOAT_TYPES(a->dtype, T, {
@@ -485,11 +518,16 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
       A.z_ready = 1;
     }
     const bool qf = a->qk_f32 != 0;
-    if (a->dk <= 32) B200_CUDA((pick_launch<T, 8, 4>(A, a->n_seqs, ch, qf, qp, st)));
-    else if (a->dk <= 64) B200_CUDA((pick_launch<T, 8, 8>(A, a->n_seqs, ch, qf, qp, st)));
-    else if (a->dk <= 128) B200_CUDA((pick_launch<T, 16, 8>(A, a->n_seqs, ch, qf, qp, st)));
-    else if (a->dk <= 256) B200_CUDA((pick_launch<T, 32, 8>(A, a->n_seqs, ch, qf, qp, st)));
-    else B200_CUDA((pick_launch<T, 32, 16>(A, a->n_seqs, ch, qf, qp, st)));
+    for (int64_t at = 0; at == 0 || at < lc.most * chunks; at += lc.fit) {   // (one launch but for long prompts in pieces on the tensor cores)
+      A.item0 = (int)at;
+      A.n_items = chunks ? (int)(lc.most - at < lc.fit ? lc.most - at : lc.fit) : 0;
+      if (a->dk <= 32) B200_CUDA((pick_launch<T, 8, 4>(A, a->n_seqs, ch, qf, qp, st)));
+      else if (a->dk <= 64) B200_CUDA((pick_launch<T, 8, 8>(A, a->n_seqs, ch, qf, qp, st)));
+      else if (a->dk <= 128) B200_CUDA((pick_launch<T, 16, 8>(A, a->n_seqs, ch, qf, qp, st)));
+      else if (a->dk <= 256) B200_CUDA((pick_launch<T, 32, 8>(A, a->n_seqs, ch, qf, qp, st)));
+      else B200_CUDA((pick_launch<T, 32, 16>(A, a->n_seqs, ch, qf, qp, st)));
+      if (!chunks) break;
+    }
   });
   return B200_OK;
 }

@@ -96,13 +96,14 @@ __global__ void __launch_bounds__(kLcThreads, 2) piece_kernel(LaArgs A, float* _
   griddep_launch();
   griddep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, h = blockIdx.y;
-  const int sidx = (int)blockIdx.z / A.n_pieces, piece = (int)blockIdx.z % A.n_pieces;
+  int piece;
+  const int sidx = seq_of_piece(A.seqs, A.n_seqs, A.least, C, A.item0 + (int)blockIdx.z, piece);
+  if (sidx < 0) return;
   const int4 sq = A.seqs[sidx];
   const int begin = piece * C, nt = min(C, sq.y - begin);
-  if (nt <= 0) return;
   const int64_t row0 = (int64_t)sq.x + begin;
   const int dk = A.dk, dv = A.dv, col0 = (int)blockIdx.x * 128;
-  const int64_t wrow = ((int64_t)sidx * A.n_pieces + piece) * A.heads + h;
+  const int64_t wrow = (int64_t)blockIdx.z * A.heads + h;
   const T* const kp = reinterpret_cast<const T*>(A.k) + row0 * A.ldk + (int64_t)h * dk;
   const T* const qp = reinterpret_cast<const T*>(A.q) + row0 * A.ldq + (int64_t)h * dk;
   const T* const vp = reinterpret_cast<const T*>(A.v) + row0 * A.ldv + (int64_t)h * dv;
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(kLcThreads, 2) piece_kernel(LaArgs A, float* _
       const float f = before[n];
 #pragma unroll
       for (int e = 0; e < 8; ++e)
-        if (8 * b + e < nt && c < dk) qp_out[((row0 + 8 * b + e) * A.heads + h) * dk + c] = qs[lc_at<DK>(8 * b + e, c)] * f;
+        if (8 * b + e < nt && c < dk) qp_out[(((int64_t)blockIdx.z * C + 8 * b + e) * A.heads + h) * dk + c] = qs[lc_at<DK>(8 * b + e, c)] * f;
       if (b == 7 && c < dk) A.ws_prod[wrow * dk + c] = f * dd[n];
     }
   }
@@ -413,13 +414,15 @@ __global__ void __launch_bounds__(kLcThreads, 2) read_kernel(LaArgs A, const flo
   griddep_launch();
   griddep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, h = blockIdx.y;
-  const int sidx = (int)blockIdx.z / A.n_pieces, piece = (int)blockIdx.z % A.n_pieces;
+  int piece;
+  const int sidx = seq_of_piece(A.seqs, A.n_seqs, A.least, C, A.item0 + (int)blockIdx.z, piece);
+  if (sidx < 0) return;
   const int4 sq = A.seqs[sidx];
+  if (piece == 0 && sq.z == 0) return;                // (from nothing)
   const int begin = piece * C, nt = min(C, sq.y - begin);
-  if (nt <= 0 || (piece == 0 && sq.z == 0)) return;   // (from nothing)
   const int64_t row0 = (int64_t)sq.x + begin;
   const int dk = A.dk, dv = A.dv, col0 = (int)blockIdx.x * 128;
-  const float* const st = A.ws_state + (((int64_t)sidx * A.n_pieces + piece) * A.heads + h) * dk * dv + col0;
+  const float* const st = A.ws_state + ((int64_t)blockIdx.z * A.heads + h) * dk * dv + col0;
   const bool q4 = (dk & 3) == 0;
   auto four = [](const float* p, int left, bool vec) {
     if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(kLcThreads, 2) read_kernel(LaArgs A, const flo
 #pragma unroll 4
   for (int i = tid * 4; i < C * DK; i += NT * 4) {
     const int t = i / DK, c = i % DK;
-    *reinterpret_cast<float4*>(qs + lc_at<DK>(t, c)) = four(qp + ((row0 + t) * A.heads + h) * dk + c, t < nt ? dk - c : 0, q4);
+    *reinterpret_cast<float4*>(qs + lc_at<DK>(t, c)) = four(qp + (((int64_t)blockIdx.z * C + t) * A.heads + h) * dk + c, t < nt ? dk - c : 0, q4);
   }
 #pragma unroll 8
   for (int i = tid * 4; i < DK * 128; i += NT * 4) {
@@ -495,13 +498,13 @@ cudaError_t piece_start(const LaArgs& A, dim3 grid, float* qp, cudaStream_t st) 
 }
 
 template <typename T, int DK>
-cudaError_t piece_launch(const LaArgs& A, int n_seqs, float* qp, cudaStream_t st) {
-  const dim3 grid((unsigned)((A.dv + 127) / 128), (unsigned)A.heads, (unsigned)(n_seqs * A.n_pieces));
+cudaError_t piece_launch(const LaArgs& A, float* qp, cudaStream_t st) {
+  const dim3 grid((unsigned)((A.dv + 127) / 128), (unsigned)A.heads, (unsigned)A.n_items);
   cudaError_t e;
   if constexpr (sizeof(T) == 2) e = A.act ? piece_start<T, DK, false>(A, grid, qp, st) : piece_start<T, DK, true>(A, grid, qp, st);
   else e = piece_start<T, DK, false>(A, grid, qp, st);
   if (e != cudaSuccess) return e;
-  e = states_launch(A, n_seqs, st);
+  e = states_launch(A, A.longs, st);
   if (e != cudaSuccess) return e;
   return launch(read_kernel<DK>, grid, dim3(kLcThreads), LcRead<DK>::kSmem, st, A, (const float*)qp);
 }

@@ -1158,7 +1158,7 @@ def linear_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.
         raise C.B200Error("linear_attn: unit inner strides, contiguous states")
     n, lib = q.shape[0], C.load_core()
     out = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
-    need = lib.b200_linear_attn_workspace_bytes(n, max_rows, seqs.shape[0], heads, dk, dv)
+    need = lib.b200_linear_attn_workspace_bytes_ex(n, max_rows, seqs.shape[0], heads, dk, dv, int(decay_in is not None))
     ws = _ws("linear_attn", q.device, need) if need else None
     args = C.LinearAttnArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), ldq=q.stride(0), ldk=k.stride(0), ldv=v.stride(0), act=int(silu),
                             q_scale=float(q_scale), decay_in=C.ptr(decay_in), ld_decay=0 if decay_in is None else decay_in.stride(0),
