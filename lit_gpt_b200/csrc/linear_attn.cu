@@ -49,6 +49,7 @@ struct LaArgs {
   int pair_o;                       // 8-byte ones on the read-out (and the states)
   // pieces on the tensor cores, counted through the sequences: how many there are sequences, from how many rows on they have pieces, how many can, and this launch's pieces
   int n_seqs, least, longs, item0, n_items;
+  int below;                        // > 0: only sequences of fewer rows (MODE 0)
 };
 
 typedef unsigned long long f2;   // two packed floats
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(kLaThreads, sizeof(TQ) == 2 && KPL <= 8 ? 5 : 
   const int h = blockIdx.y;
   const int sidx = MODE == 0 ? (int)blockIdx.z : (int)blockIdx.z / A.n_pieces, piece = MODE == 0 ? 0 : (int)blockIdx.z % A.n_pieces;
   const int4 sq = A.seqs[sidx];
+  if (MODE == 0 && A.below > 0 && sq.y >= A.below) return;
   const int begin = MODE == 0 ? 0 : piece * A.piece, end = MODE == 0 ? sq.y : min(sq.y, begin + A.piece);
   if (begin >= end) return;
   const int first = sq.x + begin, len = end - begin;
@@ -388,7 +390,13 @@ namespace {
 template <typename T, typename TQ, int LK, int KPL, bool CHANNEL>
 cudaError_t scan_launch(const LaArgs& A, int n_seqs, float* qp, cudaStream_t st) {
   if constexpr (CHANNEL && LK * KPL <= 128) {
-    if (qp) return piece_launch<T, LK * KPL <= 64 ? 64 : 128>(A, qp, st);
+    if (qp) {
+      if (A.below > 0 && A.item0 == 0) {   // single rows and short portions beside a prompt: a launch of the walk, slot state to slot state
+        const cudaError_t e = walk_launch<T, TQ, LK, KPL, CHANNEL, 0>(A, n_seqs, st);
+        if (e != cudaSuccess) return e;
+      }
+      return piece_launch<T, LK * KPL <= 64 ? 64 : 128>(A, qp, st);
+    }
   }
   if (A.n_pieces <= 1) return walk_launch<T, TQ, LK, KPL, CHANNEL, 0>(A, n_seqs, st);
   cudaError_t e = walk_launch<T, TQ, LK, KPL, CHANNEL, 1>(A, n_seqs, st);
@@ -428,20 +436,32 @@ size_t la_walk_floats(int64_t rows, int max_rows, int n_seqs, int heads, int dk,
 // Pieces of kLcC tokens on the tensor cores, for decays per channel
 struct LaChunks {
   int least = 1, longs = 0;   // rows from which on a sequence has pieces, sequences that can have that many
+  bool shorts = false;        // there can be sequences of fewer
   int64_t most = 0, fit = 0;  // pieces there can be, pieces of one launch (0: not for this shape)
   size_t floats = 0;          // states and decays, and the rows' queries from their piece's start
 };
+constexpr int kLcLeast = 16;
 constexpr int64_t kLcMaxBytes = 256ll << 20;   // scratch of one launch's pieces: long prompts go in several, the state passed on in its slot
 LaChunks la_chunks(int64_t rows, int max_rows, int n_seqs, int heads, int dk, int dv) {
   LaChunks c;
   if (g_la_piece > 0 || dk > 128 || max_rows < 2 * kLcC || n_seqs > 65535) return c;
-  // Where they are the shorter way (us, walk and pieces, bf16).  128 x 128 per head: 8 heads of 768 rows 58 / 63, of 1024 66 / 64, of 2048 118 / 71,
-  // of 8192 393 / 264; 64 heads of 130 rows 69 / 67, of 256 113 / 70.  64 x 64: 4 heads of 700 rows 29 / 31, of 1024 33 / 29, of 2048 43 / 39.
+  // Where they are the shorter way (us, walk and pieces, bf16).  128 x 128 per head: 8 heads of 768 rows 58 / 63, of 1024 66 / 64, of 2048 119 / 72,
+  // of 8192 396 / 264; 64 heads of 130 rows 69 / 67, of 256 113 / 70.  64 x 64: 4 heads of 1300 rows 34 / 37, of 2048 44 / 39, of 4096 64 / 46.
   // A CTA's time does not fall with what it leaves empty of its tile, the walk's does: 96 x 96, 8 heads of 2048 rows 98 / 71, but 64 x 64, 8 heads of
   // 4096 rows (two waves of CTAs) 72 / 76 and 32 x 32, 8 heads of 2048 rows 35 / 41.
-  const int64_t work = rows * heads * dk * dv, tile = (int64_t)(dk <= 64 ? 64 : 128) * ((dv + 127) / 128 * 128);
-  if (work < (dk <= 64 ? 1 << 24 : 1 << 27) || 2 * (int64_t)dk * dv < tile) return c;
-  if (4 * (int64_t)dk * dv < 3 * tile && (rows + kLcC - 1) / kLcC * heads * ((dv + 127) / 128) > 2 * sm_count()) return c;
+  // Single rows and short portions beside a prompt (as many as there may be beside sequences of the longest one's length) have tiles too where those are few and fit
+  // into the last wave of CTAs.  Else sequences of fewer than kLcLeast rows keep the walk, in a launch of its own: 9 us, and 0.4 a token.  The walk of all of them has CTAs for
+  // the longest one's pieces in every sequence, so that many single rows cost it more than that and a few do not.  8 heads of 128 x 128, 2048 rows beside 4, 24
+  // and 128 single rows: walk 122, 187, 695, tiles for all 76, 141, 506, a walk of the short ones and tiles 85, 91, 178; 4 heads of 64 x 64: 46, 44, 91; 43, 44, 102;
+  // 51, 53, 55.
+  const int64_t beside = n_seqs > (rows + max_rows - 1) / max_rows ? n_seqs - (rows + max_rows - 1) / max_rows : 0, long_rows = rows - beside;
+  const int64_t work = long_rows * heads * dk * dv, tile = (int64_t)(dk <= 64 ? 64 : 128) * ((dv + 127) / 128 * 128), slots = 2 * sm_count();
+  const int64_t row_ctas = (int64_t)heads * ((dv + 127) / 128), ctas = (long_rows + kLcC - 1) / kLcC * row_ctas;
+  if (2 * (int64_t)dk * dv < tile || (4 * (int64_t)dk * dv < 3 * tile && ctas > slots)) return c;
+  const bool apart = (ctas + beside * row_ctas + slots - 1) / slots > (ctas + slots - 1) / slots || 4 * beside * row_ctas > slots, few = apart && beside < (dk <= 64 ? 64 : 16);
+  if (work < (dk <= 64 ? (few ? 12 << 22 : 7 << 22) : (few ? 5 << 25 : 4 << 25))) return c;
+  if (apart) c.least = kLcLeast;
+  c.shorts = apart && rows - (int64_t)(n_seqs - 1) * max_rows < c.least;
   // n sequences of `rows` rows in all have at most (rows + 63 n) / 64 pieces
   c.longs = (int)(rows / c.least < n_seqs ? rows / c.least : n_seqs);
   c.most = (rows + (int64_t)(kLcC - 1) * c.longs) / kLcC;
@@ -504,7 +524,7 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
            ws, ws ? ws + states : nullptr,
            al(a->q, a->ldq * qsz) && al(a->k, a->ldk * qsz) && a->dk % 8 == 0, a->decay_in && al(a->decay_in, a->ld_decay * 4) && a->dk % 8 == 0,
            al(a->v, a->ldv * esz) && a->dv % 8 == 0, al(a->state, a->state_slot_stride * 4) && al(ws, 0) && a->dv % 4 == 0,
-           a->dv % 2 == 0 && a->ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 7) == 0, a->n_seqs, lc.least, lc.longs, 0, 0};
+           a->dv % 2 == 0 && a->ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 7) == 0, a->n_seqs, lc.least, lc.longs, 0, 0, 0};
   float* const qp = chunks ? ws + (lc.floats - (size_t)lc.fit * kLcC * a->heads * a->dk) : nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   const bool ch = a->decay_in != nullptr;
@@ -517,6 +537,7 @@ int b200_linear_attn(const b200_linear_attn_args* a, b200_stream_t stream) {
                        a->heads * a->dk, A.inv_tau));
       A.z_ready = 1;
     }
+    A.below = chunks && lc.shorts ? lc.least : 0;
     const bool qf = a->qk_f32 != 0;
     for (int64_t at = 0; at == 0 || at < lc.most * chunks; at += lc.fit) {   // (one launch but for long prompts in pieces on the tensor cores)
       A.item0 = (int)at;

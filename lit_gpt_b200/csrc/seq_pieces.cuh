@@ -10,6 +10,10 @@ __device__ __forceinline__ int seq_pieces(const int4& sq, int least, int C) { re
 
 // the sequence of piece `at` and the piece's number there; -1: there are not that many
 __device__ __forceinline__ int seq_of_piece(const int4* seqs, int n_seqs, int least, int C, int at, int& piece) {
+  if (n_seqs == 1) {
+    piece = at;
+    return at < seq_pieces(seqs[0], least, C) ? 0 : -1;
+  }
   const int lane = threadIdx.x & 31;
   int before = 0;
   for (int s0 = 0; s0 < n_seqs; s0 += 32) {
