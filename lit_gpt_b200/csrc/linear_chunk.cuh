@@ -28,9 +28,11 @@ struct LcPiece {
   static constexpr int kQ = kRow > kLcC * kLcC ? kRow : kLcC * kLcC, kK = kRow > kValues ? kRow : kValues;   // (B and the values take their places)
   static constexpr int kFloats = kQ + kK + kRow + 3 * 8 * DK;
   static constexpr int kSmem = kFloats * 4;
+  static_assert(kFloats >= DK * 128 + 3 * DK + 128, "walk_piece");
 };
 template <int DK>
 struct LcRead {
+  static_assert(kLcC * DK + DK * kLcPV >= DK * 128 + 3 * DK + 128, "walk_piece");
   static constexpr int kSmem = (kLcC * DK + DK * kLcPV) * 4;
 };
 
@@ -79,9 +81,57 @@ struct LcCols {
   }
 };
 
+// A piece with numbers that are not finite, token by token as in the walk, whose infinities stay what they are (halves of an infinity give NaN): from `src` (null: from
+// nothing), with read-out, the state at its end to `dst` if there is one.  A function of its own: inlined it takes registers from the kernels (8 heads of 8192
+// rows 282 us, 270 so, 267 without it).  smem: DK rows of 128 columns of the state, a token's key, query and decays, 128 sums.
+template <typename T, int DK>
+__device__ __noinline__ void walk_piece(const LaArgs& A, float* smem, int64_t row0, int nt, int h, int col0, const float* src, float* dst) {
+  constexpr int HALF = DK / 2;
+  const int tid = threadIdx.x, c = tid & 127, k0 = (tid >> 7) * HALF, dk = A.dk, dv = A.dv;
+  const bool in = col0 + c < dv;
+  float* const S = smem + k0 * 128 + c;
+  float* const tok = smem + DK * 128;        // key | query | decays
+  float* const sum = tok + 3 * DK;
+#pragma unroll 1
+  for (int i = 0; i < HALF; ++i) S[i * 128] = src && in && k0 + i < dk ? src[(int64_t)(k0 + i) * dv + c] : 0.f;
+#pragma unroll 1
+  for (int t = 0; t < nt; ++t) {
+    const int64_t row = row0 + t;
+    if (tid < DK) {
+      float k = 0.f, q = 0.f, g = 1.f;
+      if (tid < dk) {
+        const int64_t at = (int64_t)h * dk + tid;
+        k = load_as_float(reinterpret_cast<const T*>(A.k), row * A.ldk + at);
+        q = load_as_float(reinterpret_cast<const T*>(A.q), row * A.ldq + at);
+        if (A.act) { k = silu_f<T>(k); q = silu_f<T>(q); }
+        q *= A.q_scale;
+        g = channel_decay(A.z[row * A.ldz + at] + load_as_float(reinterpret_cast<const T*>(A.bias), at), A.inv_tau);
+      }
+      tok[tid] = k;
+      tok[DK + tid] = q;
+      tok[2 * DK + tid] = g;
+    }
+    float v = in ? load_as_float(reinterpret_cast<const T*>(A.v), row * A.ldv + (int64_t)h * dv + col0 + c) : 0.f, o = 0.f;
+    if (A.act) v = silu_f<T>(v);
+    __syncthreads();
+#pragma unroll 1
+    for (int i = k0; i < k0 + HALF && i < dk; ++i) {
+      float& x = smem[i * 128 + c];
+      x = fmaf(tok[2 * DK + i], x, tok[i] * v);
+      o = fmaf(x, tok[DK + i], o);
+    }
+    if (k0) sum[c] = o;
+    __syncthreads();
+    if (!k0 && in) A.out[row * A.ldo + (int64_t)h * dv + col0 + c] = o + sum[c];
+  }
+#pragma unroll 1
+  for (int i = 0; i < HALF && dst; ++i)
+    if (in && k0 + i < dk) dst[(int64_t)(k0 + i) * dv + c] = S[i * 128];
+}
+
 // EXACT: the values are 16-bit numbers and pass no activation
 template <typename T, int DK, bool EXACT>
-__global__ void __launch_bounds__(kLcThreads, 2) piece_kernel(LaArgs A, float* __restrict__ qp_out) {
+__global__ void __launch_bounds__(kLcThreads, 2) piece_kernel(const __grid_constant__ LaArgs A, float* __restrict__ qp_out) {
   using Y = LcPiece<DK>;
   constexpr int C = kLcC, NT = kLcThreads;
   extern __shared__ __align__(128) float lc_smem[];
@@ -329,20 +379,13 @@ __global__ void __launch_bounds__(kLcThreads, 2) piece_kernel(LaArgs A, float* _
 #pragma unroll
     for (int e = 0; e < 8; ++e) gs[lc_at<DK>(8 * b + e, c)] *= f;
   }
-  odd = __syncthreads_or(odd) != 0;
+  if (__syncthreads_or(odd)) {
+    walk_piece<T, DK>(A, lc_smem, row0, nt, h, col0, nullptr, A.ws_state + wrow * dk * dv + col0);
+    return;
+  }
 
   // ---- the read-out of the piece's own writes: B v ----
   float* const orow = A.out + row0 * A.ldo + (int64_t)h * dv + col0;
-  if (odd) {                                 // in order, so that nothing of a later token enters
-#pragma unroll 1
-    for (int n = tid; n < C * 128; n += NT) {
-      const int i = n / 128, c = n % 128;
-      float s = 0.f;
-#pragma unroll 1
-      for (int j = 0; j <= i; ++j) s = fmaf(bm[bat(i, j)], vb[j * kLcPV + c], s);
-      if (i < nt && col0 + c < dv) orow[(int64_t)i * A.ldo + c] = s;
-    }
-  }
   // a warp's thirty-two columns: row tiles 0 and 3 or 1 and 2 of B v, then every second tile of sixteen keys of the contribution to the state, keys by
   // values; what is read of the values serves all of a warp's tiles
   const int n0 = (warp & 3) * 4, half = warp >> 2;
@@ -363,7 +406,7 @@ __global__ void __launch_bounds__(kLcThreads, 2) piece_kernel(LaArgs A, float* _
       }
   };
   LcCols<EXACT> v;
-  if (!odd) {
+  {
     const int a0 = half, a1 = 3 - half;      // a0 < a1
     float acc[2][4][4] = {};
 #pragma unroll 1
@@ -405,8 +448,8 @@ __global__ void __launch_bounds__(kLcThreads, 2) piece_kernel(LaArgs A, float* _
 }
 
 // out += (P q)^T S0: a piece's rows from its starting state
-template <int DK>
-__global__ void __launch_bounds__(kLcThreads, 2) read_kernel(LaArgs A, const float* __restrict__ qp) {
+template <typename T, int DK>
+__global__ void __launch_bounds__(kLcThreads, 2) read_kernel(const __grid_constant__ LaArgs A, const float* __restrict__ qp) {
   constexpr int C = kLcC, NT = kLcThreads;
   extern __shared__ __align__(128) float lc_smem[];
   float* const qs = lc_smem;                 // [C][DK]
@@ -424,6 +467,8 @@ __global__ void __launch_bounds__(kLcThreads, 2) read_kernel(LaArgs A, const flo
   const int dk = A.dk, dv = A.dv, col0 = (int)blockIdx.x * 128;
   const float* const st = A.ws_state + ((int64_t)blockIdx.z * A.heads + h) * dk * dv + col0;
   const bool q4 = (dk & 3) == 0;
+  bool odd = false;                          // a number that is not finite
+  auto seen = [&](const float4& x) { odd = odd || !(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) <= 3.4028234e38f); };
   auto four = [](const float* p, int left, bool vec) {
     if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
     if (vec) return *reinterpret_cast<const float4*>(p);
@@ -432,17 +477,23 @@ __global__ void __launch_bounds__(kLcThreads, 2) read_kernel(LaArgs A, const flo
 #pragma unroll 4
   for (int i = tid * 4; i < C * DK; i += NT * 4) {
     const int t = i / DK, c = i % DK;
-    *reinterpret_cast<float4*>(qs + lc_at<DK>(t, c)) = four(qp + (((int64_t)blockIdx.z * C + t) * A.heads + h) * dk + c, t < nt ? dk - c : 0, q4);
+    const float4 x = four(qp + (((int64_t)blockIdx.z * C + t) * A.heads + h) * dk + c, t < nt ? dk - c : 0, q4);
+    seen(x);
+    *reinterpret_cast<float4*>(qs + lc_at<DK>(t, c)) = x;
   }
 #pragma unroll 8
   for (int i = tid * 4; i < DK * 128; i += NT * 4) {
     const int k = i / 128, c = i % 128;
     const float4 x = four(st + (int64_t)k * dv + c, k < dk ? dv - col0 - c : 0, A.vec_s);
+    seen(x);
     float* const d = ss + k * kLcPV + c;
     *reinterpret_cast<float2*>(d) = make_float2(x.x, x.y);
     *reinterpret_cast<float2*>(d + 2) = make_float2(x.z, x.w);
   }
-  __syncthreads();
+  if (__syncthreads_or(odd)) {               // from the starting state: what the piece wrote of its own cannot be told from it any more
+    walk_piece<T, DK>(A, lc_smem, row0, nt, h, col0, st, nullptr);
+    return;
+  }
   float* const orow = A.out + row0 * A.ldo + (int64_t)h * dv + col0;
   const int n0 = (warp & 3) * 4, half = warp >> 2;   // a warp's thirty-two columns; its row tiles half, half + 2
   float acc[2][4][4];
@@ -490,7 +541,7 @@ cudaError_t piece_start(const LaArgs& A, dim3 grid, float* qp, cudaStream_t st) 
   static PerDeviceOnce once;
   if (once.need()) {
     cudaError_t e = cudaFuncSetAttribute(piece_kernel<T, DK, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcPiece<DK>::kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(read_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcRead<DK>::kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(read_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcRead<DK>::kSmem);
     if (e != cudaSuccess) return e;
     once.done();
   }
@@ -506,7 +557,7 @@ cudaError_t piece_launch(const LaArgs& A, float* qp, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   e = states_launch(A, A.longs, st);
   if (e != cudaSuccess) return e;
-  return launch(read_kernel<DK>, grid, dim3(kLcThreads), LcRead<DK>::kSmem, st, A, (const float*)qp);
+  return launch(read_kernel<T, DK>, grid, dim3(kLcThreads), LcRead<DK>::kSmem, st, A, (const float*)qp);
 }
 
 }  // namespace
