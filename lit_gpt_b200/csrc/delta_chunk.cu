@@ -8,14 +8,17 @@
 // so everything but S0 is computed for all chunks side by side (delta_chunk_kernel), and what is left to do in order per chunk is three
 // small products on a slice of S0's columns (delta_carry_kernel; the columns never mix).
 //
-// All numbers are fp32 and products of them are formed on the tensor cores as three products of tf32 halves (tf32x3.cuh).  The decays enter as running
-// products, as in the token-by-token walk: no logarithm or quotient is taken, so any decay in [0, 1] is safe.
-// Error of the read-out and of the state against 64 bits, relative, mean over ten shapes of 64 to 2048 tokens: 2.52e-7 and 2.28e-7; with the products as
-// fp32 multiply-adds 2.60e-7 and 2.62e-7, token by token 2.37e-7 and 2.33e-7.
+// All numbers are fp32 and products of them are formed on the tensor cores as three products of tf32 halves (tf32x3.cuh); those of T and B T with the
+// right-hand sides, whose errors all results share, give back what the tensor core cuts off and keep the last bit of the right-hand sides, and B T itself is fp32
+// multiply-adds.  The decays enter as running products, as in the token-by-token walk: no logarithm or quotient is taken, so any decay in [0, 1] is safe.
+// Error against 64 bits, relative, 1e-7, mean of six shapes of 96 to 2048 tokens, read-out and state: this / every product as fp32 multiply-adds / token by token
+//   decays per channel, q, k, v of either sign  2.37, 2.29 / 2.56, 2.64 / 2.38, 2.37    past a silu  1.57, 2.34 / 1.69, 2.66 / 1.52, 2.44    with a mean of 1  0.87, 2.45 / 0.94, 2.74 / 0.69, 2.60
+//   decays per head                             2.26, 1.97 / 2.32, 2.27 / 2.17, 2.00                 1.63, 1.92 / 1.67, 2.21 / 1.46, 1.97                      1.01, 1.87 / 1.05, 2.04 / 0.74, 1.82
+// (with plain products of halves everywhere, read-outs of numbers of one sign with decays per head 1.19).
 //
 // Bound: the chain of chunks (1.6 us each at sixteen columns a CTA, a third of it tensor pipe, the rest latency between its two products and three
-// barriers), then the per-chunk work (two CTAs an SM; issue slots).  16 heads of 128 x 128 with decays per channel, 2048 tokens: 343 -> 202 us (chunks
-// 155 -> 90, chain 180 -> 108) against all of it in fp32 multiply-adds read from shared memory, 1640 token by token.
+// barriers), then the per-chunk work (two CTAs an SM; issue slots).  16 heads of 128 x 128 with decays per channel, 2048 tokens: 344 -> 209 us (chunks
+// 155 -> 97, chain 180 -> 108) against all of it in fp32 multiply-adds read from shared memory, 1640 token by token.
 #include "seq_pieces.cuh"
 #include "tc05.cuh"
 #include "tf32x3.cuh"
@@ -359,8 +362,8 @@ __global__ void __launch_bounds__(kDcChunkThreads, 2) delta_chunk_kernel(DcArgs 
   }
   __syncthreads();
 
-  // ---- B T: a tile of sixteen rows and eight columns per warp ----
-  auto dot = [&](const float* m, int i, const float* x, int pitch) {   // sum over j <= i of m_ij x_j, in order: nothing of a later token enters
+  // ---- B T: a warp's rows warp, warp + 8, .., a lane's column, in fp32 multiply-adds (B T is a factor of Q and O, and its sums are few) ----
+  auto dot = [&](const float* m, int i, const float* x, int pitch) {   // sum over j <= i of m_ij x_j
     float s = 0.f;
     for (int j = 0; j <= i; ++j) s = fmaf(m[dc_at32(i, j)], x[j * pitch], s);
     return s;
@@ -373,23 +376,23 @@ __global__ void __launch_bounds__(kDcChunkThreads, 2) delta_chunk_kernel(DcArgs 
       tm[dc_at32(C + i, j)] = s;
     }
   } else {
-    const int mt = warp & 1, col = (warp >> 1) * 8 + g8;
-    float d[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int kk = 0; kk <= mt; ++kk) {
-      x3::Split<8> a;
-      x3::Split<4> b;
-      a.set4(0, *reinterpret_cast<const float4*>(bm + dc_at32(16 * mt + g8, 16 * kk + 4 * t4)));
-      a.set4(4, *reinterpret_cast<const float4*>(bm + dc_at32(16 * mt + g8 + 8, 16 * kk + 4 * t4)));
+    float s[C / 8];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) b.set(e, tm[dc_at32(16 * kk + 4 * t4 + e, col)]);
-      float s[4];
-      x3::mma16(s, a, b);
+    for (int r = 0; r < C / 8; ++r) s[r] = 0.f;
+#pragma unroll 2
+    for (int l = 0; l < C; l += 4) {                    // (T is zero above its diagonal, B above its own)
+      float4 m[C / 8];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) d[e] += s[e];
+      for (int r = 0; r < C / 8; ++r) m[r] = *reinterpret_cast<const float4*>(bm + dc_at32(warp + 8 * r, l));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float t = tm[dc_at32(l + e, lane)];
+#pragma unroll
+        for (int r = 0; r < C / 8; ++r) s[r] = fmaf(e == 0 ? m[r].x : e == 1 ? m[r].y : e == 2 ? m[r].z : m[r].w, t, s[r]);
+      }
     }
-    const int c = (warp >> 1) * 8 + 2 * t4, row = C + 16 * mt + g8;
-    *reinterpret_cast<float2*>(tm + dc_at32(row, c)) = make_float2(d[0], d[1]);
-    *reinterpret_cast<float2*>(tm + dc_at32(row + 8, c)) = make_float2(d[2], d[3]);
+#pragma unroll
+    for (int r = 0; r < C / 8; ++r) tm[dc_at32(C + warp + 8 * r, lane)] = s[r];
   }
   __syncthreads();
 
@@ -419,7 +422,7 @@ __global__ void __launch_bounds__(kDcChunkThreads, 2) delta_chunk_kernel(DcArgs 
         const bool keys = p * 16 < DK;
         const float* const src = keys ? pk + p * 16 : vb + p * 16 - DK;
         const int pitch = keys ? Y::kPK : Y::kPV;
-        x3::Split<4> b[2][2];
+        x3::Split3<4> b[2][2];
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
@@ -435,7 +438,7 @@ __global__ void __launch_bounds__(kDcChunkThreads, 2) delta_chunk_kernel(DcArgs 
             a.set4(0, *reinterpret_cast<const float4*>(tm + dc_at32(16 * mt + g8, 16 * kk + 4 * t4)));
             a.set4(4, *reinterpret_cast<const float4*>(tm + dc_at32(16 * mt + g8 + 8, 16 * kk + 4 * t4)));
             float s[2][4];
-            x3::mma16<2>(s, {&a, &a}, {&b[kk][0], &b[kk][1]});
+            x3::mma16_mean<2, x3::Split3<4>>(s, {&a, &a}, {&b[kk][0], &b[kk][1]});
 #pragma unroll
             for (int n = 0; n < 2; ++n)
 #pragma unroll
