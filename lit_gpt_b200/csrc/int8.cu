@@ -567,6 +567,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
               if (n0 + c0 + e < p.N) yr[e] = __float2half_rn(out[e]);
           }
         }
+        __syncwarp();   // (the next load of tensor memory wants the whole warp, lanes without a row too)
       }
       tc::fence_before();
       __syncwarp();

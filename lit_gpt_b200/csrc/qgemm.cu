@@ -247,23 +247,25 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
             tc::ld16(u, acc + c0 + half);
             tc::wait_ld(v);
             tc::wait_ld(u);
-            if (m >= p.M) continue;
+            if (m < p.M) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 8) {
-              const int64_t n = t.n0 + c0 + j;
-              if (n < p.N) {
-                uint32_t o[4];
+              for (int j = 0; j < 16; j += 8) {
+                const int64_t n = t.n0 + c0 + j;
+                if (n < p.N) {
+                  uint32_t o[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  auto act = [](uint32_t g, uint32_t w) {
-                    const float a = round_bf16(__uint_as_float(g));
-                    return round_bf16(a / (1.0f + expf(-a))) * round_bf16(__uint_as_float(w));
-                  };
-                  o[e] = pack_bf16(act(v[j + 2 * e], u[j + 2 * e]), act(v[j + 2 * e + 1], u[j + 2 * e + 1]));
+                  for (int e = 0; e < 4; ++e) {
+                    auto act = [](uint32_t g, uint32_t w) {
+                      const float a = round_bf16(__uint_as_float(g));
+                      return round_bf16(a / (1.0f + expf(-a))) * round_bf16(__uint_as_float(w));
+                    };
+                    o[e] = pack_bf16(act(v[j + 2 * e], u[j + 2 * e]), act(v[j + 2 * e + 1], u[j + 2 * e + 1]));
+                  }
+                  *reinterpret_cast<uint4*>(p.y + m * p.N + n) = make_uint4(o[0], o[1], o[2], o[3]);
                 }
-                *reinterpret_cast<uint4*>(p.y + m * p.N + n) = make_uint4(o[0], o[1], o[2], o[3]);
               }
             }
+            __syncwarp();   // (the next loads of tensor memory want the whole warp, lanes without a row too)
           }
           continue;
         }
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
               }
             }
           }
+          __syncwarp();
         }
       }
       tc::fence_before();
