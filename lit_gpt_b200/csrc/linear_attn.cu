@@ -467,8 +467,11 @@ LaChunks la_chunks(int64_t rows, int max_rows, int n_seqs, int heads, int dk, in
   c.most = (rows + (int64_t)(kLcC - 1) * c.longs) / kLcC;
   const int64_t per = (int64_t)heads * dk * (dv + 1 + kLcC);
   c.fit = kLcMaxBytes / 4 / per;
-  if (c.fit > c.most) c.fit = c.most;
   if (c.fit > 65535) c.fit = 65535;
+  if (c.fit > 0) {   // launches of about as many pieces each (8 heads of 128 x 128, 32768 rows, two launches: 1103 us with as many as fit in the first)
+    const int64_t launches = (c.most + c.fit - 1) / c.fit;
+    c.fit = (c.most + launches - 1) / launches;
+  }
   c.floats = (((size_t)c.fit * heads * dk * (dv + 1) + 3) & ~(size_t)3) + (size_t)c.fit * kLcC * heads * dk;
   if (c.most > 0x3fffffff) c.fit = 0;
   if (c.fit == 0) c.floats = 0;
