@@ -12,6 +12,9 @@
 // One CTA = 4 warps; warp w takes the 32-key tiles w, w+4, .. of the split's range, double-buffered in its private
 // shared-memory stages by cp.async; S = Q K^T and O += P V on mma.sync.m16n8k16 with ldmatrix operand loads from
 // XOR-swizzled tiles (mma_tile.cuh); the new key is patched into its tile from shared memory, never re-read from HBM.
+// P enters as two 16-bit numbers, the nearest one and what is left: with the nearest alone only the keys that set a running maximum are exact (their P is 1), so that
+// the result came the further from 64 bits the fewer ranges the keys are cut into (3000 keys, the final rounding to bf16 1.65e-3 by itself: 2.20e-3, 2.16e-3, 2.14e-3,
+// 2.08e-3 for 1, 2, 3, 8 ranges).  With up to eight heads a group the second numbers are the rows that no head uses.
 #include "attn_body.cuh"
 #include "mma_tile.cuh"
 
@@ -29,7 +32,8 @@ constexpr int kGqSmem = 4 * kGqWarpBytes + kGqQBytes + 2 * kGqHS * 2;
 
 // CLUSTER: the nsplit (<= 8) CTAs of a (batch, group) are one thread-block cluster; split partials stay in shared memory
 // and cluster rank 0 merges them through distributed shared memory (no workspace, fence or ticket).
-template <bool CLUSTER>
+// SPARE: at most eight heads a group; rows 8 .. 15 of a tile hold the second numbers of rows 0 .. 7.
+template <bool CLUSTER, bool SPARE>
 __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParams p) {
   extern __shared__ __align__(128) uint8_t gq_smem[];
   constexpr int HS = kGqHS;
@@ -122,6 +126,9 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
   float o_acc[HS / 8][4];
 #pragma unroll
   for (int i = 0; i < HS / 8; ++i) o_acc[i][0] = o_acc[i][1] = o_acc[i][2] = o_acc[i][3] = 0.f;
+  float o_rest[SPARE ? 1 : HS / 8][4];                        // the second numbers' sums (SPARE: o_acc's rows g + 8)
+#pragma unroll
+  for (int i = 0; i < (SPARE ? 1 : HS / 8); ++i) o_rest[i][0] = o_rest[i][1] = o_rest[i][2] = o_rest[i][3] = 0.f;
   float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // m in the scaled (log2) domain
 
   int it = 0;
@@ -162,21 +169,35 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
     }
     tmA = fmaxf(tmA, __shfl_xor_sync(0xffffffffu, tmA, 1)); tmA = fmaxf(tmA, __shfl_xor_sync(0xffffffffu, tmA, 2));
     tmB = fmaxf(tmB, __shfl_xor_sync(0xffffffffu, tmB, 1)); tmB = fmaxf(tmB, __shfl_xor_sync(0xffffffffu, tmB, 2));
+    if (SPARE) tmB = tmA;
     const float nmA = fmaxf(mA, tmA), nmB = fmaxf(mB, tmB);     // finite: every tile holds at least one valid key
-    const float cA = exp2f(mA - nmA), cB = exp2f(mB - nmB);     // exp2(-inf) = 0 the first time
+    const float cA = exp2f(mA - nmA), cB = SPARE ? cA : exp2f(mB - nmB);     // exp2(-inf) = 0 the first time
     mA = nmA; mB = nmB;
     float rsA = 0.f, rsB = 0.f;
-    uint32_t pfr[kGqTile / 16][4];
+    uint32_t pfr[kGqTile / 16][4], prest[SPARE ? 1 : kGqTile / 16][4];
+    auto rest = [](float x, float y, uint32_t w) { return pack_bf16(x - bf16lo(w), y - bf16hi(w)); };
 #pragma unroll
     for (int i = 0; i < kGqTile / 8; ++i) {
-      const float p0 = exp2f(s[i][0] - nmA), p1 = exp2f(s[i][1] - nmA), p2 = exp2f(s[i][2] - nmB), p3 = exp2f(s[i][3] - nmB);
-      rsA += p0 + p1; rsB += p2 + p3;
-      pfr[i >> 1][(i & 1) * 2 + 0] = pack_bf16(p0, p1);
-      pfr[i >> 1][(i & 1) * 2 + 1] = pack_bf16(p2, p3);
+      const int e = (i & 1) * 2;
+      const float p0 = exp2f(s[i][0] - nmA), p1 = exp2f(s[i][1] - nmA);
+      rsA += p0 + p1;
+      pfr[i >> 1][e] = pack_bf16(p0, p1);
+      if constexpr (SPARE) {
+        pfr[i >> 1][e + 1] = rest(p0, p1, pfr[i >> 1][e]);
+      } else {
+        const float p2 = exp2f(s[i][2] - nmB), p3 = exp2f(s[i][3] - nmB);
+        rsB += p2 + p3;
+        pfr[i >> 1][e + 1] = pack_bf16(p2, p3);
+        prest[i >> 1][e] = rest(p0, p1, pfr[i >> 1][e]);
+        prest[i >> 1][e + 1] = rest(p2, p3, pfr[i >> 1][e + 1]);
+      }
     }
     lA = lA * cA + rsA; lB = lB * cB + rsB;
 #pragma unroll
-    for (int i = 0; i < HS / 8; ++i) { o_acc[i][0] *= cA; o_acc[i][1] *= cA; o_acc[i][2] *= cB; o_acc[i][3] *= cB; }
+    for (int i = 0; i < HS / 8; ++i) {
+      o_acc[i][0] *= cA; o_acc[i][1] *= cA; o_acc[i][2] *= cB; o_acc[i][3] *= cB;
+      if constexpr (!SPARE) { o_rest[i][0] *= cA; o_rest[i][1] *= cA; o_rest[i][2] *= cB; o_rest[i][3] *= cB; }
+    }
 #pragma unroll
     for (int ks = 0; ks < kGqTile / 16; ++ks) {
 #pragma unroll
@@ -185,9 +206,26 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
         ldsm_x4_t(vf, vb + sw<HS>(ks * 16 + (((lane >> 3) & 1) << 3) + (lane & 7), dp * 2 + (lane >> 4)));
         pf_mma(o_acc[2 * dp], pfr[ks], vf[0], vf[1]);
         pf_mma(o_acc[2 * dp + 1], pfr[ks], vf[2], vf[3]);
+        if constexpr (!SPARE) {
+          pf_mma(o_rest[2 * dp], prest[ks], vf[0], vf[1]);
+          pf_mma(o_rest[2 * dp + 1], prest[ks], vf[2], vf[3]);
+        }
       }
     }
     __syncwarp();   // the stage just read is refilled two iterations from now, by this warp's own cp.async
+  }
+
+  // (an infinite value times a rest of zero is no number: such a sum stays what the nearest numbers make of it)
+  auto add = [](float& x, float y) { x = fabsf(x) <= 3.4028234e38f ? x + y : x; };
+#pragma unroll
+  for (int i = 0; i < HS / 8; ++i) {
+    if constexpr (SPARE) {
+      add(o_acc[i][0], o_acc[i][2]);
+      add(o_acc[i][1], o_acc[i][3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) add(o_acc[i][e], o_rest[i][e]);
+    }
   }
 
   // ---- per-warp partial (m, l, acc) -> shared memory (each warp reuses ITS OWN stage memory), merge the 4 warps ----
@@ -200,7 +238,7 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
     for (int i = 0; i < HS / 8; ++i) *reinterpret_cast<float2*>(my_acc + g * HS + i * 8 + 2 * tq) = make_float2(o_acc[i][0], o_acc[i][1]);
     if (tq == 0) { s_m[warp][g] = mA; s_l[warp][g] = lA; }
   }
-  if (g + 8 < nh) {
+  if (!SPARE && g + 8 < nh) {
 #pragma unroll
     for (int i = 0; i < HS / 8; ++i) *reinterpret_cast<float2*>(my_acc + (g + 8) * HS + i * 8 + 2 * tq) = make_float2(o_acc[i][2], o_acc[i][3]);
     if (tq == 0) { s_m[warp][g + 8] = mB; s_l[warp][g + 8] = lB; }
@@ -351,8 +389,8 @@ static int gqa_clusters(int splits) {
   if (n == 0) {
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t cfg = gqa_cluster_config(splits, dim3((unsigned)splits, 1, 1), nullptr, attr);
-    if (cudaFuncSetAttribute(attn_decode_gqa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, attn_decode_gqa_kernel<true>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaFuncSetAttribute(attn_decode_gqa_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, attn_decode_gqa_kernel<true, true>, &cfg) != cudaSuccess || n <= 0) {
       (void)cudaGetLastError();
       n = sm_count() / (splits * 2);
     }
@@ -380,7 +418,9 @@ int attn_decode_gqa_splits(int pairs, int max_seq, int64_t bytes) {
 
 cudaError_t launch_attn_decode_gqa(const AttnParams& p, dim3 grid, cudaStream_t st) {
   const bool cluster = grid.x >= 2 && grid.x <= 8;
-  auto kernel = cluster ? attn_decode_gqa_kernel<true> : attn_decode_gqa_kernel<false>;
+  const bool spare = p.qpk <= kGqRows / 2;
+  auto kernel = cluster ? (spare ? attn_decode_gqa_kernel<true, true> : attn_decode_gqa_kernel<true, false>)
+                        : (spare ? attn_decode_gqa_kernel<false, true> : attn_decode_gqa_kernel<false, false>);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem);
   if (e != cudaSuccess) return e;
   if (!cluster) return launch(kernel, grid, dim3(128), (size_t)kGqSmem, st, p);

@@ -67,3 +67,32 @@ def test_ranges_under_capture():
         got = K.attn_decode(qkv, cos, sin, pos, kc, vc, 32, 8, HS, HS)
     graph.replay()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("B,G,qpk,max_seq,pos", [(4, 8, 4, 3008, 3000), (2, 2, 8, 1024, 1000), (1, 4, 16, 2048, 2000), (1, 2, 9, 700, 600)])
+@pytest.mark.parametrize("splits", [0, 1, 3, 12])
+def test_close_to_64_bits_whatever_the_ranges(B, G, qpk, max_seq, pos, splits):
+    """P enters as two 16-bit numbers: what is left is the rounding of the result, and 2^-17 of P and fp32 sums beside it."""
+    case = _case(B, G, qpk, max_seq, pos)
+    qkv, _, _, p, kc, vc = case
+    one, zero = torch.ones(max_seq, HS, device="cuda"), torch.zeros(max_seq, HS, device="cuda")   # (no rotation: the queries as they are)
+    y, k, v = _run((qkv, one, zero, p, kc, vc), G, qpk, splits)
+    q = qkv.view(B, G, qpk + 2, HS)[:, :, :qpk].double()
+    att = torch.softmax(torch.einsum("bgqd,bgkd->bgqk", q, k[:, :, : pos + 1].double()) * HS**-0.5, -1)
+    want = torch.einsum("bgqk,bgkd->bgqd", att, v[:, :, : pos + 1].double()).reshape(B, -1)
+    rounding = (want.bfloat16().double() - want).norm()
+    assert (y.double() - want).norm() <= 1.02 * rounding + 2**-15 * want.norm()
+
+
+@pytest.mark.parametrize("qpk", [4, 12])
+def test_infinite_values(qpk):
+    """An infinite value in one column: that column's outputs, and no other's."""
+    B, G, max_seq, pos = 2, 2, 512, 500
+    case = _case(B, G, qpk, max_seq, pos)
+    want = _run(case, G, qpk, 0)[0].view(B, G, qpk, HS)
+    case[5][1, 0, 77, 9] = float("inf")
+    got = _run(case, G, qpk, 0)[0].view(B, G, qpk, HS)
+    assert (got[1, 0, :, 9] == float("inf")).all()
+    keep = torch.ones(B, G, qpk, HS, dtype=torch.bool, device="cuda")
+    keep[1, 0, :, 9] = False
+    assert torch.equal(got[keep], want[keep])
