@@ -35,7 +35,7 @@ int attn_fused_params(const b200_attn_decode_args* a, int nsplit, AttnParams* ou
 // grouped-query kernel on mma.sync (attn_decode_gqa.cu)
 bool attn_decode_gqa_supported(int head_size, int qpk);
 cudaError_t launch_attn_decode_gqa(const AttnParams& p, dim3 grid, cudaStream_t st);
-int attn_decode_gqa_splits(int pairs, int max_seq, int64_t bytes);   // key ranges per (sequence, group)
+int attn_decode_gqa_splits(int pairs, int heads, int max_seq, int64_t bytes);   // key ranges per (sequence, group of `heads` heads)
 
 __device__ __forceinline__ float table_at(const void* tab, int is_bf16, int64_t i) {
   return is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(tab)[i]) : reinterpret_cast<const float*>(tab)[i];

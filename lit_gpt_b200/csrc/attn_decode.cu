@@ -203,7 +203,7 @@ int b200_attn_decode(const b200_attn_decode_args* a, b200_stream_t stream) {
     const int ctas = a->batch * a->n_groups * head_chunks;
     // measured (tools/attn_bench.py --splits): the scalar kernel is bound by dependent round trips, so short key ranges per
     // CTA win until the merge grows, at about 3 CTAs per SM; the tensor-core one has one CTA an SM and a rule of its own
-    nsplit = gqa ? attn_decode_gqa_splits(ctas, a->max_seq, (int64_t)ctas * a->max_seq * a->head_size * 4) : (3 * sm_count() + ctas - 1) / ctas;
+    nsplit = gqa ? attn_decode_gqa_splits(ctas, qpk, a->max_seq, (int64_t)ctas * a->max_seq * a->head_size * 4) : (3 * sm_count() + ctas - 1) / ctas;
     const int by_len = (a->max_seq + 31) / 32;
     if (nsplit > by_len) nsplit = by_len;
     // many sequences x heads over a long cache (13B, batch 16, 2048 positions: 640 CTAs of 1 MB each): three key ranges per (sequence,

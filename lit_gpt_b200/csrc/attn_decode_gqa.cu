@@ -14,7 +14,8 @@
 // XOR-swizzled tiles (mma_tile.cuh); the new key is patched into its tile from shared memory, never re-read from HBM.
 // P enters as two 16-bit numbers, the nearest one and what is left: with the nearest alone only the keys that set a running maximum are exact (their P is 1), so that
 // the result came the further from 64 bits the fewer ranges the keys are cut into (3000 keys, the final rounding to bf16 1.65e-3 by itself: 2.20e-3, 2.16e-3, 2.14e-3,
-// 2.08e-3 for 1, 2, 3, 8 ranges).  With up to eight heads a group the second numbers are the rows that no head uses.
+// 2.08e-3 for 1, 2, 3, 8 ranges).  With up to eight heads a group the second numbers are the rows that no head uses; with more they take products of their own (1 us),
+// where the ranges are fewer than fill the SMs.
 #include "attn_body.cuh"
 #include "mma_tile.cuh"
 
@@ -32,8 +33,9 @@ constexpr int kGqSmem = 4 * kGqWarpBytes + kGqQBytes + 2 * kGqHS * 2;
 
 // CLUSTER: the nsplit (<= 8) CTAs of a (batch, group) are one thread-block cluster; split partials stay in shared memory
 // and cluster rank 0 merges them through distributed shared memory (no workspace, fence or ticket).
-// SPARE: at most eight heads a group; rows 8 .. 15 of a tile hold the second numbers of rows 0 .. 7.
-template <bool CLUSTER, bool SPARE>
+// REST: where the second numbers of P go.  Rows 8 .. 15 of a tile for those of rows 0 .. 7 (at most eight heads a group), products of their own, or nowhere.
+constexpr int kRestNone = 0, kRestSpare = 1, kRestOwn = 2;
+template <bool CLUSTER, int REST>
 __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParams p) {
   extern __shared__ __align__(128) uint8_t gq_smem[];
   constexpr int HS = kGqHS;
@@ -126,9 +128,10 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
   float o_acc[HS / 8][4];
 #pragma unroll
   for (int i = 0; i < HS / 8; ++i) o_acc[i][0] = o_acc[i][1] = o_acc[i][2] = o_acc[i][3] = 0.f;
-  float o_rest[SPARE ? 1 : HS / 8][4];                        // the second numbers' sums (SPARE: o_acc's rows g + 8)
+  constexpr bool SPARE = REST == kRestSpare;
+  float o_rest[REST == kRestOwn ? HS / 8 : 1][4];             // the second numbers' sums (spare rows: o_acc's rows g + 8)
 #pragma unroll
-  for (int i = 0; i < (SPARE ? 1 : HS / 8); ++i) o_rest[i][0] = o_rest[i][1] = o_rest[i][2] = o_rest[i][3] = 0.f;
+  for (int i = 0; i < (REST == kRestOwn ? HS / 8 : 1); ++i) o_rest[i][0] = o_rest[i][1] = o_rest[i][2] = o_rest[i][3] = 0.f;
   float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // m in the scaled (log2) domain
 
   int it = 0;
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
     const float cA = exp2f(mA - nmA), cB = SPARE ? cA : exp2f(mB - nmB);     // exp2(-inf) = 0 the first time
     mA = nmA; mB = nmB;
     float rsA = 0.f, rsB = 0.f;
-    uint32_t pfr[kGqTile / 16][4], prest[SPARE ? 1 : kGqTile / 16][4];
+    uint32_t pfr[kGqTile / 16][4], prest[REST == kRestOwn ? kGqTile / 16 : 1][4];
     auto rest = [](float x, float y, uint32_t w) { return pack_bf16(x - bf16lo(w), y - bf16hi(w)); };
 #pragma unroll
     for (int i = 0; i < kGqTile / 8; ++i) {
@@ -188,15 +191,17 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
         const float p2 = exp2f(s[i][2] - nmB), p3 = exp2f(s[i][3] - nmB);
         rsB += p2 + p3;
         pfr[i >> 1][e + 1] = pack_bf16(p2, p3);
-        prest[i >> 1][e] = rest(p0, p1, pfr[i >> 1][e]);
-        prest[i >> 1][e + 1] = rest(p2, p3, pfr[i >> 1][e + 1]);
+        if constexpr (REST == kRestOwn) {
+          prest[i >> 1][e] = rest(p0, p1, pfr[i >> 1][e]);
+          prest[i >> 1][e + 1] = rest(p2, p3, pfr[i >> 1][e + 1]);
+        }
       }
     }
     lA = lA * cA + rsA; lB = lB * cB + rsB;
 #pragma unroll
     for (int i = 0; i < HS / 8; ++i) {
       o_acc[i][0] *= cA; o_acc[i][1] *= cA; o_acc[i][2] *= cB; o_acc[i][3] *= cB;
-      if constexpr (!SPARE) { o_rest[i][0] *= cA; o_rest[i][1] *= cA; o_rest[i][2] *= cB; o_rest[i][3] *= cB; }
+      if constexpr (REST == kRestOwn) { o_rest[i][0] *= cA; o_rest[i][1] *= cA; o_rest[i][2] *= cB; o_rest[i][3] *= cB; }
     }
 #pragma unroll
     for (int ks = 0; ks < kGqTile / 16; ++ks) {
@@ -206,7 +211,7 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
         ldsm_x4_t(vf, vb + sw<HS>(ks * 16 + (((lane >> 3) & 1) << 3) + (lane & 7), dp * 2 + (lane >> 4)));
         pf_mma(o_acc[2 * dp], pfr[ks], vf[0], vf[1]);
         pf_mma(o_acc[2 * dp + 1], pfr[ks], vf[2], vf[3]);
-        if constexpr (!SPARE) {
+        if constexpr (REST == kRestOwn) {
           pf_mma(o_rest[2 * dp], prest[ks], vf[0], vf[1]);
           pf_mma(o_rest[2 * dp + 1], prest[ks], vf[2], vf[3]);
         }
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(128, 1) attn_decode_gqa_kernel(const AttnParam
     if constexpr (SPARE) {
       add(o_acc[i][0], o_acc[i][2]);
       add(o_acc[i][1], o_acc[i][3]);
-    } else {
+    } else if constexpr (REST == kRestOwn) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) add(o_acc[i][e], o_rest[i][e]);
     }
@@ -389,8 +394,8 @@ static int gqa_clusters(int splits) {
   if (n == 0) {
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t cfg = gqa_cluster_config(splits, dim3((unsigned)splits, 1, 1), nullptr, attr);
-    if (cudaFuncSetAttribute(attn_decode_gqa_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, attn_decode_gqa_kernel<true, true>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaFuncSetAttribute(attn_decode_gqa_kernel<true, kRestSpare>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, attn_decode_gqa_kernel<true, kRestSpare>, &cfg) != cudaSuccess || n <= 0) {
       (void)cudaGetLastError();
       n = sm_count() / (splits * 2);
     }
@@ -399,18 +404,29 @@ static int gqa_clusters(int splits) {
   return n;
 }
 
+// as many ranges as it takes to have a CTA on every SM (rounded up), two 32-key tiles per warp at least
+static int gqa_filling(int pairs, int max_seq) {
+  const int fill = (sm_count() + pairs - 1) / pairs, by_len = (max_seq + 255) / 256;
+  return fill < by_len ? (fill < 64 ? fill : 64) : (by_len < 64 ? by_len : 64);
+}
+
 // Key ranges per (sequence, group): whatever runs in ONE round of CTAs, by what a CTA takes for its keys (6.3 ns each, all of them together at 6.2 TB/s) and the
 // merge (1.8 to 2.7 us in a cluster, 4 through the workspace).  A second round costs as much as the first: eight sequences, 8 groups of 4 heads,
 // 3000 positions in 1, 2, 3, 4 ranges (64, 128, 192, 256 CTAs) 24.8, 22.3, 30.7, 28.6 us; 1000 positions 11.3, 12.2, 19.6, 18.6; two sequences, 3900 positions in 4, 6, 8, 10
 // ranges (16 clusters of 8 do not fit at once) 13.7, 12.9, 21.0, 19.7; one sequence, 3000 positions in 4, 8, 16, 19 11.6, 9.2, 10.0, 10.0.
-int attn_decode_gqa_splits(int pairs, int max_seq, int64_t bytes) {
+// With more than eight heads a group a cluster's merge, in one CTA, is the longer one, and ranges that fill the SMs in one round do without P's second numbers:
+// 4 sequences, 2 groups of 16, 3000 positions in 1, 4, 8, 12 ranges 35.1, 22.7, 20.2, 17.1; one pair over 16000 positions in 8, 16, 24, 32, 48 (with them) 33.0, 23.9, 23.3,
+// 24.0, 26.7, in 63 27.7.  (Eight heads: 1 x 8 groups, 4000 positions in 8, 16 14.1, 14.0.)
+int attn_decode_gqa_splits(int pairs, int heads, int max_seq, int64_t bytes) {
   const int by_len = (max_seq + 255) / 256;   // two 32-key tiles per warp at least
+  if (const int fill = gqa_filling(pairs, max_seq); heads > 8 && fill <= 24 && (int64_t)pairs * fill <= sm_count()) return fill;
   int best = 1;
   double best_t = -1.0;
   for (int ns = 1; ns <= by_len && ns <= 64; ++ns) {
     if (ns > 1 && (ns <= 8 ? gqa_clusters(ns) < pairs : (int64_t)pairs * ns > sm_count())) continue;
     const double keys = 6.3e-3 * max_seq / ns * (double)((int64_t)pairs * ns > sm_count() ? ((int64_t)pairs * ns + sm_count() - 1) / sm_count() : 1), all = (double)bytes / 6.2e6;
-    const double t = (keys > all ? keys : all) + (ns == 1 ? 0.0 : ns <= 8 ? 1.6 + 0.13 * ns : 3.5 + 0.05 * ns);
+    const double merge = heads > 8 ? (ns <= 8 ? 4.4 : 2.4 + 0.08 * ns) : (ns <= 8 ? 1.6 + 0.13 * ns : 3.5 + 0.05 * ns);
+    const double t = (keys > all ? keys : all) + (ns == 1 ? 0.0 : merge);
     if (best_t < 0.0 || t < best_t) { best_t = t; best = ns; }
   }
   return best;
@@ -418,9 +434,10 @@ int attn_decode_gqa_splits(int pairs, int max_seq, int64_t bytes) {
 
 cudaError_t launch_attn_decode_gqa(const AttnParams& p, dim3 grid, cudaStream_t st) {
   const bool cluster = grid.x >= 2 && grid.x <= 8;
-  const bool spare = p.qpk <= kGqRows / 2;
-  auto kernel = cluster ? (spare ? attn_decode_gqa_kernel<true, true> : attn_decode_gqa_kernel<true, false>)
-                        : (spare ? attn_decode_gqa_kernel<false, true> : attn_decode_gqa_kernel<false, false>);
+  const int rest = p.qpk <= kGqRows / 2 ? kRestSpare : (int)grid.x >= gqa_filling((int)(grid.y * grid.z), p.max_seq) ? kRestNone : kRestOwn;
+  auto kernel = rest == kRestSpare ? (cluster ? attn_decode_gqa_kernel<true, kRestSpare> : attn_decode_gqa_kernel<false, kRestSpare>)
+                : rest == kRestOwn ? (cluster ? attn_decode_gqa_kernel<true, kRestOwn> : attn_decode_gqa_kernel<false, kRestOwn>)
+                                   : (cluster ? attn_decode_gqa_kernel<true, kRestNone> : attn_decode_gqa_kernel<false, kRestNone>);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGqSmem);
   if (e != cudaSuccess) return e;
   if (!cluster) return launch(kernel, grid, dim3(128), (size_t)kGqSmem, st, p);

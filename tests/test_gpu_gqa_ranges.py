@@ -72,7 +72,8 @@ def test_ranges_under_capture():
 @pytest.mark.parametrize("B,G,qpk,max_seq,pos", [(4, 8, 4, 3008, 3000), (2, 2, 8, 1024, 1000), (1, 4, 16, 2048, 2000), (1, 2, 9, 700, 600)])
 @pytest.mark.parametrize("splits", [0, 1, 3, 12])
 def test_close_to_64_bits_whatever_the_ranges(B, G, qpk, max_seq, pos, splits):
-    """P enters as two 16-bit numbers: what is left is the rounding of the result, and 2^-17 of P and fp32 sums beside it."""
+    """P enters as two 16-bit numbers: what is left is the rounding of the result, and 2^-17 of P and fp32 sums beside it.  (With more than eight heads a group and ranges
+    that fill the SMs it is one number, good to 2^-9: as much again.)"""
     case = _case(B, G, qpk, max_seq, pos)
     qkv, _, _, p, kc, vc = case
     one, zero = torch.ones(max_seq, HS, device="cuda"), torch.zeros(max_seq, HS, device="cuda")   # (no rotation: the queries as they are)
@@ -81,7 +82,8 @@ def test_close_to_64_bits_whatever_the_ranges(B, G, qpk, max_seq, pos, splits):
     att = torch.softmax(torch.einsum("bgqd,bgkd->bgqk", q, k[:, :, : pos + 1].double()) * HS**-0.5, -1)
     want = torch.einsum("bgqk,bgkd->bgqd", att, v[:, :, : pos + 1].double()).reshape(B, -1)
     rounding = (want.bfloat16().double() - want).norm()
-    assert (y.double() - want).norm() <= 1.02 * rounding + 2**-15 * want.norm()
+    one_number = qpk > 8 and (splits == 0 or splits >= min(-(-148 // (B * G)), -(-max_seq // 256)))
+    assert (y.double() - want).norm() <= 1.02 * rounding + (2**-9 if one_number else 2**-15) * want.norm()
 
 
 @pytest.mark.parametrize("qpk", [4, 12])
