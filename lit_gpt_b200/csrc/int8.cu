@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kI8Threads) int8_gemv_kernel(const I8Params p)
 //   copies are the limit of the int8 pipe: an SM takes 48.7 bytes a clock of 128-byte boxes from L2 (measured with copies alone), the pair's products at
 //   full rate 64, a CTA alone on 128 x 128 twice that.  777 x 4096 -> 11008 with its preparing kernels, six outlier columns: 780 us with fragments read
 //   from L2, 100 us with 128 x 128 tiles, 66.6 us with pairs of 256 features and eight epilogue warps, 62.7 with sixteen and 224 features (4096 rows ->
-//   12288: 338, 220 and 221 us, 1.9 POP/s).
+//   12288: 338, 220 and 221 us, 1.9 POP/s).  The list of outlier columns beside the row quantisation takes 2 us off all of these.
 //   PAIR = false: one CTA on 128 x 128, for up to 128 rows, where the second half of a pair's rows would be padding.
 constexpr int kI8EpiWarps = 16, kI8GemmThreads = (kI8EpiWarps + 2) * 32;
 constexpr int kI8KB = 128;                       // int8 columns per stage: one 128-byte swizzle row

@@ -517,7 +517,9 @@ static cudaError_t launch_plan(const GemmParams& p, const GemmPlan& g, cudaStrea
 // with its best tile, against one, nf4 / int4: 4096 -> 11008 at 203 rows 83 -> 76 / 70 -> 65, at 400 115 -> 95 / 116 -> 101, at 1000 223 -> 158 / 228 -> 171;
 // 5120 -> 13824 at 300 131 -> 124 / 134 -> 133, at 2000 470 -> 435 / 462 -> 438; 4096 -> 14336 at 4096 859 -> 769 / 883 -> 776.  Up to 512 rows the two ways' times
 // as modelled decide.  Beyond, whether one launch saves a round of tiles with all their features: the second of two launches starts on the SMs that the
-// first one's last round leaves idle, which the model does not know, so a twentieth has to be won.
+// first one's last round leaves idle, which the model does not know, so a twentieth has to be won.  That line counts in clocks of an older kernel (1500 and 1130 a
+// k-block of full tiles) and not the tile that then runs, and errs towards two launches: of 132 shapes and types measured beyond 512 rows one launch is shorter
+// in all, and 32 run apart, 5 to 32 % longer (4096 -> 11008, nf4, at 513 rows 184 against 145, at 4096 629 / 573).
 static GemmPlan swiglu_plan(int64_t M, int64_t N, int64_t K, bool int4) {
   const GemmPlan none{2, 0, 1, 256};
   if (M <= 128) return none;
