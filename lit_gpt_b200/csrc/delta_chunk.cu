@@ -716,12 +716,11 @@ cudaError_t carry_launch(const DcArgs& A, int L, int vec_o, cudaStream_t st) {
 }
 
 template <typename T, int DK>
-cudaError_t segment_launch(const DcArgs& A, bool channel, int vec, int vec_v, int vec_o, int L, cudaStream_t st) {
+cudaError_t segment_launch(const DcArgs& A, bool channel, int vec, int vec_v, int vec_o, int L, int64_t walks, cudaStream_t st) {
   const cudaError_t e = channel ? chunk_launch<T, DK, true>(A, vec, vec_v, st) : chunk_launch<T, DK, false>(A, vec, vec_v, st);
   if (e != cudaSuccess) return e;
   // The fewest columns a CTA with which all CTAs run at once, one an SM.  us of both kernels, 512 tokens with decays per channel, 8, 16 (one or two column
   // tiles in one group) and 32 (two groups) columns a CTA: 8 heads 44, 55, 71; 16 heads 65, 57, 73; 32 heads 128, 112, 98.
-  const int64_t walks = (int64_t)A.heads * A.longs;
   if (walks * ((A.dv + 7) / 8) <= sm_count()) return carry_launch<DK, 1, 1>(A, L, vec_o, st);
   if (walks * ((A.dv + 15) / 16) <= sm_count()) return carry_launch<DK, 2, 1>(A, L, vec_o, st);
   return carry_launch<DK, 2, 2>(A, L, vec_o, st);
@@ -814,14 +813,19 @@ int b200_delta_rule_chunked(const b200_delta_rule_args* a, void* workspace, size
   const int vec = a->dk % 4 == 0 && al(a->q, a->ldq) && al(a->k, a->ldk);
   const int vec_v = a->dv % 4 == 0 && al(a->v, a->ldv), vec_o = a->dv % 2 == 0 && a->ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 7) == 0;
   const int L = a->dk <= 64 ? 4 : 8;   // the stored layout of a state (delta.cu)
+  // Chains that go on side by side.  Sequences that have chunks are as many as there can be, unless most of the others are too short to have any: one of 1000 rows
+  // beside 40 single ones, 4 heads of 64 x 64, decays per channel, 94 us with slices for sixteen, 58 for one.
+  int64_t chains = longs;
+  if (a->max_rows > 0 && a->n_seqs > 1 && a->rows - a->max_rows < (int64_t)(a->n_seqs - 1) * kDcMinRows) chains = 1 + (a->rows > a->max_rows ? (a->rows - a->max_rows) / a->max_rows : 0);
+  if (chains > longs) chains = longs;
   const bool ch = a->channel_decay != 0;
   cudaStream_t st = (cudaStream_t)stream;
   for (int64_t at = 0; at < most; at += fit) {
     A.item0 = (int)at;
     A.n_items = (int)(most - at < fit ? most - at : fit);
     B200_FLOAT_TYPES(a->dtype, T, {
-      if (a->dk <= 64) B200_CUDA((segment_launch<T, 64>(A, ch, vec, vec_v, vec_o, L, st)));
-      else B200_CUDA((segment_launch<T, 128>(A, ch, vec, vec_v, vec_o, L, st)));
+      if (a->dk <= 64) B200_CUDA((segment_launch<T, 64>(A, ch, vec, vec_v, vec_o, L, chains * a->heads, st)));
+      else B200_CUDA((segment_launch<T, 128>(A, ch, vec, vec_v, vec_o, L, chains * a->heads, st)));
     });
   }
   return B200_OK;
