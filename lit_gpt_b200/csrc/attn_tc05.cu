@@ -68,9 +68,8 @@ struct AtTile {
 
 // V tile as the right operand: N = HS contiguous (MN-major), 64 numbers per 128-byte row, one row per key: 8-key groups 1024 bytes apart
 // (stride offset), the second panel of 64 numbers 16 KB on (leading offset).  +128 in the address field is 16 keys.
-__device__ __forceinline__ uint64_t desc_v(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(16384 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
+// The low word of the descriptor; the high one is tc::kDescSw128High.
+__device__ __forceinline__ uint32_t desc_v_low(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((16384u >> 4) << 16); }
 
 // Rows [first, first + 128) of a matrix into a swizzled tile by N threads (this one `id`), zeros from row `end` on
 template <int HS, int N>
@@ -96,7 +95,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   __shared__ float s_shrink[2 * kAtBM];   // per row: what its O and sum shrink by in this step
   __shared__ uint32_t s_tmem;
   __shared__ int s_max[8];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be the same in all lanes)
   const int h = blockIdx.y, b = blockIdx.z, grp = h / (A.n_head / A.n_groups);
   const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * A.span;   // late rows, which see most keys, are scheduled first
   const uint32_t smem = (tc::smem_u32(at_smem) + 1023u) & ~1023u;
@@ -199,18 +198,19 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
     for (int e = max(i - 2, 0); e < i; ++e) ok = __all_sync(0xffffffffu, tc::mbar_wait(full + 8 * (e & 1), (uint32_t)(e >> 1) & 1u)) && ok;
   } else if (warp == 12) {
     // ================================ products ================================
-    if (lane == 0) {
+    if (tc::elect()) {
+      const uint32_t q_low = tc::desc_sw128_low(sq_), k_low = tc::desc_sw128_low(sk_), v_low = desc_v_low(sv_);
       auto scores = [&](int t, int s) {                    // S of query tile t with the keys of stage s
-        const uint32_t q = sq_ + t * C::kBytes, k = sk_ + s * C::kBytes;
+        const uint32_t q = q_low + t * (C::kBytes >> 4), k = k_low + s * (C::kBytes >> 4);
 #pragma unroll
         for (int e = 0; e < HS / 16; ++e) {
-          const uint32_t off = (uint32_t)(e >> 2) * 16384u + (uint32_t)(e & 3) * 32u;
-          mma_ss(tmem + C::kS + t * 128, tc::desc_sw128(q + off), tc::desc_sw128(k + off), C::kIdescS, e != 0);
+          const uint32_t off = ((uint32_t)(e >> 2) * 16384u + (uint32_t)(e & 3) * 32u) >> 4;
+          mma_ss(tmem + C::kS + t * 128, tc::desc_of(q + off, tc::kDescSw128High), tc::desc_of(k + off, tc::kDescSw128High), C::kIdescS, e != 0);
         }
         tc::commit(s_full + 8 * t);
       };
       uint32_t n[2] = {0u, 0u};                            // steps of either tile so far
-      ok = tc::mbar_wait(q_full, 0) && tc::mbar_wait(k_full, 0);
+      ok = tc::mbar_wait_here(q_full, 0) && tc::mbar_wait_here(k_full, 0);
       if (ok) {
         tc::fence_after();
 #pragma unroll
@@ -221,20 +221,20 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
       for (int j = t_lo; j < t_hi && ok; ++j) {
         const int i = j - t_lo, s = i & 1, s1 = s ^ 1;
         const bool more = j + 1 < t_hi;
-        ok = tc::mbar_wait(v_full + 8 * s, (uint32_t)(i >> 1) & 1u) && (!more || tc::mbar_wait(k_full + 8 * s1, (uint32_t)((i + 1) >> 1) & 1u));
+        ok = tc::mbar_wait_here(v_full + 8 * s, (uint32_t)(i >> 1) & 1u) && (!more || tc::mbar_wait_here(k_full + 8 * s1, (uint32_t)((i + 1) >> 1) & 1u));
         if (!ok) break;
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (j >= lo[t] && j < hi[t]) {
-            const uint64_t dv = desc_v(sv_ + s * C::kBytes);
+            const uint32_t dv = v_low + s * (C::kBytes >> 4);
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-              ok = ok && tc::mbar_wait((half ? p_full : p_half) + 8 * t, n[t] & 1u);
+              ok = ok && tc::mbar_wait_here((half ? p_full : p_half) + 8 * t, n[t] & 1u);
               if (!ok) break;
               tc::fence_after();
 #pragma unroll
               for (int e = 4 * half; e < 4 * half + 4; ++e)
-                mma_ts(tmem + C::kO + t * HS, tmem + C::kS + t * 128 + e * 8, dv + 128 * e, C::kIdescO, (n[t] | (uint32_t)e) != 0);
+                mma_ts(tmem + C::kO + t * HS, tmem + C::kS + t * 128 + e * 8, tc::desc_of(dv + 128 * e, tc::kDescSw128High), C::kIdescO, (n[t] | (uint32_t)e) != 0);
             }
             if (!ok) break;
             tc::commit(o_done + 8 * t);

@@ -347,7 +347,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
   __shared__ uint32_t s_tmem;
   __shared__ __align__(16) float s_feat[10][BN];               // per feature of the tile: weight scale, bias, weight in the first eight outlier columns
   __shared__ __align__(16) float s_more[kI8EpiWarps][8][16];   // per epilogue warp: the weights of 16 features in the next eight
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be the same in all lanes)
   const uint32_t rank = PAIR ? tc::cluster_rank() : 0u;
   const uint32_t tiles = (tc::smem_u32(i8_smem) + 1023u) & ~1023u;
   const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[kI8Stages]);
@@ -377,7 +377,7 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
 
   if (warp == kI8EpiWarps) {
     // ---- copies: 128 rows of either operand into this CTA's stage, counted on the issuing CTA's barrier ----
-    if (lane == 0) {
+    if (tc::elect()) {
       int s = 0;
       uint32_t ph = 1;
       for (int t = first; t < total && ok; t += step) {
@@ -406,20 +406,20 @@ int8_gemm_kernel(const I8Params p, const __grid_constant__ CUtensorMap map_a, co
     }
   } else if (warp == kI8EpiWarps + 1) {
     // ---- products ----
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && tc::elect()) {
+      auto wait_here = [](uint32_t bar, uint32_t parity) { return PAIR ? tc::mbar_wait_cluster_here(bar, parity) : tc::mbar_wait_here(bar, parity); };
       int s = 0, acc = 0;
       uint32_t ph = 0, aph = 1;
       for (int t = first; t < total && ok; t += step) {
-        ok = PAIR ? tc::mbar_wait_cluster(acc_empty + 8 * acc, aph) : tc::mbar_wait(acc_empty + 8 * acc, aph);
-        tc::fence_after();
+        ok = wait_here(acc_empty + 8 * acc, aph);
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = PAIR ? tc::mbar_wait_cluster(full + 8 * s, ph) : tc::mbar_wait(full + 8 * s, ph);
+          ok = wait_here(full + 8 * s, ph);
           if (!ok) break;
           tc::fence_after();
-          const uint32_t st = tiles + s * kI8Stage;
-          const uint64_t da = tc::desc_sw128(st), db = tc::desc_sw128(st + 128 * kI8KB);
+          const uint32_t da = tc::desc_sw128_low(tiles + s * kI8Stage), db = da + (128 * kI8KB >> 4);
 #pragma unroll
-          for (int k = 0; k < kI8KB / 32; ++k) umma_i8<PAIR>(tmem + acc * BN, da + 2 * k, db + 2 * k, bn, (kb | k) != 0);
+          for (int k = 0; k < kI8KB / 32; ++k)
+            umma_i8<PAIR>(tmem + acc * BN, tc::desc_of(da + 2 * k, tc::kDescSw128High), tc::desc_of(db + 2 * k, tc::kDescSw128High), bn, (kb | k) != 0);
           if constexpr (PAIR) tc::commit_pair(empty + 8 * s);
           else tc::commit(empty + 8 * s);
           if (++s == kI8Stages) { s = 0; ph ^= 1u; }

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
   __shared__ uint32_t s_tmem;
   __shared__ uint4 s_token[CTAS == 2 ? C::kStages : 1][8];   // where the bytes of the other CTA's warps land
   __shared__ float s_code[16 * 32];                 // fp32 code book, one copy per lane (conflict-free look-ups)
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be the same in all lanes)
   const uint32_t rank = CTAS == 2 ? tc::cluster_rank() : 0u;
   const uint32_t tiles = (tc::smem_u32(g_smem) + 1023u) & ~1023u;
   const uint32_t full = tc::smem_u32(&s_bars[0]), empty = tc::smem_u32(&s_bars[C::kStages]), acc_full = tc::smem_u32(&s_bars[2 * C::kStages]), acc_free = acc_full + 8, idle = acc_full + 16;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     }
   } else if (warp == kGDequantWarps) {
     // =========================================== ACTIVATIONS ====================================================
-    if (lane == 0) {
+    if (tc::elect()) {
       for (int i = first; i < total && ok; i += step) {
         const Item t = item(i);
         for (int l = 0; l < t.nkb; ++l, ++q) {
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
     }
   } else if (warp == kGDequantWarps + 2) {
     // =========================================== PACKED WEIGHTS =================================================
-    if (lane == 0) {   // ahead of the stages by as many k-blocks as the buffers hold
+    if (tc::elect()) {   // ahead of the stages by as many k-blocks as the buffers hold
       int pair = 0;
       for (int i = first; i < total && ok; i += step) {
         const Item t = item(i);
@@ -348,29 +348,30 @@ __global__ void __launch_bounds__(kGThreads, 1) qgemm_tcgen05_kernel(const GemmP
       for (int i = 0; i < C::kPairs; ++i)   // (a buffer never used: the phase before the first)
         ok = tc::mbar_wait(w_full + 8 * i, (uint32_t)((pair + C::kPairs - 1 - i) / C::kPairs + 1) & 1u) && ok;
     }
-  } else if (lane == 0 && rank == 0) {
+  } else if (rank == 0 && tc::elect()) {
     // =========================================== PRODUCTS =======================================================
-    uint32_t free_ph = 1;
+    auto wait_here = [](uint32_t bar, uint32_t parity) { return CTAS == 2 ? tc::mbar_wait_cluster_here(bar, parity) : tc::mbar_wait_here(bar, parity); };
+    uint32_t free_ph = 1, ph = 0;
+    int s = 0;
     for (int i = first; i < total && ok; i += step) {
       const Item t = item(i);
-      ok = wait(acc_free, free_ph);
+      ok = wait_here(acc_free, free_ph);
       free_ph ^= 1u;
-      tc::fence_after();
-      for (int l = 0; l < t.nkb && ok; ++l, ++q) {
-        const int s = q % C::kStages;
-        ok = wait(full + 8 * s, (uint32_t)(q / C::kStages) & 1u);
+      for (int l = 0; l < t.nkb && ok; ++l) {
+        ok = wait_here(full + 8 * s, ph);
         if (!ok) break;
         tc::fence_after();
-        const uint32_t st = tiles + s * C::kStage;
-        const uint64_t db = tc::desc_sw128(st + MT * kTileBytes);
-        for (int mt = 0; mt < t.mts; ++mt) {
-          const uint64_t da = tc::desc_sw128(st + mt * kTileBytes);
+        const uint32_t st = tc::desc_sw128_low(tiles + s * C::kStage), db = st + MT * (kTileBytes >> 4);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          if (mt > 0 && t.mts == 1) break;
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)  // +32 B along K inside the swizzle atom = +2 in the address field
-            umma_bf16<CTAS>(tmem + mt * BN, da + 2 * k, db + 2 * k, bn, (l | k) != 0);
+            umma_bf16<CTAS>(tmem + mt * BN, tc::desc_of(st + mt * (kTileBytes >> 4) + 2 * k, tc::kDescSw128High), tc::desc_of(db + 2 * k, tc::kDescSw128High), bn, (l | k) != 0);
         }
         if constexpr (CTAS == 2) tc::commit_pair(empty + 8 * s);   // the stage is free once these products have read it
         else tc::commit(empty + 8 * s);
+        if (++s == C::kStages) { s = 0; ph ^= 1u; }
       }
       if (ok) {
         if constexpr (CTAS == 2) tc::commit_pair(acc_full);

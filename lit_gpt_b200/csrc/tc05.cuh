@@ -60,14 +60,16 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarri
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+constexpr uint32_t kTrySleepNs = 100000;   // how long one try may sleep: waiting threads that come back sooner take issue slots from those that work (14336 <- 4096 int4, 64 rows: 28.5 -> 27.1 us)
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(bar), "r"(parity), "r"(kTrySleepNs) : "memory");
   return done != 0;
 }
 // (64 tries take far less than 50 ms: where more went by, the GPU was held up, and the time does not count)
-static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) {
+__device__ __forceinline__ bool mbar_wait_here(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) {
+  if (mbar_try(bar, parity)) return true;
   uint64_t last, t, spent = 0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(last));
   for (;;) {
@@ -79,11 +81,23 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity
     if (spent > limit_ns) return false;
   }
 }
+// The same behind a call, which keeps it out of the way of the code around.  Where that code issues products, mbar_wait_here is the better one: no value stays in a
+// uniform register across a call.
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) { return mbar_wait_here(bar, parity, limit_ns); }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_try(bar, parity) || mbar_try(bar, parity) || mbar_wait_slow(bar, parity); }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// True in one lane of a warp whose 32 lanes are all here, the same one every time.  Products, commits and copies are issued behind `if (elect())` in code that the
+// whole warp walks: the compiler then knows their operands, which these instructions take from uniform registers, to be uniform.  In a branch on the lane's
+// number it does not, and spends a loop over the lanes on each: 55 to 130 clk a product and as much a commit, where the tensor core takes 32 for 128 x 64 x 16 and 128 for
+// 128 x 256 x 16 (four products and a commit of 128 x 64 x 16: 235 clk, 129 this way).
+__device__ __forceinline__ bool elect() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r)::"memory");
+  return r != 0;
 }
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 
@@ -107,6 +121,14 @@ __device__ __forceinline__ void tmem_free(uint32_t tmem) {
 // address / 16 | leading offset (unused: 1) | stride offset / 16 | version 1 | SWIZZLE_128B.  +2 in the address field is 32 bytes along K.
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+// The two words apart: the high one is the same for every address, so that the low one, 32-bit sums, is all that a loop over operands moves.
+constexpr uint32_t kDescSw128High = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_sw128_low(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
+__device__ __forceinline__ uint64_t desc_of(uint32_t low, uint32_t high) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(low), "r"(high));
+  return d;
 }
 __device__ __forceinline__ void commit(uint32_t bar) {   // arrives on `bar` once every MMA issued so far has completed
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -135,6 +157,9 @@ __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) 
 // a wait on a barrier that the other CTA of the pair arrives on
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
   return mbar_try_cluster(bar, parity) || mbar_try_cluster(bar, parity) || (mbar_wait_slow(bar, parity) && mbar_try_cluster(bar, parity));
+}
+__device__ __forceinline__ bool mbar_wait_cluster_here(uint32_t bar, uint32_t parity) {
+  return mbar_try_cluster(bar, parity) || (mbar_wait_here(bar, parity) && mbar_try_cluster(bar, parity));
 }
 // a box into this CTA's shared memory whose bytes count on a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
