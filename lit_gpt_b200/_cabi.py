@@ -295,6 +295,8 @@ _SIGNATURES = {
     "b200_qgemm": (c_int, [ctypes.POINTER(QGemmArgs), c_void_p]),
     "b200_qgemm_swiglu_supported": (c_int, [c_int64, c_int64, c_int64, c_int, c_int]),
     "b200_qgemm_swiglu": (c_int, [ctypes.POINTER(QGemmArgs), c_void_p, c_void_p, c_void_p]),
+    "b200_qgemm_pair_workspace": (c_int64, [c_int64, c_int64, c_int64, c_int, c_int]),
+    "b200_qgemm_pair": (c_int, [ctypes.POINTER(QGemmArgs), c_void_p, c_void_p, c_void_p]),
     "b200_qgemm_tune": (c_int, [c_int]),
 }
 

@@ -25,6 +25,7 @@
 // thread holds both halves of its outputs and stores silu(gate) * up, with the roundings of the separate launches.
 // Bound: long prompts by power (1.3 GHz and 80 % tensor pipe at 4096 tokens, 4096 -> 14336, int4: 1106 clk a k-block of 512 tokens, 1024 of them products);
 // one sub-tile by the look-ups and stores of a tile's features (606 clk a k-block without, at 256 features int4 about 800 and nf4 950).
+#include "qgemm_short.cuh"
 #include "tc05.cuh"
 
 namespace b200 {
@@ -479,6 +480,12 @@ static GemmPlan gemm_plan(int64_t M, int64_t N, int64_t K, bool int4, bool split
   return best;
 }
 
+// What gemm_time is off by at up to 256 rows since its products are issued by an elected thread (measured over the sizes that short_time was fitted to)
+static double short_margin(bool int4, const GemmPlan& g) {
+  const double off = !int4 ? (g.mt == 2 ? 0.92 : 1.0) : g.ctas == 2 ? 0.96 : g.mt == 2 ? 0.87 : g.ksplit > 1 ? 0.97 : 0.88;
+  return off * 0.97;
+}
+
 template <int CTAS, int MT, bool INT4, bool SWIGLU = false>
 static cudaError_t launch_gemm(GemmParams p, cudaStream_t st) {
   constexpr int smem = GemmTile<MT>::kSmem;
@@ -557,7 +564,9 @@ size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   // accumulators live in tensor memory; only a launch split over k ranges (short prompts: too few output tiles for the SMs) stages fp32 partial sums
   if (M <= 0 || N <= 0 || K < kBK) return 0;
   const int nf4 = gemm_plan(M, N, K, false, true).ksplit, int4 = gemm_plan(M, N, K, true, true).ksplit, s = nf4 > int4 ? nf4 : int4;   // either type's
-  return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
+  const size_t ranges = s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
+  const size_t a = short_scratch_bytes(M, short_plan(M, N, K, B200_Q_NF4, false, true), false), b = short_scratch_bytes(M, short_plan(M, N, K, B200_Q_INT4, false, true), false);
+  return ranges > a ? (ranges > b ? ranges : b) : (a > b ? a : b);
 }
 
 static int gemm_args(const b200_qgemm_args* a, GemmParams& p) {
@@ -593,12 +602,58 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
   if (g.ksplit > 1 && (a->workspace == nullptr || a->workspace_bytes < (size_t)g.ksplit * a->M * a->N * sizeof(float) ||
                        (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
     g = gemm_plan(a->M, a->N, a->K, int4, false);
+  // Up to 256 rows the kernel with the weights on the left is the shorter way but for some matrices of 2560 x 7680 and less and int4 from 200 rows: us, this one / that
+  // one, 4096 -> 14336 at 17 / 64 / 129 / 203 rows nf4 35 / 21, 36 / 23, 42 / 27, 42 / 32, int4 26 / 21, 27 / 23, 34 / 27, 34 / 31; 14336 -> 4096 nf4 36 / 22,
+  // 37 / 25, 47 / 31, 47 / 35; 2048 -> 5632 int4 at 128 rows 13.4 / 15.3.  Each has a model of its times.
+  const ShortArgs sa{{p.packed, nullptr}, {p.scale, nullptr}, p.x, p.bias, p.y, reinterpret_cast<float*>(a->workspace), p.M, p.N, p.K, p.qtype};
+  if (short_takes(sa, false)) {
+    ShortPlan s = short_plan(p.M, p.N, p.K, p.qtype, false, true);
+    if (s.shared && (a->workspace == nullptr || a->workspace_bytes < short_scratch_bytes(p.M, s, false) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
+      s = short_plan(p.M, p.N, p.K, p.qtype, false, false);
+    if (s.ctas && s.time < gemm_time(p.M, p.N, p.K, int4, g, g.bn) * short_margin(int4, g)) {
+      const cudaError_t e = launch_short(sa, s, false, (cudaStream_t)stream);
+      if (e != cudaSuccess) {
+        set_error("b200_qgemm: launch failed: %s", cudaGetErrorString(e));
+        return B200_ERR_CUDA;
+      }
+      return B200_OK;
+    }
+  }
   p.ksplit = g.ksplit;
   p.bn = g.bn;
   p.partial = reinterpret_cast<float*>(a->workspace);
   const cudaError_t e = int4 ? launch_plan<true>(p, g, (cudaStream_t)stream) : launch_plan<false>(p, g, (cudaStream_t)stream);
   if (e != cudaSuccess) {
     set_error("b200_qgemm: launch failed: %s", cudaGetErrorString(e));
+    return B200_ERR_CUDA;
+  }
+  return B200_OK;
+}
+
+int64_t b200_qgemm_pair_workspace(int64_t M, int64_t N, int64_t K, int qtype, int blocksize) {
+  const int block = qtype == B200_Q_INT4 ? 128 : 64;
+  if ((qtype != B200_Q_NF4 && qtype != B200_Q_FP4 && qtype != B200_Q_INT4) || blocksize != block || M <= 0 || N <= 0 || K <= 0) return -1;
+  const ShortPlan s = short_plan(M, N, K, qtype, true, true);
+  return s.ctas ? (int64_t)short_scratch_bytes(M, s, true) : -1;
+}
+
+int b200_qgemm_pair(const b200_qgemm_args* a, const void* packed2, const void* scale2, b200_stream_t stream) {
+  GemmParams p{};
+  if (const int rc = gemm_args(a, p)) return rc;
+  B200_CHECK_ARG(packed2 && scale2 && (reinterpret_cast<uintptr_t>(packed2) & 15) == 0, "b200_qgemm_pair: null or misaligned second matrix");
+  B200_CHECK_ARG(!a->bias, "b200_qgemm_pair: takes no bias");
+  ShortArgs sa{{p.packed, reinterpret_cast<const uint8_t*>(packed2)}, {p.scale, reinterpret_cast<const uint32_t*>(scale2)}, p.x, nullptr, p.y,
+               reinterpret_cast<float*>(a->workspace), p.M, p.N, p.K, p.qtype};
+  ShortPlan s = short_plan(p.M, p.N, p.K, p.qtype, true, true);
+  if (s.shared && (a->workspace == nullptr || a->workspace_bytes < short_scratch_bytes(p.M, s, true) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
+    s = short_plan(p.M, p.N, p.K, p.qtype, true, false);
+  if (s.ctas == 0 || !short_takes(sa, true)) {
+    set_error("b200_qgemm_pair: (M=%lld N=%lld K=%lld) or its addresses run as two b200_qgemm and b200_swiglu", (long long)a->M, (long long)a->N, (long long)a->K);
+    return B200_ERR_UNSUPPORTED;
+  }
+  const cudaError_t e = launch_short(sa, s, true, (cudaStream_t)stream);
+  if (e != cudaSuccess) {
+    set_error("b200_qgemm_pair: launch failed: %s", cudaGetErrorString(e));
     return B200_ERR_CUDA;
   }
   return B200_OK;

@@ -60,11 +60,18 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarri
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-constexpr uint32_t kTrySleepNs = 100000;   // how long one try may sleep: waiting threads that come back sooner take issue slots from those that work (14336 <- 4096 int4, 64 rows: 28.5 -> 27.1 us)
+constexpr uint32_t kTrySleepNs = 100000;   // how long one try may sleep: waiting threads that come back sooner take issue slots from those that work (qgemm.cu, 4096 -> 14336 int4, 64 rows: 28.5 -> 27.1 us)
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                : "=r"(done) : "r"(bar), "r"(parity), "r"(kTrySleepNs) : "memory");
+  return done != 0;
+}
+// without waiting at all
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
 // (64 tries take far less than 50 ms: where more went by, the GPU was held up, and the time does not count)

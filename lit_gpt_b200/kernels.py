@@ -452,6 +452,29 @@ def qgemm_swiglu(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, pac
     return y
 
 
+def qgemm_pair_workspace(M: int, N: int, K: int, quant_type: str = "nf4", blocksize: int = 64) -> int:
+    """Bytes of scratch ``qgemm_pair`` takes (allocated by it on each call), or -1 for a size it does not run."""
+    return C.load().b200_qgemm_pair_workspace(M, N, K, QTYPES[quant_type], blocksize)
+
+
+def qgemm_pair(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, packed2: torch.Tensor, scale2: torch.Tensor, N: int, K: int,
+               quant_type: str = "nf4", blocksize: int = 64) -> torch.Tensor:
+    """``qgemm_swiglu`` for up to 128 rows, on the kernel of short prompts (csrc/qgemm_short.cu).  Raises NotImplementedError where
+    ``qgemm_pair_workspace`` is negative."""
+    C.require_cuda(x, packed, scale, packed2, scale2)
+    x = _bf16c(x, "x")
+    if x.shape[-1] != K:
+        raise C.B200Error(f"qgemm_pair: x has rows of {x.shape[-1]} numbers, the weights take {K}")
+    M = x.numel() // K
+    y = torch.empty(tuple(x.shape[:-1]) + (N,), dtype=torch.bfloat16, device=x.device)
+    need = qgemm_pair_workspace(M, N, K, quant_type, blocksize)
+    ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need > 0 else None   # (as in qgemm)
+    args = C.QGemmArgs(packed=packed.data_ptr(), scale=scale.data_ptr(), qtype=QTYPES[quant_type], blocksize=blocksize, M=M, N=N, K=K,
+                       x=x.data_ptr(), y=y.data_ptr(), workspace=C.ptr(ws), workspace_bytes=0 if ws is None else ws.numel())
+    C.check(C.load().b200_qgemm_pair(ctypes.byref(args), packed2.data_ptr(), scale2.data_ptr(), C.stream_ptr(x.device)), "qgemm_pair")
+    return y
+
+
 def qgemm_tune(wide: bool = True) -> None:
     """development switch: long prompts may use tiles of 512 tokens (default) or keep to 256"""
     C.check(C.load().b200_qgemm_tune(1 if wide else 0), "qgemm_tune")

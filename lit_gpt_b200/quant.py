@@ -410,15 +410,23 @@ def _called_plainly(m: nn.Module) -> bool:
                      or every._global_forward_pre_hooks or every._global_backward_hooks or every._global_backward_pre_hooks))
 
 
-def prefill_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
-    """True where the two projections of a gated MLP can be one launch with the product in its epilogue: plain 4-bit modules of one layout
-    without a bias or a hook (a hook wants the projections' own outputs) whose reference layouts are resident, at sizes the library calls the shorter way."""
+def _plain_pair(gate: nn.Module, up: nn.Module) -> bool:
+    """Plain 4-bit modules of one layout without a bias or a hook (a hook wants the projections' own outputs) whose reference layouts are resident."""
     if not all(isinstance(m, QLinear) and _called_plainly(m) and m.is_quantized and not m.released and m.quant_type != "int8" and m.bias is None
                for m in (gate, up)):
         return False
     return (gate.quant_type == up.quant_type and gate.blocksize == up.blocksize and gate.in_features == up.in_features
-            and gate.out_features == up.out_features
-            and K.qgemm_swiglu_supported(rows, gate.out_features, gate.in_features, gate.quant_type, gate.blocksize))
+            and gate.out_features == up.out_features)
+
+
+def prefill_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
+    """True where the two projections of a gated MLP can be one launch with the product in its epilogue, at sizes the library calls the shorter way."""
+    return _plain_pair(gate, up) and K.qgemm_swiglu_supported(rows, gate.out_features, gate.in_features, gate.quant_type, gate.blocksize)
+
+
+def short_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
+    """``prefill_pair`` for the kernel of short prompts."""
+    return _plain_pair(gate, up) and K.qgemm_pair_workspace(rows, gate.out_features, gate.in_features, gate.quant_type, gate.blocksize) >= 0
 
 
 class QuantPrecision:

@@ -1,0 +1,62 @@
+"""Prompt GEMM of up to 256 rows with the weights in tensor memory (csrc/qgemm_short.cu): edges of its tiles, of its stages of rows and of the ranges of k."""
+import pytest
+import torch
+
+from tests.test_gpu_kernels import K, _gemv_case  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+# rows on both sides of what a stage of rows holds (64, 128) and of a multiple of 16; features that end inside a tile of 128; one unit of 256 k, an odd number of them,
+# fewer and more than SMs (ranges of several tiles, tiles of several ranges)
+@pytest.mark.parametrize("M", [1, 16, 17, 64, 65, 128, 129, 241, 256])
+@pytest.mark.parametrize("N,Kdim", [(136, 256), (264, 1280), (1000, 768), (4104, 2304), (19208, 256)])
+@pytest.mark.parametrize("qt", ["nf4", "fp4", "int4"])
+def test_one_hot_rows_read_the_weights(K, qt, M, N, Kdim):  # noqa: F811
+    _, _, packed, scale, bs, deq = _gemv_case(K, N, Kdim, 1, qt, seed=M + N)
+    hot = torch.randint(0, Kdim, (M,), generator=torch.Generator().manual_seed(N))
+    x = torch.nn.functional.one_hot(hot, Kdim).to(torch.bfloat16).cuda()
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    want = deq.to(torch.bfloat16).T[hot]
+    assert torch.equal(K.qgemm(x, packed, scale, N, Kdim, qt, bs).cpu(), want)
+    assert torch.equal(K.qgemm(x, packed, scale, N, Kdim, qt, bs, bias=bias.cuda()).cpu(), (want.float() + bias.float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("M", [1, 17, 64, 65, 128])
+@pytest.mark.parametrize("N,Kdim", [(136, 256), (1000, 1280), (11008, 4096), (19208, 512)])
+@pytest.mark.parametrize("qt", ["nf4", "fp4", "int4"])
+def test_pair_is_the_separate_launches(K, qt, M, N, Kdim):  # noqa: F811
+    """Both projections and their product in one launch against two GEMMs and the product: sums in another order of k ranges, so some bf16 roundings of either
+    projection go the other way by one unit, 2^-8 of the number at most."""
+    _, _, p1, s1, bs, _ = _gemv_case(K, N, Kdim, 1, qt, seed=M)
+    _, _, p2, s2, _, _ = _gemv_case(K, N, Kdim, 1, qt, seed=N)
+    x = torch.randn(M, Kdim, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    assert K.qgemm_pair_workspace(M, N, Kdim, qt, bs) >= 0
+    y = K.qgemm_pair(x, p1, s1, p2, s2, N, Kdim, qt, bs)
+    ref = K.swiglu(K.qgemm(x, p1, s1, N, Kdim, qt, bs), K.qgemm(x, p2, s2, N, Kdim, qt, bs))
+    assert (y.double() - ref.double()).norm() <= 2.0 ** -8 * ref.double().norm()
+    assert torch.equal(y, K.qgemm_pair(x, p1, s1, p2, s2, N, Kdim, qt, bs))
+
+
+def test_pair_refuses(K):  # noqa: F811
+    for M, N, Kdim in ((1000, 512, 512), (32, 512, 320), (32, 500, 512)):
+        assert K.qgemm_pair_workspace(M, N, Kdim, "nf4", 64) < 0
+        x, w = torch.zeros(M, Kdim, dtype=torch.bfloat16, device="cuda"), torch.zeros(N * Kdim // 2, dtype=torch.uint8, device="cuda")
+        s = torch.zeros(N * Kdim // 64, dtype=torch.float32, device="cuda")
+        with pytest.raises(NotImplementedError):
+            K.qgemm_pair(x, w, s, w, s, N, Kdim, "nf4", 64)
+
+
+@pytest.mark.parametrize("zero", [7.53, 0.0, 16.0, 17.0, -2.25])
+def test_int4_scales(K, zero):  # noqa: F811
+    """Scales and zero points that need all eleven bits of a half, whole zero points up to 16 and others: bf16_rn(scale * (q - zero)) with an exact product."""
+    N, Kdim, M = 264, 512, 40
+    g = torch.Generator().manual_seed(3)
+    packed = torch.randint(0, 256, (N * Kdim // 2,), dtype=torch.uint8, generator=g)
+    scale = torch.stack([(torch.rand(N * 4, generator=g) * 0.1 + 1e-3).half(), torch.full((N * 4,), zero).half()], 1).contiguous()
+    q = torch.stack([packed & 15, packed >> 4], 1).view(N, Kdim).double()   # element e of a word in bits 4 e
+    w = (scale[:, 0].double().view(N, 4, 1) * (q.view(N, 4, 128) - scale[:, 1].double().view(N, 4, 1))).view(N, Kdim)
+    hot = torch.randint(0, Kdim, (M,), generator=g)
+    x = torch.nn.functional.one_hot(hot, Kdim).to(torch.bfloat16)
+    y = K.qgemm(x.cuda(), packed.cuda(), scale.cuda().view(torch.int32).view(-1), N, Kdim, "int4", 128)
+    assert torch.equal(y.cpu(), w.T[hot].to(torch.float32).to(torch.bfloat16))
