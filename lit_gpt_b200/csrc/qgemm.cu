@@ -552,6 +552,18 @@ static GemmPlan swiglu_plan(int64_t M, int64_t N, int64_t K, bool int4) {
   return (pair1 < pair2 ? pair1 : pair2) < worth ? best : none;
 }
 
+// Gate, up projection and product of 129 to 256 rows by the kernels of this file, as modelled.  us, in one launch here / in one of qgemm_short.cu, 4096 -> 14336 at 129 / 203 rows
+// nf4 80 / 50, 80 / 66, int4 63 / 52, 63 / 65; 4096 -> 6144 39 / 36, 39 / 44, 31 / 34, 31 / 42; 2048 -> 5632 23 / 26, 23 / 32, 19 / 26, 19 / 32.
+static double swiglu_time(int64_t M, int64_t N, int64_t K, bool int4) {
+  const GemmPlan one = gemm_plan(M, N, K, int4, true);
+  double best = 2.0 * gemm_time(M, N, K, int4, one, one.bn) - gemm_cost(int4, one.ctas, one.mt).start + 4.0 + 1e-6 * (double)M * (double)N;
+  for (int bn = 256; bn >= 128; bn -= 32) {
+    const double t = gemm_time(M, N, K, int4, GemmPlan{2, 1, 1, bn}, bn / 2);
+    if (t < best) best = t;
+  }
+  return best * (int4 ? 0.93 : 0.97);   // (int4: what the model is off by since an elected thread issues the products; and something has to be won)
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -634,7 +646,9 @@ int64_t b200_qgemm_pair_workspace(int64_t M, int64_t N, int64_t K, int qtype, in
   const int block = qtype == B200_Q_INT4 ? 128 : 64;
   if ((qtype != B200_Q_NF4 && qtype != B200_Q_FP4 && qtype != B200_Q_INT4) || blocksize != block || M <= 0 || N <= 0 || K <= 0) return -1;
   const ShortPlan s = short_plan(M, N, K, qtype, true, true);
-  return s.ctas ? (int64_t)short_scratch_bytes(M, s, true) : -1;
+  // (up to 128 rows there is no other launch for both; from 129 it is b200_qgemm_swiglu's or two)
+  if (s.ctas == 0 || (M > 128 && s.time >= swiglu_time(M, N, K, qtype == B200_Q_INT4))) return -1;
+  return (int64_t)short_scratch_bytes(M, s, true);
 }
 
 int b200_qgemm_pair(const b200_qgemm_args* a, const void* packed2, const void* scale2, b200_stream_t stream) {
@@ -647,7 +661,7 @@ int b200_qgemm_pair(const b200_qgemm_args* a, const void* packed2, const void* s
   ShortPlan s = short_plan(p.M, p.N, p.K, p.qtype, true, true);
   if (s.shared && (a->workspace == nullptr || a->workspace_bytes < short_scratch_bytes(p.M, s, true) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
     s = short_plan(p.M, p.N, p.K, p.qtype, true, false);
-  if (s.ctas == 0 || !short_takes(sa, true)) {
+  if (s.ctas == 0 || !short_takes(sa, true) || b200_qgemm_pair_workspace(p.M, p.N, p.K, p.qtype, a->blocksize) < 0) {
     set_error("b200_qgemm_pair: (M=%lld N=%lld K=%lld) or its addresses run as two b200_qgemm and b200_swiglu", (long long)a->M, (long long)a->N, (long long)a->K);
     return B200_ERR_UNSUPPORTED;
   }

@@ -17,7 +17,8 @@
 // Bound: the rebuilding warps, issue slots and the latency of their chain (wait, codes, arithmetic, tensor memory, hand-over): 0.87 us a unit of 256 k, nf4 and int4, at 17
 // rows, 1.3 at 203, where 0.42 is what the weights take from HBM.  us, qgemm.cu / here, weights in turn: 4096 -> 14336 nf4 at 17, 64, 129, 203 rows 35 / 21, 36 / 23,
 // 42 / 27, 42 / 32, int4 26 / 21, 27 / 22, 34 / 27, 34 / 31; 14336 -> 4096 at 64 nf4 37 / 25, int4 29 / 24; the pair of 4096 -> 14336 in one launch, against two and the
-// product, at 17 / 64 rows nf4 74 / 37, 75 / 41, int4 55 / 38, 57 / 41.
+// product, at 17 / 64 rows nf4 74 / 37, 75 / 41, int4 55 / 38, 57 / 41,
+// and against one launch of qgemm.cu at 129 / 203 80 / 50, 80 / 66, int4 63 / 52, 63 / 65.
 #include "qgemm_short.cuh"
 #include "tc05.cuh"
 
@@ -29,14 +30,14 @@ constexpr int kShGroups = 4, kShWarps = 4 * kShGroups, kShThreads = (kShWarps + 
 constexpr int kShStage = 128 * 128 + 128 * 16;        // 256 k of 128 features: packed codes and scales
 constexpr int kShLow = 3;                             // stages below the table of byte pairs
 constexpr int kShTable = 256 * 256;
-constexpr int kShMaxPair = 128;                       // rows of a gate / up pair: two accumulators beside the rebuilt weights
+constexpr int kShMaxPair = 208;                       // rows of a gate / up pair: two accumulators beside the rebuilt weights
 constexpr int kShSmem = 227 * 1024 - 2048;            // dynamic shared memory (static: barriers)
-constexpr int kShMaxW = 8, kShMaxB = 8, kShA = 2;     // most stages of weights and rows; stages of rebuilt weights (256 k: 128 columns each, handed over in halves)
+constexpr int kShMaxW = 8, kShMaxB = 8, kShA = 2, kShMaxRing = 8;   // most stages of weights and rows; stages of rebuilt weights (256 k: 128 columns each, handed over in halves)
 
 struct ShortParams {
   ShortArgs a;
   int tiles, nq, shared, nb;                          // tiles of 128 features, units (256 k) a tile, ..., accumulator columns (rows up to a multiple of 16)
-  int ws, bs;                                         // stages of weights and of rows
+  int ws, bs, ring;                                   // stages of weights and of rows; of single rebuilt k-blocks (a pair of more than 128 rows)
 };
 
 __device__ __forceinline__ int64_t unit_begin(int64_t c, int64_t ctas, int64_t tiles, int64_t nq, bool shared) {
@@ -113,8 +114,9 @@ __global__ void __launch_bounds__(kShThreads, 1)
 qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ CUtensorMap map_w2, unsigned* err) {
   constexpr int NACC = PAIR ? 2 : 1;
+  constexpr bool RING = PAIR && BQ == 1;   // accumulators that leave less than two stages of rebuilt weights: single k-blocks in turn (p.ring of them)
   extern __shared__ __align__(1024) uint8_t sh_smem[];
-  __shared__ __align__(8) uint64_t s_bars[2 * (kShMaxW + kShMaxB + 2 * kShA) + 3];
+  __shared__ __align__(8) uint64_t s_bars[2 * (kShMaxW + kShMaxB + kShMaxRing) + 3];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform, and known to be)
   const uint32_t base = (tc::smem_u32(sh_smem) + 1023u) & ~1023u;
@@ -126,7 +128,7 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
   const uint32_t row_block = (uint32_t)p.nb * 128u, row_stage = BQ * row_block;
   const uint32_t bars = tc::smem_u32(s_bars);
   const uint32_t w_full = bars, w_empty = w_full + 8 * kShMaxW, b_full = w_empty + 8 * kShMaxW, b_empty = b_full + 8 * kShMaxB, a_full = b_empty + 8 * kShMaxB,
-                 a_empty = a_full + 16 * kShA, acc_full = a_empty + 16 * kShA, acc_free = acc_full + 8, idle = acc_full + 16;
+                 a_empty = a_full + 8 * kShMaxRing, acc_full = a_empty + 8 * kShMaxRing, acc_free = acc_full + 8, idle = acc_full + 16;
   if (rows + (uint32_t)p.bs * row_stage > tc::smem_u32(sh_smem) + (uint32_t)kShSmem) {   // (a layout of shared memory other than the host counts with)
     if (tid == 0) *err = 1u;
     return;
@@ -134,7 +136,7 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
   if (tid == 0) {
     for (int i = 0; i < p.ws; ++i) { tc::mbar_init(w_full + 8 * i, 1 + 32); tc::mbar_init(w_empty + 8 * i, 1); }
     for (int i = 0; i < p.bs; ++i) { tc::mbar_init(b_full + 8 * i, 1); tc::mbar_init(b_empty + 8 * i, 1); }
-    for (int i = 0; i < 2 * kShA; ++i) { tc::mbar_init(a_full + 8 * i, kShWarps / 2); tc::mbar_init(a_empty + 8 * i, 1); }
+    for (int i = 0; i < (RING ? 8 : 2 * kShA); ++i) { tc::mbar_init(a_full + 8 * i, RING ? 4 : kShWarps / 2); tc::mbar_init(a_empty + 8 * i, 1); }
     tc::mbar_init(acc_full, 1);
     tc::mbar_init(acc_free, kShWarps);
     tc::mbar_init(idle, 1);
@@ -161,7 +163,7 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const uint32_t tmem = s_tmem, acc0 = tmem + 128u * kShA;   // rebuilt weights, then the accumulators
+  const uint32_t tmem = s_tmem, acc0 = tmem + (RING ? 32u * (uint32_t)p.ring : 128u * kShA);   // rebuilt weights, then the accumulators
   struct Segment { int tile, q0, n; };
   auto segment = [&](int64_t u) {
     Segment s;
@@ -199,12 +201,20 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc) : "r"(st + scale0));
       if (++sw == p.ws) { sw = 0; pw ^= 1u; }
     };
+    // A ring's k-blocks stand in the order of their products: of a unit the gate's and the up projection's first two, then their last two.  Number n takes the room of
+    // n - ring; either's hand-overs go by barrier n % 8, so that no wait is for a phase but the present one: a group's steps from one k-block to its next are 2 and 6.
+    int n = (g >> 1) * 4 + (g & 1);
     fetch();
     for (int64_t u = u0; ok;) {
-      ok = __all_sync(0xffffffffu, tc::mbar_wait_here(half_empty + 16 * (i & 1u), ((i >> 1) & 1u) ^ 1u));
+      const uint32_t full = RING ? a_full + 8 * (n & 7) : half_full + 16 * (i & 1u), to = RING ? tmem + lanes + 32u * (uint32_t)(n % p.ring) : to0 + 128u * (i & 1u);
+      if constexpr (RING) {
+        const int before = n - p.ring;
+        if (before >= 0) ok = __all_sync(0xffffffffu, tc::mbar_wait_here(a_empty + 8 * (before & 7), (uint32_t)(before >> 3) & 1u));
+      } else {
+        ok = __all_sync(0xffffffffu, tc::mbar_wait_here(half_empty + 16 * (i & 1u), ((i >> 1) & 1u) ^ 1u));
+      }
       if (!ok) break;
       tc::fence_after();
-      const uint32_t to = to0 + 128u * (i & 1u);
       if constexpr (INT4) {
         rebuild_int4(to, qw, sc);
       } else {
@@ -226,7 +236,8 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc::fence_before();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(half_full + 16 * (i & 1u));
+      if (lane == 0) tc::mbar_arrive(full);
+      if (RING) n += i & 1u ? 6 : 2;
       ++i;
       ++done;
       if (left > 0 && at + done < (int)nq * NACC) continue;
@@ -342,6 +353,45 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
     int sb = 0, sw = 0, at = (int)(u0 - (u0 / nq) * nq);      // the unit's first stage of rows; next stage of weights; unit within the tile
     uint32_t pa = 0u, pb = 0u, free_ph = 1u, fresh = 1u;      // fresh: a segment's first unit
     int left = (int)(u1 - u0);
+    if constexpr (RING) {
+      int slot = 0;
+      for (; left > 0 && ok; --left) {
+        if (fresh) {
+          ok = tc::mbar_wait_here(acc_free, free_ph);
+          free_ph ^= 1u;
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {                         // k-blocks 0 and 1 of the gate, of the up projection, 2 and 3 likewise
+          const int l = (c >> 2) * 2 + (c & 1), m = (c >> 1) & 1;
+          int s = sb + l;
+          uint32_t ph = pb;
+          if (s >= p.bs) { s -= p.bs; ph ^= 1u; }
+          if (m == 0) ok = ok && tc::mbar_wait_here(b_full + 8 * s, ph);
+          ok = ok && tc::mbar_wait_here(a_full + 8 * c, pa);
+          if (!ok) break;
+          tc::fence_after();
+          const uint32_t db = row_desc + s * stage_step, ta = tmem + 32u * (uint32_t)slot;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_ts(acc0 + (m ? (uint32_t)p.nb : 0u), ta + (uint32_t)(8 * k), db + 2 * k, idesc, l | k ? 1u : fresh ^ 1u);
+          tc::commit(a_empty + 8 * c);
+          if (m == 1) tc::commit(b_empty + 8 * s);
+          if (l == 3) {
+            tc::commit(w_empty + 8 * sw);
+            if (++sw == p.ws) sw = 0;
+          }
+          if (++slot == p.ring) slot = 0;
+        }
+        pa ^= 1u;
+        sb += 4;
+        while (sb >= p.bs) { sb -= p.bs; pb ^= 1u; }
+        fresh = 0u;
+        if (++at == p.nq || left == 1) {
+          if (ok) tc::commit(acc_full);
+          at = 0;
+          fresh = 1u;
+        }
+      }
+    }
     while (left > 0 && ok) {
 #pragma unroll
       for (int sa = 0; sa < kShA; ++sa) {                     // one unit a stage; of a pair one unit, its gate and its up projection
@@ -453,6 +503,7 @@ cudaError_t launch_kind(const ShortArgs& a, const ShortPlan& plan, cudaStream_t 
   const int stage = BQ * p.nb * 128;
   p.bs = (all - (INT4 ? 4 : PAIR ? 1 : 0) * kShStage) / stage;
   if (p.bs > 4) p.bs = 4;
+  p.ring = (512 - 2 * p.nb) / 32 < kShMaxRing ? (512 - 2 * p.nb) / 32 : kShMaxRing;
   p.ws = (INT4 ? 0 : kShLow) + (all - p.bs * stage) / kShStage;
   if (p.ws > kShMaxW) p.ws = kShMaxW;
   alignas(64) CUtensorMap mx, mw, mw2;
@@ -471,8 +522,7 @@ cudaError_t launch_kind(const ShortArgs& a, const ShortPlan& plan, cudaStream_t 
 template <bool INT4, bool PAIR>
 cudaError_t launch_rows(const ShortArgs& a, const ShortPlan& plan, cudaStream_t st) {
   if (a.M <= 64) return launch_kind<INT4, PAIR, 4>(a, plan, st);
-  if (PAIR || a.M <= 128) return launch_kind<INT4, PAIR, 2>(a, plan, st);
-  return launch_kind<INT4, PAIR, PAIR ? 2 : 1>(a, plan, st);
+  return a.M <= 128 ? launch_kind<INT4, PAIR, 2>(a, plan, st) : launch_kind<INT4, PAIR, 1>(a, plan, st);
 }
 
 }  // namespace
@@ -494,20 +544,21 @@ static double short_time(int64_t units, int64_t ctas, int nb, const ShortCost& c
 }
 
 ShortPlan short_plan(int64_t M, int64_t N, int64_t K, int qtype, bool pair, bool scratch) {
-  // [int4][rows up to 64, 128, 256][whole tiles, shared]; pairs [int4][whole, shared]
+  // [int4][rows up to 64, 128, 256][whole tiles, shared]; pairs [int4][rows up to 128, 208][whole, shared]
   static const ShortCost one[2][3][2] = {{{{4.53, 0.856, 0.0018, 0.512}, {7.04, 1.028, 0.0025, 0.275}},
                                           {{5.40, 0.766, 0.0024, 0.298}, {7.32, 0.980, 0.0036, 0.217}},
                                           {{7.44, 0.433, 0.0041, 0.218}, {6.17, 1.159, 0.0033, 0.241}}},
                                          {{{4.71, 0.930, 0.0, 0.547}, {6.96, 1.108, 0.0, 0.273}},
                                           {{5.75, 0.839, 0.0012, 0.306}, {7.30, 1.004, 0.0022, 0.218}},
                                           {{7.53, 0.584, 0.0029, 0.234}, {5.95, 1.058, 0.0031, 0.246}}}};
-  static const ShortCost two[2][2] = {{{3.79, 2.009, 0.00335, 0.17}, {9.85, 1.836, 0.00676, 0.29}}, {{2.43, 2.244, 0.00124, 0.25}, {9.13, 2.103, 0.00399, 0.29}}};
+  static const ShortCost two[2][2][2] = {{{{3.79, 2.009, 0.00335, 0.17}, {9.85, 1.836, 0.00676, 0.29}}, {{10.91, 0.202, 0.0143, 0.222}, {8.19, 2.219, 0.0086, 0.373}}},
+                                         {{{2.43, 2.244, 0.00124, 0.25}, {9.13, 2.103, 0.00399, 0.29}}, {{10.76, 0.703, 0.0112, 0.246}, {8.19, 2.117, 0.0089, 0.328}}}};
   ShortPlan best{0, false, 0.0};
   if (M < 1 || M > (pair ? kShMaxPair : 256) || N < 1 || K < 256 || K % 256 || N % 8) return best;
   const int64_t tiles = (N + 127) / 128, nq = K / 256, sms = sm_count(), total = tiles * nq;
   const int nb = (int)((M + 15) / 16 * 16), rows = M <= 64 ? 0 : M <= 128 ? 1 : 2;
   const bool int4 = qtype == B200_Q_INT4;
-  const ShortCost* const cost = pair ? two[int4] : one[int4][rows];
+  const ShortCost* const cost = pair ? two[int4][rows == 2] : one[int4][rows];
   best.ctas = (int)(tiles < sms ? tiles : sms);
   best.time = short_time((tiles + sms - 1) / sms * nq, best.ctas, nb, cost[0]);
   if (scratch) {

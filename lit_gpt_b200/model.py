@@ -657,11 +657,11 @@ class LLaMAMLP(nn.Module):
                 and f1.quant_type == f2.quant_type and f1.quant_type != "int8" and not torch.compiler.is_compiling()):
             # gate and up projections + SwiGLU in one pass over both weight matrices
             return self.proj(f1.gemv(x, other=f2))
-        if (rows > 16 and x.is_cuda and x.dtype == torch.bfloat16 and not torch.compiler.is_compiling()
-                and (short_pair if rows <= 128 else prefill_pair)(f1, f2, rows) and x.size(-1) == f1.in_features):
-            (pw, ps), (pw2, ps2) = f1.packed(), f2.packed()
-            both = K.qgemm_pair if rows <= 128 else K.qgemm_swiglu
-            return self.proj(both(x, pw, ps, pw2, ps2, f1.out_features, f1.in_features, f1.quant_type, f1.blocksize))
+        if rows > 16 and x.is_cuda and x.dtype == torch.bfloat16 and not torch.compiler.is_compiling() and x.size(-1) == getattr(f1, "in_features", None):
+            both = K.qgemm_pair if rows <= 208 and short_pair(f1, f2, rows) else K.qgemm_swiglu if rows > 128 and prefill_pair(f1, f2, rows) else None
+            if both is not None:
+                (pw, ps), (pw2, ps2) = f1.packed(), f2.packed()
+                return self.proj(both(x, pw, ps, pw2, ps2, f1.out_features, f1.in_features, f1.quant_type, f1.blocksize))
         x_fc_1 = self.fc_1(x)
         x_fc_2 = self.fc_2(x)
         if (x_fc_1.is_cuda and x_fc_1.dtype == torch.bfloat16 and x_fc_1.numel() % 8 == 0 and not torch.compiler.is_compiling()

@@ -22,8 +22,8 @@ def test_one_hot_rows_read_the_weights(K, qt, M, N, Kdim):  # noqa: F811
     assert torch.equal(K.qgemm(x, packed, scale, N, Kdim, qt, bs, bias=bias.cuda()).cpu(), (want.float() + bias.float()).to(torch.bfloat16))
 
 
-@pytest.mark.parametrize("M", [1, 17, 64, 65, 128])
-@pytest.mark.parametrize("N,Kdim", [(136, 256), (1000, 1280), (11008, 4096), (19208, 512)])
+@pytest.mark.parametrize("M", [1, 17, 64, 65, 128, 129, 160, 176, 192, 203, 208])
+@pytest.mark.parametrize("N,Kdim", [(136, 256), (1000, 1280), (11008, 4096), (19208, 512), (18952, 1280)])
 @pytest.mark.parametrize("qt", ["nf4", "fp4", "int4"])
 def test_pair_is_the_separate_launches(K, qt, M, N, Kdim):  # noqa: F811
     """Both projections and their product in one launch against two GEMMs and the product: sums in another order of k ranges, so some bf16 roundings of either
@@ -31,7 +31,9 @@ def test_pair_is_the_separate_launches(K, qt, M, N, Kdim):  # noqa: F811
     _, _, p1, s1, bs, _ = _gemv_case(K, N, Kdim, 1, qt, seed=M)
     _, _, p2, s2, _, _ = _gemv_case(K, N, Kdim, 1, qt, seed=N)
     x = torch.randn(M, Kdim, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
-    assert K.qgemm_pair_workspace(M, N, Kdim, qt, bs) >= 0
+    if K.qgemm_pair_workspace(M, N, Kdim, qt, bs) < 0:
+        assert M > 128
+        pytest.skip("another launch is the shorter way")
     y = K.qgemm_pair(x, p1, s1, p2, s2, N, Kdim, qt, bs)
     ref = K.swiglu(K.qgemm(x, p1, s1, N, Kdim, qt, bs), K.qgemm(x, p2, s2, N, Kdim, qt, bs))
     assert (y.double() - ref.double()).norm() <= 2.0 ** -8 * ref.double().norm()
@@ -39,7 +41,7 @@ def test_pair_is_the_separate_launches(K, qt, M, N, Kdim):  # noqa: F811
 
 
 def test_pair_refuses(K):  # noqa: F811
-    for M, N, Kdim in ((1000, 512, 512), (32, 512, 320), (32, 500, 512)):
+    for M, N, Kdim in ((209, 512, 512), (1000, 512, 512), (32, 512, 320), (32, 500, 512)):
         assert K.qgemm_pair_workspace(M, N, Kdim, "nf4", 64) < 0
         x, w = torch.zeros(M, Kdim, dtype=torch.bfloat16, device="cuda"), torch.zeros(N * Kdim // 2, dtype=torch.uint8, device="cuda")
         s = torch.zeros(N * Kdim // 64, dtype=torch.float32, device="cuda")
