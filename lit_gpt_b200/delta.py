@@ -14,6 +14,8 @@ rows of q | k | v and the state matrices, laid out as the recurrence kernel read
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -35,6 +37,11 @@ class DeltaState(nn.Module):
 
     def tensors(self):
         return [self.tail, self.matrices]
+
+
+@functools.lru_cache(maxsize=256)
+def _conv_plan(heads: int, kv_heads: int, dk: int, dv: int) -> K.ConvPlan:
+    return K.ConvPlan([(kv_heads, dk, dict(act=1, post=2, post_scale=dk ** -0.5, eps=1e-6)), (kv_heads, dk, dict(act=1, post=2, eps=1e-6)), (heads, dv, dict(act=1))])
 
 
 class GatedDeltaRule(nn.Module):
@@ -71,15 +78,9 @@ class GatedDeltaRule(nn.Module):
         s, n = self.spec, h.shape[0]
         H, G, dk, dv = s.heads, s.kv_heads, s.dim, s.vdim
         proj = F.linear(h, self.w_in)
-        qkv = torch.empty((n, self.conv_cols), dtype=torch.float32, device=h.device)
-        q, k, v = qkv[:, : G * dk], qkv[:, G * dk : 2 * G * dk], qkv[:, 2 * G * dk :]
-        cw = self.conv
-        groups = [
-            K.conv_group(cw[: G * dk], q, 0, G, dk, act=1, post=2, post_scale=dk ** -0.5, eps=1e-6),
-            K.conv_group(cw[G * dk : 2 * G * dk], k, G * dk, G, dk, act=1, post=2, eps=1e-6),
-            K.conv_group(cw[2 * G * dk :], v, 2 * G * dk, H, dv, act=1),
-        ]
-        K.short_conv(proj, groups, s.conv, state.tail, batch.seq_state, batch.row_seq)
+        qkv = h.new_empty((n, self.conv_cols), dtype=torch.float32)
+        q, k, v = qkv.split((G * dk, G * dk, H * dv), 1)
+        K.short_conv_plan(proj, self.conv, qkv, _conv_plan(H, G, dk, dv), s.conv, state.tail, batch.seq_state, batch.row_seq)
         beta_in = proj[:, self.off_beta :]
         if s.channel:
             decay_in = F.linear(proj[:, self.off_decay : self.off_beta], self.w_decay2)

@@ -420,14 +420,22 @@ def qgemm(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, N: int, K:
     M = x.numel() // K
     if out is not None and (out.numel() != M * N or out.dtype != torch.bfloat16 or not out.is_contiguous()):
         raise C.B200Error(f"qgemm: out must be {M} x {N} contiguous bfloat16 numbers")
-    y = out if out is not None else torch.empty(tuple(x.shape[:-1]) + (N,), dtype=torch.bfloat16, device=x.device)
-    need = C.load().b200_qgemm_workspace_bytes(M, N, K)   # fp32 partial sums of a launch split over k ranges; 0 otherwise
+    y, device = out if out is not None else x.new_empty((*x.shape[:-1], N)), x.device
+    need = _qgemm_workspace_bytes(M, N, K, device.index)   # fp32 partial sums of a launch split over k ranges; 0 otherwise
     # (from the allocator on every call: safe on any stream and inside a capture, whose graph then keeps it)
-    ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
-    args = C.QGemmArgs(packed=packed.data_ptr(), scale=scale.data_ptr(), qtype=QTYPES[quant_type], blocksize=blocksize, M=M, N=N, K=K,
-                       x=x.data_ptr(), bias=C.ptr(bias), y=y.data_ptr(), workspace=C.ptr(ws), workspace_bytes=0 if ws is None else ws.numel())
-    C.check(C.load().b200_qgemm(ctypes.byref(args), C.stream_ptr(x.device)), "qgemm")
+    ws = x.new_empty(need, dtype=torch.uint8) if need else None
+    args = C.QGemmArgs(packed.data_ptr(), scale.data_ptr(), QTYPES[quant_type], blocksize, M, N, K, x.data_ptr(), None if bias is None else bias.data_ptr(),
+                       y.data_ptr(), None if ws is None else ws.data_ptr(), need)
+    rc = C.load().b200_qgemm(ctypes.byref(args), C.stream_ptr(device))
+    if rc:
+        C.check(rc, "qgemm")
     return y
+
+
+@functools.lru_cache(maxsize=4096)
+def _qgemm_workspace_bytes(M: int, N: int, K: int, device: Optional[int]) -> int:
+    """Asked once for a size (the host is what bounds a call of a few dozen rows).  The device is part of the key: the ranges are for its SMs."""
+    return C.load().b200_qgemm_workspace_bytes(M, N, K)
 
 
 def qgemm_swiglu_supported(M: int, N: int, K: int, quant_type: str = "nf4", blocksize: int = 64) -> bool:
@@ -478,6 +486,7 @@ def qgemm_pair(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, packe
 def qgemm_tune(wide: bool = True) -> None:
     """development switch: long prompts may use tiles of 512 tokens (default) or keep to 256"""
     C.check(C.load().b200_qgemm_tune(1 if wide else 0), "qgemm_tune")
+    _qgemm_workspace_bytes.cache_clear()
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, delta: Optional[torch.Tensor] = None,
@@ -1108,6 +1117,52 @@ def short_conv(inp: torch.Tensor, groups: Sequence["C.ConvGroup"], taps: int, ta
                                           _code(inp), st), "conv_tail_update")
 
 
+class ConvPlan:
+    """Neighbouring groups of heads of one convolution, without their addresses: what ``short_conv_plan`` copies and completes on each call."""
+
+    def __init__(self, groups: Sequence[Tuple[int, int, dict]]) -> None:
+        """groups: (heads, dim, keywords of ``conv_group``) in the order of their columns."""
+        self.kind, col = C.ConvGroup * len(groups), 0
+        self.template, self.rot_dims = self.kind(), max(kw.get("rot_dims", 0) for _, _, kw in groups)
+        for g, (heads, dim, kw) in zip(self.template, groups):
+            g.col0, g.heads, g.dim, g.act, g.post, g.rot_dims = col, heads, dim, kw.get("act", 0), kw.get("post", 0), kw.get("rot_dims", 0)
+            g.rot_mscale, g.post_scale, g.eps = kw.get("rot_mscale", 1.0), kw.get("post_scale", 1.0), kw.get("eps", 0.0)
+            col += heads * dim
+        self.cols, self.starts = col, [g.col0 for g in self.template]
+
+
+def short_conv_plan(inp: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: ConvPlan, taps: int, tail: torch.Tensor, seqs: torch.Tensor,
+                    row_seq: torch.Tensor, inv_freq: Optional[torch.Tensor] = None) -> None:
+    """``short_conv`` of all columns of w (cols, taps) into out (rows, cols).  The host is what bounds a layer of a few hundred rows: three ``conv_group``s on slices
+    and ``short_conv`` took 22 us of it, this 11."""
+    C.require_cuda(inp, w, out, tail, seqs, row_seq, inv_freq)
+    if not w.is_contiguous() or out.stride(-1) != 1 or out.dtype not in (w.dtype, torch.float32) or w.numel() != plan.cols * taps or out.shape[-1] != plan.cols:
+        raise C.B200Error("short_conv_plan: contiguous weights (cols, taps), output rows of as many columns in the model dtype or fp32")
+    if (inv_freq is not None or plan.rot_dims) and (inv_freq is None or inv_freq.dtype != torch.float64 or inv_freq.numel() < plan.rot_dims // 2):
+        raise C.B200Error("short_conv_plan: inv_freq must be a CUDA float64 tensor of rot_dims / 2 entries")
+    if inp.stride(-1) != 1 or seqs.dtype != torch.int32 or row_seq.dtype != torch.int32 or not seqs.is_contiguous():
+        raise C.B200Error("short_conv_plan: unit inner stride, int32 seqs and row_seq")
+    if tail.dtype != inp.dtype or not tail.is_contiguous():
+        raise C.B200Error("short_conv_plan: the tail must be contiguous in the model dtype")
+    arr = plan.kind.from_buffer_copy(plan.template)
+    wp, op, ld, wsize, osize = w.data_ptr(), out.data_ptr(), out.stride(0), w.element_size() * taps, out.element_size()
+    f32, freq = int(osize != w.element_size()), None if inv_freq is None else inv_freq.data_ptr()
+    for g, col in zip(arr, plan.starts):
+        g.w, g.out, g.ld_out, g.out_f32 = wp + col * wsize, op + col * osize, ld, f32
+        if freq is not None and g.rot_dims:
+            g.inv_freq = freq
+    lib, st, code = C.load_core(), C.stream_ptr(inp.device), _code(inp)
+    ip, il, tp, stride, cols, sp = inp.data_ptr(), inp.stride(0), tail.data_ptr(), tail.stride(0), tail.shape[-1], seqs.data_ptr()
+    rc = lib.b200_short_conv(ip, il, arr, len(arr), taps, tp, stride, cols, sp, row_seq.data_ptr(), inp.shape[0], code, st)
+    if rc:
+        C.check(rc, "short_conv")
+    if taps > 1:
+        rc = lib.b200_conv_tail_update(ip, il, tp, stride, cols, taps, sp, seqs.shape[0], code, st)
+        if rc:
+            C.check(rc, "conv_tail_update")
+
+
+@functools.lru_cache(maxsize=None)
 def delta_rule_state_floats(dk: int, dv: int) -> int:
     """fp32 numbers one head's state takes in the kernel's own order."""
     return int(C.load_core().b200_delta_rule_state_floats(dk, dv))
@@ -1132,15 +1187,13 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_in: torch
             raise C.B200Error("delta_rule: unit inner strides")
     if state.stride(0) < heads * delta_rule_state_floats(dk, dv) or not state.is_contiguous():
         raise C.B200Error("delta_rule: the state slots are too small")
-    out = torch.empty((q.shape[0], heads * dv), dtype=torch.float32, device=q.device)
-    args = C.DeltaRuleArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), ldq=q.stride(0), ldk=k.stride(0), ldv=v.stride(0),
-                           beta_in=beta_in.data_ptr(), ld_beta=beta_in.stride(0), decay_in=decay_in.data_ptr(), ld_decay=decay_in.stride(0),
-                           a_log=a_log.data_ptr(), dt_bias=dt_bias.data_ptr(), state=state.data_ptr(), state_slot_stride=state.stride(0),
-                           out=out.data_ptr(), ldo=out.stride(0), seqs=seqs.data_ptr(), n_seqs=seqs.shape[0], heads=heads, kv_heads=kv_heads,
-                           dk=dk, dv=dv, channel_decay=int(channel_decay), dtype=_code(beta_in), max_rows=int(max_rows), rows=q.shape[0])
-    lib, n_seqs = C.load_core(), seqs.shape[0]
+    n, n_seqs = q.shape[0], seqs.shape[0]
+    out = q.new_empty((n, heads * dv))
+    args = C.DeltaRuleArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), beta_in.data_ptr(), beta_in.stride(0),
+                           decay_in.data_ptr(), decay_in.stride(0), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), state.stride(0), out.data_ptr(),
+                           heads * dv, seqs.data_ptr(), n_seqs, heads, kv_heads, dk, dv, int(channel_decay), _code(beta_in), int(max_rows), n)
     # a prompt goes 32 tokens at a time; max_rows says whether that pays, the rows there are how much scratch it takes
-    n, ws = q.shape[0], None
+    lib, ws = C.load_core(), None
     chunks = DELTA_CHUNKED
     if chunks is None:
         chunks = lib.b200_delta_rule_in_chunks(n, int(max_rows), n_seqs, heads, dk, dv, int(channel_decay)) != 0
@@ -1251,18 +1304,19 @@ def window_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_ring: torch
         raise C.B200Error("window_attn: one dtype, contiguous rings")
     if q.stride(-1) != 1 or k.stride(-1) != 1 or v.stride(-1) != 1 or seqs.dtype != torch.int32 or not seqs.is_contiguous():
         raise C.B200Error("window_attn: unit inner strides, int32 seqs")
-    ring = k_ring.shape[1] - keep
-    out = _out_rows(out, q.shape[0], n_head * dv, q, "window_attn")
+    ring, n = k_ring.shape[1] - keep, q.shape[0]
+    out = _out_rows(out, n, n_head * dv, q, "window_attn")
     lib, st = C.load_core(), C.stream_ptr(q.device)
     mma = from_start and max_q_len > 1 and WINDOW_PREFILL_MMA and q.dtype == torch.bfloat16
-    if (mma and keep == 0 and softcap == 0.0 and out_scale == 1.0 and dk == dv and dk in (64, 128)
-            and not (q.stride(0) | k.stride(0) | v.stride(0)) & 7 and not (q.data_ptr() | k.data_ptr() | v.data_ptr() | seqs.data_ptr()) & 15):
-        C.check(lib.b200_attn_prefill_window_ex(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), seqs.data_ptr(),
-                                                seqs.shape[0], max_q_len, out.data_ptr(), out.stride(0), n_head, n_kv_head, dk, float(scale), window,
-                                                C.ptr(sink), C.ptr(r1), C.ptr(r2), C.ptr(gate), ldg, gate_mode, st), "attn_prefill_window")
-        C.check(lib.b200_ring_store(k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), k_ring.data_ptr(), v_ring.data_ptr(), ring, n_kv_head * dk,
-                                    n_kv_head * dv, seqs.data_ptr(), row_seq.data_ptr(), q.shape[0], _code(q), st), "ring_store")
-        return out
+    if mma and keep == 0 and softcap == 0.0 and out_scale == 1.0 and dk == dv and dk in (64, 128):
+        qp, kp, vp, sp, ldq, ldk, ldv = q.data_ptr(), k.data_ptr(), v.data_ptr(), seqs.data_ptr(), q.stride(0), k.stride(0), v.stride(0)
+        if not ((ldq | ldk | ldv) & 7 or (qp | kp | vp | sp) & 15):
+            rc = lib.b200_attn_prefill_window_ex(qp, ldq, kp, ldk, vp, ldv, sp, seqs.shape[0], max_q_len, out.data_ptr(), out.stride(0), n_head, n_kv_head, dk,
+                                                 float(scale), window, C.ptr(sink), C.ptr(r1), C.ptr(r2), C.ptr(gate), ldg, gate_mode, st)
+            C.check(rc, "attn_prefill_window")
+            C.check(lib.b200_ring_store(kp, ldk, vp, ldv, k_ring.data_ptr(), v_ring.data_ptr(), ring, n_kv_head * dk, n_kv_head * dv, sp, row_seq.data_ptr(), n,
+                                        _code(q), st), "ring_store")
+            return out
     # the any-size kernels store the step's rows into the rings themselves (single rows: inside the attention kernel)
     args = C.WindowAttnArgs(row_seq=row_seq.data_ptr(), rows=q.shape[0], q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=out.data_ptr(),
                             ldq=q.stride(0), ldk=k.stride(0), ldv=v.stride(0), ldo=out.stride(0), k_ring=k_ring.data_ptr(), v_ring=v_ring.data_ptr(), sink=C.ptr(sink), seqs=seqs.data_ptr(),

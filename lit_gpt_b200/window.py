@@ -22,6 +22,7 @@ own ahead of the ring's.
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -46,6 +47,12 @@ class WindowState(nn.Module):
 
     def tensors(self):
         return [self.tail, self.k_ring, self.v_ring]
+
+
+@functools.lru_cache(maxsize=256)
+def _conv_plan(heads: int, kv_heads: int, dk: int, dv: int, rot_dims: int, magnitude: float, eps: float) -> K.ConvPlan:
+    turned = dict(post=1, rot_dims=rot_dims, rot_mscale=magnitude, eps=eps)
+    return K.ConvPlan([(heads, dk, turned), (kv_heads, dk, turned), (kv_heads, dv, {})])
 
 
 class WindowAttention(nn.Module):
@@ -82,18 +89,11 @@ class WindowAttention(nn.Module):
         s, n = self.spec, h.shape[0]
         H, G, dk, dv = s.heads, s.kv_heads, s.dim, s.vdim
         qkv = F.linear(h, self.w_qkv, self.b_qkv)
-        out = torch.empty((n, self.cols), dtype=h.dtype, device=h.device)
-        q, k, v = out[:, : H * dk], out[:, H * dk : (H + G) * dk], out[:, (H + G) * dk :]
+        out = h.new_empty((n, self.cols))
+        q, k, v = out.split((H * dk, G * dk, G * dv), 1)
         rot = s.rot
-        rd = rot.dims if rot is not None else 0
-        mag = rot.magnitude if rot is not None else 1.0
-        cw, fr = self.conv, self.inv_freq(h.device)
-        groups = [
-            K.conv_group(cw[: H * dk], q, 0, H, dk, post=1, rot_dims=rd, inv_freq=fr, rot_mscale=mag, eps=self.eps),
-            K.conv_group(cw[H * dk : (H + G) * dk], k, H * dk, G, dk, post=1, rot_dims=rd, inv_freq=fr, rot_mscale=mag, eps=self.eps),
-            K.conv_group(cw[(H + G) * dk :], v, (H + G) * dk, G, dv),
-        ]
-        K.short_conv(qkv, groups, s.conv, state.tail, batch.seq_state, batch.row_seq)
+        plan = _conv_plan(H, G, dk, dv, rot.dims if rot is not None else 0, rot.magnitude if rot is not None else 1.0, self.eps)
+        K.short_conv_plan(qkv, self.conv, out, plan, s.conv, state.tail, batch.seq_state, batch.row_seq, self.inv_freq(h.device))
         y = K.window_attn(q, k, v, state.k_ring, state.v_ring, self.sink, batch.seq_state, batch.row_seq, batch.max_q_len, H, G, dk, dv,
                           s.window, s.scale, from_start=batch.identity_ctx)
         return F.linear(y, self.w_o, self.b_o)
