@@ -107,8 +107,8 @@ attn_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   __shared__ int s_maxpos[kPfThreads / 32];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
-  const int mt = (int)gridDim.x - 1 - (int)blockIdx.x;     // long (late) query tiles are scheduled first
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int late = (int)blockIdx.x / n_head;               // long (late) query tiles are scheduled first, those of all heads before any head's earlier ones
+  const int h = (int)blockIdx.x - late * n_head, b = blockIdx.y, mt = (int)gridDim.x / n_head - 1 - late;
   const int grp = h / (n_head / n_groups);
   const int r0 = mt * kPfBM;
   griddep_launch();
@@ -445,7 +445,7 @@ cudaError_t launch_prefill(const void* q, const void* kc, const void* vc, const 
     if (e != cudaSuccess) return e;
     once.done();
   }
-  dim3 grid((T + kPfBM - 1) / kPfBM, H, B);
+  dim3 grid((T + kPfBM - 1) / kPfBM * H, B);
   return launch(attn_prefill_kernel<HS, PosT, HK2, MODE, HV, EX>, grid, dim3(kPfThreads), smem, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)kc,
                 (const __nv_bfloat16*)vc, (const PosT*)pos, (__nv_bfloat16*)y, T, H, G, max_seq, scale * 1.4426950408889634f, vw);
 }

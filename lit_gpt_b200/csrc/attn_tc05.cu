@@ -16,8 +16,8 @@
 // summed as rounded, as they multiply V (the sum of the unrounded ones makes the error against 64 bits 0.1 to 0.4 % larger).  (Moving the maximum only when it grew by 2^8 saves a tenth of the time and raises the error against 64 bits by half.)
 //
 // Bound: the chain of one tile -- 128 exponentials a row on the special-function units (16 a clock and SM), then its two products, 1270 clocks
-// where shared memory feeds them -- of which the other tile's fills the gaps.  32 heads of 128 over 8 key-value heads, 4096 rows: 230 us, 598
-// TFLOP/s of the causal half (589 us with the mma.sync tiles of attn_prefill.cu).
+// where shared memory feeds them -- of which the other tile's fills the gaps.  32 heads of 128 over 8 key-value heads, 4096 rows: 158 us, 870
+// TFLOP/s of the causal half (589 us with the mma.sync tiles of attn_prefill.cu).  Taking a quarter of the exponentials with multiply-adds instead: 225 us, issue slots.
 #include "attn_tc05.cuh"
 #include "tc05.cuh"
 
@@ -96,8 +96,10 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   __shared__ uint32_t s_tmem;
   __shared__ int s_max[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be the same in all lanes)
-  const int h = blockIdx.y, b = blockIdx.z, grp = h / (A.n_head / A.n_groups);
-  const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * A.span;   // late rows, which see most keys, are scheduled first
+  // Late rows, which see most keys, are scheduled first, those of all heads before any head's earlier ones: with a head's rows next to each other the last heads'
+  // late rows started when the others were nearly done (32 heads of 128, 4096 rows: 512 CTAs on 148 SMs, 196 us; 158 in this order).
+  const int late = (int)blockIdx.x / A.n_head, h = (int)blockIdx.x - late * A.n_head, b = blockIdx.y, grp = h / (A.n_head / A.n_groups);
+  const int r0 = ((int)gridDim.x / A.n_head - 1 - late) * A.span;
   const uint32_t smem = (tc::smem_u32(at_smem) + 1023u) & ~1023u;
   const uint32_t sq_ = smem, sk_ = smem + 2 * C::kBytes, sv_ = smem + 4 * C::kBytes;
   const uint32_t bars = tc::smem_u32(s_bars);
@@ -448,7 +450,7 @@ cudaError_t launch_hs(AttnTc05Args a, int batch, cudaStream_t st) {
   // one: 12.6, 10.8 / 13.2, 11.3 / 17.9, 16.0; from position 4000 80.6, 70.6 / 84.9, 72.6 / 86.7, 77.4.
   const int64_t pairs = (int64_t)((a.T + 2 * kAtBM - 1) / (2 * kAtBM)) * a.n_head * batch;
   a.span = pairs * 2 <= sm_count() ? kAtBM : 2 * kAtBM;
-  const dim3 grid((unsigned)((a.T + a.span - 1) / a.span), (unsigned)a.n_head, (unsigned)batch);
+  const dim3 grid((unsigned)(((int64_t)a.T + a.span - 1) / a.span * a.n_head), (unsigned)batch);
   unsigned* const err = wait_error_word();
   if (!err) return cudaErrorMemoryAllocation;
   return launch(attn_tc05_kernel<HS>, grid, dim3(kAtThreads), (size_t)smem, st, a, mk, mv, err);
