@@ -521,18 +521,9 @@ static cudaError_t launch_plan(const GemmParams& p, const GemmPlan& g, cudaStrea
   return g.mt == 2 ? launch_gemm<2, 2, INT4>(p, st) : launch_gemm<2, 1, INT4>(p, st);
 }
 
-// Tile of a gate / up pair in one launch; no sub-tiles (mt 0) where two launches and the product are the shorter way.  us, two launches and the product, each
-// with its best tile, against one, nf4 / int4: 4096 -> 11008 at 203 rows 83 -> 76 / 70 -> 65, at 400 115 -> 95 / 116 -> 101, at 1000 223 -> 158 / 228 -> 171;
-// 5120 -> 13824 at 300 131 -> 124 / 134 -> 133, at 2000 470 -> 435 / 462 -> 438; 4096 -> 14336 at 4096 859 -> 769 / 883 -> 776.  Up to 512 rows the two ways' times
-// as modelled decide.  Beyond, whether one launch saves a round of tiles with all their features: the second of two launches starts on the SMs that the
-// first one's last round leaves idle, which the model does not know, so a twentieth has to be won.  That line counts in clocks of an older kernel (1500 and 1130 a
-// k-block of full tiles) and not the tile that then runs, and errs towards two launches: of 132 shapes and types measured beyond 512 rows one launch is shorter
-// in all, and 32 run apart, 5 to 32 % longer (4096 -> 11008, nf4, at 513 rows 184 against 145, at 4096 629 / 573).
-static GemmPlan swiglu_plan(int64_t M, int64_t N, int64_t K, bool int4) {
-  const GemmPlan none{2, 0, 1, 256};
-  if (M <= 128) return none;
-  const int64_t units = sm_count() / 2, n = (N + 127) / 128, nkb = K / kBK;
-  GemmPlan best = none;
+// Tile of a gate / up pair in one launch (from 129 rows)
+static GemmPlan swiglu_tile(int64_t M, int64_t N, int64_t K, bool int4) {
+  GemmPlan best{2, 0, 1, 256};
   double best_t = -1.0;
   for (int mt = 1; mt <= (M > 256 && g_gemm_wide.load() ? 2 : 1); ++mt)
     for (int bn = 256; bn >= 128; bn -= 32) {
@@ -540,6 +531,21 @@ static GemmPlan swiglu_plan(int64_t M, int64_t N, int64_t K, bool int4) {
       const double t = gemm_time(M, N, K, int4, g, bn / 2);
       if (best_t < 0.0 || t < best_t) { best_t = t; best = g; }
     }
+  return best;
+}
+
+// The same, no sub-tiles (mt 0) where b200_qgemm_swiglu refuses.  us, two launches and the product, each
+// with its best tile, against one, nf4 / int4: 4096 -> 11008 at 203 rows 83 -> 76 / 70 -> 65, at 400 115 -> 95 / 116 -> 101, at 1000 223 -> 158 / 228 -> 171;
+// 5120 -> 13824 at 300 131 -> 124 / 134 -> 133, at 2000 470 -> 435 / 462 -> 438; 4096 -> 14336 at 4096 859 -> 769 / 883 -> 776.  Up to 512 rows the two ways' times
+// as modelled decide.  Beyond, an older line stands, which counts rounds of full tiles in clocks of an older kernel (1500 and 1130 a k-block).  One launch is shorter
+// where it refuses too, in all of 104 shapes and types measured, and b200_qgemm_pair takes those: 4096 -> 11008 at 513 rows 180 / 137 (nf4), 139 / 118 (int4),
+// at 2400 378 / 336; 4096 -> 14336 at 1024 219 / 201, 205 / 185; 5120 -> 13824 at 2000 446 / 412, 433 / 408.
+static GemmPlan swiglu_plan(int64_t M, int64_t N, int64_t K, bool int4) {
+  const GemmPlan none{2, 0, 1, 256};
+  if (M <= 128) return none;
+  const int64_t units = sm_count() / 2, n = (N + 127) / 128, nkb = K / kBK;
+  const GemmPlan best = swiglu_tile(M, N, K, int4);
+  const double best_t = gemm_time(M, N, K, int4, best, best.bn / 2);
   if (M <= 512) {
     const GemmPlan one = gemm_plan(M, N, K, int4, true);
     const double apart = 2.0 * gemm_time(M, N, K, int4, one, one.bn) - gemm_cost(int4, one.ctas, one.mt).start + 4.0 + 1e-6 * (double)M * (double)N;   // (and the product)
@@ -642,9 +648,26 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
   return B200_OK;
 }
 
+static int launch_swiglu(const b200_qgemm_args* a, GemmParams p, const GemmPlan& g, const void* packed2, const void* scale2, b200_stream_t stream, const char* what) {
+  p.packed2 = reinterpret_cast<const uint8_t*>(packed2);
+  p.scale2 = reinterpret_cast<const uint32_t*>(scale2);
+  p.ksplit = 1;
+  p.bn = g.bn;
+  const cudaStream_t st = (cudaStream_t)stream;
+  const bool int4 = a->qtype == B200_Q_INT4;
+  const cudaError_t e = g.mt == 2 ? (int4 ? launch_gemm<2, 2, true, true>(p, st) : launch_gemm<2, 2, false, true>(p, st))
+                                : (int4 ? launch_gemm<2, 1, true, true>(p, st) : launch_gemm<2, 1, false, true>(p, st));
+  if (e != cudaSuccess) {
+    set_error("%s: launch failed: %s", what, cudaGetErrorString(e));
+    return B200_ERR_CUDA;
+  }
+  return B200_OK;
+}
+
 int64_t b200_qgemm_pair_workspace(int64_t M, int64_t N, int64_t K, int qtype, int blocksize) {
   const int block = qtype == B200_Q_INT4 ? 128 : 64;
   if ((qtype != B200_Q_NF4 && qtype != B200_Q_FP4 && qtype != B200_Q_INT4) || blocksize != block || M <= 0 || N <= 0 || K <= 0) return -1;
+  if (M > 512) return K % block == 0 && N % 8 == 0 && N <= 65535LL * 128 && M <= 65535LL * 128 && swiglu_plan(M, N, K, qtype == B200_Q_INT4).mt == 0 ? 0 : -1;
   const ShortPlan s = short_plan(M, N, K, qtype, true, true);
   // (up to 128 rows there is no other launch for both; from 129 it is b200_qgemm_swiglu's or two)
   if (s.ctas == 0 || (M > 128 && s.time >= swiglu_time(M, N, K, qtype == B200_Q_INT4))) return -1;
@@ -656,6 +679,8 @@ int b200_qgemm_pair(const b200_qgemm_args* a, const void* packed2, const void* s
   if (const int rc = gemm_args(a, p)) return rc;
   B200_CHECK_ARG(packed2 && scale2 && (reinterpret_cast<uintptr_t>(packed2) & 15) == 0, "b200_qgemm_pair: null or misaligned second matrix");
   B200_CHECK_ARG(!a->bias, "b200_qgemm_pair: takes no bias");
+  if (p.M > 512 && b200_qgemm_pair_workspace(p.M, p.N, p.K, p.qtype, a->blocksize) >= 0)
+    return launch_swiglu(a, p, swiglu_tile(p.M, p.N, p.K, p.qtype == B200_Q_INT4), packed2, scale2, stream, "b200_qgemm_pair");
   ShortArgs sa{{p.packed, reinterpret_cast<const uint8_t*>(packed2)}, {p.scale, reinterpret_cast<const uint32_t*>(scale2)}, p.x, nullptr, p.y,
                reinterpret_cast<float*>(a->workspace), p.M, p.N, p.K, p.qtype};
   ShortPlan s = short_plan(p.M, p.N, p.K, p.qtype, true, true);
@@ -685,24 +710,12 @@ int b200_qgemm_swiglu(const b200_qgemm_args* a, const void* packed2, const void*
   if (const int rc = gemm_args(a, p)) return rc;
   B200_CHECK_ARG(packed2 && scale2 && (reinterpret_cast<uintptr_t>(packed2) & 15) == 0, "b200_qgemm_swiglu: null or misaligned second matrix");
   B200_CHECK_ARG(!a->bias, "b200_qgemm_swiglu: takes no bias");
-  const bool int4 = a->qtype == B200_Q_INT4;
-  const GemmPlan g = swiglu_plan(a->M, a->N, a->K, int4);
+  const GemmPlan g = swiglu_plan(a->M, a->N, a->K, a->qtype == B200_Q_INT4);
   if (g.mt == 0) {
     set_error("b200_qgemm_swiglu: (M=%lld N=%lld K=%lld) runs as two b200_qgemm and b200_swiglu", (long long)a->M, (long long)a->N, (long long)a->K);
     return B200_ERR_UNSUPPORTED;
   }
-  p.packed2 = reinterpret_cast<const uint8_t*>(packed2);
-  p.scale2 = reinterpret_cast<const uint32_t*>(scale2);
-  p.ksplit = 1;
-  p.bn = g.bn;
-  const cudaStream_t st = (cudaStream_t)stream;
-  const cudaError_t e = g.mt == 2 ? (int4 ? launch_gemm<2, 2, true, true>(p, st) : launch_gemm<2, 2, false, true>(p, st))
-                                : (int4 ? launch_gemm<2, 1, true, true>(p, st) : launch_gemm<2, 1, false, true>(p, st));
-  if (e != cudaSuccess) {
-    set_error("b200_qgemm_swiglu: launch failed: %s", cudaGetErrorString(e));
-    return B200_ERR_CUDA;
-  }
-  return B200_OK;
+  return launch_swiglu(a, p, g, packed2, scale2, stream, "b200_qgemm_swiglu");
 }
 
 }  // extern "C"

@@ -658,7 +658,9 @@ class LLaMAMLP(nn.Module):
             # gate and up projections + SwiGLU in one pass over both weight matrices
             return self.proj(f1.gemv(x, other=f2))
         if rows > 16 and x.is_cuda and x.dtype == torch.bfloat16 and not torch.compiler.is_compiling() and x.size(-1) == getattr(f1, "in_features", None):
-            both = K.qgemm_pair if rows <= 208 and short_pair(f1, f2, rows) else K.qgemm_swiglu if rows > 128 and prefill_pair(f1, f2, rows) else None
+            both = K.qgemm_swiglu if rows > 208 and prefill_pair(f1, f2, rows) else K.qgemm_pair if short_pair(f1, f2, rows) else None
+            if both is None and 128 < rows <= 208 and prefill_pair(f1, f2, rows):
+                both = K.qgemm_swiglu
             if both is not None:
                 (pw, ps), (pw2, ps2) = f1.packed(), f2.packed()
                 return self.proj(both(x, pw, ps, pw2, ps2, f1.out_features, f1.in_features, f1.quant_type, f1.blocksize))

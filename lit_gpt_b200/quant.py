@@ -425,7 +425,7 @@ def prefill_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
 
 
 def short_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
-    """``prefill_pair`` for the kernel of short prompts."""
+    """``prefill_pair`` for what else the library does in one launch: up to 208 rows, and beyond 512 where ``prefill_pair`` says no."""
     return _plain_pair(gate, up) and K.qgemm_pair_workspace(rows, gate.out_features, gate.in_features, gate.quant_type, gate.blocksize) >= 0
 
 

@@ -40,8 +40,20 @@ def test_pair_is_the_separate_launches(K, qt, M, N, Kdim):  # noqa: F811
     assert torch.equal(y, K.qgemm_pair(x, p1, s1, p2, s2, N, Kdim, qt, bs))
 
 
+@pytest.mark.parametrize("M,N,Kdim", [(513, 11008, 4096), (700, 5632, 4096), (1281, 11008, 1024)])
+@pytest.mark.parametrize("qt", ["nf4", "fp4", "int4"])
+def test_pair_takes_long_prompts_that_swiglu_refuses(K, qt, M, N, Kdim):  # noqa: F811
+    """The same sums in the same order as two GEMMs without k ranges: the same bits."""
+    _, _, p1, s1, bs, _ = _gemv_case(K, N, Kdim, 1, qt, seed=M)
+    _, _, p2, s2, _, _ = _gemv_case(K, N, Kdim, 1, qt, seed=N)
+    x = torch.randn(M, Kdim, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    assert (K.qgemm_pair_workspace(M, N, Kdim, qt, bs) == 0) != K.qgemm_swiglu_supported(M, N, Kdim, qt, bs)
+    one = K.qgemm_swiglu if K.qgemm_swiglu_supported(M, N, Kdim, qt, bs) else K.qgemm_pair
+    assert torch.equal(one(x, p1, s1, p2, s2, N, Kdim, qt, bs), K.swiglu(K.qgemm(x, p1, s1, N, Kdim, qt, bs), K.qgemm(x, p2, s2, N, Kdim, qt, bs)))
+
+
 def test_pair_refuses(K):  # noqa: F811
-    for M, N, Kdim in ((209, 512, 512), (1000, 512, 512), (32, 512, 320), (32, 500, 512)):
+    for M, N, Kdim in ((209, 512, 512), (512, 512, 512), (32, 512, 320), (32, 500, 512), (1000, 500, 512)):
         assert K.qgemm_pair_workspace(M, N, Kdim, "nf4", 64) < 0
         x, w = torch.zeros(M, Kdim, dtype=torch.bfloat16, device="cuda"), torch.zeros(N * Kdim // 2, dtype=torch.uint8, device="cuda")
         s = torch.zeros(N * Kdim // 64, dtype=torch.float32, device="cuda")
