@@ -79,9 +79,12 @@ __global__ void __launch_bounds__(128) rope_kv_append_kernel(const __nv_bfloat16
 // one unit -- eight elements and the eight they are turned with -- and walks the heads, so its cosines and sines are read once per token.
 // Bound: bytes (the projection read, q and the cache rows written), and how many loads are under way: those of a thread's first heads are issued
 // before the position and the tables that depend on it have arrived.  4096 tokens, 32 + 32 + 32 heads of 128 (201 MB: 31 us at the copy rate): 60 -> 53 us,
-// fp32 tables 50 -> 43; 32 + 8 + 8 heads 41 -> 34 and 32 -> 30 (the kernel above, with an element per thread and two barriers per head, 116).
+// fp32 tables 50 -> 43; 32 + 8 + 8 heads 41 -> 34 and 32 -> 30 (with fewer threads a CTA, b200_rope_kv_append, 29 and 22; the kernel above, with an element per thread and two barriers per head, 116).
 // Two heads at a time with bf16 tables, three with fp32 ones, whose turns take fewer registers: three with bf16 tables 51 us, but 13.1 instead
 // of 11.8 for 613 tokens of 40 + 40 + 40 heads; two with fp32 ones 51.
+template <bool TB>
+constexpr int kRopeHeads = TB ? 2 : 3;   // heads of a thread whose loads are under way together
+
 template <typename PosT, bool TB>
 __global__ void __launch_bounds__(256, 3) rope_kv_append_vec_kernel(const __nv_bfloat16* __restrict__ qkv, const void* __restrict__ cos,
                                                                  const void* __restrict__ sin, int table_presel, int rope_n,
@@ -90,10 +93,10 @@ __global__ void __launch_bounds__(256, 3) rope_kv_append_vec_kernel(const __nv_b
                                                                  int n_head, int n_groups, int hs, int max_seq) {
   griddep_launch();
   griddep_wait();
-  const int t = blockIdx.x, b = blockIdx.y, units = hs >> 4, lanes = 256 / units;
+  const int t = blockIdx.x, b = blockIdx.y, units = hs >> 4, lanes = (int)blockDim.x / units;
   const int u = (int)threadIdx.x % units, hl = (int)threadIdx.x / units;
   if (hl >= lanes) return;
-  constexpr int R = TB ? 2 : 3;   // heads of a thread whose loads are under way together
+  constexpr int R = kRopeHeads<TB>;
   const int64_t p0 = (int64_t)pos[t];
   const int half = rope_n >> 1, rope_units = rope_n >> 4;
   const bool turns = u < rope_units;
@@ -337,8 +340,13 @@ int b200_rope_kv_append(const void* qkv, const void* cos, const void* sin, int t
   const uintptr_t all = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin) |
                         reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(q_out);
   if (head_size % 16 == 0 && head_size <= 4096 && rope_n_elem % 16 == 0 && (all & 15) == 0) {
+    // From two rounds of CTAs on no more threads than give each as many heads as it has under way together: on 256 threads 32 + 8 + 8 heads are one or two of three.
+    // us, 256 threads / this: 4096 tokens, fp32 tables 30.0 / 21.9, bf16 33.6 / 29.5; 1000 tokens of 40 + 40 + 40 14.3 / 13.4; but 200 of 32 + 8 + 8 3.4 / 4.3, 613 of 40 + 40 + 40 10.2 / 10.9
+    const int units = head_size / 16, most = 256 / units, heads = n_head + 2 * n_groups, R = tb ? kRopeHeads<true> : kRopeHeads<false>;
+    const int turns = (heads + R * most - 1) / (R * most), lanes = (heads + R * turns - 1) / (R * turns);
+    const int threads = (int64_t)T * batch > 6 * sm_count() ? (lanes * units + 31) / 32 * 32 : 256;
     auto go = [&](auto kernel, auto p) {
-      return launch(kernel, dim3((unsigned)T, (unsigned)batch), dim3(256), 0, st, (const __nv_bfloat16*)qkv, cos, sin, table_preselected, rope_n_elem, p,
+      return launch(kernel, dim3((unsigned)T, (unsigned)batch), dim3((unsigned)threads), 0, st, (const __nv_bfloat16*)qkv, cos, sin, table_preselected, rope_n_elem, p,
                     (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, (__nv_bfloat16*)q_out, T, n_head, n_groups, head_size, max_seq);
     };
     if (pos_is_int64) B200_CUDA(tb ? go(rope_kv_append_vec_kernel<int64_t, true>, (const int64_t*)pos) : go(rope_kv_append_vec_kernel<int64_t, false>, (const int64_t*)pos));

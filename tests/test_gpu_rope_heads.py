@@ -15,3 +15,12 @@ def test_rope_kv_append_heads(H, G, hs, n, table):
     from lit_gpt_b200 import kernels
 
     base.test_rope_kv_append_units(kernels, 2, 3, H, G, hs, n, 9, table, torch.int64, False)
+
+
+# launches of more than 6 CTAs per SM take no more threads than the heads need: one lane of heads, an odd number of units, part of a warp at the end
+@pytest.mark.parametrize("table", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,T,H,G,hs,n", [(1, 1200, 1, 1, 128, 128), (2, 600, 32, 8, 128, 128), (1, 1000, 40, 40, 64, 32), (3, 400, 5, 1, 80, 48)])
+def test_rope_kv_append_long_launches(B, T, H, G, hs, n, table):
+    from lit_gpt_b200 import kernels
+
+    base.test_rope_kv_append_units(kernels, B, T, H, G, hs, n, T + 7, table, torch.int64, True)
