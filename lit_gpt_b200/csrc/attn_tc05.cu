@@ -99,7 +99,8 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   // Late rows, which see most keys, are scheduled first, those of all heads before any head's earlier ones: with a head's rows next to each other the last heads'
   // late rows started when the others were nearly done (32 heads of 128, 4096 rows: 512 CTAs on 148 SMs, 196 us; 158 in this order).
   const int late = (int)blockIdx.x / A.n_head, h = (int)blockIdx.x - late * A.n_head, b = blockIdx.y, grp = h / (A.n_head / A.n_groups);
-  const int r0 = ((int)gridDim.x / A.n_head - 1 - late) * A.span;
+  const int block = (int)gridDim.x / A.n_head - 1 - late;                   // the first A.pairs blocks of rows have two tiles, those behind one
+  const int r0 = (block + min(block, A.pairs)) * kAtBM, r1 = r0 + (block < A.pairs ? 2 * kAtBM : kAtBM);
   const uint32_t smem = (tc::smem_u32(at_smem) + 1023u) & ~1023u;
   const uint32_t sq_ = smem, sk_ = smem + 2 * C::kBytes, sv_ = smem + 4 * C::kBytes;
   const uint32_t bars = tc::smem_u32(s_bars);
@@ -140,7 +141,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   int lim = -1;
   if (warp < 8) {
     const int r = r0 + tid;
-    if (r < T && tid < A.span) {
+    if (r < T && r < r1) {
       const int64_t p = A.seqs ? (int64_t)pos0 + r : (A.pos64 ? reinterpret_cast<const int64_t*>(A.pos)[r] : (int64_t)reinterpret_cast<const int32_t*>(A.pos)[r]);
       lim = (int)(p < 0 ? 0 : (p >= max_seq ? max_seq - 1 : p));
     }
@@ -292,7 +293,7 @@ attn_tc05_kernel(const AttnTc05Args A, const __grid_constant__ CUtensorMap map_k
   } else {
     // ================================ softmax: a row per thread ================================
     const int t = warp >> 2, r = r0 + tid;
-    copy_tile<HS, 128>(sq_ + t * C::kBytes, A.q + (int64_t)b * A.q_b + (int64_t)h * A.q_h + qrow0 * A.q_r, A.q_r, r0 + t * kAtBM, min(T, r0 + A.span), tid & 127);
+    copy_tile<HS, 128>(sq_ + t * C::kBytes, A.q + (int64_t)b * A.q_b + (int64_t)h * A.q_h + qrow0 * A.q_r, A.q_r, r0 + t * kAtBM, min(T, r1), tid & 127);
     asm volatile("cp.async.wait_all;" ::: "memory");
     tc::fence_smem_async();
     __syncwarp();
@@ -445,12 +446,14 @@ cudaError_t launch_hs(AttnTc05Args a, int batch, cudaStream_t st) {
   if (!tensor_map_2d(&mk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.k, rows, cols, a.k_r * 2, 128) ||
       !tensor_map_2d(&mv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.v, rows, cols, a.v_r * 2, 128))
     return cudaErrorInvalidValue;
-  // One tile of rows per CTA while twice the CTAs are no more than the SMs: two tiles take turns on one SM's special-function units, and the second
-  // one's longer key range would be all that is left of the launch.  32 heads of 128, 160 / 256 / 400 rows from position 0, us with two tiles and with
-  // one: 12.6, 10.8 / 13.2, 11.3 / 17.9, 16.0; from position 4000 80.6, 70.6 / 84.9, 72.6 / 86.7, 77.4.
-  const int64_t pairs = (int64_t)((a.T + 2 * kAtBM - 1) / (2 * kAtBM)) * a.n_head * batch;
-  a.span = pairs * 2 <= sm_count() ? kAtBM : 2 * kAtBM;
-  const dim3 grid((unsigned)(((int64_t)a.T + a.span - 1) / a.span * a.n_head), (unsigned)batch);
+  // Two tiles take turns on one SM's issue slots and special-function units; a CTA with one goes through its keys in 0.85 of the time.  So as many blocks of rows have
+  // one tile as still run at once, the late ones, which see most keys; where even pairs take more than a round, all are pairs.  32 heads of 128, 160 / 256 / 400 rows
+  // from position 0, us with two tiles and with one: 12.6, 10.8 / 13.2, 11.3 / 17.9, 16.0; from position 4000 80.6, 70.6 / 84.9, 72.6 / 86.7, 77.4.  A pair and three of one,
+  // all pairs before: 613 rows of 32 heads from position 1500 44.9, 41.4, 500 of 40 heads from 700 34.0, 30.3; 300 of 40 heads from 0, one each, 14.2, 12.9.
+  const int64_t tiles = ((int64_t)a.T + kAtBM - 1) / kAtBM, chains = (int64_t)a.n_head * batch, fit = sm_count() / chains;
+  const int64_t pairs = tiles <= fit ? 0 : tiles - fit <= tiles / 2 ? tiles - fit : tiles / 2;
+  a.pairs = (int)pairs;
+  const dim3 grid((unsigned)((tiles - pairs) * a.n_head), (unsigned)batch);
   unsigned* const err = wait_error_word();
   if (!err) return cudaErrorMemoryAllocation;
   return launch(attn_tc05_kernel<HS>, grid, dim3(kAtThreads), (size_t)smem, st, a, mk, mv, err);

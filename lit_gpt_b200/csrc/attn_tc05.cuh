@@ -15,7 +15,7 @@ struct AttnTc05Args {
   int kv_first_row;       // ragged: the keys start at the sequence's first query row
   int T, n_head, n_groups, max_seq;   // ragged: T is the longest sequence's rows
   float scale_log2;
-  int span;               // set by launch_attn_tc05: query rows per CTA, two tiles of 128 or one
+  int pairs;              // set by launch_attn_tc05: blocks of 256 query rows, one CTA's, before those of 128
 };
 
 cudaError_t launch_attn_tc05(const AttnTc05Args& a, int head_size, int batch, cudaStream_t st);
