@@ -20,6 +20,7 @@
 // barriers), then the per-chunk work (two CTAs an SM; issue slots).  16 heads of 128 x 128 with decays per channel, 2048 tokens: 344 -> 209 us (chunks
 // 155 -> 97, chain 180 -> 108) against all of it in fp32 multiply-adds read from shared memory, 1640 token by token.
 #include "seq_pieces.cuh"
+#define B200_TRY_SLEEP_NS 0
 #include "tc05.cuh"
 #include "tf32x3.cuh"
 

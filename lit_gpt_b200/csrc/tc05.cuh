@@ -60,28 +60,32 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarri
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-constexpr uint32_t kTrySleepNs = 100000;   // how long one try may sleep: waiting threads that come back sooner take issue slots from those that work (qgemm.cu, 4096 -> 14336 int4, 64 rows: 28.5 -> 27.1 us)
+// SLEEP: how long one try may sleep, ns.  Waiting threads that come back sooner take issue slots from those that work (qgemm.cu, 4096 -> 14336 int4, 64 rows: 28.5 -> 27.1 us
+// with 100000); 0 is the hardware's own limit, for warps that wait in turns for short times (delta rule per head, fp32, two prompts of 1900 rows in all, 16 heads: the layer 875 us, 882 with 100000).
+#ifndef B200_TRY_SLEEP_NS   // (a source file may set it before this header)
+#define B200_TRY_SLEEP_NS 100000
+#endif
+constexpr uint32_t kTrySleepNs = B200_TRY_SLEEP_NS;
+template <uint32_t SLEEP = kTrySleepNs>
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done) : "r"(bar), "r"(parity), "r"(kTrySleepNs) : "memory");
-  return done != 0;
-}
-// without waiting at all
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  if constexpr (SLEEP > 0)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(bar), "r"(parity), "r"(SLEEP) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
 // (64 tries take far less than 50 ms: where more went by, the GPU was held up, and the time does not count)
+template <uint32_t SLEEP = kTrySleepNs>
 __device__ __forceinline__ bool mbar_wait_here(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) {
-  if (mbar_try(bar, parity)) return true;
+  if (mbar_try<SLEEP>(bar, parity)) return true;
   uint64_t last, t, spent = 0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(last));
   for (;;) {
     for (int i = 0; i < 64; ++i)
-      if (mbar_try(bar, parity)) return true;
+      if (mbar_try<SLEEP>(bar, parity)) return true;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     spent += t - last < 50000000ull ? t - last : 50000000ull;
     last = t;
@@ -90,8 +94,12 @@ __device__ __forceinline__ bool mbar_wait_here(uint32_t bar, uint32_t parity, ui
 }
 // The same behind a call, which keeps it out of the way of the code around.  Where that code issues products, mbar_wait_here is the better one: no value stays in a
 // uniform register across a call.
-static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) { return mbar_wait_here(bar, parity, limit_ns); }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_try(bar, parity) || mbar_try(bar, parity) || mbar_wait_slow(bar, parity); }
+template <uint32_t SLEEP = kTrySleepNs>
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) { return mbar_wait_here<SLEEP>(bar, parity, limit_ns); }
+template <uint32_t SLEEP = kTrySleepNs>
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  return mbar_try<SLEEP>(bar, parity) || mbar_try<SLEEP>(bar, parity) || mbar_wait_slow<SLEEP>(bar, parity);
+}
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
