@@ -344,8 +344,9 @@ int b200_qgemm(const b200_qgemm_args* args, b200_stream_t stream);
  * the shorter way (nothing is launched); elsewhere the call returns B200_ERR_UNSUPPORTED. */
 int b200_qgemm_swiglu_supported(int64_t M, int64_t N, int64_t K, int qtype, int blocksize);
 int b200_qgemm_swiglu(const b200_qgemm_args* args, const void* packed2, const void* scale2, b200_stream_t stream);
-/* The same of up to 208 rows, from 129 where it is the shorter way, and of more than 512 rows where b200_qgemm_swiglu refuses.  pair_workspace: bytes of scratch the call wants in args->workspace (0: none; without it the launch leaves SMs idle), or -1 where it
- * returns B200_ERR_UNSUPPORTED. */
+/* The same of up to 208 rows, from 129 where it is the shorter way, and of more than 512 rows where b200_qgemm_swiglu refuses.  pair_workspace: bytes of scratch the call
+ * wants in args->workspace (0: none; without it the launch leaves SMs idle), or -1 where it returns B200_ERR_UNSUPPORTED.  Up to 208 rows it returns that too where scale or
+ * scale2 is not 16-byte aligned, which b200_qgemm and b200_qgemm_swiglu do not ask for. */
 int64_t b200_qgemm_pair_workspace(int64_t M, int64_t N, int64_t K, int qtype, int blocksize);
 int b200_qgemm_pair(const b200_qgemm_args* args, const void* packed2, const void* scale2, b200_stream_t stream);
 /* tuning: wide = 1 (default): long prompts may share each dequantised weight tile among 512 tokens; 0: among 256 */

@@ -425,8 +425,10 @@ def prefill_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
 
 
 def short_pair(gate: nn.Module, up: nn.Module, rows: int) -> bool:
-    """``prefill_pair`` for what else the library does in one launch: up to 208 rows, and beyond 512 where ``prefill_pair`` says no."""
-    return _plain_pair(gate, up) and K.qgemm_pair_workspace(rows, gate.out_features, gate.in_features, gate.quant_type, gate.blocksize) >= 0
+    """``prefill_pair`` for what else the library does in one launch: up to 208 rows, and beyond 512 where ``prefill_pair`` says no.  Up to 208 rows that launch copies
+    scales 16 bytes at a time: those that begin elsewhere (views into a larger buffer) are left to the other launches, which read them one by one."""
+    return (_plain_pair(gate, up) and K.qgemm_pair_workspace(rows, gate.out_features, gate.in_features, gate.quant_type, gate.blocksize) >= 0
+            and (rows > 208 or all(m.packed()[1].data_ptr() % 16 == 0 for m in (gate, up))))
 
 
 class QuantPrecision:

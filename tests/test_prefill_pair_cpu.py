@@ -46,13 +46,24 @@ def test_hooks_of_all_modules(pair, register):
     assert quant.prefill_pair(*pair, 300)
 
 
+@pytest.mark.parametrize("offsets,rows,taken", [((0, 0), 17, True), ((4, 0), 17, False), ((0, 4), 208, False), ((4, 4), 64, False), ((4, 4), 600, True)])
+def test_scales_inside_a_larger_buffer(pair, monkeypatch, offsets, rows, taken):
+    """The launch for up to 208 rows copies scales 16 bytes at a time: scales elsewhere keep to the launches that read them one by one."""
+    monkeypatch.setattr(K, "qgemm_pair_workspace", lambda *a: 0)
+    buffer = torch.zeros(64)
+    first = -buffer.data_ptr() % 16 // 4   # the first number on a 16-byte boundary
+    for m, bytes_on in zip(pair, offsets):
+        monkeypatch.setattr(m, "packed", lambda scale=buffer[first + bytes_on // 4:]: (None, scale))
+    assert quant.short_pair(*pair, rows) == taken
+
+
 class _Cuda(torch.Tensor):
     """a CPU tensor that passes for a CUDA one: the checks come before anything reads it"""
 
     is_cuda = True
 
 
-@pytest.mark.parametrize("call", ["qgemm", "qgemm_swiglu"])
+@pytest.mark.parametrize("call", ["qgemm", "qgemm_swiglu", "qgemm_pair"])
 @pytest.mark.parametrize("shape", [(4, 256), (4, 64), (2, 2, 64)])
 def test_rows_of_another_length_are_refused(call, shape):
     """Elements enough for whole rows are not enough: the output has a row per row of x."""
