@@ -583,7 +583,7 @@ size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K < kBK) return 0;
   const int nf4 = gemm_plan(M, N, K, false, true).ksplit, int4 = gemm_plan(M, N, K, true, true).ksplit, s = nf4 > int4 ? nf4 : int4;   // either type's
   const size_t ranges = s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
-  const size_t a = short_scratch_bytes(M, short_plan(M, N, K, B200_Q_NF4, false, true), false), b = short_scratch_bytes(M, short_plan(M, N, K, B200_Q_INT4, false, true), false);
+  const size_t a = short_scratch_bytes(M, N, short_plan(M, N, K, B200_Q_NF4, false, true), false), b = short_scratch_bytes(M, N, short_plan(M, N, K, B200_Q_INT4, false, true), false);
   return ranges > a ? (ranges > b ? ranges : b) : (a > b ? a : b);
 }
 
@@ -626,7 +626,7 @@ int b200_qgemm(const b200_qgemm_args* a, b200_stream_t stream) {
   const ShortArgs sa{{p.packed, nullptr}, {p.scale, nullptr}, p.x, p.bias, p.y, reinterpret_cast<float*>(a->workspace), p.M, p.N, p.K, p.qtype};
   if (short_takes(sa, false)) {
     ShortPlan s = short_plan(p.M, p.N, p.K, p.qtype, false, true);
-    if (s.shared && (a->workspace == nullptr || a->workspace_bytes < short_scratch_bytes(p.M, s, false) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
+    if (s.shared && (a->workspace == nullptr || a->workspace_bytes < short_scratch_bytes(p.M, p.N, s, false) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
       s = short_plan(p.M, p.N, p.K, p.qtype, false, false);
     if (s.ctas && s.time < gemm_time(p.M, p.N, p.K, int4, g, g.bn) * short_margin(int4, g)) {
       const cudaError_t e = launch_short(sa, s, false, (cudaStream_t)stream);
@@ -671,7 +671,7 @@ int64_t b200_qgemm_pair_workspace(int64_t M, int64_t N, int64_t K, int qtype, in
   const ShortPlan s = short_plan(M, N, K, qtype, true, true);
   // (up to 128 rows there is no other launch for both; from 129 it is b200_qgemm_swiglu's or two)
   if (s.ctas == 0 || (M > 128 && s.time >= swiglu_time(M, N, K, qtype == B200_Q_INT4))) return -1;
-  return (int64_t)short_scratch_bytes(M, s, true);
+  return (int64_t)short_scratch_bytes(M, N, s, true);
 }
 
 int b200_qgemm_pair(const b200_qgemm_args* a, const void* packed2, const void* scale2, b200_stream_t stream) {
@@ -684,7 +684,7 @@ int b200_qgemm_pair(const b200_qgemm_args* a, const void* packed2, const void* s
   ShortArgs sa{{p.packed, reinterpret_cast<const uint8_t*>(packed2)}, {p.scale, reinterpret_cast<const uint32_t*>(scale2)}, p.x, nullptr, p.y,
                reinterpret_cast<float*>(a->workspace), p.M, p.N, p.K, p.qtype};
   ShortPlan s = short_plan(p.M, p.N, p.K, p.qtype, true, true);
-  if (s.shared && (a->workspace == nullptr || a->workspace_bytes < short_scratch_bytes(p.M, s, true) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
+  if (s.shared && (a->workspace == nullptr || a->workspace_bytes < short_scratch_bytes(p.M, p.N, s, true) || (reinterpret_cast<uintptr_t>(a->workspace) & 15)))
     s = short_plan(p.M, p.N, p.K, p.qtype, true, false);
   if (s.ctas == 0 || !short_takes(sa, true) || b200_qgemm_pair_workspace(p.M, p.N, p.K, p.qtype, a->blocksize) < 0) {
     set_error("b200_qgemm_pair: (M=%lld N=%lld K=%lld) or its addresses run as two b200_qgemm and b200_swiglu", (long long)a->M, (long long)a->N, (long long)a->K);

@@ -40,6 +40,10 @@ struct ShortParams {
   int ws, bs, ring;                                   // stages of weights and of rows; of single rebuilt k-blocks (a pair of more than 128 rows)
 };
 
+// Room for the partial sums of CTA c's part of tile t.  Parts in the order of their k step on by a CTA, a tile or both, so that c + t is another number for each; where
+// tiles are more than CTAs, a CTA has two cut ones at most: the one its range begins in and the one (`head`) that it ends in.
+__device__ __forceinline__ int64_t part_slot(int64_t c, int64_t t, bool head, int64_t ctas, int64_t tiles) { return tiles <= ctas ? c + t : 2 * c + head; }
+
 __device__ __forceinline__ int64_t unit_begin(int64_t c, int64_t ctas, int64_t tiles, int64_t nq, bool shared) {
   return shared ? c * (tiles * nq) / ctas : (c * tiles / ctas) * nq;
 }
@@ -250,7 +254,7 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
       tc::fence_after();
       const bool whole = t.n == p.nq;
       const int64_t n = (int64_t)t.tile * 128 + row, M = p.a.M, N = p.a.N;
-      float* const part = p.a.partial + ((int64_t)(2 * blockIdx.x + (t.q0 == 0)) * NACC * M) * 128 + row;
+      float* const part = p.a.partial + part_slot(blockIdx.x, t.tile, t.q0 == 0, gridDim.x, p.tiles) * NACC * M * 128 + row;
       const float bias = !PAIR && whole && p.a.bias && n < N ? __bfloat162float(p.a.bias[n]) : 0.f;
 #pragma unroll 1
       for (int c0 = g * 16; c0 < p.nb; c0 += kShGroups * 16) {
@@ -466,7 +470,7 @@ __global__ void __launch_bounds__(256) short_reduce_kernel(const ShortArgs a, in
   for (int64_t c = first; c <= last; ++c) {
 #pragma unroll
     for (int m = 0; m < NACC; ++m) {
-      const float4 v = *reinterpret_cast<const float4*>(a.partial + (((2 * c + (c == first)) * NACC + m) * a.M + r) * 128 + f);
+      const float4 v = *reinterpret_cast<const float4*>(a.partial + ((part_slot(c, t, c == first, ctas, tiles) * NACC + m) * a.M + r) * 128 + f);
       s[m][0] += v.x; s[m][1] += v.y; s[m][2] += v.z; s[m][3] += v.w;
     }
   }
@@ -570,8 +574,9 @@ ShortPlan short_plan(int64_t M, int64_t N, int64_t K, int qtype, bool pair, bool
   return best;
 }
 
-size_t short_scratch_bytes(int64_t M, const ShortPlan& plan, bool pair) {
-  return plan.shared ? (size_t)plan.ctas * 2 * (pair ? 2 : 1) * (size_t)M * 128 * sizeof(float) : 0;
+size_t short_scratch_bytes(int64_t M, int64_t N, const ShortPlan& plan, bool pair) {
+  const int64_t tiles = (N + 127) / 128, slots = tiles <= plan.ctas ? plan.ctas + tiles - 1 : 2 * (int64_t)plan.ctas;   // (part_slot)
+  return plan.shared ? (size_t)slots * (pair ? 2 : 1) * (size_t)M * 128 * sizeof(float) : 0;
 }
 
 cudaError_t launch_short(const ShortArgs& a, const ShortPlan& plan, bool pair, cudaStream_t st) {
