@@ -340,8 +340,9 @@ typedef struct b200_qgemm_args {
 size_t b200_qgemm_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200_qgemm(const b200_qgemm_args* args, b200_stream_t stream);
 /* y = silu(gate) * up of two projections of the same x (bf16 each, silu to bf16, product to bf16: the roundings of two b200_qgemm and
- * b200_swiglu, and their bits where those run without k ranges), `args` holding the gate and packed2 / scale2 the up projection in the same layout; no bias.  supported: 1 where one launch is
- * the shorter way (nothing is launched); elsewhere the call returns B200_ERR_UNSUPPORTED. */
+ * b200_swiglu, and their bits where those run without k ranges), `args` holding the gate and packed2 / scale2 the up projection in the same layout; no bias.  supported: 1 where the call
+ * runs, 129 rows and more at sizes where one launch is the shorter way (nothing is launched); elsewhere, also at some sizes of more than 512 rows where one launch would be
+ * shorter (b200_qgemm_pair's), the call returns B200_ERR_UNSUPPORTED. */
 int b200_qgemm_swiglu_supported(int64_t M, int64_t N, int64_t K, int qtype, int blocksize);
 int b200_qgemm_swiglu(const b200_qgemm_args* args, const void* packed2, const void* scale2, b200_stream_t stream);
 /* The same of up to 208 rows, from 129 where it is the shorter way, and of more than 512 rows where b200_qgemm_swiglu refuses.  pair_workspace: bytes of scratch the call
@@ -349,6 +350,9 @@ int b200_qgemm_swiglu(const b200_qgemm_args* args, const void* packed2, const vo
  * scale2 is not 16-byte aligned, which b200_qgemm and b200_qgemm_swiglu do not ask for. */
 int64_t b200_qgemm_pair_workspace(int64_t M, int64_t N, int64_t K, int qtype, int blocksize);
 int b200_qgemm_pair(const b200_qgemm_args* args, const void* packed2, const void* scale2, b200_stream_t stream);
+/* development: the kernel of up to 256 rows (a pair, packed2 not NULL: 208) whatever the times that the calls above go by; ranges 0: whole tiles, 1: equal ranges of k. */
+int64_t b200_qgemm_short_workspace(int64_t M, int64_t N, int64_t K, int pair, int ranges);
+int b200_qgemm_short(const b200_qgemm_args* args, const void* packed2, const void* scale2, int ranges, b200_stream_t stream);
 /* tuning: wide = 1 (default): long prompts may share each dequantised weight tile among 512 tokens; 0: among 256 */
 int b200_qgemm_tune(int wide);
 

@@ -297,6 +297,8 @@ _SIGNATURES = {
     "b200_qgemm_swiglu": (c_int, [ctypes.POINTER(QGemmArgs), c_void_p, c_void_p, c_void_p]),
     "b200_qgemm_pair_workspace": (c_int64, [c_int64, c_int64, c_int64, c_int, c_int]),
     "b200_qgemm_pair": (c_int, [ctypes.POINTER(QGemmArgs), c_void_p, c_void_p, c_void_p]),
+    "b200_qgemm_short_workspace": (c_int64, [c_int64, c_int64, c_int64, c_int, c_int]),
+    "b200_qgemm_short": (c_int, [ctypes.POINTER(QGemmArgs), c_void_p, c_void_p, c_int, c_void_p]),
     "b200_qgemm_tune": (c_int, [c_int]),
 }
 

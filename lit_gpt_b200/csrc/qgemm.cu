@@ -698,6 +698,29 @@ int b200_qgemm_pair(const b200_qgemm_args* a, const void* packed2, const void* s
   return B200_OK;
 }
 
+int64_t b200_qgemm_short_workspace(int64_t M, int64_t N, int64_t K, int pair, int ranges) {
+  if (M < 1 || N < 1 || K < 256) return -1;
+  return (int64_t)short_scratch_bytes(M, N, short_shape(N, K, ranges != 0), pair != 0);
+}
+
+int b200_qgemm_short(const b200_qgemm_args* a, const void* packed2, const void* scale2, int ranges, b200_stream_t stream) {
+  GemmParams p{};
+  if (const int rc = gemm_args(a, p)) return rc;
+  const bool pair = packed2 != nullptr;
+  B200_CHECK_ARG(!pair || (scale2 && !a->bias), "b200_qgemm_short: a pair takes scale2 and no bias");
+  const ShortArgs sa{{p.packed, reinterpret_cast<const uint8_t*>(packed2)}, {p.scale, reinterpret_cast<const uint32_t*>(scale2)}, p.x, p.bias, p.y,
+                     reinterpret_cast<float*>(a->workspace), p.M, p.N, p.K, p.qtype};
+  if (!short_takes(sa, pair)) {
+    set_error("b200_qgemm_short: (M=%lld N=%lld K=%lld) or its addresses are not the kernel's", (long long)a->M, (long long)a->N, (long long)a->K);
+    return B200_ERR_UNSUPPORTED;
+  }
+  const ShortPlan s = short_shape(p.N, p.K, ranges != 0);
+  B200_CHECK_ARG(!s.shared || (a->workspace && a->workspace_bytes >= short_scratch_bytes(p.M, p.N, s, pair) && (reinterpret_cast<uintptr_t>(a->workspace) & 15) == 0),
+                 "b200_qgemm_short: ranges of k want b200_qgemm_short_workspace bytes on a 16-byte boundary");
+  B200_CUDA(launch_short(sa, s, pair, (cudaStream_t)stream));
+  return B200_OK;
+}
+
 int b200_qgemm_swiglu_supported(int64_t M, int64_t N, int64_t K, int qtype, int blocksize) {
   const int block = qtype == B200_Q_INT4 ? 128 : 64;
   if ((qtype != B200_Q_NF4 && qtype != B200_Q_FP4 && qtype != B200_Q_INT4) || blocksize != block) return 0;

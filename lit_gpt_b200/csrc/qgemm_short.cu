@@ -32,7 +32,7 @@ constexpr int kShLow = 3;                             // stages below the table 
 constexpr int kShTable = 256 * 256;
 constexpr int kShMaxPair = 208;                       // rows of a gate / up pair: two accumulators beside the rebuilt weights
 constexpr int kShSmem = 227 * 1024 - 2048;            // dynamic shared memory (static: barriers)
-constexpr int kShMaxW = 8, kShMaxB = 8, kShA = 2, kShMaxRing = 8;   // most stages of weights and rows; stages of rebuilt weights (256 k: 128 columns each, handed over in halves)
+constexpr int kShMaxW = 8, kShMaxB = 4, kShA = 2, kShMaxRing = 8;   // most stages of weights and rows; stages of rebuilt weights (256 k: 128 columns each, handed over in halves)
 
 struct ShortParams {
   ShortArgs a;
@@ -51,7 +51,7 @@ __device__ __forceinline__ int64_t unit_begin(int64_t c, int64_t ctas, int64_t t
 // b: the low word of a tc::desc_sw128 descriptor, whose high word is the same for every address
 __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 bd, {%2, %5};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %3, p;\n\t}"
-               ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"((1024 >> 4) | (1 << 14) | (2 << 29)) : "memory");
+               ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"(tc::kDescSw128High) : "memory");
 }
 __device__ __forceinline__ void st8(uint32_t addr, const uint32_t (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
@@ -502,11 +502,11 @@ cudaError_t launch_kind(const ShortArgs& a, const ShortPlan& plan, cudaStream_t 
   p.nq = (int)(a.K / 256);
   p.shared = plan.shared;
   p.nb = (int)((a.M + 15) / 16 * 16);
-  // rows: up to eight stages; what they leave is the weights'
+  // rows: up to kShMaxB stages; what they leave is the weights'
   const int all = INT4 ? kShSmem - 2048 : kShSmem + 1024 - 0x20000;   // (int4: no table; else what lies above it, at 128 KB, whatever the kernel's own first address)
   const int stage = BQ * p.nb * 128;
   p.bs = (all - (INT4 ? 4 : PAIR ? 1 : 0) * kShStage) / stage;
-  if (p.bs > 4) p.bs = 4;
+  if (p.bs > kShMaxB) p.bs = kShMaxB;
   p.ring = (512 - 2 * p.nb) / 32 < kShMaxRing ? (512 - 2 * p.nb) / 32 : kShMaxRing;
   p.ws = (INT4 ? 0 : kShLow) + (all - p.bs * stage) / kShStage;
   if (p.ws > kShMaxW) p.ws = kShMaxW;
@@ -547,6 +547,11 @@ static double short_time(int64_t units, int64_t ctas, int nb, const ShortCost& c
   return c.start + (double)units * (c.unit + c.column * nb) + c.out * 1e-3 * (double)ctas * nb;
 }
 
+ShortPlan short_shape(int64_t N, int64_t K, bool shared) {
+  const int64_t tiles = (N + 127) / 128, sms = sm_count(), most = shared ? tiles * (K / 256) : tiles;
+  return {(int)(most < sms ? most : sms), shared, 0.0};
+}
+
 ShortPlan short_plan(int64_t M, int64_t N, int64_t K, int qtype, bool pair, bool scratch) {
   // [int4][rows up to 64, 128, 256][whole tiles, shared]; pairs [int4][rows up to 128, 208][whole, shared]
   static const ShortCost one[2][3][2] = {{{{4.53, 0.856, 0.0018, 0.512}, {7.04, 1.028, 0.0025, 0.275}},
@@ -563,13 +568,13 @@ ShortPlan short_plan(int64_t M, int64_t N, int64_t K, int qtype, bool pair, bool
   const int nb = (int)((M + 15) / 16 * 16), rows = M <= 64 ? 0 : M <= 128 ? 1 : 2;
   const bool int4 = qtype == B200_Q_INT4;
   const ShortCost* const cost = pair ? two[int4][rows == 2] : one[int4][rows];
-  best.ctas = (int)(tiles < sms ? tiles : sms);
+  best = short_shape(N, K, false);
   best.time = short_time((tiles + sms - 1) / sms * nq, best.ctas, nb, cost[0]);
   if (scratch) {
-    const int64_t ctas = total < sms ? total : sms;
-    const int64_t units = (total + ctas - 1) / ctas;
-    const double t = short_time(units, ctas, nb, cost[1]);
-    if (units < (tiles + sms - 1) / sms * nq && t < best.time) best = {(int)ctas, true, t};
+    ShortPlan s = short_shape(N, K, true);
+    const int64_t units = (total + s.ctas - 1) / s.ctas;
+    s.time = short_time(units, s.ctas, nb, cost[1]);
+    if (units < (tiles + sms - 1) / sms * nq && s.time < best.time) best = s;
   }
   return best;
 }

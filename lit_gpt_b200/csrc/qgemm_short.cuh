@@ -23,6 +23,7 @@ struct ShortPlan {
 };
 
 bool short_takes(const ShortArgs& a, bool pair);                              // pointers and sizes
+ShortPlan short_shape(int64_t N, int64_t K, bool shared);                      // the CTAs of either way, no time
 ShortPlan short_plan(int64_t M, int64_t N, int64_t K, int qtype, bool pair, bool scratch);
 size_t short_scratch_bytes(int64_t M, int64_t N, const ShortPlan& plan, bool pair);
 cudaError_t launch_short(const ShortArgs& a, const ShortPlan& plan, bool pair, cudaStream_t st);

@@ -484,6 +484,23 @@ def qgemm_pair(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, packe
     return y
 
 
+def qgemm_short(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, N: int, K: int, quant_type: str = "nf4", blocksize: int = 64, *, ranges: bool,
+                bias: Optional[torch.Tensor] = None, up: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> torch.Tensor:
+    """Development call: ``qgemm``, or with `up` (packed, scale) ``qgemm_pair``, by the kernel of short prompts whatever the library's times say; `ranges`: k in
+    equal ranges over the SMs, else whole tiles."""
+    C.require_cuda(x, packed, scale, bias, *(up or ()))
+    x, bias = _bf16c(x, "x"), _bf16c(bias, "bias")
+    if x.shape[-1] != K:
+        raise C.B200Error(f"qgemm_short: x has rows of {x.shape[-1]} numbers, the weights take {K}")
+    M = x.numel() // K
+    y, lib = x.new_empty((*x.shape[:-1], N)), C.load()
+    ws = x.new_empty(max(lib.b200_qgemm_short_workspace(M, N, K, int(up is not None), int(ranges)), 0), dtype=torch.uint8)
+    args = C.QGemmArgs(packed.data_ptr(), scale.data_ptr(), QTYPES[quant_type], blocksize, M, N, K, x.data_ptr(), C.ptr(bias), y.data_ptr(), C.ptr(ws), ws.numel())
+    p2, s2 = (None, None) if up is None else (up[0].data_ptr(), up[1].data_ptr())
+    C.check(lib.b200_qgemm_short(ctypes.byref(args), p2, s2, int(ranges), C.stream_ptr(x.device)), "qgemm_short")
+    return y
+
+
 def qgemm_tune(wide: bool = True) -> None:
     """development switch: long prompts may use tiles of 512 tokens (default) or keep to 256"""
     C.check(C.load().b200_qgemm_tune(1 if wide else 0), "qgemm_tune")
