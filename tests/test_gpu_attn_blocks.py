@@ -17,11 +17,8 @@ def test_blocks_of_rows(K, H, G, T, start, hs):  # noqa: F811
     k, v = (torch.randn(1, G, S, hs, generator=g).to(torch.bfloat16) for _ in range(2))
     pos = torch.arange(start, S)
     y = K.attn_prefill(q.cuda(), k.cuda(), v.cuda(), pos.cuda()).cpu().view(T, H, hs)
-    heads = sorted({0, 1, H // 2, H - 1})
-    want = _attn_exact(q[0, heads].transpose(0, 1), k[0, [h // (H // G) for h in heads]].transpose(0, 1), v[0, [h // (H // G) for h in heads]].transpose(0, 1), pos, torch.zeros(T),
-                       hs ** -0.5).view(T, len(heads), hs)
-    # weights and result rounded to bf16: two halves of a unit, the weights' as their root mean square over the keys at most
-    err = (y[:, heads].double() - want).norm() / want.norm()
+    of = [h // (H // G) for h in range(H)]   # every head, so that no block of rows can stand in for another's
+    want = _attn_exact(q[0].transpose(0, 1), k[0, of].transpose(0, 1), v[0, of].transpose(0, 1), pos, torch.zeros(T), hs ** -0.5).view(T, H, hs)
+    # weights and result rounded to bf16: two halves of a unit, the weights' as their root mean square over the keys at most; of a head, whichever
+    err = ((y.double() - want).norm(dim=(0, 2)) / want.norm(dim=(0, 2))).max()
     assert err <= 2.0 ** -8, err
-    for h in range(H):   # every row of every head is written
-        assert y[:, h].abs().sum(1).gt(0).all()

@@ -50,6 +50,20 @@ def routes(monkeypatch):
     return seen
 
 
+@pytest.mark.parametrize("rows", [17, 64, 128, 129, 203, 208, 209, 300, 512, 513, 700])
+@pytest.mark.parametrize("mode", ["nf4", "int4"])
+def test_routes(routes, mode, rows):
+    from lit_gpt_b200 import kernels as K
+
+    mlp = _mlp(mode)
+    x = torch.randn(rows, 512, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).cuda()
+    bs = 128 if mode == "int4" else 64
+    swiglu, pair = K.qgemm_swiglu_supported(rows, 1024, 512, mode, bs), K.qgemm_pair_workspace(rows, 1024, 512, mode, bs) >= 0
+    _check(mlp, x)
+    assert routes == (["qgemm_pair"] if pair else ["qgemm_swiglu"] if swiglu else [])
+    assert routes or 128 < rows <= 512   # up to 128 rows and beyond 512 there is one launch at every size
+
+
 @pytest.mark.parametrize("rows", [17, 128, 203, 600])
 @pytest.mark.parametrize("mode", ["nf4", "int4"])
 def test_scales_off_a_16_byte_boundary(routes, mode, rows):
@@ -60,3 +74,20 @@ def test_scales_off_a_16_byte_boundary(routes, mode, rows):
         setattr(m, name, _off_boundary(getattr(m, name)))
     _check(mlp, torch.randn(rows, 512, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).cuda())
     assert "qgemm_pair" not in routes or rows > 208
+
+
+@pytest.mark.parametrize("rows", [40, 203, 600])
+def test_hooks_and_released_layouts_keep_the_separate_launches(routes, rows):
+    x = torch.randn(rows, 512, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).cuda()
+    mlp, outs = _mlp("nf4"), []
+    handle = mlp.fc_2.register_forward_hook(lambda m, a, y: outs.append(y))
+    mlp(x)
+    assert not routes and outs[0].shape == (rows, 1024)
+    handle.remove()
+    want = mlp(x)
+    assert routes
+    del routes[:]
+    assert all(m.release_reference_layout() for m in (mlp.fc_1, mlp.fc_2))
+    y = mlp(x)
+    assert not routes
+    assert (y.double() - want.double()).norm() <= 2.0 ** -7 * want.double().norm()
