@@ -20,7 +20,6 @@
 // barriers), then the per-chunk work (two CTAs an SM; issue slots).  16 heads of 128 x 128 with decays per channel, 2048 tokens: 344 -> 209 us (chunks
 // 155 -> 97, chain 180 -> 108) against all of it in fp32 multiply-adds read from shared memory, 1640 token by token.
 #include "seq_pieces.cuh"
-#define B200_TRY_SLEEP_NS 0
 #include "tc05.cuh"
 #include "tf32x3.cuh"
 
@@ -568,7 +567,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   bool ok = true;
   for (int c = 0; c < chunks; ++c) {
     const float* const sg = dc_smem + (c % STAGES) * Y::kStage;
-    if (!tc::mbar_wait(full + 8 * (c % STAGES), (uint32_t)(c / STAGES) & 1u)) *(volatile int*)&s_gave_up[group] = 1;
+    if (!tc::mbar_wait<0>(full + 8 * (c % STAGES), (uint32_t)(c / STAGES) & 1u)) *(volatile int*)&s_gave_up[group] = 1;
     float acc[NT][4];
     const float* const wr = sg + (mt >> 1) * I::kMat + row * DK;
 #pragma unroll
@@ -682,7 +681,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   if (!ok) {   // given up: the copies under way land before the CTA leaves
     if (tid == 0) {
       *A.err = 1u;
-      for (int e = 0; e < chunks && e < STAGES; ++e) tc::mbar_wait(full + 8 * e, *(volatile unsigned*)&s_done[e] / G & 1u);   // (sent once and once per G counts)
+      for (int e = 0; e < chunks && e < STAGES; ++e) tc::mbar_wait<0>(full + 8 * e, *(volatile unsigned*)&s_done[e] / G & 1u);   // (sent once and once per G counts)
     }
   }
   for (int i = tid; i < DK * NC; i += 256) {

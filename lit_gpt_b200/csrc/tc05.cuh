@@ -61,11 +61,8 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 // SLEEP: how long one try may sleep, ns.  Waiting threads that come back sooner take issue slots from those that work (qgemm.cu, 4096 -> 14336 int4, 64 rows: 28.5 -> 27.1 us
-// with 100000); 0 is the hardware's own limit, for warps that wait in turns for short times (delta rule per head, fp32, two prompts of 1900 rows in all, 16 heads: the layer 875 us, 882 with 100000).
-#ifndef B200_TRY_SLEEP_NS   // (a source file may set it before this header)
-#define B200_TRY_SLEEP_NS 100000
-#endif
-constexpr uint32_t kTrySleepNs = B200_TRY_SLEEP_NS;
+// with 100000); 0 is the hardware's own limit, for warps that wait in turns for short times (delta_chunk.cu: delta rule per head, fp32, two prompts of 1900 rows in all, 16 heads: the layer 875 us, 882 with 100000).
+constexpr uint32_t kTrySleepNs = 100000;
 template <uint32_t SLEEP = kTrySleepNs>
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t done;
