@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(128) gated_rms_heads_kernel(const float* __res
   }
 }
 
-// the same for heads of up to 256 numbers, a multiple of four, on 16-byte boundaries (8 for 16-bit ones): four neighbouring numbers a lane, everything read once and kept,
+// the same for heads of fewer than 256 numbers, a multiple of four, on 16-byte boundaries (8 for 16-bit ones): four neighbouring numbers a lane, everything read once and kept,
 // several heads of fewer than 128 numbers a warp.  Bound: the exponential and the quotient of a number, beside the bytes.  us, a number per access and o read twice /
 // this: 2048 rows of 16 heads of 128, bf16 (34 MB) 12.9 / 12.1, of 8 7.2 / 6.6, one row 2.85 / 2.45, 300 rows of 8 heads of 64 3.1 / 2.5, fp32 1000 rows of 16 of 64 6.6 / 4.2.
 template <typename T>

@@ -1,4 +1,5 @@
-// Prefill GEMM: y (M, N) = x (M, K) . dequant(W)^T on the 5th-generation tensor cores (tcgen05 + TMEM).
+// Prefill GEMM: y (M, N) = x (M, K) . dequant(W)^T on the 5th-generation tensor cores (tcgen05 + TMEM).  Up to 256 rows most sizes run in qgemm_short.cu, which
+// b200_qgemm picks by the times of both (K a multiple of 256, addresses on 16 bytes); this kernel takes the others and every longer prompt.
 //
 // Replaces, for T > 16 rows, bnb.nn.Linear4bit.forward's "dequantize_4bit of the WHOLE weight to bf16, then F.linear"
 // (call sites lit_gpt/model.py:519,619,656,713,714,716): the bf16 weight is never materialised in HBM.
@@ -430,8 +431,9 @@ struct GemmPlan {
 
 // Tile and k ranges by the time of the last SM to finish, us.  A k-block takes `block + feature * bn` -- products and hand-overs, and the look-ups or
 // conversions of a tile's features, which its tokens share -- a launch `start`, a further round of tiles `round` more, k ranges 0.88 and 2.3 for every
-// million partial sums.  Fitted to some 700 launches of one to three rounds (24 shapes of 64 to 2000 rows, every tile and count of ranges: 4 % rms), in
-// which the plan's choice is within 4 % of the best one, but for 4096 -> 6144 at 150 rows, nf4 (8 %).
+// million partial sums.  Fitted to some 700 launches of one to three rounds (24 shapes of 64 to 2000 rows, every tile and count of ranges: 4 % rms) from before an
+// elected thread issued the products.  Against every tile and count of ranges timed since at 257 to 3000 rows (8 shapes, 160 sizes and types) the choice is 1.2 % off the best on
+// average and more than 5 % in 17: int4 5120 -> 5120 at 257 rows 29 %, 5120 -> 15360 at 613 17 %, 4096 -> 4096 at 257 14 %; nf4 4096 -> 4096 at 512 13 %.
 // Fewer features than 128 per CTA pay where they fill SMs that would have idled: 4096 -> 11008, nf4 / int4, at 64 rows 86 CTAs of 128 features and 138 of 80 39.0
 // and 30.8 / 30.6 and 25.6; at 203 rows 43 pairs of 256 and 69 of 160 46.2 and 38.0 / 36.7 and 31.6.
 // k ranges are for launches that leave SMs idle all the same: at least four k-blocks per range, at most 16 ranges and 64 MB of partial sums, and no more

@@ -349,7 +349,7 @@ qgemm_short_kernel(const __grid_constant__ ShortParams p, const __grid_constant_
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (tc::elect()) {
     // =========================================== PRODUCTS =======================================================
-    // One thread, chosen by elect: its operands are uniform to the compiler.  A stage's number is a constant of its copy of the code, and addresses are 32-bit
+    // One thread, chosen by tc::elect.  A stage's number is a constant of its copy of the code, and addresses are 32-bit
     // sums of constants and what stands before the loop.  (Two and four issuing warps with an accumulator each took as long: a stage's
     // chain of wait, rebuilding and hand-over in the sixteen warps is what a unit takes.)
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.nb >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);

@@ -1,4 +1,5 @@
-// tcgen05 / TMA / mbarrier helpers shared by the kernels that keep their accumulators in tensor memory (int8.cu, attn_tc05.cu).
+// tcgen05 / TMA / mbarrier helpers: the kernels that keep their accumulators in tensor memory (qgemm.cu, qgemm_short.cu, int8.cu, attn_tc05.cu), and delta_chunk.cu, whose
+// chain of chunks takes the barriers and the report of waits.
 //
 // Every wait is bounded: after about two seconds mbar_wait() gives up and returns false, the kernel raises the word wait_error_word()
 // hands out and leaves through its ordinary teardown, so that a mistake costs one wrong result and not a hung GPU.  The host reports it: the
@@ -89,8 +90,7 @@ __device__ __forceinline__ bool mbar_wait_here(uint32_t bar, uint32_t parity, ui
     if (spent > limit_ns) return false;
   }
 }
-// The same behind a call, which keeps it out of the way of the code around.  Where that code issues products, mbar_wait_here is the better one: no value stays in a
-// uniform register across a call.
+// The same behind a call, which keeps it out of the way of the code around.  Where that code issues products, mbar_wait_here took part in what elect() below gained.
 template <uint32_t SLEEP = kTrySleepNs>
 static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) { return mbar_wait_here<SLEEP>(bar, parity, limit_ns); }
 template <uint32_t SLEEP = kTrySleepNs>
@@ -102,10 +102,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
-// True in one lane of a warp whose 32 lanes are all here, the same one every time.  Products, commits and copies are issued behind `if (elect())` in code that the
-// whole warp walks: the compiler then knows their operands, which these instructions take from uniform registers, to be uniform.  In a branch on the lane's
-// number it does not, and spends a loop over the lanes on each: 55 to 130 clk a product and as much a commit, where the tensor core takes 32 for 128 x 64 x 16 and 128 for
-// 128 x 256 x 16 (four products and a commit of 128 x 64 x 16: 235 clk, 129 this way).
+// True in one lane of a warp whose 32 lanes are all here, the same one every time.  Products and commits, and the copies of the GEMMs, are issued behind `if (elect())` in code
+// that the whole warp walks (attn_tc05.cu's two copies for 128 keys stand behind a test of the lane).  Measured: four products and a commit issued behind `lane == 0` take
+// 235 clk whatever their width, this way 129 for 128 x 64 x 16 and 502 for 128 x 256 x 16, the tensor core's own time.  The likely cause is that the compiler
+// has to take operands of a branch on the lane's number for different ones in each lane.
 __device__ __forceinline__ bool elect() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r)::"memory");

@@ -468,8 +468,7 @@ def qgemm_pair_workspace(M: int, N: int, K: int, quant_type: str = "nf4", blocks
 def qgemm_pair(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor, packed2: torch.Tensor, scale2: torch.Tensor, N: int, K: int,
                quant_type: str = "nf4", blocksize: int = 64) -> torch.Tensor:
     """``qgemm_swiglu`` for up to 208 rows, on the kernel of short prompts (csrc/qgemm_short.cu), and for more than 512 where that one
-    refuses.  Raises NotImplementedError where
-    ``qgemm_pair_workspace`` is negative."""
+    refuses.  Raises NotImplementedError where ``qgemm_pair_workspace`` is negative, and up to 208 rows for scales off a 16-byte boundary."""
     C.require_cuda(x, packed, scale, packed2, scale2)
     x = _bf16c(x, "x")
     if x.shape[-1] != K:

@@ -388,8 +388,8 @@ class QLinear(nn.Module):
 
 
 def prefill_linear(q: QLinear, x: torch.Tensor) -> torch.Tensor:
-    """T > 16 rows: the tcgen05 / TMEM dequant-GEMM (csrc/qgemm.cu): weights are dequantised tile by tile in shared
-    memory, the bf16 matrix never exists in HBM.  Shapes it does not cover (K not a multiple of the quantisation
+    """T > 16 rows: the tcgen05 / TMEM dequant-GEMM: weights are dequantised tile by tile, in tensor memory (csrc/qgemm_short.cu,
+    most calls of up to 256 rows) or in shared memory (csrc/qgemm.cu), the bf16 matrix never exists in HBM.  Shapes it does not cover (K not a multiple of the quantisation
     block, N % 8 != 0: toy configs only) take the reference's own formulation -- dequantize_4bit to bf16, then a
     library GEMM -- with the dequantisation done by this library's kernel."""
     if x.dtype == torch.bfloat16:

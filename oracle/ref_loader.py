@@ -1,10 +1,10 @@
-"""Import the UNMODIFIED reference (``/root/reference``) in this container.
+"""Import the UNMODIFIED reference from ``B200GPT_REFERENCE_ROOT``.
 
-TEST INFRASTRUCTURE (see oracle/__init__.py).  ``/root/reference`` does not
-exist on the GPU box, so nothing here may be used at GPU run time; it is used
+TEST INFRASTRUCTURE (see oracle/__init__.py).  The reference need not be
+where the GPU is, so nothing here may be used at GPU run time; it is used
 only by ``tests/golden/make_golden.py`` (fixture generation), by the ``not gpu``
 tests that cross-check the restatement when the reference is present, and by
-``bench.py --impl reference`` when run inside this container.
+``bench.py --impl reference`` where the reference is there.
 
 The reference hard-fails at import without ``lightning`` (lit_gpt/__init__.py:9-16,
 lit_gpt/utils.py:12-17).  None of the imported names is *executed* on the

@@ -1,8 +1,8 @@
-"""Generate golden vectors by running the UNMODIFIED reference (/root/reference) in this container.
+"""Generate golden vectors by running the UNMODIFIED reference, wherever ``oracle.ref_loader`` finds it.
 
     python tests/golden/make_golden.py            # rewrites tests/golden/*.npz
 
-The reference cannot travel to the GPU box, so its outputs are committed as small fixtures.  Weights are
+The reference is not part of this repository, so its outputs are committed as small fixtures.  Weights are
 produced by ``oracle.model_ref.init_weights(seed)`` (a seeded torch CPU generator) and loaded into the
 reference's own ``GPT`` with ``load_state_dict``; the fixture stores a sha256 of the weights so RNG drift is
 detected, plus inputs and the reference's logits / tokens.  Reference entry points exercised:
@@ -103,7 +103,7 @@ def main() -> None:
         np.savez_compressed(os.path.join(HERE, f"{name}.npz"), **out)
         print(name, "logits", out["fwd_logits"].shape, "tokens", out["gen_tokens"][-5:])
 
-    # unit vectors: RMSNorm, rope tables (fp32 and the bf16-default-dtype aliasing of SURVEY F5), apply_rope
+    # unit vectors: RMSNorm, rope tables (fp32 and under a bf16 default dtype, where neighbouring positions round to one number), apply_rope
     g = torch.Generator().manual_seed(99)
     u = {}
     xx = torch.randn(3, 7, 96, generator=g)
