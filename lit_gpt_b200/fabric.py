@@ -30,8 +30,8 @@ class Fabric:
         self.world_size = int(os.environ.get("WORLD_SIZE", 1)) if strategy == "ddp" else 1
         use_cuda = torch.cuda.is_available() and accelerator in ("auto", "cuda", "gpu")
         # B200_TP_SHARED_DEVICE=1: every rank drives cuda:0 and the control plane is gloo (two NCCL ranks cannot share a
-        # device).  The peer-memory hand-off works unchanged between processes on one GPU (CUDA IPC, time-sliced contexts);
-        # this is how the tensor-parallel decode path is tested on a one-GPU box (tests/test_gpu_tp_shared.py).
+        # device).  The ranks' kernels wait for one another with nothing to guarantee that they run at the same time
+        # (time-sliced contexts): for a GPU of one's own, and no test does it.
         self.shared_device = strategy == "ddp" and os.environ.get("B200_TP_SHARED_DEVICE", "0") == "1"
         index = self.local_rank if strategy == "ddp" and not self.shared_device else 0
         self.device = torch.device("cuda", index) if use_cuda else torch.device("cpu")

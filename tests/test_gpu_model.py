@@ -321,22 +321,26 @@ def test_sampling_path_in_graph(golden):
         assert torch.equal(a, b)
 
 
-@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs 2 GPUs (the one-GPU variant is tests/test_gpu_tp_shared.py)")
-@pytest.mark.parametrize("mode,inter", [("nf4", 0), ("int4", 0), ("nf4", 2112)])
-def test_tp2_matches_oracle_multi_gpu(mode, inter):
-    """Two ranks on two GPUs over NCCL / NVLink: the sharded model (peer-memory hand-off in the GEMVs) against the oracle on
+# (a GPU for each rank: their kernels wait for one another, and nothing guarantees that launches of several processes on one GPU run at the same time)
+@pytest.mark.parametrize("world,mode,groups,seq0,inter,head", [(2, "nf4", 4, 0, 0, 0), (2, "int4", 4, 0, 0, 0), (2, "nf4", 4, 0, 2112, 0), (2, "nf4", 4, 65535 - 20, 0, 0), (2, "nf4", 4, 0, 0, 1),
+                                                               (4, "int4", 4, 0, 0, 0), (4, "int4", 4, 0, 0, 1), (8, "nf4", 8, 0, 11008, 0)])
+def test_tp_matches_oracle_multi_gpu(world, mode, groups, seq0, inter, head):
+    """Ranks on as many GPUs over NCCL / NVLink: the sharded model (peer-memory hand-off in the GEMVs) against the oracle on
     identically sharded-then-quantized weights, identical logits on every rank, and agreement with the all-NCCL path
-    (B200_TP_NCCL=1).  inter = 2112: the mlp.proj shard (1056 columns) is not block-aligned -> folded tiled layout."""
+    (B200_TP_NCCL=1).  inter = 2112 at two ranks, 11008 at eight: the mlp.proj shard (1056, 1376 columns) is not block-aligned -> folded tiled layout.
+    Four ranks over four groups: one kv group a rank.  seq0: sequence counters just below the 16-bit tag's wrap.  head: lm_head in row shards, gathered over peer memory."""
     import os
     import subprocess
     import sys
 
+    if torch.cuda.device_count() < world:
+        pytest.skip(f"needs {world} GPUs")
     root = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
-    env = dict(os.environ, B200_TP_SHARED_DEVICE="0", B200_TP_NCCL="0", OMP_NUM_THREADS="4")
-    cmd = [sys.executable, "-m", "torch.distributed.run", "--nnodes=1", "--nproc-per-node=2", "--master-addr", "127.0.0.1",
-           "--master-port", "29631", os.path.join(root, "tests", "tp_shared_worker.py"), root, mode, "8", "4", "0", str(inter)]
+    env = dict(os.environ, B200_TP_NCCL="0", OMP_NUM_THREADS="4", B200_TP_SHARD_LM_HEAD=str(head))
+    cmd = [sys.executable, "-m", "torch.distributed.run", "--nnodes=1", f"--nproc-per-node={world}", "--master-addr", "127.0.0.1",
+           "--master-port", "29631", os.path.join(root, "tests", "tp_worker.py"), root, mode, "8", str(groups), str(seq0), str(inter)]
     out = subprocess.run(cmd, capture_output=True, text=True, timeout=600, env=env)
-    assert out.returncode == 0 and "TP_SHARED_OK" in out.stdout, out.stdout[-2000:] + out.stderr[-4000:]
+    assert out.returncode == 0 and "TP_OK" in out.stdout, out.stdout[-2000:] + out.stderr[-4000:]
     print(out.stdout[-500:])
 
 

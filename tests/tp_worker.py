@@ -1,5 +1,4 @@
-"""Launched by tests/test_gpu_tp_shared.py under torchrun: WORLD ranks that all drive cuda:0 (B200_TP_SHARED_DEVICE=1, gloo
-control plane), so that a ONE-GPU box exercises the tensor-parallel decode path end to end: shard-then-quantize
+"""Launched by tests/test_gpu_model.py under torchrun, a rank per GPU over NCCL: the tensor-parallel decode path end to end: shard-then-quantize
 (generate/tp.py:28-92, 163-192), the peer-memory hand-off inside the GEMV kernels (b200_tp_handoff: CUDA-IPC slots,
 self-validating packets, buffer alternation, tag wrap-around) and the captured decode graph.
 
@@ -70,11 +69,7 @@ def main() -> None:
     fabric = Fabric(devices="auto", strategy="ddp", plugins=QuantPrecision(mode, torch.bfloat16))
     fabric.launch()
     world, rank = fabric.world_size, fabric.global_rank
-    shared = os.environ.get("B200_TP_SHARED_DEVICE", "0") == "1"
-    if shared:
-        assert fabric.device == torch.device("cuda", 0) and dist.get_backend() == "gloo"
-    else:  # one GPU per rank, NCCL control plane (tests/test_gpu_model.py::test_tp2_matches_oracle_multi_gpu)
-        assert fabric.device == torch.device("cuda", fabric.local_rank) and dist.get_backend() == "nccl"
+    assert fabric.device == torch.device("cuda", fabric.local_rank) and dist.get_backend() == "nccl"
     cfg_kw = dict(n_layer=2, n_head=n_head, n_query_groups=n_groups, n_embd=128 * n_head, intermediate_size=inter or 256 * world * 2,
                   padded_vocab_size=1024, vocab_size=1024, block_size=64)
     cfg = Config.from_name("Llama-2-7b-hf", **cfg_kw)
@@ -146,7 +141,7 @@ def main() -> None:
         agree = got.argmax(-1) == logits32.argmax(-1)
         assert bool(agree[decisive].all()), agree.tolist()
         # ---- every rank holds the same logits bit for bit (no broadcast in tp.py:200) ----------------------------------
-        got_d = got if shared else got.to(dev)   # gloo gathers host tensors, NCCL device tensors
+        got_d = got.to(dev)   # NCCL gathers device tensors
         gathered = [torch.empty_like(got_d) for _ in range(world)]
         dist.all_gather(gathered, got_d)
         assert all(torch.equal(gathered[0], t) for t in gathered)
@@ -158,12 +153,12 @@ def main() -> None:
         div = next((i for i in range(T, n_total) if out[i].item() != toks32[i].item()), None)
         if div is not None:
             assert not bool(decisive[div - T]), f"rollout diverged at decisive step {div}"
-        out_d = out if shared else out.to(dev)
+        out_d = out.to(dev)
         outs = [torch.empty_like(out_d) for _ in range(world)]
         dist.all_gather(outs, out_d)
         assert all(torch.equal(outs[0], t) for t in outs)
         e_n = None
-        if not shared:
+        if not seq0 and not head_sharded:
             # the same sharded model with every row-parallel sum by NCCL all-reduce (generate/tp.py:73-74): the peer-memory
             # hand-off must agree with it to bf16 rounding of the partial sums
             os.environ["B200_TP_NCCL"] = "1"
@@ -179,7 +174,7 @@ def main() -> None:
             assert e_n <= 2 ** -6 * scale, (e_n, scale)
         seq_now = int(raw_u32(comm._flags(comm._local, 0), 1, dev).item())
     if rank == 0:
-        print(f"[tp{world}/{'shared-gpu' if shared else 'multi-gpu'}/{mode}/H{n_head}G{n_groups}/I{cfg.intermediate_size}{'/lm_head-sharded' if head_sharded else ''}] bf16-reference err {e_ref:.4f} cuda err {e_k:.4f} tol {tol:.4f} "
+        print(f"[tp{world}/{mode}/H{n_head}G{n_groups}/I{cfg.intermediate_size}{'/lm_head-sharded' if head_sharded else ''}] bf16-reference err {e_ref:.4f} cuda err {e_k:.4f} tol {tol:.4f} "
               f"(|logit| max {scale:.2f}); top-1 {int(agree.sum())}/{len(agree)} (decisive {int(decisive.sum())}); "
               f"greedy prefix {(div or n_total) - T}/{n_total - T}; hand-off seq {seq0} -> {seq_now}"
               + ("" if e_n is None else f"; |p2p - nccl| {e_n:.4f}"), flush=True)
@@ -190,7 +185,7 @@ def main() -> None:
     model.__dict__.pop("_decode_graphs", None)
     comm.close()
     if rank == 0:
-        print("TP_SHARED_OK", flush=True)
+        print("TP_OK", flush=True)
     dist.destroy_process_group()
 
 
