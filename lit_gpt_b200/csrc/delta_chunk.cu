@@ -31,6 +31,8 @@ constexpr int kDcC = 32;            // tokens per chunk
 constexpr int kDcChunkThreads = 256;
 constexpr int kDcMinRows = 64;
 
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return tc::mbar_wait<0>(bar, parity); }   // (a try's length: tc05.cuh)
+
 struct DcArgs {
   const float* q; const float* k; const float* v;
   int64_t ldq, ldk, ldv;
@@ -567,7 +569,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   bool ok = true;
   for (int c = 0; c < chunks; ++c) {
     const float* const sg = dc_smem + (c % STAGES) * Y::kStage;
-    if (!tc::mbar_wait<0>(full + 8 * (c % STAGES), (uint32_t)(c / STAGES) & 1u)) *(volatile int*)&s_gave_up[group] = 1;
+    if (!mbar_wait(full + 8 * (c % STAGES), (uint32_t)(c / STAGES) & 1u)) *(volatile int*)&s_gave_up[group] = 1;
     float acc[NT][4];
     const float* const wr = sg + (mt >> 1) * I::kMat + row * DK;
 #pragma unroll
@@ -681,7 +683,7 @@ __global__ void __launch_bounds__(256 * G, 1) delta_carry_kernel(DcArgs A, int L
   if (!ok) {   // given up: the copies under way land before the CTA leaves
     if (tid == 0) {
       *A.err = 1u;
-      for (int e = 0; e < chunks && e < STAGES; ++e) tc::mbar_wait<0>(full + 8 * e, *(volatile unsigned*)&s_done[e] / G & 1u);   // (sent once and once per G counts)
+      for (int e = 0; e < chunks && e < STAGES; ++e) mbar_wait(full + 8 * e, *(volatile unsigned*)&s_done[e] / G & 1u);   // (sent once and once per G counts)
     }
   }
   for (int i = tid; i < DK * NC; i += 256) {
